@@ -29,7 +29,7 @@ def build_library(force=False):
     """compile every source under csrc/ that belongs to the shared library"""
     out = HERE / 'libvesta_b200.so'
     srcs = sorted(list((HERE / 'csrc').glob('*.cpp')) + list((HERE / 'csrc').glob('*.cu')))
-    newest = max(s.stat().st_mtime for s in srcs + [ROOT / 'include' / 'vesta_b200.h'])
+    newest = max(s.stat().st_mtime for s in srcs + list((HERE / 'csrc').glob('pass*.cuh')) + [HERE / 'csrc' / 'rt_internal.h', ROOT / 'include' / 'vesta_b200.h'])
     if out.exists() and out.stat().st_mtime >= newest and not force:
         return out
     cmd = [NVCC, '-O2', '-std=c++17', '-shared', '-Xcompiler', '-fPIC', *ARCH_FLAGS, '-I', str(ROOT / 'include'),

@@ -1,0 +1,303 @@
+// Host side of the forward pass over rows (pass_kernels.cuh): sizes, workspace, tensor maps, the launches of a pass and,
+// for decode steps, the CUDA graph that holds them.
+#include <cuda.h>
+#include <cuda_runtime.h>
+#include <algorithm>
+#include <string>
+#include <vector>
+
+#include "pass_kernels.cuh"
+#include "rt_internal.h"
+#include "vesta_b200.h"
+
+using namespace vesta_pass;
+using vesta_rt::fail;
+
+namespace {
+
+int cuda_fail(cudaError_t e, const char* what) { return fail((int)e, std::string(what) + ": " + cudaGetErrorString(e)); }
+#define TRY(x) do { cudaError_t e_ = (x); if (e_ != cudaSuccess) return cuda_fail(e_, #x); } while (0)
+
+int up(long long v, int a) { return (int)((v + a - 1) / a * a); }
+
+enum Kind { K_QKV = 0, K_PROJ = 1, K_FC = 2, K_P2 = 3, K_LOGITS = 4 };
+
+struct Tile { int bm, bn, stages, splits; };
+
+struct Layout { size_t z, q, act, att, gelu, part, fin, best, rowoff, pos, skip, total; };
+
+struct Pass {
+    vesta_pass_desc d;
+    int rp;                                    // rows of an operand plane when head and remainder are kept, else 0
+    int planes;                                // operand rows: rp * 2, or the rows rounded up to whole tiles
+    int fplanes;                               // the same for the rows that want logits
+    Layout o;
+    unsigned char* ws;
+    Tile tile[5];
+    CUtensorMap w[5], a[5];                    // weights and operand of every contraction
+    int max_parts;
+    std::vector<cudaGraphExec_t> graphs;       // decode: one step
+    int sms;
+};
+
+// rows of an operand: one product column per row; up to 16 rows at fp32 accuracy take two planes of 8 or 16
+int plane_rows(int rows, bool exact) { return !exact ? 0 : rows <= 8 ? 8 : 16; }
+
+// Tile sizes of a contraction of `feat` features over `kb` blocks of 64 for `rows` rows (columns of the product).
+Tile choose(int kind, int rows, int rp, int feat, int kb, int sms) {
+    Tile t;
+    const int cols = rp ? 2 * rp : rows;
+    t.bn = cols <= 16 ? 16 : cols <= 32 ? 32 : cols <= 64 ? 64 : 128;
+    t.bm = t.bn <= 64 ? 64 : 128;
+    const int tiles = ((feat + t.bm - 1) / t.bm) * (rp ? 1 : (rows + t.bn - 1) / t.bn);
+    t.splits = 1;
+    if (kind == K_PROJ || kind == K_P2) t.splits = std::max(1, std::min(std::min(8, kb), (sms + tiles / 2) / tiles));
+    const int per = (kb + t.splits - 1) / t.splits;
+    t.splits = (kb + per - 1) / per;
+    const int stage = (t.bm + t.bn) * 128;
+    t.stages = std::max(2, std::min(per, (112 * 1024 - 1024 - 5120) / (stage + 16)));
+    return t;
+}
+
+Layout layout(const Pass& p, int D, int F, int rows, int lrows) {
+    Layout o{};
+    size_t at = 0;
+    auto take = [&](size_t bytes) { const size_t r = at; at += (bytes + 255) / 256 * 256; return r; };
+    o.z = take((size_t)rows * D * 4);
+    o.q = take((size_t)rows * D * 4);
+    o.act = take((size_t)p.planes * D * 2);
+    o.att = take((size_t)p.planes * D * 2);
+    o.gelu = take((size_t)p.planes * F * 2);
+    o.part = take((size_t)p.max_parts * rows * D * 4);
+    o.fin = take((size_t)p.fplanes * D * 2);
+    o.best = take((size_t)lrows * 8);
+    o.rowoff = take((size_t)rows * 8);
+    o.pos = take((size_t)rows * 4);
+    o.skip = take(4);
+    o.total = at;
+    return o;
+}
+
+int plan(Pass& p, const vesta_pass_desc* d) {
+    if (!d || d->rows < 1 || d->logit_rows < 1 || d->logit_rows > d->rows) return fail(-1, "vesta_pass: bad row counts");
+    if (d->L < 1 || d->D % 64 || d->D > 4096 || d->H * 64 != d->D || d->F % 16 || d->N < 1) return fail(-1, "vesta_pass: sizes outside the supported family");
+    if (d->exact && d->rows > 16) return fail(-1, "vesta_pass: fp32-accurate operands are kept for at most 16 rows");
+    p.d = *d;
+    int dev = 0;
+    p.sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&p.sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaGetLastError();                          // (sizes can be asked for without a device)
+    p.rp = plane_rows(d->rows, d->exact != 0);
+    const int frp = plane_rows(d->logit_rows, d->exact != 0);
+    p.planes = p.rp ? 2 * p.rp : up(d->rows, 128);
+    p.fplanes = p.rp ? 2 * p.rp : up(d->logit_rows, 128);
+    (void)frp;
+    const int kbd = d->D / 64, kbf = (d->F + 63) / 64;
+    p.tile[K_QKV] = choose(K_QKV, d->rows, p.rp, 3 * d->D, kbd, p.sms);
+    p.tile[K_PROJ] = choose(K_PROJ, d->rows, p.rp, d->D, kbd, p.sms);
+    p.tile[K_FC] = choose(K_FC, d->rows, p.rp, d->F, kbd, p.sms);
+    p.tile[K_P2] = choose(K_P2, d->rows, p.rp, d->D, kbf, p.sms);
+    p.tile[K_LOGITS] = choose(K_LOGITS, d->logit_rows, p.rp, d->N, kbd, p.sms);
+    p.max_parts = std::max(p.tile[K_PROJ].splits, p.tile[K_P2].splits);
+    p.o = layout(p, d->D, d->F, d->rows, d->logit_rows);
+    return 0;
+}
+
+template <int BM, int BN, int EPI>
+cudaError_t launch_gemm(const cudaLaunchConfig_t& c, const CUtensorMap& w, const CUtensorMap& a, const GemmArgs& g) {
+    return cudaLaunchKernelEx(&c, pass_gemm<BM, BN, EPI>, w, a, g);
+}
+template <int BM, int BN, int EPI>
+cudaError_t prepare_gemm(int stages) {
+    return cudaFuncSetAttribute(pass_gemm<BM, BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<BM, BN>::bytes(stages));
+}
+// one case per tile shape and epilogue
+#define SHAPES(X, EPI) X(64, 16, EPI) X(64, 32, EPI) X(64, 64, EPI) X(128, 128, EPI)
+#define EACH(X) SHAPES(X, EPI_QKV) SHAPES(X, EPI_PART) SHAPES(X, EPI_GELU) SHAPES(X, EPI_LOGITS)
+
+cudaError_t gemm(int epi, const Tile& t, cudaLaunchConfig_t c, const CUtensorMap& w, const CUtensorMap& a, const GemmArgs& g) {
+#define ONE(M, N, E) if (epi == E && t.bm == M && t.bn == N) { c.dynamicSmemBytes = GemmSmem<M, N>::bytes(t.stages); return launch_gemm<M, N, E>(c, w, a, g); }
+    EACH(ONE)
+#undef ONE
+    return cudaErrorInvalidValue;
+}
+cudaError_t gemm_prepare(int epi, const Tile& t) {
+#define ONE(M, N, E) if (epi == E && t.bm == M && t.bn == N) return prepare_gemm<M, N, E>(t.stages);
+    EACH(ONE)
+#undef ONE
+    return cudaErrorInvalidValue;
+}
+const int EPI_OF[5] = {EPI_QKV, EPI_PART, EPI_GELU, EPI_PART, EPI_LOGITS};
+
+// launch attributes: `dependent` = may start while the kernel before it runs
+struct Config {
+    cudaLaunchConfig_t c = {};
+    cudaLaunchAttribute at[2];
+    Config(dim3 grid, int block, cudaStream_t st, bool dependent, int cluster = 1) {
+        c.gridDim = grid; c.blockDim = dim3(block); c.stream = st; c.attrs = at; c.numAttrs = 0;
+        if (dependent) { at[c.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[c.numAttrs].val.programmaticStreamSerializationAllowed = 1; c.numAttrs++; }
+        if (cluster > 1) { at[c.numAttrs].id = cudaLaunchAttributeClusterDimension; at[c.numAttrs].val.clusterDim.x = 1; at[c.numAttrs].val.clusterDim.y = 1; at[c.numAttrs].val.clusterDim.z = cluster; c.numAttrs++; }
+    }
+};
+
+// The launches of one pass over `rows` rows. Prompts: `tiles` runs of rows for the attention, `lrows` rows that want logits
+// (listed in d.want; none: the pass ends after the last layer's cache rows).
+int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles) {
+    const vesta_pass_desc& d = p.d;
+    const int D = d.D, F = d.F, L = d.L, kbd = D / 64, kbf = (F + 63) / 64;
+    const bool many = d.tiles != 0;
+    auto u = [&](size_t off) { return p.ws + off; };
+    float* z = (float*)u(p.o.z);
+    u16 *act = (u16*)u(p.o.act), *att = (u16*)u(p.o.att), *fin = (u16*)u(p.o.fin);
+    const int nthr = up(D / 4, 32);
+    auto f16 = [](const void* q, size_t off) { return (const u16*)q + off; };
+    auto norm = [&](int mode, int l, int nparts) {
+        NormArgs n = {};
+        n.D = D; n.nparts = nparts; n.rp = p.rp; n.eps = d.eps; n.z = z;
+        n.part = (const float*)u(p.o.part); n.part_stride = (size_t)d.rows * D;
+        n.x = (const int*)d.x; n.t = (const int*)d.t; n.seq = (const int*)d.seq; n.t_stride = d.t_stride; n.N = d.N; n.cpos = d.cpos; n.tmax = d.tmax; n.L = L;
+        n.wte = (const u16*)d.wte; n.wpe = (const u16*)d.wpe;
+        n.rowoff = (long long*)u(p.o.rowoff); n.pos = (int*)u(p.o.pos); n.skip = (int*)u(p.o.skip); n.bar = (u32*)d.bar;
+        n.want = (const int*)d.want;
+        n.act = act;
+        if (mode == 0) { n.gain = f16(d.ln1w, 0); n.shift = f16(d.ln1b, 0); }
+        else if (mode == 1) { n.gain = f16(d.ln2w, (size_t)l * D); n.shift = f16(d.ln2b, (size_t)l * D); n.bias = f16(d.ob, (size_t)l * D); }
+        else if (mode == 2) { n.gain = f16(d.ln1w, (size_t)(l + 1) * D); n.shift = f16(d.ln1b, (size_t)(l + 1) * D); n.bias = f16(d.pb, (size_t)l * D); }
+        else { n.gain = f16(d.lnfw, 0); n.shift = f16(d.lnfb, 0); n.bias = f16(d.pb, (size_t)l * D); n.act = fin; }
+        Config c(dim3(mode == 3 ? lrows : rows), nthr, st, mode != 0);
+        return mode == 0 ? cudaLaunchKernelEx(&c.c, pass_norm<NORM_EMBED>, n) : mode == 3 ? cudaLaunchKernelEx(&c.c, pass_norm<NORM_FINAL>, n) : cudaLaunchKernelEx(&c.c, pass_norm<NORM_MID>, n);
+    };
+    auto mul = [&](int kind, int l) {
+        const Tile& t = p.tile[kind];
+        GemmArgs g = {};
+        g.layer = l; g.D = D; g.rp = p.rp; g.stages = t.stages; g.status = (u32*)d.bar; g.skip = (const int*)u(p.o.skip);
+        g.rows = kind == K_LOGITS ? lrows : rows;
+        g.kblocks = kind == K_P2 ? kbf : kbd; g.kb_per = (g.kblocks + t.splits - 1) / t.splits;
+        g.nfeat = kind == K_QKV ? 3 * D : kind == K_FC ? F : kind == K_LOGITS ? d.N : D;
+        if (kind == K_QKV) {
+            g.bias = f16(d.qkvb, (size_t)l * 3 * D); g.of = (float*)u(p.o.q); g.rowoff = (const long long*)u(p.o.rowoff);
+            g.kc = (u16*)d.keys + (size_t)l * d.tmax * D; g.vc = (u16*)d.vals + (size_t)l * d.tmax * D;
+        } else if (kind == K_FC) {
+            g.bias = f16(d.fcb, (size_t)l * F); g.oh = (u16*)u(p.o.gelu); g.ga = d.gelu_a; g.gb = d.gelu_b; g.gc = d.gelu_c;
+        } else if (kind == K_LOGITS) { g.of = (float*)d.logits; g.best = (u64*)u(p.o.best); }
+        else { g.of = (float*)u(p.o.part); g.part_stride = (size_t)d.rows * D; }
+        Config c(dim3((g.nfeat + t.bm - 1) / t.bm, p.rp ? 1 : (g.rows + t.bn - 1) / t.bn, t.splits), 192, st, true);
+        return gemm(EPI_OF[kind], t, c.c, p.w[kind], p.a[kind], g);
+    };
+    auto attend = [&](int l) {
+        const float* q = (const float*)u(p.o.q);
+        const u16 *kc = (const u16*)d.keys + (size_t)l * d.tmax * D, *vc = (const u16*)d.vals + (size_t)l * d.tmax * D;
+        const long long ss = (long long)L * d.tmax * D;
+        int e = 0;
+        const int pow2 = frexpf(d.scale, &e) == 0.5f;
+        if (many) {
+            AttManyArgs a = {q, kc, vc, ss, (const int4*)d.tiles, D, pow2, d.scale, att};
+            Config c(dim3(tiles, d.H), 128, st, true);
+            return cudaLaunchKernelEx(&c.c, pass_attend_many, a);
+        }
+        AttArgs a = {q, kc, vc, ss, (const int*)u(p.o.pos), (const int*)d.seq, D, pow2, p.rp, d.scale, att};
+        int C = 1;
+        while (C < 8 && rows * d.H * C * 2 <= 2 * p.sms && d.tmax > C * ATT_WARPS * 32) C *= 2;
+        Config c(dim3(d.H, rows, C), ATT_WARPS * 32, st, true, C);
+        return cudaLaunchKernelEx(&c.c, pass_attend, a);
+    };
+    TRY(norm(0, 0, 0));
+    for (int l = 0; l < L; l++) {
+        TRY(mul(K_QKV, l));
+        if (l == L - 1 && lrows == 0) break;
+        TRY(attend(l));
+        TRY(mul(K_PROJ, l));
+        TRY(norm(1, l, p.tile[K_PROJ].splits));
+        TRY(mul(K_FC, l));
+        TRY(mul(K_P2, l));
+        TRY(norm(l + 1 < L ? 2 : 3, l, p.tile[K_P2].splits));
+    }
+    if (lrows) TRY(mul(K_LOGITS, 0));
+    FinishArgs f = {};
+    f.rows = lrows; f.best = (u64*)u(p.o.best); f.skip = (int*)u(p.o.skip); f.next = (float*)d.next; f.pos = (const int*)u(p.o.pos);
+    f.t_stride = d.t_stride; f.tstep = d.tstep; f.N = d.N; f.dst = (const int*)d.dst;
+    if (d.dst) f.x = (int*)d.x_out;
+    else if (d.feedback) { f.x = (int*)d.x; f.t = (int*)d.t; f.prompt = (const int*)d.prompt; f.plen = (const int*)d.plen; f.plen_cap = d.prompt_len; }
+    Config c(dim3(1), 256, st, true);
+    TRY(cudaLaunchKernelEx(&c.c, pass_finish, f));
+    return 0;
+}
+
+}  // namespace
+
+namespace vesta_rt {
+int pass_steps(void* pass, void* stream, int steps) {
+    Pass* p = (Pass*)pass;
+    cudaStream_t st = (cudaStream_t)stream;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    TRY(cudaStreamIsCapturing(st, &cap));
+    for (int i = 0; i < steps; i++) {
+        if (cap != cudaStreamCaptureStatusNone || p->graphs.empty()) { if (int e = enqueue(*p, st, p->d.rows, p->d.logit_rows, 0)) return e; }
+        else TRY(cudaGraphLaunch(p->graphs[0], st));
+    }
+    return 0;
+}
+}  // namespace vesta_rt
+
+extern "C" {
+
+int vesta_pass_workspace(const vesta_pass_desc* d, size_t* bytes) {
+    Pass p{};
+    if (!bytes) return fail(-1, "vesta_pass_workspace: null argument");
+    if (int e = plan(p, d)) return e;
+    *bytes = p.o.total;
+    return 0;
+}
+
+int vesta_pass_create(const vesta_pass_desc* d, void* workspace, int graph, void** out) {
+    if (!out || !workspace) return fail(-1, "vesta_pass_create: null argument");
+    Pass* p = new Pass{};
+    int e = plan(*p, d);
+    p->ws = (unsigned char*)workspace;
+    const int D = d->D, F = d->F;
+    const void* w[5] = {d->qkvw, d->ow, d->fcw, d->pw, d->wte};
+    const int fold[5] = {D, D, D, F, D}, feat[5] = {3 * D, D, F, D, d->N};
+    unsigned char* op[5] = {p->ws + p->o.act, p->ws + p->o.att, p->ws + p->o.act, p->ws + p->o.gelu, p->ws + p->o.fin};
+    for (int k = 0; k < 5 && !e; k++) {
+        if (k == K_LOGITS) e = vesta_rt::tensor_map(&p->w[k], w[k], D, feat[k], 1, p->tile[k].bm);
+        else e = vesta_rt::tensor_map(&p->w[k], w[k], feat[k], fold[k], d->L, 64);
+        if (!e) e = vesta_rt::tensor_map(&p->a[k], op[k], fold[k], k == K_LOGITS ? p->fplanes : p->planes, 1, p->tile[k].bn);
+        if (!e) { const cudaError_t ce = gemm_prepare(EPI_OF[k], p->tile[k]); if (ce != cudaSuccess) e = cuda_fail(ce, "cudaFuncSetAttribute"); }
+    }
+    if (!e && graph) {
+        // a decode step as a graph, captured on a stream of its own
+        cudaStream_t st = nullptr;
+        cudaGraph_t g = nullptr;
+        cudaGraphExec_t ge = nullptr;
+        cudaError_t ce = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+        if (ce == cudaSuccess) ce = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
+        if (ce == cudaSuccess) {
+            e = enqueue(*p, st, d->rows, d->logit_rows, 0);
+            ce = cudaStreamEndCapture(st, &g);
+        }
+        if (ce == cudaSuccess && !e) ce = cudaGraphInstantiate(&ge, g, 0);
+        if (ge) p->graphs.push_back(ge);
+        if (g) cudaGraphDestroy(g);
+        if (st) cudaStreamDestroy(st);
+        if (ce != cudaSuccess && !e) e = cuda_fail(ce, "vesta_pass_create: graph of a step");
+    }
+    if (e) { vesta_pass_release(p); return e; }
+    *out = p;
+    return 0;
+}
+
+int vesta_pass_run(void* pass, void* stream, int rows, int logit_rows, int tiles) {
+    Pass* p = (Pass*)pass;
+    if (!p) return fail(-1, "vesta_pass_run: no pass");
+    if (rows < 1 || rows > p->d.rows || logit_rows < 0 || logit_rows > p->d.logit_rows || tiles < 0) return fail(-1, "vesta_pass_run: row counts outside what the pass was created for");
+    return enqueue(*p, (cudaStream_t)stream, rows, logit_rows, tiles);
+}
+
+void vesta_pass_release(void* pass) {
+    Pass* p = (Pass*)pass;
+    if (!p) return;
+    for (auto g : p->graphs) cudaGraphExecDestroy(g);
+    delete p;
+}
+
+}  // extern "C"

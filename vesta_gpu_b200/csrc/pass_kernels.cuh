@@ -1,0 +1,683 @@
+// Kernels of one forward pass over a set of rows, written for sm_100a: the rows are the sequences of a decode step or the
+// (sequence, position) pairs of prompts. A pass is a chain of small kernels per layer,
+//
+//     norm | QKV | attention | projection | norm | FC | MLP projection
+//
+// launched with programmatic stream serialization: a kernel starts while its predecessor runs, does what does not depend
+// on it (barriers, tensor memory, its weights into shared memory) and waits (griddepcontrol.wait) before it touches what
+// the predecessor writes. Measured on B200 in a CUDA graph: 1.15 to 1.25 us per kernel of such a chain, a load from L2
+// and a store included (148 blocks; 1.4 without the early start, 2.4 us and more for a barrier across one persistent
+// kernel), and the weights of several kernels ahead stream in meanwhile, as far as shared memory goes.
+//
+// Contractions (pass_gemm) run on tcgen05.mma with the output features as the rows of the product (operand A: the
+// weights as they are stored, [fold][feature], i.e. M-major; the table of the logits K-major) and the rows of the pass as
+// its columns (operand B, fp16 [row][fold]). So few rows cost few columns, and a weight element is read by one block (per tile of rows).
+// Rows whose activations are multiplied at fp32 accuracy (`rp` > 0) pass as two planes, fp16 head and fp16 remainder,
+// in the columns [0, rp) and [rp, 2 rp) of the same product.
+// No sum depends on the order in which blocks run: a fold that is cut over blocks leaves its parts in separate buffers and
+// the next norm kernel adds them in order, so a pass gives the same bits every time.
+#pragma once
+#include <cuda.h>
+#include <cuda_runtime.h>
+
+namespace vesta_pass {
+
+typedef unsigned int u32;
+typedef unsigned long long u64;
+typedef unsigned short u16;
+
+// ---- small wrappers -------------------------------------------------------------------------------------------------
+__device__ __forceinline__ u32 smem_u32(const void* p) { return (u32)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ u64 now_ns() { u64 t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); return t; }
+__device__ __forceinline__ u32 pack_h2(float lo, float hi) { u32 r; asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo)); return r; }
+__device__ __forceinline__ float h_lo(u32 w) { float f; asm("{.reg .b16 l,h; mov.b32 {l,h}, %1; cvt.f32.f16 %0, l;}" : "=f"(f) : "r"(w)); return f; }
+__device__ __forceinline__ float h_hi(u32 w) { float f; asm("{.reg .b16 l,h; mov.b32 {l,h}, %1; cvt.f32.f16 %0, h;}" : "=f"(f) : "r"(w)); return f; }
+__device__ __forceinline__ float h2f(u16 h) { float f; asm("cvt.f32.f16 %0, %1;" : "=f"(f) : "h"(h)); return f; }
+__device__ __forceinline__ u16 f2h(float f) { u16 h; asm("cvt.rn.f16.f32 %0, %1;" : "=h"(h) : "f"(f)); return h; }
+__device__ __forceinline__ float fast_exp(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f)); return y; }
+__device__ __forceinline__ void dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void mbar_init(u32 bar, u32 count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bar), "r"(count) : "memory"); }
+__device__ __forceinline__ void mbar_expect(u32 bar, u32 bytes) { asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(bytes) : "memory"); }
+__device__ __forceinline__ bool mbar_try(u32 bar, u32 parity) {
+    u32 ok;
+    asm volatile("{.reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p;}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ void tma3(u32 dst, const CUtensorMap* m, int x, int y, int z, u32 bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 :: "r"(dst), "l"(m), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
+}
+__device__ __forceinline__ u32 elect_one() {
+    u32 leader;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(leader));
+    return leader;
+}
+
+// Every wait gives up after half a second: it leaves a code in the status word and a flag that ends the block's other
+// waits, and the block runs to its end.
+#define PASS_WAIT_NS 500000000ull
+struct Wait { volatile int* dead; u32* status; };
+__device__ __noinline__ bool mbar_wait_slow(u32 bar, u32 parity, const Wait& w, u32 code) {
+    const u64 t0 = now_ns();
+    u32 spins = 0;
+    while (!mbar_try(bar, parity)) {
+        if (*w.dead) return false;
+        if ((++spins & 63u) == 0 && now_ns() - t0 > PASS_WAIT_NS) {
+            atomicCAS(w.status, 0u, code | (blockIdx.x << 16));
+            *w.dead = 1;
+            return false;
+        }
+    }
+    return true;
+}
+__device__ __forceinline__ bool mbar_wait(u32 bar, u32 parity, const Wait& w, u32 code) { return mbar_try(bar, parity) || mbar_wait_slow(bar, parity, w, code); }
+
+// ---- contractions ---------------------------------------------------------------------------------------------------
+enum { EPI_QKV = 0, EPI_PART = 1, EPI_GELU = 2, EPI_LOGITS = 3 };
+
+struct GemmArgs {
+    int layer, nfeat, kblocks, kb_per, rows, rp, stages;
+    int D;
+    const u16* bias;                 // QKV, FC: of the layer
+    float* of;                       // QKV: queries [row][D]; PART: sums [part][row][nfeat]; LOGITS: logits [row][nfeat]
+    size_t part_stride;              // floats between two parts
+    u16* oh;                         // GELU: [row][nfeat], the remainder plane rp rows further
+    u16 *kc, *vc;                    // QKV: the caches at this layer
+    const long long* rowoff;         // QKV: element offset of every row's position in the caches (-1: none)
+    const int* skip;                 // not zero: the pass was refused, nothing may be written that outlives it
+    u64* best;                       // LOGITS: packed (value, ~index) maximum of every row
+    u32* status;
+    float ga, gb, gc;
+};
+
+// shared-memory operand descriptors, 128-byte swizzle. K-major: rows of 128 bytes (64 fold indices), groups of eight rows
+// 1024 bytes apart. M-major: rows of 128 bytes hold 64 features of one fold index, groups of eight fold indices 1024
+// bytes apart, the next 64 features 8192 bytes further (one box of 64 x 64).
+__device__ __forceinline__ u64 desc_k(u32 a) { return (u64)((a & 0x3FFFFu) >> 4) | ((u64)1 << 16) | ((u64)(1024 >> 4) << 32) | ((u64)1 << 46) | ((u64)2 << 61); }
+__device__ __forceinline__ u64 desc_m(u32 a) { return (u64)((a & 0x3FFFFu) >> 4) | ((u64)(8192 >> 4) << 16) | ((u64)(1024 >> 4) << 32) | ((u64)1 << 46) | ((u64)2 << 61); }
+
+__device__ __forceinline__ void tm_ld16(u32 (&r)[16], u32 addr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
+                   "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(addr) : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+// tanh-GELU: a v (1 + tanh(b (v + c v^3))), tanh(u) = 1 - 2 / (1 + e^(2u))
+__device__ __forceinline__ float gelu_tanh(float v, float ga, float gb, float gc) {
+    const float u = gb * (v + gc * v * v * v);
+    float e, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(u * 2.8853900817779268f));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+    return ga * v * (2.0f - 2.0f * r);
+}
+// orderable key of (value, index): larger value wins, then the lower index
+__device__ __forceinline__ u64 best_key(int ordered, u32 n) { return ((u64)((u32)ordered ^ 0x80000000u) << 32) | (u64)(0xFFFFFFFFu - n); }
+
+template <int BM, int BN> struct GemmSmem {
+    static constexpr int A = BM * 128, B = BN * 128, STAGE = A + B;
+    // after the stages: full and empty barriers, "done", tensor-memory address, dead flag; row offsets or the warps' best keys
+    static constexpr int tail(int stages) { return 2 * stages * 8 + 16 + 16 + BN * 8 * 4; }
+    static constexpr int bytes(int stages) { return stages * STAGE + tail(stages) + 1024; }
+};
+
+// One tile of BM features x BN rows over kb_per blocks of 64 fold indices (blockIdx.z: which part of the fold).
+// Warp 0 loads (one lane), warp 1 issues the products (one lane), warps 2..5 read the accumulators.
+template <int BM, int BN, int EPI>
+__global__ void __launch_bounds__(192) pass_gemm(const __grid_constant__ CUtensorMap wm, const __grid_constant__ CUtensorMap am, const __grid_constant__ GemmArgs g) {
+    using S = GemmSmem<BM, BN>;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    const int st = g.stages;
+    const u32 sbase = smem_u32(smem), bars = sbase + st * S::STAGE, done = bars + 2 * st * 8;
+    unsigned char* tail = smem + st * S::STAGE + 2 * st * 8 + 16;
+    volatile int* dead = reinterpret_cast<volatile int*>(tail + 4);
+    volatile u32* tmem_p = reinterpret_cast<volatile u32*>(tail);
+    u64* side = reinterpret_cast<u64*>(tail + 16);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int TCOLS = BN < 32 ? 32 : BN;
+    const Wait w{dead, g.status};
+    if (threadIdx.x == 0) {
+        *dead = 0;
+        for (int i = 0; i < st; i++) { mbar_init(bars + i * 8, 1); mbar_init(bars + (st + i) * 8, 1); }
+        mbar_init(done, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(tail)), "n"(TCOLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    }
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (threadIdx.x == 0) dep_launch();              // (after the allocation: the blocks of the next kernel queue behind it)
+    const u32 tmem = *tmem_p;
+    const int kb0 = blockIdx.z * g.kb_per, nkb = min(g.kb_per, g.kblocks - kb0);
+    const int f0 = blockIdx.x * BM, row0 = blockIdx.y * BN;
+
+    if (warp == 0) {
+        if (elect_one()) {
+            auto load_w = [&](int s, int kb) {
+                const u32 dst = sbase + s * S::STAGE, bar = bars + s * 8;
+                if (EPI == EPI_LOGITS) tma3(dst, &wm, kb * 64, f0, 0, bar);
+                else {
+                    tma3(dst, &wm, f0, kb * 64, g.layer, bar);
+                    if (BM == 128) tma3(dst + 8192, &wm, f0 + 64, kb * 64, g.layer, bar);
+                }
+            };
+            const int pre = min(st, nkb);
+            for (int i = 0; i < pre; i++) { mbar_expect(bars + i * 8, S::STAGE); load_w(i, kb0 + i); }
+            dep_wait();
+            for (int i = 0; i < pre; i++) tma3(sbase + i * S::STAGE + S::A, &am, (kb0 + i) * 64, row0, 0, bars + i * 8);
+            int s = 0, ph = 0;
+            for (int i = pre; i < nkb; i++) {
+                if (!mbar_wait(bars + (st + s) * 8, ph, w, 0xB00u)) break;
+                mbar_expect(bars + s * 8, S::STAGE);
+                load_w(s, kb0 + i);
+                tma3(sbase + s * S::STAGE + S::A, &am, (kb0 + i) * 64, row0, 0, bars + s * 8);
+                if (++s == st) { s = 0; ph ^= 1; }
+            }
+        }
+    } else if (warp == 1) {
+        // fp32 accumulators, fp16 operands; A M-major (bit 15) except for the table of the logits
+        constexpr u32 idesc = (1u << 4) | (EPI == EPI_LOGITS ? 0u : (1u << 15)) | ((u32)(BN >> 3) << 17) | ((u32)(BM >> 4) << 24);
+        int s = 0, ph = 0;
+        const u32 leader = elect_one();
+        for (int i = 0; i < nkb; i++) {
+            const bool ok = mbar_wait(bars + s * 8, ph, w, 0xB10u);
+            if (!__all_sync(0xffffffffu, ok)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const u32 a = sbase + s * S::STAGE;
+            const u64 ad = EPI == EPI_LOGITS ? desc_k(a) : desc_m(a), bd = desc_k(a + S::A);
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                             :: "r"(tmem), "l"(ad + (EPI == EPI_LOGITS ? 2 : 128) * k), "l"(bd + 2 * k), "r"(idesc), "r"((i | k) ? 1u : 0u), "r"(leader) : "memory");
+            if (leader) {
+                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bars + (st + s) * 8) : "memory");
+                if (i == nkb - 1) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(done) : "memory");
+            }
+            __syncwarp();
+            if (++s == st) { s = 0; ph ^= 1; }
+        }
+    } else {
+        const int quarter = warp & 3, ew = warp - 2, et = threadIdx.x - 64;
+        const int fl = BM == 128 ? quarter * 32 + lane : quarter * 16 + lane;      // (a product of 64 rows leaves row m in lane 32 (m / 16) + m % 16)
+        const int f = f0 + fl;
+        const bool own = (BM == 128 || lane < 16) && f < g.nfeat;
+        float bias = 0.f;
+        if ((EPI == EPI_QKV || EPI == EPI_GELU) && own) bias = h2f(__ldg(g.bias + f));
+        dep_wait();
+        const bool skip = (EPI == EPI_QKV || EPI == EPI_LOGITS) ? __ldcg(g.skip) != 0 : false;
+        const int live = min(g.rp ? g.rp : BN, g.rows - row0);                     // rows of this tile
+        if (EPI == EPI_QKV) {
+            for (int i = et; i < BN; i += 128) side[i] = i < live ? (u64)__ldcg(g.rowoff + row0 + i) : ~0ull;
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+        }
+        const bool ok = mbar_wait(done, 0, w, 0xB20u);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (__all_sync(0xffffffffu, ok)) {
+            const u32 ta = tmem + ((u32)(quarter * 32) << 16);
+            const int part = EPI == EPI_QKV ? f / g.D : 0;                         // 0 query, 1 key, 2 value (a warp never straddles two)
+            u16* cache = EPI == EPI_QKV ? (part == 1 ? g.kc : g.vc) + (f - part * g.D) : (u16*)0;
+#pragma unroll 1
+            for (int c0 = 0; c0 < live; c0 += 16) {
+                u32 r[16];
+                tm_ld16(r, ta + c0);
+                int n = min(16, live - c0);
+                if (g.rp) {
+                    u32 q[16];
+                    if (BN >= 32) tm_ld16(q, ta + 16);
+                    n = live;
+#pragma unroll
+                    for (int i = 0; i < 16; i++) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(BN >= 32 ? q[i] : r[(i + 8) & 15]));
+                }
+#pragma unroll
+                for (int i = 0; i < 16; i++) {
+                    if (i < n) {
+                        const int row = row0 + c0 + i;
+                        float v = __uint_as_float(r[i]) + bias;
+                        if (EPI == EPI_QKV) {
+                            if (own) {
+                                if (part == 0) g.of[(size_t)row * g.D + f] = v;
+                                else {
+                                    const long long o = (long long)side[c0 + i];
+                                    if (o >= 0 && !skip) cache[o] = f2h(v);
+                                }
+                            }
+                        } else if (EPI == EPI_PART) {
+                            if (own) g.of[blockIdx.z * g.part_stride + (size_t)row * g.nfeat + f] = v;
+                        } else if (EPI == EPI_GELU) {
+                            v = gelu_tanh(v, g.ga, g.gb, g.gc);
+                            if (own) {
+                                const u16 h = f2h(v);
+                                g.oh[(size_t)row * g.nfeat + f] = h;
+                                if (g.rp) g.oh[(size_t)(g.rp + row) * g.nfeat + f] = f2h(v - h2f(h));
+                            }
+                        } else {
+                            if (own && !skip) g.of[(size_t)row * g.nfeat + f] = v;
+                            // the warp's best feature of this row: maximum by redux, lowest feature among the equal ones by ballot
+                            int kv = own ? __float_as_int(v) : __float_as_int(-3.0e38f);
+                            kv = kv >= 0 ? kv : kv ^ 0x7fffffff;
+                            const int km = __reduce_max_sync(0xffffffffu, kv);
+                            const u32 who = __ballot_sync(0xffffffffu, kv == km && own);
+                            if (lane == 0) side[ew * BN + c0 + i] = who ? best_key(km, (u32)(f - lane + (__ffs(who) - 1))) : 0ull;
+                        }
+                    }
+                }
+            }
+            if (EPI == EPI_LOGITS) {
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+                if (!skip)
+                    for (int i = et; i < live; i += 128) {
+                        u64 k = side[i];
+#pragma unroll
+                        for (int x = 1; x < 4; x++) if (side[x * BN + i] > k) k = side[x * BN + i];
+                        if (k) atomicMax(g.best + row0 + i, k);
+                    }
+            }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    }
+    __syncthreads();
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "n"(TCOLS) : "memory");
+    if (*dead && threadIdx.x == 0) {
+        // a wait ran out: let copies in flight land (bounded) before the block's shared memory goes to another
+        const u64 t0 = now_ns();
+        while (now_ns() - t0 < 2000000ull) { }
+    }
+}
+
+// ---- norm: residual sums, LayerNorm, operand ---------------------------------------------------------------------------
+enum { NORM_EMBED = 0, NORM_MID = 1, NORM_FINAL = 2 };
+struct NormArgs {
+    int D, nparts, rp;
+    float eps;
+    float* z;                        // residual stream [row][D], updated in place
+    const float* part;               // [part][row][D]: sums of the projection before this norm
+    size_t part_stride;
+    const u16 *bias, *gain, *shift;
+    u16* act;                        // [row][D] fp16 (and the remainder plane rp rows further)
+    // EMBED: tokens and positions
+    const int *x, *t, *seq;
+    int t_stride, N, cpos, tmax, L;
+    const u16 *wte, *wpe;
+    long long* rowoff;
+    int *pos, *skip;
+    u32* bar;                        // [0] status, [2] abort flag
+    const int* want;                 // FINAL: rows that want logits (0: all)
+};
+
+// One row per block, four elements per thread (the row stays in registers: one read, one write).
+template <int MODE>
+__global__ void __launch_bounds__(1024) pass_norm(const __grid_constant__ NormArgs a) {
+    __shared__ float red[2][32];
+    const int tid = threadIdx.x, d = tid * 4, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
+    const bool own = d < a.D;
+    if (tid == 0) dep_launch();
+    uint2 gw = make_uint2(0, 0), sw = make_uint2(0, 0), bw = make_uint2(0, 0);
+    if (own) {
+        gw = __ldg(reinterpret_cast<const uint2*>(a.gain + d)); sw = __ldg(reinterpret_cast<const uint2*>(a.shift + d));
+        if (MODE != NORM_EMBED) bw = __ldg(reinterpret_cast<const uint2*>(a.bias + d));
+    }
+    if (MODE != NORM_EMBED) dep_wait();
+    const int out = blockIdx.x;
+    int row = out;
+    if (MODE == NORM_FINAL && a.want) row = __ldcg(a.want + out);
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (MODE == NORM_EMBED) {
+        // tokens and positions outside their ranges would index outside the tables and the caches: the pass is refused
+        // (a negative position: a sequence that has not started, its row is carried along and writes no cache)
+        const int x = __ldcg(a.x + row), t = __ldcg(a.t + row * a.t_stride), sq = a.seq ? __ldcg(a.seq + row) : row;
+        const bool aborted = __ldcg(a.bar + 2) != 0u;
+        const bool bad = t >= a.tmax || t >= a.cpos || x < 0 || x >= a.N || aborted;
+        if (tid == 0) {
+            if (bad) { atomicExch(a.skip, 1); atomicCAS(a.bar, 0u, 0x900u); }
+            a.rowoff[row] = (bad || t < 0) ? -1ll : ((long long)sq * a.L * a.tmax + t) * a.D;
+            a.pos[row] = bad ? -1 : t;
+        }
+        if (own) {
+            const uint2 e = __ldg(reinterpret_cast<const uint2*>(a.wte + (size_t)(bad ? 0 : x) * a.D + d)), p = __ldg(reinterpret_cast<const uint2*>(a.wpe + (size_t)(bad ? 0 : max(t, 0)) * a.D + d));
+            v = make_float4(h_lo(e.x) + h_lo(p.x), h_hi(e.x) + h_hi(p.x), h_lo(e.y) + h_lo(p.y), h_hi(e.y) + h_hi(p.y));
+        }
+    } else if (own) {
+        v = __ldcg(reinterpret_cast<const float4*>(a.z + (size_t)row * a.D + d));
+        v.x += h_lo(bw.x); v.y += h_hi(bw.x); v.z += h_lo(bw.y); v.w += h_hi(bw.y);
+#pragma unroll 4
+        for (int s = 0; s < a.nparts; s++) {
+            const float4 p = __ldcg(reinterpret_cast<const float4*>(a.part + s * a.part_stride + (size_t)row * a.D + d));
+            v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
+        }
+    }
+    if (MODE != NORM_FINAL && own) *reinterpret_cast<float4*>(a.z + (size_t)row * a.D + d) = v;
+    float s = (v.x + v.y) + (v.z + v.w);
+#pragma unroll
+    for (int m = 16; m; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+    if (lane == 0) red[0][warp] = s;
+    __syncthreads();
+    s = 0.f;
+    for (int i = 0; i < nw; i++) s += red[0][i];
+    const float mean = s / a.D;
+    const float x0 = v.x - mean, x1 = v.y - mean, x2 = v.z - mean, x3 = v.w - mean;
+    float q = own ? (x0 * x0 + x1 * x1) + (x2 * x2 + x3 * x3) : 0.f;
+#pragma unroll
+    for (int m = 16; m; m >>= 1) q += __shfl_xor_sync(0xffffffffu, q, m);
+    if (lane == 0) red[1][warp] = q;
+    __syncthreads();
+    q = 0.f;
+    for (int i = 0; i < nw; i++) q += red[1][i];
+    const float rs = rsqrtf(q / a.D + a.eps);
+    if (own) {
+        const float o0 = x0 * rs * h_lo(gw.x) + h_lo(sw.x), o1 = x1 * rs * h_hi(gw.x) + h_hi(sw.x);
+        const float o2 = x2 * rs * h_lo(gw.y) + h_lo(sw.y), o3 = x3 * rs * h_hi(gw.y) + h_hi(sw.y);
+        const u32 p0 = pack_h2(o0, o1), p1 = pack_h2(o2, o3);
+        *reinterpret_cast<uint2*>(a.act + (size_t)out * a.D + d) = make_uint2(p0, p1);
+        if (a.rp) *reinterpret_cast<uint2*>(a.act + (size_t)(a.rp + out) * a.D + d) = make_uint2(pack_h2(o0 - h_lo(p0), o1 - h_hi(p0)), pack_h2(o2 - h_lo(p1), o3 - h_hi(p1)));
+    }
+}
+
+// ---- attention of one position per row (decode) -----------------------------------------------------------------------
+struct AttArgs {
+    const float* q;                  // [row][D] fp32
+    const u16 *kc, *vc;              // the caches at this layer
+    long long seq_stride;            // elements between two sequences
+    const int *pos, *seq;
+    int D, pow2, rp;
+    float scale;
+    u16* out;                        // [row][D] fp16 (and the remainder plane)
+};
+#define ATT_WARPS 4
+// Block = one (row, head), or 1 / C of its positions where C blocks form a cluster; warps take runs of 32 positions in
+// turn. A group of eight lanes reads one position's 128 bytes (16 per lane), eight positions per group and step are in flight
+// for K and for V. fp32 arithmetic on the ordinary cores: 9 warp instructions per position and head, 11 us per layer
+// at 256 sequences of 290 positions where reading the cache takes 35.
+__global__ void __launch_bounds__(ATT_WARPS * 32) pass_attend(const __grid_constant__ AttArgs a) {
+    __shared__ float part[ATT_WARPS + 1][66];
+    const int h = blockIdx.x, row = blockIdx.y, C = gridDim.z, cr = blockIdx.z;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, pl = lane >> 3, dl = lane & 7;
+    if (threadIdx.x == 0) dep_launch();
+    dep_wait();
+    const int n = __ldcg(a.pos + row) + 1, sq = a.seq ? __ldcg(a.seq + row) : row;
+    float q[8];
+    {
+        const float4* qp = reinterpret_cast<const float4*>(a.q + (size_t)row * a.D + h * 64 + dl * 8);
+        const float4 q0 = __ldcg(qp), q1 = __ldcg(qp + 1);
+        const float sc = a.pow2 ? 1.0f / a.scale : 1.0f;
+        q[0] = q0.x * sc; q[1] = q0.y * sc; q[2] = q0.z * sc; q[3] = q0.w * sc; q[4] = q1.x * sc; q[5] = q1.y * sc; q[6] = q1.z * sc; q[7] = q1.w * sc;
+    }
+    const u16* kp = a.kc + sq * a.seq_stride + h * 64 + dl * 8;
+    const u16* vp = a.vc + sq * a.seq_stride + h * 64 + dl * 8;
+    float m = -3.0e38f, den = 0.f, o[8];
+#pragma unroll
+    for (int e = 0; e < 8; e++) o[e] = 0.f;
+#pragma unroll 1
+    for (int p0 = (cr * ATT_WARPS + warp) * 32; p0 < n; p0 += C * ATT_WARPS * 32) {
+        uint4 k[8], v[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const int p = min(p0 + j * 4 + pl, n - 1);
+            k[j] = __ldcg(reinterpret_cast<const uint4*>(kp + (size_t)p * a.D));
+        }
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const int p = min(p0 + j * 4 + pl, n - 1);
+            v[j] = __ldcg(reinterpret_cast<const uint4*>(vp + (size_t)p * a.D));
+        }
+        float s[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+            s[j] = (q[0] * h_lo(k[j].x) + q[1] * h_hi(k[j].x)) + (q[2] * h_lo(k[j].y) + q[3] * h_hi(k[j].y)) +
+                   ((q[4] * h_lo(k[j].z) + q[5] * h_hi(k[j].z)) + (q[6] * h_lo(k[j].w) + q[7] * h_hi(k[j].w)));
+        // sums over the eight lanes of a group, transposed: lane dl ends with the score of position p0 + 4 dl + pl
+#pragma unroll
+        for (int j = 0; j < 4; j++) { const float keep = (dl & 4) ? s[j + 4] : s[j], give = (dl & 4) ? s[j] : s[j + 4]; s[j] = keep + __shfl_xor_sync(0xffffffffu, give, 4); }
+#pragma unroll
+        for (int j = 0; j < 2; j++) { const float keep = (dl & 2) ? s[j + 2] : s[j], give = (dl & 2) ? s[j] : s[j + 2]; s[j] = keep + __shfl_xor_sync(0xffffffffu, give, 2); }
+        { const float keep = (dl & 1) ? s[1] : s[0], give = (dl & 1) ? s[0] : s[1]; s[0] = keep + __shfl_xor_sync(0xffffffffu, give, 1); }
+        float sc = a.pow2 ? s[0] : s[0] / a.scale;
+        const bool live = p0 + dl * 4 + pl < n;
+        int km = __float_as_int(live ? sc : -3.0e38f);
+        km = __reduce_max_sync(0xffffffffu, km >= 0 ? km : km ^ 0x7fffffff);
+        const float mn = fmaxf(m, __int_as_float(km >= 0 ? km : km ^ 0x7fffffff));
+        const float corr = fast_exp(m - mn), p = live ? fast_exp(sc - mn) : 0.f;
+        m = mn;
+        den = den * corr + p;
+#pragma unroll
+        for (int e = 0; e < 8; e++) o[e] *= corr;
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const float pj = __shfl_sync(0xffffffffu, p, (lane & 24) | j);
+            o[0] += pj * h_lo(v[j].x); o[1] += pj * h_hi(v[j].x); o[2] += pj * h_lo(v[j].y); o[3] += pj * h_hi(v[j].y);
+            o[4] += pj * h_lo(v[j].z); o[5] += pj * h_hi(v[j].z); o[6] += pj * h_lo(v[j].w); o[7] += pj * h_hi(v[j].w);
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < 8; e++) { o[e] += __shfl_xor_sync(0xffffffffu, o[e], 8); o[e] += __shfl_xor_sync(0xffffffffu, o[e], 16); }
+#pragma unroll
+    for (int x = 16; x; x >>= 1) den += __shfl_xor_sync(0xffffffffu, den, x);
+    if (lane == 0) { part[warp][64] = m; part[warp][65] = den; }
+    if (lane < 8)
+#pragma unroll
+        for (int e = 0; e < 8; e++) part[warp][dl * 8 + e] = o[e];
+    __syncthreads();
+    float M = -3.0e38f, dd = 0.f, num = 0.f;
+    if (threadIdx.x < 64) {
+#pragma unroll
+        for (int i = 0; i < ATT_WARPS; i++) M = fmaxf(M, part[i][64]);
+#pragma unroll
+        for (int i = 0; i < ATT_WARPS; i++) { const float c = fast_exp(part[i][64] - M); dd += part[i][65] * c; num += part[i][threadIdx.x] * c; }
+    }
+    if (C > 1) {
+        // the blocks of a cluster: their results meet in the first one
+        if (threadIdx.x < 64) { part[ATT_WARPS][threadIdx.x] = num; if (threadIdx.x == 0) { part[ATT_WARPS][64] = M; part[ATT_WARPS][65] = dd; } }
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (cr == 0 && threadIdx.x < 64) {
+            float mm[8], de[8], nu[8];
+            const u32 mine = smem_u32(&part[ATT_WARPS][0]);
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                mm[i] = -3.0e38f; de[i] = 0.f; nu[i] = 0.f;
+                if (i < C) {
+                    u32 r;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(mine), "r"(i));
+                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(mm[i]) : "r"(r + 64 * 4) : "memory");
+                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(de[i]) : "r"(r + 65 * 4) : "memory");
+                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(nu[i]) : "r"(r + threadIdx.x * 4) : "memory");
+                }
+            }
+            M = -3.0e38f; dd = 0.f; num = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; i++) M = fmaxf(M, mm[i]);
+#pragma unroll
+            for (int i = 0; i < 8; i++) { const float c = fast_exp(mm[i] - M); dd += de[i] * c; num += nu[i] * c; }
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (cr != 0) return;
+    }
+    if (threadIdx.x < 64) {
+        const float r = dd > 0.f ? __fdividef(num, dd) : 0.f;                      // a sequence that has not started attends to nothing
+        const u16 hi = f2h(r);
+        a.out[(size_t)row * a.D + h * 64 + threadIdx.x] = hi;
+        if (a.rp) a.out[(size_t)(a.rp + row) * a.D + h * 64 + threadIdx.x] = f2h(r - h2f(hi));
+    }
+}
+
+// ---- attention of many positions (prompts) ----------------------------------------------------------------------------
+struct AttManyArgs {
+    const float* q;
+    const u16 *kc, *vc;
+    long long seq_stride;
+    const int4* tiles;               // (first row, rows, sequence, first position) of every run of at most 64 rows of one sequence
+    int D, pow2;
+    float scale;
+    u16* out;
+};
+__device__ __forceinline__ int kv_off(int row, int piece) { return row * 128 + ((piece ^ (row & 7)) << 4); }
+__device__ __forceinline__ void cp16(u32 dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ void ldsm4(u32 (&r)[4], u32 p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(p) : "memory");
+}
+__device__ __forceinline__ void ldsm4t(u32 (&r)[4], u32 p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(p) : "memory");
+}
+__device__ __forceinline__ void mma16816(float (&c)[4], const u32 (&a)[4], u32 b0, u32 b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// Block = up to 64 consecutive positions of one sequence x one head, sixteen per warp; the cache in tiles of 64 positions,
+// double buffered; causal. Queries and weights enter the products as fp16 head and fp16 remainder (two products each),
+// as in the decode kernels: scores and output at fp32 accuracy over the fp16 cache.
+__global__ void __launch_bounds__(128) pass_attend_many(const __grid_constant__ AttManyArgs a) {
+    __shared__ __align__(128) unsigned char kv[2][2][64 * 128];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    if (threadIdx.x == 0) dep_launch();
+    const int4 tl = __ldg(a.tiles + blockIdx.x);
+    const int h = blockIdx.y, row0 = tl.x, nrows = tl.y, pos0 = tl.w;
+    dep_wait();
+    const u16* kp = a.kc + tl.z * a.seq_stride + h * 64;
+    const u16* vp = a.vc + tl.z * a.seq_stride + h * 64;
+    const int total = pos0 + nrows, ntiles = (total + 63) / 64;
+    auto fetch = [&](int j) {
+        const u32 ks = smem_u32(kv[j & 1][0]), vs = smem_u32(kv[j & 1][1]);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int e = threadIdx.x + i * 128, r = e >> 3, c = e & 7;
+            const size_t off = (size_t)min(j * 64 + r, total - 1) * a.D + c * 8;
+            cp16(ks + kv_off(r, c), kp + off);
+            cp16(vs + kv_off(r, c), vp + off);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0);
+    u32 qh[4][4], ql[4][4];
+    const int rA = warp * 16 + g, rB = rA + 8;
+    {
+        const float sc = a.pow2 ? 1.0f / a.scale : 1.0f;
+        const float* qa = a.q + (size_t)(row0 + min(rA, nrows - 1)) * a.D + h * 64 + 2 * t;
+        const float* qb = a.q + (size_t)(row0 + min(rB, nrows - 1)) * a.D + h * 64 + 2 * t;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            float2 x[4];
+            x[0] = __ldcg(reinterpret_cast<const float2*>(qa + k * 16)); x[1] = __ldcg(reinterpret_cast<const float2*>(qb + k * 16));
+            x[2] = __ldcg(reinterpret_cast<const float2*>(qa + k * 16 + 8)); x[3] = __ldcg(reinterpret_cast<const float2*>(qb + k * 16 + 8));
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float u = x[i].x * sc, v = x[i].y * sc;
+                qh[k][i] = pack_h2(u, v);
+                ql[k][i] = pack_h2(u - h_lo(qh[k][i]), v - h_hi(qh[k][i]));
+            }
+        }
+    }
+    float mA = -3.0e38f, mB = -3.0e38f, dA = 0.f, dB = 0.f, o[8][4];
+#pragma unroll
+    for (int n = 0; n < 8; n++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) o[n][i] = 0.f;
+#pragma unroll 1
+    for (int j = 0; j < ntiles; j++) {
+        if (j + 1 < ntiles) { fetch(j + 1); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+        else asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        const u32 ks = smem_u32(kv[j & 1][0]), vs = smem_u32(kv[j & 1][1]);
+        float s[8][4];
+#pragma unroll
+        for (int n = 0; n < 8; n++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) s[n][i] = 0.f;
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+#pragma unroll
+            for (int n = 0; n < 8; n += 2) {
+                u32 b[4];
+                ldsm4(b, ks + kv_off(n * 8 + (lane & 7) + ((lane >> 4) << 3), k * 2 + ((lane >> 3) & 1)));
+                mma16816(s[n], qh[k], b[0], b[1]); mma16816(s[n + 1], qh[k], b[2], b[3]);
+                mma16816(s[n], ql[k], b[0], b[1]); mma16816(s[n + 1], ql[k], b[2], b[3]);
+            }
+        const int pA = pos0 + rA - j * 64, pB = pA + 8;                            // last position of the tile that the rows see
+        float xA = -3.0e38f, xB = -3.0e38f;
+#pragma unroll
+        for (int n = 0; n < 8; n++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                if (!a.pow2) s[n][i] /= a.scale;
+                if (n * 8 + 2 * t + (i & 1) > ((i & 2) ? pB : pA)) s[n][i] = -3.0e38f;
+                if (i & 2) xB = fmaxf(xB, s[n][i]); else xA = fmaxf(xA, s[n][i]);
+            }
+        xA = fmaxf(xA, __shfl_xor_sync(0xffffffffu, xA, 1)); xA = fmaxf(xA, __shfl_xor_sync(0xffffffffu, xA, 2));
+        xB = fmaxf(xB, __shfl_xor_sync(0xffffffffu, xB, 1)); xB = fmaxf(xB, __shfl_xor_sync(0xffffffffu, xB, 2));
+        const float nA = fmaxf(mA, xA), nB = fmaxf(mB, xB), cA = fast_exp(mA - nA), cB = fast_exp(mB - nB);
+        mA = nA; mB = nB; dA *= cA; dB *= cB;
+#pragma unroll
+        for (int n = 0; n < 8; n++) {
+            o[n][0] *= cA; o[n][1] *= cA; o[n][2] *= cB; o[n][3] *= cB;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                s[n][i] = s[n][i] > -1.0e38f ? fast_exp(s[n][i] - ((i & 2) ? nB : nA)) : 0.f;
+                if (i & 2) dB += s[n][i]; else dA += s[n][i];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            u32 ph[4], pr[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float u = s[2 * k + (i >> 1)][(i & 1) * 2], v = s[2 * k + (i >> 1)][(i & 1) * 2 + 1];
+                ph[i] = pack_h2(u, v);
+                pr[i] = pack_h2(u - h_lo(ph[i]), v - h_hi(ph[i]));
+            }
+#pragma unroll
+            for (int n = 0; n < 8; n += 2) {
+                u32 b[4];
+                ldsm4t(b, vs + kv_off(k * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, n + (lane >> 4)));
+                mma16816(o[n], ph, b[0], b[1]); mma16816(o[n + 1], ph, b[2], b[3]);
+                mma16816(o[n], pr, b[0], b[1]); mma16816(o[n + 1], pr, b[2], b[3]);
+            }
+        }
+        __syncthreads();
+    }
+    dA += __shfl_xor_sync(0xffffffffu, dA, 1); dA += __shfl_xor_sync(0xffffffffu, dA, 2);
+    dB += __shfl_xor_sync(0xffffffffu, dB, 1); dB += __shfl_xor_sync(0xffffffffu, dB, 2);
+    const float iA = dA > 0.f ? __fdividef(1.0f, dA) : 0.f, iB = dB > 0.f ? __fdividef(1.0f, dB) : 0.f;
+#pragma unroll
+    for (int n = 0; n < 8; n++) {
+        if (rA < nrows) *reinterpret_cast<u32*>(a.out + (size_t)(row0 + rA) * a.D + h * 64 + n * 8 + 2 * t) = pack_h2(o[n][0] * iA, o[n][1] * iA);
+        if (rB < nrows) *reinterpret_cast<u32*>(a.out + (size_t)(row0 + rB) * a.D + h * 64 + n * 8 + 2 * t) = pack_h2(o[n][2] * iB, o[n][3] * iB);
+    }
+}
+
+// ---- the end of a pass: the chosen tokens, feedback ---------------------------------------------------------------------
+struct FinishArgs {
+    int rows;
+    u64* best;
+    int* skip;
+    float* next;                     // decode: the chosen tokens as float (0: none)
+    const int* pos;
+    int *x, *t;                      // fed back (0: no feedback)
+    int t_stride, tstep, N;
+    const int *prompt, *plen;
+    int plen_cap;
+    const int *dst;                  // prompts: where in x the row's token goes
+};
+__global__ void __launch_bounds__(256) pass_finish(const __grid_constant__ FinishArgs a) {
+    dep_wait();
+    const bool skip = __ldcg(a.skip) != 0;
+    for (int b = threadIdx.x; b < a.rows; b += blockDim.x) {
+        const u64 k = __ldcg(a.best + b);
+        a.best[b] = 0ull;
+        if (skip) continue;
+        const u32 n = 0xFFFFFFFFu - (u32)(k & 0xFFFFFFFFull);
+        if (a.next) a.next[b] = (float)n;
+        if (a.dst) { a.x[__ldg(a.dst + b)] = (n >= (u32)a.N) ? 0 : (int)n; continue; }
+        if (a.x) {
+            int nx = (int)n;
+            const int tn = a.pos[b] + a.tstep;
+            if (a.plen && tn >= 0 && tn < a.plen[b]) nx = a.prompt[(size_t)b * a.plen_cap + tn];
+            a.x[b] = (nx < 0 || nx >= a.N) ? 0 : nx;
+            if (a.t_stride || b == 0) a.t[b * a.t_stride] = tn;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) *a.skip = 0;
+}
+
+}  // namespace vesta_pass

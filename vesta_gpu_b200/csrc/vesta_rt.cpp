@@ -10,6 +10,7 @@
 #include <string>
 #include <vector>
 
+#include "rt_internal.h"
 #include "vesta_b200.h"
 
 namespace {
@@ -123,6 +124,7 @@ int rtc_open() {
 }
 
 struct Bound {
+    void* pass = nullptr;            // a decode step as a chain of kernels (pass.cu) instead of one function
     CUfunction fn;
     unsigned grid, block, smem;
     std::vector<unsigned long long> vals;
@@ -130,6 +132,29 @@ struct Bound {
 };
 
 }  // namespace
+
+namespace vesta_rt {
+int fail(int code, const std::string& what) { return ::fail(code, what); }
+
+int tensor_map(void* out, const void* base, unsigned long long d0, unsigned long long d1, unsigned long long d2, unsigned box1) {
+    if (!out || !base) return ::fail(-1, "tensor map: null argument");
+    if (int e = driver()) return e;
+    if (box1 == 0 || box1 > 256u || (d0 * 2ull) % 16ull) return ::fail(-1, "tensor map: at most 256 rows per box, rows a multiple of 16 bytes");
+    // fp16 [d2][d1][d0], box = box1 rows of 64 elements of one plane; 128-byte swizzle: the 16-byte piece c of row r lands at
+    // piece c ^ (r % 8) of its 128-byte row in shared memory
+    const cuuint64_t dims[3] = {d0, d1, d2};
+    const cuuint64_t strides[2] = {d0 * 2ull, d1 * d0 * 2ull};
+    const cuuint32_t box[3] = {64, box1, 1};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    CUtensorMap tm;
+    CUresult r = g_cu.TensorMapEncodeTiled(&tm, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return cu(r, "cuTensorMapEncodeTiled");
+    memcpy(out, &tm, sizeof(tm));
+    return 0;
+}
+}  // namespace vesta_rt
 
 extern "C" {
 
@@ -267,6 +292,7 @@ int vesta_step_run(void* bound, void* stream, int steps) {
     if (!bound) return fail(-1, "vesta_step_run: not bound");
     if (int e = driver()) return e;
     Bound* b = (Bound*)bound;
+    if (b->pass) return vesta_rt::pass_steps(b->pass, stream, steps);
     for (int i = 0; i < steps; i++) {
         CUresult r = g_cu.LaunchCooperative(b->fn, b->grid, 1, 1, b->block, 1, 1, b->smem, (CUstream)stream, b->ptrs.data());
         if (r != CUDA_SUCCESS) return cu(r, "cuLaunchCooperativeKernel");
@@ -285,8 +311,11 @@ int vesta_step_host(void* bound, void* stream, unsigned long long tokens_dev, co
         r = g_cu.MemcpyHtoDAsync((CUdeviceptr)tokens_dev, tokens_host, tokens_bytes, st);
         if (r != CUDA_SUCCESS) return cu(r, "cuMemcpyHtoDAsync");
     }
-    r = g_cu.LaunchCooperative(b->fn, b->grid, 1, 1, b->block, 1, 1, b->smem, st, b->ptrs.data());
-    if (r != CUDA_SUCCESS) return cu(r, "cuLaunchCooperativeKernel");
+    if (b->pass) { if (int e = vesta_rt::pass_steps(b->pass, stream, 1)) return e; }
+    else {
+        r = g_cu.LaunchCooperative(b->fn, b->grid, 1, 1, b->block, 1, 1, b->smem, st, b->ptrs.data());
+        if (r != CUDA_SUCCESS) return cu(r, "cuLaunchCooperativeKernel");
+    }
     if (result_host && result_bytes) {
         r = g_cu.MemcpyDtoHAsync(result_host, (CUdeviceptr)result_dev, result_bytes, st);
         if (r != CUDA_SUCCESS) return cu(r, "cuMemcpyDtoHAsync");
@@ -299,28 +328,16 @@ int vesta_step_host(void* bound, void* stream, unsigned long long tokens_dev, co
 int vesta_tensor_map_rows(void* out, const void* base, unsigned long long row_elems, unsigned long long rows,
                           unsigned long long planes, unsigned box_elems, unsigned box_rows) {
     if (!out || !base) return fail(-1, "vesta_tensor_map_rows: null argument");
-    if (int e = driver()) return e;
     if (box_elems * 2u != 128u || box_rows == 0 || box_rows > 256u || (row_elems * 2ull) % 16ull)
         return fail(-1, "vesta_tensor_map_rows: the box must be 128 bytes wide, at most 256 rows, rows a multiple of 16 bytes");
-    // fp16 [planes][rows][row_elems]; box = box_rows rows of 64 elements of one plane; 128-byte swizzle: the 16-byte
-    // piece c of row r lands at piece c ^ (r % 8) of its 128-byte row in shared memory
-    const cuuint64_t dims[3] = {row_elems, rows, planes};
-    const cuuint64_t strides[2] = {row_elems * 2ull, rows * row_elems * 2ull};
-    const cuuint32_t box[3] = {box_elems, box_rows, 1};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    CUtensorMap tm;
-    CUresult r = g_cu.TensorMapEncodeTiled(&tm, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, const_cast<void*>(base), dims, strides, box, estr,
-                                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return cu(r, "cuTensorMapEncodeTiled");
-    memcpy(out, &tm, sizeof(tm));
-    return 0;
+    return vesta_rt::tensor_map(out, base, row_elems, rows, planes, box_rows);
 }
 
 int vesta_step_run_fused(void* bound, void* stream, int steps, int per_launch) {
     if (!bound) return fail(-1, "vesta_step_run_fused: not bound");
     if (int e = driver()) return e;
     Bound* b = (Bound*)bound;
+    if (b->pass) return per_launch < 1 ? fail(-1, "vesta_step_run_fused: bad argument") : vesta_rt::pass_steps(b->pass, stream, steps);
     if (b->vals.empty() || per_launch < 1) return fail(-1, "vesta_step_run_fused: bad argument");
     while (steps > 0) {
         const int n = steps < per_launch ? steps : per_launch;
@@ -333,6 +350,18 @@ int vesta_step_run_fused(void* bound, void* stream, int steps, int per_launch) {
     return 0;
 }
 
-void vesta_step_release(void* bound) { delete (Bound*)bound; }
+int vesta_pass_bind(void* pass, void** bound) {
+    if (!pass || !bound) return fail(-1, "vesta_pass_bind: null argument");
+    Bound* b = new Bound;
+    b->pass = pass;
+    *bound = b;
+    return 0;
+}
+
+void vesta_step_release(void* bound) {
+    Bound* b = (Bound*)bound;
+    if (b && b->pass) vesta_pass_release(b->pass);
+    delete b;
+}
 
 }  // extern "C"

@@ -17,6 +17,7 @@ import torch
 from . import PROGRAMS
 from .launch import Kernel, TORCH_DT
 from .lower import lower
+from .passes import PromptPass
 from .program_text import decode_program
 from .shapes import Shape
 
@@ -42,6 +43,10 @@ def shape_of(W, heads=None):
     L, _, F = W['fcw'].shape
     H = heads or D // E_HEAD
     return Shape('model', L=L, D=D, H=H, E=D // H, F=F, N=N, C=W['wpe'].shape[0])
+
+
+# rows per dense pass of prefill(): a pass that holds more rows fills the GPU better, up to where all SMs are busy in every kernel
+PREFILL_ROWS = (128, 256, 512, 1024, 2048, 4096, 8192, 16384)
 
 
 class VestaGPT2:
@@ -109,10 +114,9 @@ class VestaGPT2:
         self.k.step_host(self.x, tokens_host, nv, next_host)
 
     def prefill(self, tokens, lengths=None, rows=None):
-        """consume whole prompts as dense passes: all prompt positions of all sequences are cut into launches of `rows`
-        (sequence, position) rows (default 1024 from 1 K positions, 256 from 256, else 128) through the large-batch kernel: tensor-core
-        contractions where the shape allows, every row's K and V written before any row attends, so a row sees the rows
-        of its own sequence before it. On return the cache holds every prompt position, x the first generated token
+        """consume whole prompts as dense passes: all prompt positions of all sequences are cut into passes of at most `rows`
+        (sequence, position) rows (default: the smallest of PREFILL_ROWS that holds them all, or its largest), see
+        passes.PromptPass. On return the cache holds every prompt position, x the first generated token
         of every sequence and t its position (= its prompt length). tokens: int array (batch, P); lengths: (batch,) or
         None for P everywhere (lengths that differ need per_sequence_t=True).
         The reference feeds the prompt one position per step (bench/g0_bench.py:172-173); prefill_stepwise does the same
@@ -128,10 +132,10 @@ class VestaGPT2:
         if self.t.numel() == 1 and lens.min() != lens.max():
             raise ValueError('prompts of different lengths need per_sequence_t=True')
         total = int(lens.sum())
-        rows = int(rows or (1024 if total >= 1024 else 256 if total >= 256 else 128))
+        rows = int(rows or next((r for r in PREFILL_ROWS if total <= r), PREFILL_ROWS[-1]))
         eng = self._prefill_engines.get(rows)
         if eng is None:
-            eng = self._prefill_engines[rows] = _PrefillRows(self, rows)
+            eng = self._prefill_engines[rows] = PromptPass(self, rows)
         self.reset()
         first = eng.run(tokens, lens)
         self.x.copy_(first)
@@ -191,56 +195,4 @@ class VestaGPT2:
         return 2 * sh.L * self.B * n_ctx * sh.D * self.keys.element_size()
 
 
-class _PrefillRows:
-    """The dense prompt pass behind VestaGPT2.prefill: a second lowering of the same program for `rows` rows of
-    (cache sequence, position) that share the model's weights and caches (lower(..., row_seq=True))."""
-
-    def __init__(self, model, rows):
-        dev, sh = model.device, model.shape
-        self.model, self.R = model, rows
-        self.x = torch.zeros(rows, dtype=torch.int32, device=dev)
-        self.t = torch.full((rows,), -1, dtype=torch.int32, device=dev)
-        self.seq = torch.zeros(rows, dtype=torch.int32, device=dev)
-        R = {'x': self.x, 't': self.t, **model.W, 'keys': model.keys, 'vals': model.vals}
-        names = {torch.int32: 'i32', torch.float16: 'f16', torch.float32: 'f32'}
-        spec = {n: (tuple(v.shape), names[v.dtype]) for n, v in R.items()}
-        sms = torch.cuda.get_device_properties(dev).multi_processor_count
-        tune = dict(model._tune or {})
-        tune.setdefault('ln_dist', True)            # rows normalised once on the grid: what the tensor-core contractions read
-        self.low = lower(model._text, spec, axis_max={'s': model.tmax}, batch=rows, per_token=('x', 'keys', 'vals', 't'),
-                         outputs=('logit', 'next'), feedback=None, grid=sms, row_seq=True, tune=tune)
-        self.k = Kernel(self.low, device=dev.index)
-        self.k.bind(dict(R, row_seq=self.seq))
-
-    def run(self, tokens, lens):
-        """tokens (B, P), lens (B,) numpy -> int32 tensor (B,) on the device: the token chosen after every prompt"""
-        import numpy as np
-        B, R = tokens.shape[0], self.R
-        seqs = np.repeat(np.arange(B, dtype=np.int32), lens)
-        pos = np.concatenate([np.arange(n, dtype=np.int32) for n in lens])
-        tok = tokens[seqs, pos].astype(np.int32)
-        first = torch.zeros(B, dtype=torch.int32, device=self.model.device)
-        for i in range(0, len(seqs), R):
-            n = min(R, len(seqs) - i)
-            x, t, s = np.zeros(R, np.int32), np.full(R, -1, np.int32), np.zeros(R, np.int32)
-            x[:n], t[:n], s[:n] = tok[i:i + n], pos[i:i + n], seqs[i:i + n]
-            # Only the last position of a prompt needs logits: those rows go first (the order of the rows is free), all
-            # others carry the kernel's "nobody reads these logits" mark, and the logits phase runs for the slabs of
-            # 64 rows that hold an unmarked row (none, in most launches of a long prompt).
-            want = np.zeros(R, bool)
-            want[:n] = t[:n] == lens[s[:n]] - 1
-            order = np.argsort(~want, kind='stable')
-            x, t, s, want = x[order], t[order], s[order], want[order]
-            self.x.copy_(torch.from_numpy(x)); self.t.copy_(torch.from_numpy(t))
-            self.seq.copy_(torch.from_numpy(np.where(want, s, s | ROW_NO_LOGITS).astype(np.int32)))
-            self.k.launch()
-            last = np.flatnonzero(want)                                # rows that are the last position of their prompt
-            if len(last):
-                rows = torch.from_numpy(last).to(self.model.device)
-                first[torch.from_numpy(s[last].astype(np.int64)).to(self.model.device)] = self.k.view('next')[rows].to(torch.int32)
-        self.k.check()
-        return first
-
-
-ROW_NO_LOGITS = 0x40000000         # mark in row_seq (csrc/step_kernel.cuh): nobody reads the logits of this row
 DEFAULT_PROGRAM = PROGRAMS / 'gpt2.vst'

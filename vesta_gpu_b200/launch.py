@@ -55,6 +55,12 @@ def lib():
         L.vesta_step_host.argtypes = [vp, vp, ctypes.c_ulonglong, vp, sz, ctypes.c_ulonglong, vp, sz]
         L.vesta_step_release.argtypes = [vp]
         L.vesta_step_release.restype = None
+        L.vesta_pass_workspace.argtypes = [vp, ctypes.POINTER(sz)]
+        L.vesta_pass_create.argtypes = [vp, vp, ci, ctypes.POINTER(vp)]
+        L.vesta_pass_run.argtypes = [vp, vp, ci, ci, ci]
+        L.vesta_pass_bind.argtypes = [vp, ctypes.POINTER(vp)]
+        L.vesta_pass_release.argtypes = [vp]
+        L.vesta_pass_release.restype = None
         _lib = L
     return _lib
 
@@ -99,7 +105,7 @@ def compile_cubin(src, arch=ARCH, cache=True):
 
 
 STATUS_WHERE = {0x100: 'grid barrier', 0x200: 'weight stream (producer)', 0x300: 'weight stream (consumer)', 0x400: 'step flag', 0x500: 'K/V tile', 0x600: 'logits operand', 0x700: 'tensor-core tile', 0x800: 'K/V stage (producer)',
-                0x900: 'token or position out of range', 0xA00: 'exchange between CTAs (tagged values)'}
+                0x900: 'token or position out of range', 0xA00: 'exchange between CTAs (tagged values)', 0xB00: 'operands of a contraction'}
 
 
 class Kernel:
