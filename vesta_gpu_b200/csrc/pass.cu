@@ -43,20 +43,42 @@ struct Pass {
 // rows of an operand: one product column per row; up to 16 rows at fp32 accuracy take two planes of 8 or 16
 int plane_rows(int rows, bool exact) { return !exact ? 0 : rows <= 8 ? 8 : 16; }
 
-// Tile sizes of a contraction of `feat` features over `kb` blocks of 64 for `rows` rows (columns of the product).
+// Tile sizes of a contraction of `feat` features over `kb` blocks of 64 for `rows` rows (columns of the product), from a
+// model of the kernel's time in microseconds, fitted to measurements on B200 (rows 16 to 16,384, folds of 768 to 6,400,
+// tiles of 16 to 256 rows; within 15 % of each):
+//   BM = 64 (one tile per block, whole share of the weights in flight): 1.75 + 0.22 per stage + the operand's rows;
+//   BM = 128: 2.2 + 0.0065 bn for the first fill and the last epilogue, then per block of the fold the larger of the products
+//     (2 bn cycles) and the loads (340 + 0.45 bn cycles), times the tiles a block takes in turn.
+// A cut fold (projections) costs its parts once more in the norm that adds them: 0.25 us and 3 MB of traffic at 4 TB/s each.
 Tile choose(int kind, int rows, int rp, int feat, int kb, int sms) {
-    Tile t;
+    Tile best = {};
+    double best_t = 1e30;
     const int cols = rp ? 2 * rp : rows;
-    t.bn = cols <= 16 ? 16 : cols <= 32 ? 32 : cols <= 64 ? 64 : 128;
-    t.bm = t.bn <= 64 ? 64 : 128;
-    const int tiles = ((feat + t.bm - 1) / t.bm) * (rp ? 1 : (rows + t.bn - 1) / t.bn);
-    t.splits = 1;
-    if (kind == K_PROJ || kind == K_P2) t.splits = std::max(1, std::min(std::min(8, kb), (sms + tiles / 2) / tiles));
-    const int per = (kb + t.splits - 1) / t.splits;
-    t.splits = (kb + per - 1) / per;
-    const int stage = (t.bm + t.bn) * 128;
-    t.stages = std::max(2, std::min(per, (112 * 1024 - 1024 - 5120) / (stage + 16)));
-    return t;
+    const bool cut = kind == K_PROJ || kind == K_P2;
+    for (int bm = 64; bm <= 128; bm += 64)
+        for (int bn = 16; bn <= (bm == 64 ? 64 : 256); bn += 16) {
+            if (rp && (bm != 64 || bn != cols)) continue;
+            if (bn > 16 && bn - 16 >= cols) continue;
+            const int ks = bm == 64 ? GemmShape<64>::KS : GemmShape<128>::KS;
+            const int stage = bm == 64 ? GemmShape<64>::stage(bn) : GemmShape<128>::stage(bn);
+            const int room = 227 * 1024 - 1024 - 1024 - bn * 32;
+            const int tiles = ((feat + bm - 1) / bm) * (rp ? 1 : (rows + bn - 1) / bn);
+            for (int sp = 1; sp <= (cut ? 8 : 1); sp++) {
+                Tile t;
+                t.bm = bm; t.bn = bn;
+                const int per = (kb + sp - 1) / sp, nst = (per + ks - 1) / ks;
+                t.splits = (kb + per - 1) / per;
+                if (t.splits != sp) continue;
+                const int waves = (tiles * sp + sms - 1) / sms;
+                t.stages = std::max(1, std::min(bm == 64 || waves == 1 ? nst : 16, room / (stage + 16)));
+                double us;
+                if (bm == 64) us = (1.75 + 0.22 * nst + 0.0023 * (bn - 16) * per) * (kind == K_LOGITS ? 1 : waves) + 0.002 * tiles * sp;
+                else us = 2.2 + 0.0065 * bn + waves * per * std::max(2.0 * bn + 30, 340 + 0.45 * bn) / 1900;
+                if (cut) us += sp * (0.25 + (double)rows * feat * 4 / 4e6);
+                if (us < best_t) { best_t = us; best = t; }
+            }
+        }
+    return best;
 }
 
 Layout layout(const Pass& p, int D, int F, int rows, int lrows) {
@@ -67,7 +89,7 @@ Layout layout(const Pass& p, int D, int F, int rows, int lrows) {
     o.q = take((size_t)rows * D * 4);
     o.act = take((size_t)p.planes * D * 2);
     o.att = take((size_t)p.planes * D * 2);
-    o.gelu = take((size_t)p.planes * F * 2);
+    o.gelu = take((size_t)p.planes * F * 2 + 128);       // (the last block of the fold may reach past the last row)
     o.part = take((size_t)p.max_parts * rows * D * 4);
     o.fin = take((size_t)p.fplanes * D * 2);
     o.best = take((size_t)lrows * 8);
@@ -103,26 +125,26 @@ int plan(Pass& p, const vesta_pass_desc* d) {
     return 0;
 }
 
-template <int BM, int BN, int EPI>
-cudaError_t launch_gemm(const cudaLaunchConfig_t& c, const CUtensorMap& w, const CUtensorMap& a, const GemmArgs& g) {
-    return cudaLaunchKernelEx(&c, pass_gemm<BM, BN, EPI>, w, a, g);
+template <int BM, int EPI>
+cudaError_t launch_gemm(cudaLaunchConfig_t& c, const Tile& t, const CUtensorMap& w, const CUtensorMap& a, const GemmArgs& g) {
+    c.dynamicSmemBytes = GemmShape<BM>::bytes(t.stages, t.bn);
+    c.blockDim = dim3(GemmShape<BM>::THREADS);
+    return cudaLaunchKernelEx(&c, pass_gemm<BM, EPI>, w, a, g);
 }
-template <int BM, int BN, int EPI>
-cudaError_t prepare_gemm(int stages) {
-    return cudaFuncSetAttribute(pass_gemm<BM, BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<BM, BN>::bytes(stages));
+template <int BM, int EPI>
+cudaError_t prepare_gemm(const Tile& t) {
+    return cudaFuncSetAttribute(pass_gemm<BM, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
 }
 // one case per tile shape and epilogue
-#define SHAPES(X, EPI) X(64, 16, EPI) X(64, 32, EPI) X(64, 64, EPI) X(128, 128, EPI)
-#define EACH(X) SHAPES(X, EPI_QKV) SHAPES(X, EPI_PART) SHAPES(X, EPI_GELU) SHAPES(X, EPI_LOGITS)
-
+#define EACH(X) X(64, EPI_QKV) X(64, EPI_PART) X(64, EPI_GELU) X(64, EPI_LOGITS) X(128, EPI_QKV) X(128, EPI_PART) X(128, EPI_GELU) X(128, EPI_LOGITS)
 cudaError_t gemm(int epi, const Tile& t, cudaLaunchConfig_t c, const CUtensorMap& w, const CUtensorMap& a, const GemmArgs& g) {
-#define ONE(M, N, E) if (epi == E && t.bm == M && t.bn == N) { c.dynamicSmemBytes = GemmSmem<M, N>::bytes(t.stages); return launch_gemm<M, N, E>(c, w, a, g); }
+#define ONE(M, E) if (epi == E && t.bm == M) return launch_gemm<M, E>(c, t, w, a, g);
     EACH(ONE)
 #undef ONE
     return cudaErrorInvalidValue;
 }
 cudaError_t gemm_prepare(int epi, const Tile& t) {
-#define ONE(M, N, E) if (epi == E && t.bm == M && t.bn == N) return prepare_gemm<M, N, E>(t.stages);
+#define ONE(M, E) if (epi == E && t.bm == M) return prepare_gemm<M, E>(t);
     EACH(ONE)
 #undef ONE
     return cudaErrorInvalidValue;
@@ -178,10 +200,11 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles) {
             g.bias = f16(d.qkvb, (size_t)l * 3 * D); g.of = (float*)u(p.o.q); g.rowoff = (const long long*)u(p.o.rowoff);
             g.kc = (u16*)d.keys + (size_t)l * d.tmax * D; g.vc = (u16*)d.vals + (size_t)l * d.tmax * D;
         } else if (kind == K_FC) {
-            g.bias = f16(d.fcb, (size_t)l * F); g.oh = (u16*)u(p.o.gelu); g.ga = d.gelu_a; g.gb = d.gelu_b; g.gc = d.gelu_c;
+            g.bias = f16(d.fcb, (size_t)l * F); g.oh = (u16*)u(p.o.gelu); g.a2 = 2 * d.gelu_a; g.k1 = d.gelu_b * 2.8853900817779268f; g.k2 = d.gelu_c * g.k1;
         } else if (kind == K_LOGITS) { g.of = (float*)d.logits; g.best = (u64*)u(p.o.best); }
         else { g.of = (float*)u(p.o.part); g.part_stride = (size_t)d.rows * D; }
-        Config c(dim3((g.nfeat + t.bm - 1) / t.bm, p.rp ? 1 : (g.rows + t.bn - 1) / t.bn, t.splits), 192, st, true);
+        g.bn = t.bn; g.ftiles = (g.nfeat + t.bm - 1) / t.bm; g.rtiles = p.rp ? 1 : (g.rows + t.bn - 1) / t.bn; g.ntiles = g.ftiles * g.rtiles * t.splits;
+        Config c(dim3(t.bm == 64 ? g.ntiles : std::min(g.ntiles, p.sms)), 192, st, true);
         return gemm(EPI_OF[kind], t, c.c, p.w[kind], p.a[kind], g);
     };
     auto attend = [&](int l) {
@@ -259,9 +282,11 @@ int vesta_pass_create(const vesta_pass_desc* d, void* workspace, int graph, void
     const int fold[5] = {D, D, D, F, D}, feat[5] = {3 * D, D, F, D, d->N};
     unsigned char* op[5] = {p->ws + p->o.act, p->ws + p->o.att, p->ws + p->o.act, p->ws + p->o.gelu, p->ws + p->o.fin};
     for (int k = 0; k < 5 && !e; k++) {
-        if (k == K_LOGITS) e = vesta_rt::tensor_map(&p->w[k], w[k], D, feat[k], 1, p->tile[k].bm);
-        else e = vesta_rt::tensor_map(&p->w[k], w[k], feat[k], fold[k], d->L, 64);
-        if (!e) e = vesta_rt::tensor_map(&p->a[k], op[k], fold[k], k == K_LOGITS ? p->fplanes : p->planes, 1, p->tile[k].bn);
+        const Tile& t = p->tile[k];
+        const int ks = t.bm == 64 ? GemmShape<64>::KS : GemmShape<128>::KS;
+        if (k == K_LOGITS) e = vesta_rt::fold_map(&p->w[k], w[k], D, feat[k], t.bm, ks);
+        else e = vesta_rt::tensor_map(&p->w[k], w[k], feat[k], fold[k], d->L, (size_t)feat[k] * 2, (size_t)feat[k] * fold[k] * 2, 64 * ks, 1);
+        if (!e) e = vesta_rt::fold_map(&p->a[k], op[k], fold[k], k == K_LOGITS ? p->fplanes : p->planes, t.bn, ks);
         if (!e) { const cudaError_t ce = gemm_prepare(EPI_OF[k], p->tile[k]); if (ce != cudaSuccess) e = cuda_fail(ce, "cudaFuncSetAttribute"); }
     }
     if (!e && graph) {

@@ -78,6 +78,7 @@ enum { EPI_QKV = 0, EPI_PART = 1, EPI_GELU = 2, EPI_LOGITS = 3 };
 
 struct GemmArgs {
     int layer, nfeat, kblocks, kb_per, rows, rp, stages;
+    int bn, ftiles, rtiles, ntiles;  // rows per tile (a multiple of 16); tiles of features, of rows, in all (with the parts of the fold)
     int D;
     const u16* bias;                 // QKV, FC: of the layer
     float* of;                       // QKV: queries [row][D]; PART: sums [part][row][nfeat]; LOGITS: logits [row][nfeat]
@@ -88,14 +89,14 @@ struct GemmArgs {
     const int* skip;                 // not zero: the pass was refused, nothing may be written that outlives it
     u64* best;                       // LOGITS: packed (value, ~index) maximum of every row
     u32* status;
-    float ga, gb, gc;
+    float a2, k1, k2;                // GELU: see gelu_tanh
 };
 
 // shared-memory operand descriptors, 128-byte swizzle. K-major: rows of 128 bytes (64 fold indices), groups of eight rows
 // 1024 bytes apart. M-major: rows of 128 bytes hold 64 features of one fold index, groups of eight fold indices 1024
-// bytes apart, the next 64 features 8192 bytes further (one box of 64 x 64).
+// bytes apart, the next 64 features `chunk` bytes further (one box).
 __device__ __forceinline__ u64 desc_k(u32 a) { return (u64)((a & 0x3FFFFu) >> 4) | ((u64)1 << 16) | ((u64)(1024 >> 4) << 32) | ((u64)1 << 46) | ((u64)2 << 61); }
-__device__ __forceinline__ u64 desc_m(u32 a) { return (u64)((a & 0x3FFFFu) >> 4) | ((u64)(8192 >> 4) << 16) | ((u64)(1024 >> 4) << 32) | ((u64)1 << 46) | ((u64)2 << 61); }
+__device__ __forceinline__ u64 desc_m(u32 a, u32 chunk) { return (u64)((a & 0x3FFFFu) >> 4) | ((u64)(chunk >> 4) << 16) | ((u64)(1024 >> 4) << 32) | ((u64)1 << 46) | ((u64)2 << 61); }
 
 __device__ __forceinline__ void tm_ld16(u32 (&r)[16], u32 addr) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -103,48 +104,68 @@ __device__ __forceinline__ void tm_ld16(u32 (&r)[16], u32 addr) {
                    "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(addr) : "memory");
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
-// tanh-GELU: a v (1 + tanh(b (v + c v^3))), tanh(u) = 1 - 2 / (1 + e^(2u))
-__device__ __forceinline__ float gelu_tanh(float v, float ga, float gb, float gc) {
-    const float u = gb * (v + gc * v * v * v);
+// tanh-GELU: a v (1 + tanh(b (v + c v^3))) with tanh(u) = 1 - 2 / (1 + e^(2u)): 2a v (1 - 1 / (1 + 2^(v (k1 + k2 v^2)))),
+// k1 = 2 b log2(e), k2 = c k1
+__device__ __forceinline__ float gelu_tanh(float v, float a2, float k1, float k2) {
     float e, r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(u * 2.8853900817779268f));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(v * fmaf(v * v, k2, k1)));
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
-    return ga * v * (2.0f - 2.0f * r);
+    const float w = a2 * v;
+    return fmaf(-w, r, w);
 }
 // orderable key of (value, index): larger value wins, then the lower index
 __device__ __forceinline__ u64 best_key(int ordered, u32 n) { return ((u64)((u32)ordered ^ 0x80000000u) << 32) | (u64)(0xFFFFFFFFu - n); }
 
-template <int BM, int BN> struct GemmSmem {
-    static constexpr int A = BM * 128, B = BN * 128, STAGE = A + B;
-    // after the stages: full and empty barriers, "done", tensor-memory address, dead flag; row offsets or the warps' best keys
-    static constexpr int tail(int stages) { return 2 * stages * 8 + 16 + 16 + BN * 8 * 4; }
-    static constexpr int bytes(int stages) { return stages * STAGE + tail(stages) + 1024; }
+// Shared memory of a block: the stages, then full and empty barriers, the accumulators' full and empty barriers, the
+// tensor-memory address and the dead flag; per accumulator the row offsets (QKV) or the warps' best keys (LOGITS).
+template <int BM> struct GemmShape {
+    static constexpr int KS = BM == 64 ? 4 : 1;          // blocks of 64 fold indices per stage
+    static constexpr int EW = BM == 64 ? 4 : 8;          // warps that read the accumulators
+    static constexpr int THREADS = 64 + 32 * EW;
+    static __host__ __device__ constexpr int stage(int bn) { return KS * (BM + bn) * 128; }
+    static __host__ __device__ constexpr int tail(int stages, int bn) { return 2 * stages * 8 + 48 + bn * 8 * 4; }
+    static __host__ __device__ constexpr int bytes(int stages, int bn) { return stages * stage(bn) + tail(stages, bn) + 1024; }
+    static __host__ __device__ constexpr int columns(int bn, bool two) { int c = 32; while (c < (two ? 2 * bn : bn)) c *= 2; return c; }
 };
+__device__ __forceinline__ void st_u16(u16* p, u16 v, bool yes) {
+    asm volatile("{.reg .pred p; setp.ne.s32 p, %2, 0; @p st.global.u16 [%0], %1;}" :: "l"(p), "h"(v), "r"((int)yes) : "memory");
+}
+__device__ __forceinline__ void st_f32(float* p, float v, bool yes) {
+    asm volatile("{.reg .pred p; setp.ne.s32 p, %2, 0; @p st.global.f32 [%0], %1;}" :: "l"(p), "f"(v), "r"((int)yes) : "memory");
+}
 
-// One tile of BM features x BN rows over kb_per blocks of 64 fold indices (blockIdx.z: which part of the fold).
-// Warp 0 loads (one lane), warp 1 issues the products (one lane), warps 2..5 read the accumulators.
-template <int BM, int BN, int EPI>
-__global__ void __launch_bounds__(192) pass_gemm(const __grid_constant__ CUtensorMap wm, const __grid_constant__ CUtensorMap am, const __grid_constant__ GemmArgs g) {
-    using S = GemmSmem<BM, BN>;
+// Tiles of BM features x bn rows over kb_per blocks of 64 fold indices; a block takes the tiles blockIdx.x,
+// blockIdx.x + gridDim.x, ... Warp 0 loads (one lane), warp 1 issues the products, the others read the accumulators; with
+// more tiles than blocks two accumulators alternate, so that a tile's epilogue runs under the next one's products.
+//   BM = 64: few rows, one tile per block. What counts is the chain wait - operand - products - epilogue: the block's
+//     whole share of the weights is in flight before it waits for its predecessor, four blocks of the fold per stage (a
+//     stage costs the issuing warps 0.1 us whatever its size: 12 blocks of 64 x 16 took 2.0 us one by one, 1.0 in fours).
+//   BM = 128: many rows. 128 x 128 tiles run at 1,215 TFLOP/s without an epilogue, 1,119 with fp32 stores.
+template <int BM, int EPI>
+__global__ void __launch_bounds__(GemmShape<BM>::THREADS) pass_gemm(const __grid_constant__ CUtensorMap wm, const __grid_constant__ CUtensorMap am, const __grid_constant__ GemmArgs g) {
+    using S = GemmShape<BM>;
+    constexpr int KS = S::KS, EW = S::EW;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    const int st = g.stages;
-    const u32 sbase = smem_u32(smem), bars = sbase + st * S::STAGE, done = bars + 2 * st * 8;
-    unsigned char* tail = smem + st * S::STAGE + 2 * st * 8 + 16;
+    const int st = g.stages, bn = g.bn, stage = S::stage(bn);
+    const u32 sbase = smem_u32(smem), bars = sbase + st * stage, tmf = bars + 2 * st * 8, tme = tmf + 16;
+    unsigned char* tail = smem + st * stage + 2 * st * 8 + 32;
     volatile int* dead = reinterpret_cast<volatile int*>(tail + 4);
     volatile u32* tmem_p = reinterpret_cast<volatile u32*>(tail);
     u64* side = reinterpret_cast<u64*>(tail + 16);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int TCOLS = BN < 32 ? 32 : BN;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const bool two = g.ntiles > (int)gridDim.x;
+    const int cols = S::columns(bn, two);
     const Wait w{dead, g.status};
     if (threadIdx.x == 0) {
         *dead = 0;
         for (int i = 0; i < st; i++) { mbar_init(bars + i * 8, 1); mbar_init(bars + (st + i) * 8, 1); }
-        mbar_init(done, 1);
+        for (int i = 0; i < 2; i++) { mbar_init(tmf + i * 8, 1); mbar_init(tme + i * 8, EW); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("prefetch.tensormap [%0];" :: "l"(&am) : "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(tail)), "n"(TCOLS) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(tail)), "r"(cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     }
@@ -152,135 +173,191 @@ __global__ void __launch_bounds__(192) pass_gemm(const __grid_constant__ CUtenso
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (threadIdx.x == 0) dep_launch();              // (after the allocation: the blocks of the next kernel queue behind it)
     const u32 tmem = *tmem_p;
-    const int kb0 = blockIdx.z * g.kb_per, nkb = min(g.kb_per, g.kblocks - kb0);
-    const int f0 = blockIdx.x * BM, row0 = blockIdx.y * BN;
+    const int per = g.ftiles * g.rtiles;
 
     if (warp == 0) {
         if (elect_one()) {
-            auto load_w = [&](int s, int kb) {
-                const u32 dst = sbase + s * S::STAGE, bar = bars + s * 8;
-                if (EPI == EPI_LOGITS) tma3(dst, &wm, kb * 64, f0, 0, bar);
-                else {
-                    tma3(dst, &wm, f0, kb * 64, g.layer, bar);
-                    if (BM == 128) tma3(dst + 8192, &wm, f0 + 64, kb * 64, g.layer, bar);
+            int s = 0, ph = 1;
+            bool first = true;
+            for (int t = blockIdx.x; t < g.ntiles; t += gridDim.x) {
+                const int z = t / per, r = t - z * per, rt = r / g.ftiles, f0 = (r - rt * g.ftiles) * BM, row0 = rt * bn;
+                const int kb0 = z * g.kb_per, nst = (min(g.kb_per, g.kblocks - kb0) + KS - 1) / KS;
+                auto load_w = [&](int slot, int i) {
+                    const u32 dst = sbase + slot * stage, bar = bars + slot * 8;
+                    mbar_expect(bar, stage);
+                    if (EPI == EPI_LOGITS) tma3(dst, &wm, 0, f0, kb0 + i * KS, bar);
+                    else {
+                        tma3(dst, &wm, f0, (kb0 + i * KS) * 64, g.layer, bar);
+                        if (BM == 128) tma3(dst + KS * 8192, &wm, f0 + 64, (kb0 + i * KS) * 64, g.layer, bar);
+                    }
+                };
+                auto load_a = [&](int slot, int i) { tma3(sbase + slot * stage + KS * BM * 128, &am, 0, row0, kb0 + i * KS, bars + slot * 8); };
+                int i = 0;
+                if (first) {
+                    // the weights do not depend on the predecessor
+                    const int pre = min(st, nst);
+                    for (; i < pre; i++) load_w(i, i);
+                    dep_wait();
+                    for (i = 0; i < pre; i++) load_a(i, i);
+                    s = pre; if (s == st) { s = 0; ph = 0; }
+                    first = false;
                 }
-            };
-            const int pre = min(st, nkb);
-            for (int i = 0; i < pre; i++) { mbar_expect(bars + i * 8, S::STAGE); load_w(i, kb0 + i); }
-            dep_wait();
-            for (int i = 0; i < pre; i++) tma3(sbase + i * S::STAGE + S::A, &am, (kb0 + i) * 64, row0, 0, bars + i * 8);
-            int s = 0, ph = 0;
-            for (int i = pre; i < nkb; i++) {
-                if (!mbar_wait(bars + (st + s) * 8, ph, w, 0xB00u)) break;
-                mbar_expect(bars + s * 8, S::STAGE);
-                load_w(s, kb0 + i);
-                tma3(sbase + s * S::STAGE + S::A, &am, (kb0 + i) * 64, row0, 0, bars + s * 8);
-                if (++s == st) { s = 0; ph ^= 1; }
+                for (; i < nst; i++) {
+                    if (!mbar_wait(bars + (st + s) * 8, ph, w, 0xB00u)) break;
+                    load_w(s, i);
+                    load_a(s, i);
+                    if (++s == st) { s = 0; ph ^= 1; }
+                }
+                if (*dead) break;
             }
         }
     } else if (warp == 1) {
         // fp32 accumulators, fp16 operands; A M-major (bit 15) except for the table of the logits
-        constexpr u32 idesc = (1u << 4) | (EPI == EPI_LOGITS ? 0u : (1u << 15)) | ((u32)(BN >> 3) << 17) | ((u32)(BM >> 4) << 24);
-        int s = 0, ph = 0;
-        const u32 leader = elect_one();
-        for (int i = 0; i < nkb; i++) {
-            const bool ok = mbar_wait(bars + s * 8, ph, w, 0xB10u);
-            if (!__all_sync(0xffffffffu, ok)) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const u32 a = sbase + s * S::STAGE;
-            const u64 ad = EPI == EPI_LOGITS ? desc_k(a) : desc_m(a), bd = desc_k(a + S::A);
+        const u32 idesc = (1u << 4) | (EPI == EPI_LOGITS ? 0u : (1u << 15)) | ((u32)(bn >> 3) << 17) | ((u32)(BM >> 4) << 24);
+        constexpr int AKB = EPI == EPI_LOGITS ? BM * 128 : 8192, AK = EPI == EPI_LOGITS ? 32 : 2048;   // bytes to the next block, to the next 16 fold indices
+        int s = 0, ph = 0, n = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; t < g.ntiles && ok; t += gridDim.x, n++) {
+            const int kb0 = (t / per) * g.kb_per, nkb = min(g.kb_per, g.kblocks - kb0), nst = (nkb + KS - 1) / KS, b = n & 1;
+            if (n >= 2) ok = !__any_sync(0xffffffffu, !mbar_wait(tme + b * 8, ((n >> 1) & 1) ^ 1, w, 0xB30u));
+            const u32 acc = tmem + (b ? bn : 0);
+            for (int i = 0; i < nst && ok; i++) {
+                ok = !__any_sync(0xffffffffu, !mbar_wait(bars + s * 8, ph, w, 0xB10u));
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                // (the elected lane is asked for here, next to the products: under a predicate that comes from further away a
+                // product costs 90 cycles instead of the 20 to 40 its operands take: the descriptors then pass to uniform
+                // registers one by one)
+                if (elect_one()) {
+                    const u32 a = sbase + s * stage;
+                    const u64 ad = EPI == EPI_LOGITS ? desc_k(a) : desc_m(a, KS * 8192), bd = desc_k(a + KS * BM * 128);
 #pragma unroll
-            for (int k = 0; k < 4; k++)
-                asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                             :: "r"(tmem), "l"(ad + (EPI == EPI_LOGITS ? 2 : 128) * k), "l"(bd + 2 * k), "r"(idesc), "r"((i | k) ? 1u : 0u), "r"(leader) : "memory");
-            if (leader) {
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bars + (st + s) * 8) : "memory");
-                if (i == nkb - 1) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(done) : "memory");
+                    for (int kb = 0; kb < KS; kb++)
+                        if (KS == 1 || i * KS + kb < nkb) {
+                            const u64 bk = bd + (u64)((kb * bn * 128) >> 4);
+#pragma unroll
+                            for (int k = 0; k < 4; k++)
+                                asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                                             :: "r"(acc), "l"(ad + (kb * AKB + k * AK) / 16), "l"(bk + 2 * k), "r"(idesc), "r"((i | kb | k) ? 1u : 0u) : "memory");
+                        }
+                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bars + (st + s) * 8) : "memory");
+                    if (i == nst - 1) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(tmf + b * 8) : "memory");
+                }
+                __syncwarp();
+                if (++s == st) { s = 0; ph ^= 1; }
             }
-            __syncwarp();
-            if (++s == st) { s = 0; ph ^= 1; }
         }
     } else {
         const int quarter = warp & 3, ew = warp - 2, et = threadIdx.x - 64;
         const int fl = BM == 128 ? quarter * 32 + lane : quarter * 16 + lane;      // (a product of 64 rows leaves row m in lane 32 (m / 16) + m % 16)
-        const int f = f0 + fl;
-        const bool own = (BM == 128 || lane < 16) && f < g.nfeat;
-        float bias = 0.f;
-        if ((EPI == EPI_QKV || EPI == EPI_GELU) && own) bias = h2f(__ldg(g.bias + f));
-        dep_wait();
-        const bool skip = (EPI == EPI_QKV || EPI == EPI_LOGITS) ? __ldcg(g.skip) != 0 : false;
-        const int live = min(g.rp ? g.rp : BN, g.rows - row0);                     // rows of this tile
-        if (EPI == EPI_QKV) {
-            for (int i = et; i < BN; i += 128) side[i] = i < live ? (u64)__ldcg(g.rowoff + row0 + i) : ~0ull;
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-        }
-        const bool ok = mbar_wait(done, 0, w, 0xB20u);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (__all_sync(0xffffffffu, ok)) {
-            const u32 ta = tmem + ((u32)(quarter * 32) << 16);
+        bool waited = false, skip = false;
+        int n = 0;
+        for (int t = blockIdx.x; t < g.ntiles; t += gridDim.x, n++) {
+            const int z = t / per, r0 = t - z * per, rt = r0 / g.ftiles, f0 = (r0 - rt * g.ftiles) * BM, row0 = rt * bn, b = n & 1;
+            const int f = f0 + fl;
+            const bool own = (BM == 128 || lane < 16) && f < g.nfeat;
+            float bias = 0.f;
+            if ((EPI == EPI_QKV || EPI == EPI_GELU) && own) bias = h2f(__ldg(g.bias + f));
+            if (!waited) {
+                dep_wait();
+                waited = true;
+                skip = (EPI == EPI_QKV || EPI == EPI_LOGITS) ? __ldcg(g.skip) != 0 : false;
+            }
+            const int live = min(g.rp ? g.rp : bn, g.rows - row0);                 // rows of this tile
+            if (EPI == EPI_QKV) {
+                // (everyone is past the previous tile's offsets but one: two buffers)
+                for (int i = et; i < bn; i += EW * 32) side[b * bn + i] = (i < live && !skip) ? (u64)__ldcg(g.rowoff + row0 + i) : ~0ull;
+                asm volatile("bar.sync 1, %0;" :: "n"(EW * 32) : "memory");
+            }
+            const bool ok = mbar_wait(tmf + b * 8, (n >> 1) & 1, w, 0xB20u);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (__any_sync(0xffffffffu, !ok)) break;
+            const u32 ta = tmem + ((u32)(quarter * 32) << 16) + (b ? bn : 0);
             const int part = EPI == EPI_QKV ? f / g.D : 0;                         // 0 query, 1 key, 2 value (a warp never straddles two)
             u16* cache = EPI == EPI_QKV ? (part == 1 ? g.kc : g.vc) + (f - part * g.D) : (u16*)0;
+            // eight warps: two per quarter of the lanes, the second takes the upper half of the rows
+            const int half = EW == 8 ? ((bn + 31) / 32) * 16 : bn;
+            const int c_lo = EW == 8 && ew >= 4 ? half : 0, c_hi = min(live, EW == 8 && ew < 4 ? half : bn);
 #pragma unroll 1
-            for (int c0 = 0; c0 < live; c0 += 16) {
+            for (int c0 = c_lo; c0 < c_hi; c0 += 16) {
                 u32 r[16];
                 tm_ld16(r, ta + c0);
-                int n = min(16, live - c0);
-                if (g.rp) {
+                int m = min(16, c_hi - c0);
+                if (BM == 64 && g.rp) {
                     u32 q[16];
-                    if (BN >= 32) tm_ld16(q, ta + 16);
-                    n = live;
+                    if (g.rp == 16) tm_ld16(q, ta + 16);
+                    m = live;
 #pragma unroll
-                    for (int i = 0; i < 16; i++) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(BN >= 32 ? q[i] : r[(i + 8) & 15]));
+                    for (int i = 0; i < 16; i++) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(g.rp == 16 ? q[i] : r[(i + 8) & 15]));
                 }
+                // (no branch per row: the sixteen chains of arithmetic overlap, only the stores are predicated)
+                const int row = row0 + c0;
+                float v[16];
 #pragma unroll
                 for (int i = 0; i < 16; i++) {
-                    if (i < n) {
-                        const int row = row0 + c0 + i;
-                        float v = __uint_as_float(r[i]) + bias;
-                        if (EPI == EPI_QKV) {
-                            if (own) {
-                                if (part == 0) g.of[(size_t)row * g.D + f] = v;
-                                else {
-                                    const long long o = (long long)side[c0 + i];
-                                    if (o >= 0 && !skip) cache[o] = f2h(v);
-                                }
-                            }
-                        } else if (EPI == EPI_PART) {
-                            if (own) g.of[blockIdx.z * g.part_stride + (size_t)row * g.nfeat + f] = v;
-                        } else if (EPI == EPI_GELU) {
-                            v = gelu_tanh(v, g.ga, g.gb, g.gc);
-                            if (own) {
-                                const u16 h = f2h(v);
-                                g.oh[(size_t)row * g.nfeat + f] = h;
-                                if (g.rp) g.oh[(size_t)(g.rp + row) * g.nfeat + f] = f2h(v - h2f(h));
-                            }
-                        } else {
-                            if (own && !skip) g.of[(size_t)row * g.nfeat + f] = v;
-                            // the warp's best feature of this row: maximum by redux, lowest feature among the equal ones by ballot
-                            int kv = own ? __float_as_int(v) : __float_as_int(-3.0e38f);
-                            kv = kv >= 0 ? kv : kv ^ 0x7fffffff;
-                            const int km = __reduce_max_sync(0xffffffffu, kv);
-                            const u32 who = __ballot_sync(0xffffffffu, kv == km && own);
-                            if (lane == 0) side[ew * BN + c0 + i] = who ? best_key(km, (u32)(f - lane + (__ffs(who) - 1))) : 0ull;
-                        }
+                    v[i] = __uint_as_float(r[i]) + bias;
+                    if (EPI == EPI_GELU) v[i] = gelu_tanh(v[i], g.a2, g.k1, g.k2);
+                }
+                if (!own) m = 0;
+                if (EPI == EPI_QKV) {
+                    if (part == 0) {
+                        float* dst = g.of + (size_t)row * g.D + f;
+#pragma unroll
+                        for (int i = 0; i < 16; i++) st_f32(dst + (size_t)i * g.D, v[i], i < m);
+                    } else {
+                        long long o[16];
+#pragma unroll
+                        for (int i = 0; i < 16; i++) o[i] = (long long)side[b * bn + c0 + i];
+#pragma unroll
+                        for (int i = 0; i < 16; i++) st_u16(cache + o[i], f2h(v[i]), i < m && o[i] >= 0);
+                    }
+                } else if (EPI == EPI_PART) {
+                    float* dst = g.of + z * g.part_stride + (size_t)row * g.nfeat + f;
+#pragma unroll
+                    for (int i = 0; i < 16; i++) st_f32(dst + (size_t)i * g.nfeat, v[i], i < m);
+                } else if (EPI == EPI_GELU) {
+                    u16* dst = g.oh + (size_t)row * g.nfeat + f;
+#pragma unroll
+                    for (int i = 0; i < 16; i++) st_u16(dst + (size_t)i * g.nfeat, f2h(v[i]), i < m);
+                    if (BM == 64 && g.rp) {
+                        dst += (size_t)g.rp * g.nfeat;
+#pragma unroll
+                        for (int i = 0; i < 16; i++) st_u16(dst + (size_t)i * g.nfeat, f2h(v[i] - h2f(f2h(v[i]))), i < m);
+                    }
+                } else {
+                    float* dst = g.of + (size_t)row * g.nfeat + f;
+#pragma unroll
+                    for (int i = 0; i < 16; i++) st_f32(dst + (size_t)i * g.nfeat, v[i], i < m && !skip);
+                    // the warp's best feature of every row: maximum by redux, lowest feature among the equal ones by ballot
+#pragma unroll
+                    for (int i = 0; i < 16; i++) {
+                        int kv = own ? __float_as_int(v[i]) : __float_as_int(-3.0e38f);
+                        kv = kv >= 0 ? kv : kv ^ 0x7fffffff;
+                        const int km = __reduce_max_sync(0xffffffffu, kv);
+                        const u32 who = __ballot_sync(0xffffffffu, kv == km && own);
+                        if (lane == 0) side[quarter * bn + c0 + i] = who ? best_key(km, (u32)(f - lane + (__ffs(who) - 1))) : 0ull;
                     }
                 }
             }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(tme + b * 8) : "memory");
             if (EPI == EPI_LOGITS) {
-                asm volatile("bar.sync 1, 128;" ::: "memory");
+                asm volatile("bar.sync 1, %0;" :: "n"(EW * 32) : "memory");
                 if (!skip)
-                    for (int i = et; i < live; i += 128) {
+                    for (int i = et; i < live; i += EW * 32) {
                         u64 k = side[i];
 #pragma unroll
-                        for (int x = 1; x < 4; x++) if (side[x * BN + i] > k) k = side[x * BN + i];
+                        for (int x = 1; x < 4; x++) if (side[x * bn + i] > k) k = side[x * bn + i];
                         if (k) atomicMax(g.best + row0 + i, k);
                     }
+                if (two) asm volatile("bar.sync 1, %0;" :: "n"(EW * 32) : "memory");
             }
         }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        if (!waited) dep_wait();
     }
     __syncthreads();
-    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "n"(TCOLS) : "memory");
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(cols) : "memory");
     if (*dead && threadIdx.x == 0) {
         // a wait ran out: let copies in flight land (bounded) before the block's shared memory goes to another
         const u64 t0 = now_ns();

@@ -136,15 +136,16 @@ struct Bound {
 namespace vesta_rt {
 int fail(int code, const std::string& what) { return ::fail(code, what); }
 
-int tensor_map(void* out, const void* base, unsigned long long d0, unsigned long long d1, unsigned long long d2, unsigned box1) {
+int tensor_map(void* out, const void* base, unsigned long long d0, unsigned long long d1, unsigned long long d2,
+               unsigned long long stride1, unsigned long long stride2, unsigned box1, unsigned box2) {
     if (!out || !base) return ::fail(-1, "tensor map: null argument");
     if (int e = driver()) return e;
-    if (box1 == 0 || box1 > 256u || (d0 * 2ull) % 16ull) return ::fail(-1, "tensor map: at most 256 rows per box, rows a multiple of 16 bytes");
-    // fp16 [d2][d1][d0], box = box1 rows of 64 elements of one plane; 128-byte swizzle: the 16-byte piece c of row r lands at
-    // piece c ^ (r % 8) of its 128-byte row in shared memory
+    if (box1 == 0 || box1 > 256u || box2 == 0 || box2 > 256u || stride1 % 16ull || stride2 % 16ull)
+        return ::fail(-1, "tensor map: at most 256 rows per box, rows a multiple of 16 bytes");
+    // 128-byte swizzle: the 16-byte piece c of row r lands at piece c ^ (r % 8) of its 128-byte row in shared memory
     const cuuint64_t dims[3] = {d0, d1, d2};
-    const cuuint64_t strides[2] = {d0 * 2ull, d1 * d0 * 2ull};
-    const cuuint32_t box[3] = {64, box1, 1};
+    const cuuint64_t strides[2] = {stride1, stride2};
+    const cuuint32_t box[3] = {64, box1, box2};
     const cuuint32_t estr[3] = {1, 1, 1};
     CUtensorMap tm;
     CUresult r = g_cu.TensorMapEncodeTiled(&tm, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, const_cast<void*>(base), dims, strides, box, estr,
@@ -330,7 +331,7 @@ int vesta_tensor_map_rows(void* out, const void* base, unsigned long long row_el
     if (!out || !base) return fail(-1, "vesta_tensor_map_rows: null argument");
     if (box_elems * 2u != 128u || box_rows == 0 || box_rows > 256u || (row_elems * 2ull) % 16ull)
         return fail(-1, "vesta_tensor_map_rows: the box must be 128 bytes wide, at most 256 rows, rows a multiple of 16 bytes");
-    return vesta_rt::tensor_map(out, base, row_elems, rows, planes, box_rows);
+    return vesta_rt::tensor_map(out, base, row_elems, rows, planes, row_elems * 2ull, rows * row_elems * 2ull, box_rows, 1);
 }
 
 int vesta_step_run_fused(void* bound, void* stream, int steps, int per_launch) {
