@@ -49,7 +49,7 @@ int plane_rows(int rows, bool exact) { return !exact ? 0 : rows <= 8 ? 8 : 16; }
 //   BM = 64 (one tile per block, whole share of the weights in flight): 1.75 + 0.22 per stage + the operand's rows;
 //   BM = 128: 2.2 + 0.0065 bn for the first fill and the last epilogue, then per block of the fold the larger of the products
 //     (2 bn cycles) and the loads (340 + 0.45 bn cycles), times the tiles a block takes in turn.
-// A cut fold (projections) costs its parts once more in the norm that adds them: 0.25 us and 3 MB of traffic at 4 TB/s each.
+// A cut fold (projections) costs its parts once more in the norm that adds them.
 Tile choose(int kind, int rows, int rp, int feat, int kb, int sms) {
     Tile best = {};
     double best_t = 1e30;
@@ -63,7 +63,7 @@ Tile choose(int kind, int rows, int rp, int feat, int kb, int sms) {
             const int stage = bm == 64 ? GemmShape<64>::stage(bn) : GemmShape<128>::stage(bn);
             const int room = 227 * 1024 - 1024 - 1024 - bn * 32;
             const int tiles = ((feat + bm - 1) / bm) * (rp ? 1 : (rows + bn - 1) / bn);
-            for (int sp = 1; sp <= (cut ? 8 : 1); sp++) {
+            for (int sp = 1; sp <= (cut ? PARTS_MAX : 1); sp++) {
                 Tile t;
                 t.bm = bm; t.bn = bn;
                 const int per = (kb + sp - 1) / sp, nst = (per + ks - 1) / ks;
@@ -72,9 +72,9 @@ Tile choose(int kind, int rows, int rp, int feat, int kb, int sms) {
                 const int waves = (tiles * sp + sms - 1) / sms;
                 t.stages = std::max(1, std::min(bm == 64 || waves == 1 ? nst : 16, room / (stage + 16)));
                 double us;
-                if (bm == 64) us = (1.75 + 0.22 * nst + 0.0023 * (bn - 16) * per) * (kind == K_LOGITS ? 1 : waves) + 0.002 * tiles * sp;
+                if (bm == 64) us = (1.75 + 0.22 * nst + 0.0023 * (bn - 16) * per) * waves + 0.002 * tiles * sp;
                 else us = 2.2 + 0.0065 * bn + waves * per * std::max(2.0 * bn + 30, 340 + 0.45 * bn) / 1900;
-                if (cut) us += sp * (0.25 + (double)rows * feat * 4 / 4e6);
+                if (cut && sp > 1) us += 0.1 * sp + (sp - 1) * (double)rows * feat * 4 / 4e6;
                 if (us < best_t) { best_t = us; best = t; }
             }
         }
@@ -136,7 +136,7 @@ cudaError_t prepare_gemm(const Tile& t) {
     return cudaFuncSetAttribute(pass_gemm<BM, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
 }
 // one case per tile shape and epilogue
-#define EACH(X) X(64, EPI_QKV) X(64, EPI_PART) X(64, EPI_GELU) X(64, EPI_LOGITS) X(128, EPI_QKV) X(128, EPI_PART) X(128, EPI_GELU) X(128, EPI_LOGITS)
+#define EACH(X) X(64, EPI_ADD) X(128, EPI_ADD) X(64, EPI_QKV) X(64, EPI_PART) X(64, EPI_GELU) X(64, EPI_LOGITS) X(128, EPI_QKV) X(128, EPI_PART) X(128, EPI_GELU) X(128, EPI_LOGITS)
 cudaError_t gemm(int epi, const Tile& t, cudaLaunchConfig_t c, const CUtensorMap& w, const CUtensorMap& a, const GemmArgs& g) {
 #define ONE(M, E) if (epi == E && t.bm == M) return launch_gemm<M, E>(c, t, w, a, g);
     EACH(ONE)
@@ -149,7 +149,7 @@ cudaError_t gemm_prepare(int epi, const Tile& t) {
 #undef ONE
     return cudaErrorInvalidValue;
 }
-const int EPI_OF[5] = {EPI_QKV, EPI_PART, EPI_GELU, EPI_PART, EPI_LOGITS};
+int epi_of(int kind, const Tile& t) { return kind == K_QKV ? EPI_QKV : kind == K_FC ? EPI_GELU : kind == K_LOGITS ? EPI_LOGITS : t.splits > 1 ? EPI_PART : EPI_ADD; }
 
 // launch attributes: `dependent` = may start while the kernel before it runs
 struct Config {
@@ -202,10 +202,11 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles) {
         } else if (kind == K_FC) {
             g.bias = f16(d.fcb, (size_t)l * F); g.oh = (u16*)u(p.o.gelu); g.a2 = 2 * d.gelu_a; g.k1 = d.gelu_b * 2.8853900817779268f; g.k2 = d.gelu_c * g.k1;
         } else if (kind == K_LOGITS) { g.of = (float*)d.logits; g.best = (u64*)u(p.o.best); }
-        else { g.of = (float*)u(p.o.part); g.part_stride = (size_t)d.rows * D; }
+        else if (t.splits > 1) { g.of = (float*)u(p.o.part); g.part_stride = (size_t)d.rows * D; }
+        else { g.of = z; g.bias = kind == K_PROJ ? f16(d.ob, (size_t)l * D) : f16(d.pb, (size_t)l * D); }
         g.bn = t.bn; g.ftiles = (g.nfeat + t.bm - 1) / t.bm; g.rtiles = p.rp ? 1 : (g.rows + t.bn - 1) / t.bn; g.ntiles = g.ftiles * g.rtiles * t.splits;
-        Config c(dim3(t.bm == 64 ? g.ntiles : std::min(g.ntiles, p.sms)), 192, st, true);
-        return gemm(EPI_OF[kind], t, c.c, p.w[kind], p.a[kind], g);
+        Config c(dim3(t.bm == 64 && kind != K_LOGITS ? g.ntiles : std::min(g.ntiles, p.sms)), 192, st, true);
+        return gemm(epi_of(kind, t), t, c.c, p.w[kind], p.a[kind], g);
     };
     auto attend = [&](int l) {
         const float* q = (const float*)u(p.o.q);
@@ -218,9 +219,9 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles) {
             Config c(dim3(tiles, d.H), 128, st, true);
             return cudaLaunchKernelEx(&c.c, pass_attend_many, a);
         }
-        AttArgs a = {q, kc, vc, ss, (const int*)u(p.o.pos), (const int*)d.seq, D, pow2, p.rp, d.scale, att};
+        AttArgs a = {q, kc, vc, ss, (const int*)d.t, (const int*)d.seq, d.t_stride, d.tmax, D, pow2, p.rp, d.scale, att};
         int C = 1;
-        while (C < 8 && rows * d.H * C * 2 <= 2 * p.sms && d.tmax > C * ATT_WARPS * 32) C *= 2;
+        while (C < 8 && rows * d.H * C * 2 <= 6 * p.sms && d.tmax > C * ATT_WARPS * ATT_RUN) C *= 2;
         Config c(dim3(d.H, rows, C), ATT_WARPS * 32, st, true, C);
         return cudaLaunchKernelEx(&c.c, pass_attend, a);
     };
@@ -230,10 +231,10 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles) {
         if (l == L - 1 && lrows == 0) break;
         TRY(attend(l));
         TRY(mul(K_PROJ, l));
-        TRY(norm(1, l, p.tile[K_PROJ].splits));
+        TRY(norm(1, l, p.tile[K_PROJ].splits > 1 ? p.tile[K_PROJ].splits : 0));
         TRY(mul(K_FC, l));
         TRY(mul(K_P2, l));
-        TRY(norm(l + 1 < L ? 2 : 3, l, p.tile[K_P2].splits));
+        TRY(norm(l + 1 < L ? 2 : 3, l, p.tile[K_P2].splits > 1 ? p.tile[K_P2].splits : 0));
     }
     if (lrows) TRY(mul(K_LOGITS, 0));
     FinishArgs f = {};
@@ -287,7 +288,7 @@ int vesta_pass_create(const vesta_pass_desc* d, void* workspace, int graph, void
         if (k == K_LOGITS) e = vesta_rt::fold_map(&p->w[k], w[k], D, feat[k], t.bm, ks);
         else e = vesta_rt::tensor_map(&p->w[k], w[k], feat[k], fold[k], d->L, (size_t)feat[k] * 2, (size_t)feat[k] * fold[k] * 2, 64 * ks, 1);
         if (!e) e = vesta_rt::fold_map(&p->a[k], op[k], fold[k], k == K_LOGITS ? p->fplanes : p->planes, t.bn, ks);
-        if (!e) { const cudaError_t ce = gemm_prepare(EPI_OF[k], p->tile[k]); if (ce != cudaSuccess) e = cuda_fail(ce, "cudaFuncSetAttribute"); }
+        if (!e) { const cudaError_t ce = gemm_prepare(epi_of(k, p->tile[k]), p->tile[k]); if (ce != cudaSuccess) e = cuda_fail(ce, "cudaFuncSetAttribute"); }
     }
     if (!e && graph) {
         // a decode step as a graph, captured on a stream of its own

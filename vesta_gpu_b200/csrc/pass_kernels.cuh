@@ -74,14 +74,14 @@ __device__ __noinline__ bool mbar_wait_slow(u32 bar, u32 parity, const Wait& w, 
 __device__ __forceinline__ bool mbar_wait(u32 bar, u32 parity, const Wait& w, u32 code) { return mbar_try(bar, parity) || mbar_wait_slow(bar, parity, w, code); }
 
 // ---- contractions ---------------------------------------------------------------------------------------------------
-enum { EPI_QKV = 0, EPI_PART = 1, EPI_GELU = 2, EPI_LOGITS = 3 };
+enum { EPI_QKV = 0, EPI_PART = 1, EPI_GELU = 2, EPI_LOGITS = 3, EPI_ADD = 4 };
 
 struct GemmArgs {
     int layer, nfeat, kblocks, kb_per, rows, rp, stages;
     int bn, ftiles, rtiles, ntiles;  // rows per tile (a multiple of 16); tiles of features, of rows, in all (with the parts of the fold)
     int D;
     const u16* bias;                 // QKV, FC: of the layer
-    float* of;                       // QKV: queries [row][D]; PART: sums [part][row][nfeat]; LOGITS: logits [row][nfeat]
+    float* of;                       // QKV: queries [row][D]; PART: sums [part][row][nfeat]; ADD: vector added to [row][nfeat]; LOGITS: logits [row][nfeat]
     size_t part_stride;              // floats between two parts
     u16* oh;                         // GELU: [row][nfeat], the remainder plane rp rows further
     u16 *kc, *vc;                    // QKV: the caches at this layer
@@ -98,11 +98,23 @@ struct GemmArgs {
 __device__ __forceinline__ u64 desc_k(u32 a) { return (u64)((a & 0x3FFFFu) >> 4) | ((u64)1 << 16) | ((u64)(1024 >> 4) << 32) | ((u64)1 << 46) | ((u64)2 << 61); }
 __device__ __forceinline__ u64 desc_m(u32 a, u32 chunk) { return (u64)((a & 0x3FFFFu) >> 4) | ((u64)(chunk >> 4) << 16) | ((u64)(1024 >> 4) << 32) | ((u64)1 << 46) | ((u64)2 << 61); }
 
-__device__ __forceinline__ void tm_ld16(u32 (&r)[16], u32 addr) {
+template <int N> struct Int { static constexpr int n = N; };
+// CH consecutive columns of this thread's tensor-memory lane
+__device__ __forceinline__ void tm_ld(float (&r)[16], u32 addr) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
-                   "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(addr) : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                 : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]), "=f"(r[8]), "=f"(r[9]), "=f"(r[10]), "=f"(r[11]),
+                   "=f"(r[12]), "=f"(r[13]), "=f"(r[14]), "=f"(r[15]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void tm_ld(float (&r)[4], u32 addr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]) : "r"(addr) : "memory");
+}
+// the loads have arrived: the values pass through here, so that nothing that uses them is moved in front of the wait
+__device__ __forceinline__ void tm_wait(float (&r)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+f"(r[0]), "+f"(r[1]), "+f"(r[2]), "+f"(r[3]), "+f"(r[4]), "+f"(r[5]), "+f"(r[6]), "+f"(r[7]), "+f"(r[8]), "+f"(r[9]), "+f"(r[10]),
+                 "+f"(r[11]), "+f"(r[12]), "+f"(r[13]), "+f"(r[14]), "+f"(r[15]) :: "memory");
+}
+__device__ __forceinline__ void tm_wait(float (&r)[4]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+f"(r[0]), "+f"(r[1]), "+f"(r[2]), "+f"(r[3]) :: "memory");
 }
 // tanh-GELU: a v (1 + tanh(b (v + c v^3))) with tanh(u) = 1 - 2 / (1 + e^(2u)): 2a v (1 - 1 / (1 + 2^(v (k1 + k2 v^2)))),
 // k1 = 2 b log2(e), k2 = c k1
@@ -257,7 +269,7 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS) pass_gemm(const __grid
             const int f = f0 + fl;
             const bool own = (BM == 128 || lane < 16) && f < g.nfeat;
             float bias = 0.f;
-            if ((EPI == EPI_QKV || EPI == EPI_GELU) && own) bias = h2f(__ldg(g.bias + f));
+            if ((EPI == EPI_QKV || EPI == EPI_GELU || EPI == EPI_ADD) && own) bias = h2f(__ldg(g.bias + f));
             if (!waited) {
                 dep_wait();
                 waited = true;
@@ -278,24 +290,30 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS) pass_gemm(const __grid
             // eight warps: two per quarter of the lanes, the second takes the upper half of the rows
             const int half = EW == 8 ? ((bn + 31) / 32) * 16 : bn;
             const int c_lo = EW == 8 && ew >= 4 ? half : 0, c_hi = min(live, EW == 8 && ew < 4 ? half : bn);
-#pragma unroll 1
-            for (int c0 = c_lo; c0 < c_hi; c0 += 16) {
-                u32 r[16];
-                tm_ld16(r, ta + c0);
-                int m = min(16, c_hi - c0);
-                if (BM == 64 && g.rp) {
-                    u32 q[16];
-                    if (g.rp == 16) tm_ld16(q, ta + 16);
-                    m = live;
+            // CH rows at a time (no branch per row: their chains of arithmetic overlap, only the stores are predicated); the last
+            // four or fewer on their own
+            auto rows_of = [&](auto CHC, int c0) {
+                constexpr int CH = decltype(CHC)::n;
+                int m = min(CH, c_hi - c0);
+                float add[CH], v[CH];
+                if (EPI == EPI_ADD) {
+                    const float* src = g.of + (size_t)(row0 + c0) * g.nfeat + f;
 #pragma unroll
-                    for (int i = 0; i < 16; i++) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(g.rp == 16 ? q[i] : r[(i + 8) & 15]));
+                    for (int i = 0; i < CH; i++) add[i] = own && i < m ? __ldcg(src + (size_t)i * g.nfeat) : 0.f;
                 }
-                // (no branch per row: the sixteen chains of arithmetic overlap, only the stores are predicated)
-                const int row = row0 + c0;
-                float v[16];
+                tm_ld(v, ta + c0);
+                if (BM == 64 && g.rp) {
+                    float q[CH];
+                    tm_ld(q, ta + g.rp + c0);
+                    tm_wait(v);
+                    tm_wait(q);
 #pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    v[i] = __uint_as_float(r[i]) + bias;
+                    for (int i = 0; i < CH; i++) v[i] += q[i];
+                } else tm_wait(v);
+                const int row = row0 + c0;
+#pragma unroll
+                for (int i = 0; i < CH; i++) {
+                    v[i] += bias;
                     if (EPI == EPI_GELU) v[i] = gelu_tanh(v[i], g.a2, g.k1, g.k2);
                 }
                 if (!own) m = 0;
@@ -303,34 +321,34 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS) pass_gemm(const __grid
                     if (part == 0) {
                         float* dst = g.of + (size_t)row * g.D + f;
 #pragma unroll
-                        for (int i = 0; i < 16; i++) st_f32(dst + (size_t)i * g.D, v[i], i < m);
+                        for (int i = 0; i < CH; i++) st_f32(dst + (size_t)i * g.D, v[i], i < m);
                     } else {
-                        long long o[16];
+                        long long o[CH];
 #pragma unroll
-                        for (int i = 0; i < 16; i++) o[i] = (long long)side[b * bn + c0 + i];
+                        for (int i = 0; i < CH; i++) o[i] = (long long)side[b * bn + c0 + i];
 #pragma unroll
-                        for (int i = 0; i < 16; i++) st_u16(cache + o[i], f2h(v[i]), i < m && o[i] >= 0);
+                        for (int i = 0; i < CH; i++) st_u16(cache + o[i], f2h(v[i]), i < m && o[i] >= 0);
                     }
-                } else if (EPI == EPI_PART) {
-                    float* dst = g.of + z * g.part_stride + (size_t)row * g.nfeat + f;
+                } else if (EPI == EPI_PART || EPI == EPI_ADD) {
+                    float* dst = g.of + (EPI == EPI_PART ? z * g.part_stride : 0) + (size_t)row * g.nfeat + f;
 #pragma unroll
-                    for (int i = 0; i < 16; i++) st_f32(dst + (size_t)i * g.nfeat, v[i], i < m);
+                    for (int i = 0; i < CH; i++) st_f32(dst + (size_t)i * g.nfeat, EPI == EPI_ADD ? v[i] + add[i] : v[i], i < m);
                 } else if (EPI == EPI_GELU) {
                     u16* dst = g.oh + (size_t)row * g.nfeat + f;
 #pragma unroll
-                    for (int i = 0; i < 16; i++) st_u16(dst + (size_t)i * g.nfeat, f2h(v[i]), i < m);
+                    for (int i = 0; i < CH; i++) st_u16(dst + (size_t)i * g.nfeat, f2h(v[i]), i < m);
                     if (BM == 64 && g.rp) {
                         dst += (size_t)g.rp * g.nfeat;
 #pragma unroll
-                        for (int i = 0; i < 16; i++) st_u16(dst + (size_t)i * g.nfeat, f2h(v[i] - h2f(f2h(v[i]))), i < m);
+                        for (int i = 0; i < CH; i++) st_u16(dst + (size_t)i * g.nfeat, f2h(v[i] - h2f(f2h(v[i]))), i < m);
                     }
                 } else {
                     float* dst = g.of + (size_t)row * g.nfeat + f;
 #pragma unroll
-                    for (int i = 0; i < 16; i++) st_f32(dst + (size_t)i * g.nfeat, v[i], i < m && !skip);
+                    for (int i = 0; i < CH; i++) st_f32(dst + (size_t)i * g.nfeat, v[i], i < m && !skip);
                     // the warp's best feature of every row: maximum by redux, lowest feature among the equal ones by ballot
 #pragma unroll
-                    for (int i = 0; i < 16; i++) {
+                    for (int i = 0; i < CH; i++) {
                         int kv = own ? __float_as_int(v[i]) : __float_as_int(-3.0e38f);
                         kv = kv >= 0 ? kv : kv ^ 0x7fffffff;
                         const int km = __reduce_max_sync(0xffffffffu, kv);
@@ -338,7 +356,11 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS) pass_gemm(const __grid
                         if (lane == 0) side[quarter * bn + c0 + i] = who ? best_key(km, (u32)(f - lane + (__ffs(who) - 1))) : 0ull;
                     }
                 }
-            }
+            };
+            int c0 = c_lo;
+#pragma unroll 1
+            for (; c0 + 4 < c_hi; c0 += 16) rows_of(Int<16>{}, c0);
+            if (c0 < c_hi) rows_of(Int<4>{}, c0);
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(tme + b * 8) : "memory");
@@ -366,12 +388,13 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS) pass_gemm(const __grid
 }
 
 // ---- norm: residual sums, LayerNorm, operand ---------------------------------------------------------------------------
+#define PARTS_MAX 8
 enum { NORM_EMBED = 0, NORM_MID = 1, NORM_FINAL = 2 };
 struct NormArgs {
     int D, nparts, rp;
     float eps;
     float* z;                        // residual stream [row][D], updated in place
-    const float* part;               // [part][row][D]: sums of the projection before this norm
+    const float* part;               // [part][row][D]: sums of the projection before this norm (nparts = 0: already in z)
     size_t part_stride;
     const u16 *bias, *gain, *shift;
     u16* act;                        // [row][D] fp16 (and the remainder plane rp rows further)
@@ -385,22 +408,25 @@ struct NormArgs {
     const int* want;                 // FINAL: rows that want logits (0: all)
 };
 
-// One row per block, four elements per thread (the row stays in registers: one read, one write).
+// One row per block, four elements per thread (the row stays in registers: one read, one write). Latency bound for few rows:
+// all parts of the sum are requested together, and mean and variance cost one exchange through shared memory: every warp
+// takes the mean and the squared deviations of its own elements, the block combines them (Chan's formula).
 template <int MODE>
 __global__ void __launch_bounds__(1024) pass_norm(const __grid_constant__ NormArgs a) {
-    __shared__ float red[2][32];
+    __shared__ float2 red[32];
     const int tid = threadIdx.x, d = tid * 4, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
     const bool own = d < a.D;
     if (tid == 0) dep_launch();
     uint2 gw = make_uint2(0, 0), sw = make_uint2(0, 0), bw = make_uint2(0, 0);
     if (own) {
         gw = __ldg(reinterpret_cast<const uint2*>(a.gain + d)); sw = __ldg(reinterpret_cast<const uint2*>(a.shift + d));
-        if (MODE != NORM_EMBED) bw = __ldg(reinterpret_cast<const uint2*>(a.bias + d));
+        if (MODE != NORM_EMBED && a.nparts) bw = __ldg(reinterpret_cast<const uint2*>(a.bias + d));
     }
+    const float rd = 1.0f / (float)a.D, rl = 1.0f / (float)(a.D - (nw - 1) * 128);   // one over the elements of the row, of the last warp
     if (MODE != NORM_EMBED) dep_wait();
     const int out = blockIdx.x;
     int row = out;
-    if (MODE == NORM_FINAL && a.want) row = __ldcg(a.want + out);
+    if (MODE == NORM_FINAL && a.want) row = __ldg(a.want + out);
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (MODE == NORM_EMBED) {
         // tokens and positions outside their ranges would index outside the tables and the caches: the pass is refused
@@ -418,35 +444,39 @@ __global__ void __launch_bounds__(1024) pass_norm(const __grid_constant__ NormAr
             v = make_float4(h_lo(e.x) + h_lo(p.x), h_hi(e.x) + h_hi(p.x), h_lo(e.y) + h_lo(p.y), h_hi(e.y) + h_hi(p.y));
         }
     } else if (own) {
+        float4 p[PARTS_MAX];
         v = __ldcg(reinterpret_cast<const float4*>(a.z + (size_t)row * a.D + d));
+#pragma unroll
+        for (int s = 0; s < PARTS_MAX; s++) p[s] = s < a.nparts ? __ldcg(reinterpret_cast<const float4*>(a.part + s * a.part_stride + (size_t)row * a.D + d)) : make_float4(0.f, 0.f, 0.f, 0.f);
         v.x += h_lo(bw.x); v.y += h_hi(bw.x); v.z += h_lo(bw.y); v.w += h_hi(bw.y);
-#pragma unroll 4
-        for (int s = 0; s < a.nparts; s++) {
-            const float4 p = __ldcg(reinterpret_cast<const float4*>(a.part + s * a.part_stride + (size_t)row * a.D + d));
-            v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
-        }
+#pragma unroll
+        for (int s = 0; s < PARTS_MAX; s++) { v.x += p[s].x; v.y += p[s].y; v.z += p[s].z; v.w += p[s].w; }
     }
-    if (MODE != NORM_FINAL && own) *reinterpret_cast<float4*>(a.z + (size_t)row * a.D + d) = v;
+    if (own && (MODE == NORM_EMBED || (MODE == NORM_MID && a.nparts))) *reinterpret_cast<float4*>(a.z + (size_t)row * a.D + d) = v;
     float s = (v.x + v.y) + (v.z + v.w);
 #pragma unroll
     for (int m = 16; m; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
-    if (lane == 0) red[0][warp] = s;
-    __syncthreads();
-    s = 0.f;
-    for (int i = 0; i < nw; i++) s += red[0][i];
-    const float mean = s / a.D;
-    const float x0 = v.x - mean, x1 = v.y - mean, x2 = v.z - mean, x3 = v.w - mean;
-    float q = own ? (x0 * x0 + x1 * x1) + (x2 * x2 + x3 * x3) : 0.f;
+    const float mw = s * (warp < nw - 1 ? 1.0f / 128.0f : rl);
+    float y0 = v.x - mw, y1 = v.y - mw, y2 = v.z - mw, y3 = v.w - mw;
+    float q = own ? (y0 * y0 + y1 * y1) + (y2 * y2 + y3 * y3) : 0.f;
 #pragma unroll
     for (int m = 16; m; m >>= 1) q += __shfl_xor_sync(0xffffffffu, q, m);
-    if (lane == 0) red[1][warp] = q;
+    if (lane == 0) red[warp] = make_float2(s, q);
     __syncthreads();
-    q = 0.f;
-    for (int i = 0; i < nw; i++) q += red[1][i];
-    const float rs = rsqrtf(q / a.D + a.eps);
+    // the block's mean, then its squared deviations: every warp's own plus its elements times (its mean - the mean)^2
+    const float2 mine = lane < nw ? red[lane] : make_float2(0.f, 0.f);
+    s = mine.x;
+#pragma unroll
+    for (int m = 16; m; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+    const float mean = s * rd;
+    const float dm = mine.x * (lane < nw - 1 ? 1.0f / 128.0f : rl) - mean;
+    q = lane < nw ? mine.y + (lane < nw - 1 ? 128.0f : (float)(a.D - (nw - 1) * 128)) * dm * dm : 0.f;
+#pragma unroll
+    for (int m = 16; m; m >>= 1) q += __shfl_xor_sync(0xffffffffu, q, m);
+    const float rs = rsqrtf(q * rd + a.eps);
     if (own) {
-        const float o0 = x0 * rs * h_lo(gw.x) + h_lo(sw.x), o1 = x1 * rs * h_hi(gw.x) + h_hi(sw.x);
-        const float o2 = x2 * rs * h_lo(gw.y) + h_lo(sw.y), o3 = x3 * rs * h_hi(gw.y) + h_hi(sw.y);
+        const float o0 = (v.x - mean) * rs * h_lo(gw.x) + h_lo(sw.x), o1 = (v.y - mean) * rs * h_hi(gw.x) + h_hi(sw.x);
+        const float o2 = (v.z - mean) * rs * h_lo(gw.y) + h_lo(sw.y), o3 = (v.w - mean) * rs * h_hi(gw.y) + h_hi(sw.y);
         const u32 p0 = pack_h2(o0, o1), p1 = pack_h2(o2, o3);
         *reinterpret_cast<uint2*>(a.act + (size_t)out * a.D + d) = make_uint2(p0, p1);
         if (a.rp) *reinterpret_cast<uint2*>(a.act + (size_t)(a.rp + out) * a.D + d) = make_uint2(pack_h2(o0 - h_lo(p0), o1 - h_hi(p0)), pack_h2(o2 - h_lo(p1), o3 - h_hi(p1)));
@@ -458,75 +488,93 @@ struct AttArgs {
     const float* q;                  // [row][D] fp32
     const u16 *kc, *vc;              // the caches at this layer
     long long seq_stride;            // elements between two sequences
-    const int *pos, *seq;
-    int D, pow2, rp;
+    const int *t, *seq;              // positions as the step began (they change only after it)
+    int t_stride, tmax, D, pow2, rp;
     float scale;
     u16* out;                        // [row][D] fp16 (and the remainder plane)
 };
 #define ATT_WARPS 4
-// Block = one (row, head), or 1 / C of its positions where C blocks form a cluster; warps take runs of 32 positions in
-// turn. A group of eight lanes reads one position's 128 bytes (16 per lane), eight positions per group and step are in flight
-// for K and for V. fp32 arithmetic on the ordinary cores: 9 warp instructions per position and head, 11 us per layer
-// at 256 sequences of 290 positions where reading the cache takes 35.
-__global__ void __launch_bounds__(ATT_WARPS * 32) pass_attend(const __grid_constant__ AttArgs a) {
+// Block = one (row, head), or 1 / C of its positions where C blocks form a cluster; warps take runs of 16 positions in
+// turn. A group of eight lanes reads one position's 128 bytes (16 per lane), four positions per group are in flight for K
+// and for V, the next run's while one is computed. fp32 arithmetic on the ordinary cores: about 10 warp instructions per
+// position and head. The rows before the current position are there since earlier steps: a warp's first run is in its
+// registers, and the rest of its rows on the way to L2, before the block waits for the kernel that computes the query and the
+// current position's row. Six blocks per SM (64 sequences x 12 heads are resident at once; runs of 32 positions took 128
+// registers, four blocks per SM, and a second round).
+#define ATT_RUN 16
+__global__ void __launch_bounds__(ATT_WARPS * 32, 6) pass_attend(const __grid_constant__ AttArgs a) {
     __shared__ float part[ATT_WARPS + 1][66];
     const int h = blockIdx.x, row = blockIdx.y, C = gridDim.z, cr = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, pl = lane >> 3, dl = lane & 7;
     if (threadIdx.x == 0) dep_launch();
+    const int n = min(__ldcg(a.t + row * a.t_stride) + 1, a.tmax), sq = a.seq ? __ldcg(a.seq + row) : row;
+    const u16* kp = a.kc + sq * a.seq_stride + h * 64 + dl * 8;
+    const u16* vp = a.vc + sq * a.seq_stride + h * 64 + dl * 8;
+    const int step = C * ATT_WARPS * ATT_RUN;
+    int p0 = (cr * ATT_WARPS + warp) * ATT_RUN;
+    uint4 k[4], v[4];
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int j = 0; j < 4; j++) { const int p = p0 + j * 4 + pl; k[j] = p < n - 1 ? __ldcg(reinterpret_cast<const uint4*>(kp + (size_t)p * a.D)) : zero; }
+#pragma unroll
+    for (int j = 0; j < 4; j++) { const int p = p0 + j * 4 + pl; v[j] = p < n - 1 ? __ldcg(reinterpret_cast<const uint4*>(vp + (size_t)p * a.D)) : zero; }
+#pragma unroll 1
+    for (int p = p0 + step + (lane & 15); p < n - 1; p += step)
+        asm volatile("prefetch.global.L2 [%0];" :: "l"((lane < 16 ? kp : vp) - dl * 8 + (size_t)p * a.D));
     dep_wait();
-    const int n = __ldcg(a.pos + row) + 1, sq = a.seq ? __ldcg(a.seq + row) : row;
     float q[8];
     {
         const float4* qp = reinterpret_cast<const float4*>(a.q + (size_t)row * a.D + h * 64 + dl * 8);
         const float4 q0 = __ldcg(qp), q1 = __ldcg(qp + 1);
+        const int at = n - 1 - p0;                                                 // the current position, if it is in this run
+        if (n > 0 && at >= 0 && at < ATT_RUN) {
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (at == j * 4 + pl) {
+                    k[j] = __ldcg(reinterpret_cast<const uint4*>(kp + (size_t)(n - 1) * a.D));
+                    v[j] = __ldcg(reinterpret_cast<const uint4*>(vp + (size_t)(n - 1) * a.D));
+                }
+        }
         const float sc = a.pow2 ? 1.0f / a.scale : 1.0f;
         q[0] = q0.x * sc; q[1] = q0.y * sc; q[2] = q0.z * sc; q[3] = q0.w * sc; q[4] = q1.x * sc; q[5] = q1.y * sc; q[6] = q1.z * sc; q[7] = q1.w * sc;
     }
-    const u16* kp = a.kc + sq * a.seq_stride + h * 64 + dl * 8;
-    const u16* vp = a.vc + sq * a.seq_stride + h * 64 + dl * 8;
     float m = -3.0e38f, den = 0.f, o[8];
 #pragma unroll
     for (int e = 0; e < 8; e++) o[e] = 0.f;
 #pragma unroll 1
-    for (int p0 = (cr * ATT_WARPS + warp) * 32; p0 < n; p0 += C * ATT_WARPS * 32) {
-        uint4 k[8], v[8];
+    while (p0 < n) {
+        float s[4];
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const int p = min(p0 + j * 4 + pl, n - 1);
-            k[j] = __ldcg(reinterpret_cast<const uint4*>(kp + (size_t)p * a.D));
-        }
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const int p = min(p0 + j * 4 + pl, n - 1);
-            v[j] = __ldcg(reinterpret_cast<const uint4*>(vp + (size_t)p * a.D));
-        }
-        float s[8];
-#pragma unroll
-        for (int j = 0; j < 8; j++)
+        for (int j = 0; j < 4; j++)
             s[j] = (q[0] * h_lo(k[j].x) + q[1] * h_hi(k[j].x)) + (q[2] * h_lo(k[j].y) + q[3] * h_hi(k[j].y)) +
                    ((q[4] * h_lo(k[j].z) + q[5] * h_hi(k[j].z)) + (q[6] * h_lo(k[j].w) + q[7] * h_hi(k[j].w)));
-        // sums over the eight lanes of a group, transposed: lane dl ends with the score of position p0 + 4 dl + pl
+        const int p1 = p0 + step;
 #pragma unroll
-        for (int j = 0; j < 4; j++) { const float keep = (dl & 4) ? s[j + 4] : s[j], give = (dl & 4) ? s[j] : s[j + 4]; s[j] = keep + __shfl_xor_sync(0xffffffffu, give, 4); }
+        for (int j = 0; j < 4; j++) { const int p = p1 + j * 4 + pl; if (p < n) k[j] = __ldcg(reinterpret_cast<const uint4*>(kp + (size_t)p * a.D)); }
+        // sums over the eight lanes of a group, transposed: lane dl ends with the score of position p0 + 4 (dl / 2) + pl
 #pragma unroll
-        for (int j = 0; j < 2; j++) { const float keep = (dl & 2) ? s[j + 2] : s[j], give = (dl & 2) ? s[j] : s[j + 2]; s[j] = keep + __shfl_xor_sync(0xffffffffu, give, 2); }
-        { const float keep = (dl & 1) ? s[1] : s[0], give = (dl & 1) ? s[0] : s[1]; s[0] = keep + __shfl_xor_sync(0xffffffffu, give, 1); }
-        float sc = a.pow2 ? s[0] : s[0] / a.scale;
-        const bool live = p0 + dl * 4 + pl < n;
+        for (int j = 0; j < 2; j++) { const float keep = (dl & 4) ? s[j + 2] : s[j], give = (dl & 4) ? s[j] : s[j + 2]; s[j] = keep + __shfl_xor_sync(0xffffffffu, give, 4); }
+        { const float keep = (dl & 2) ? s[1] : s[0], give = (dl & 2) ? s[0] : s[1]; s[0] = keep + __shfl_xor_sync(0xffffffffu, give, 2); }
+        s[0] += __shfl_xor_sync(0xffffffffu, s[0], 1);
+        const float sc = a.pow2 ? s[0] : s[0] / a.scale;
+        const bool live = p0 + (dl >> 1) * 4 + pl < n;
         int km = __float_as_int(live ? sc : -3.0e38f);
         km = __reduce_max_sync(0xffffffffu, km >= 0 ? km : km ^ 0x7fffffff);
         const float mn = fmaxf(m, __int_as_float(km >= 0 ? km : km ^ 0x7fffffff));
         const float corr = fast_exp(m - mn), p = live ? fast_exp(sc - mn) : 0.f;
         m = mn;
-        den = den * corr + p;
+        den = den * corr + ((dl & 1) ? 0.f : p);
 #pragma unroll
         for (int e = 0; e < 8; e++) o[e] *= corr;
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const float pj = __shfl_sync(0xffffffffu, p, (lane & 24) | j);
+        for (int j = 0; j < 4; j++) {
+            const float pj = __shfl_sync(0xffffffffu, p, (lane & 24) | (2 * j));
             o[0] += pj * h_lo(v[j].x); o[1] += pj * h_hi(v[j].x); o[2] += pj * h_lo(v[j].y); o[3] += pj * h_hi(v[j].y);
             o[4] += pj * h_lo(v[j].z); o[5] += pj * h_hi(v[j].z); o[6] += pj * h_lo(v[j].w); o[7] += pj * h_hi(v[j].w);
         }
+        p0 = p1;
+#pragma unroll
+        for (int j = 0; j < 4; j++) { const int p = p0 + j * 4 + pl; if (p < n) v[j] = __ldcg(reinterpret_cast<const uint4*>(vp + (size_t)p * a.D)); }
     }
 #pragma unroll
     for (int e = 0; e < 8; e++) { o[e] += __shfl_xor_sync(0xffffffffu, o[e], 8); o[e] += __shfl_xor_sync(0xffffffffu, o[e], 16); }

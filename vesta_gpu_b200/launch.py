@@ -1,5 +1,6 @@
-"""Compile a Lowered program with NVRTC for sm_100a and run it as one cooperative launch per
-decode step, through the C ABI of libvesta_b200.so (include/vesta_b200.h) bound with ctypes.
+"""Run a Lowered program through the C ABI of libvesta_b200.so (include/vesta_b200.h) bound with ctypes: a decode step as a
+chain of kernels of the library (passes.py), or, where the lowering asks for it (tune options, timing), as one persistent
+kernel compiled with NVRTC for sm_100a and launched cooperatively.
 
 Mirrors the reference run-time (vesta/launch.py:10-73): `TORCH_DT`, `ok`, `compile_cubin`,
 and `Kernel` with `view`, `bind`, `launch`, `__call__` and the attributes `mod, fn, smem, sms,
@@ -130,13 +131,7 @@ class Kernel:
                 raise RuntimeError(f'program was placed for {lowered.grid} SMs, device has {self.sms}: '
                                    f'call lower(..., grid={self.sms})')
             self.lowered = lowered
-            self.cubin = compile_cubin(lowered.src, ARCH)
-            self._cubin_buf = ctypes.create_string_buffer(self.cubin, len(self.cubin))
-            mod, fn, pk = ctypes.c_void_p(), ctypes.c_void_p(), ctypes.c_void_p()
-            ok(L.vesta_module_load(ctypes.cast(self._cubin_buf, ctypes.c_void_p), ctypes.byref(mod)))
-            ok(L.vesta_module_get_function(mod, b'vesta_step', ctypes.byref(fn)))
-            ok(L.vesta_module_get_function(mod, b'vesta_pack', ctypes.byref(pk)))
-            self.mod, self.fn, self.pack_fn = mod, fn, pk
+            self.chain = bool(lowered.dims.get('chain'))         # a step is a chain of kernels (passes.py), not one persistent kernel
             self.smem = lowered.shared_bytes
             # The reference's signature defaults to block=256 (vesta/launch.py:30) and callers pass it along: 256 and
             # None both mean "the block size the program was lowered for" (8 consumer warps + the producer warp).
@@ -147,21 +142,54 @@ class Kernel:
                 import warnings
                 warnings.warn(f'blocks_per_sm={blocks_per_sm} is ignored: the step kernel is placed for one persistent block per SM',
                               RuntimeWarning, stacklevel=2)
-            ok(L.vesta_func_set_max_dynamic_smem(fn, self.smem))
-            per_sm = ctypes.c_int()
-            ok(L.vesta_occupancy(fn, self.block, self.smem, ctypes.byref(per_sm)))
-            if per_sm.value < 1:
-                raise RuntimeError('kernel cannot be resident at this block size')
             self.grid = self.sms                                 # one persistent CTA per SM
             self.S = torch.zeros(lowered.scratch_floats, dtype=torch.float32, device=self.device)
             self.bar = torch.zeros(lowered.counters, dtype=torch.int32, device=self.device)
             self.TS = torch.zeros(2048, dtype=torch.int64, device=self.device)
-            self.PT = torch.from_numpy(np.ascontiguousarray(lowered.place)).to(self.device)
-            self.WP = torch.empty(max(lowered.packed_bytes, 512), dtype=torch.uint8, device=self.device)
+            self._module = self._packed = None
             self.args, self.keep, self._bound = None, None, None
             self.fuse = 16                                       # decode steps per launch in launch(steps > 1)
             self.feeds_back = '#define V_FEEDBACK 1' in lowered.src
             self.launches = 0
+            if not self.chain:
+                self._load()
+
+    def _load(self):
+        """compile and load the persistent kernel -> (module, step function, packing function). A kernel that runs its steps
+        as a chain does this only for callers that ask for the function (e.g. vesta_step_static)."""
+        if self._module is None:
+            with torch.cuda.device(self.device):
+                L = lib()
+                self.cubin = compile_cubin(self.lowered.src, ARCH)
+                self._cubin_buf = ctypes.create_string_buffer(self.cubin, len(self.cubin))
+                mod, fn, pk = ctypes.c_void_p(), ctypes.c_void_p(), ctypes.c_void_p()
+                ok(L.vesta_module_load(ctypes.cast(self._cubin_buf, ctypes.c_void_p), ctypes.byref(mod)))
+                ok(L.vesta_module_get_function(mod, b'vesta_step', ctypes.byref(fn)))
+                ok(L.vesta_module_get_function(mod, b'vesta_pack', ctypes.byref(pk)))
+                ok(L.vesta_func_set_max_dynamic_smem(fn, self.smem))
+                per_sm = ctypes.c_int()
+                ok(L.vesta_occupancy(fn, self.block, self.smem, ctypes.byref(per_sm)))
+                if per_sm.value < 1:
+                    raise RuntimeError('kernel cannot be resident at this block size')
+                self._module = (mod, fn, pk)
+        return self._module
+
+    mod = property(lambda self: self._load()[0])
+    fn = property(lambda self: self._load()[1])
+    pack_fn = property(lambda self: self._load()[2])
+
+    def _pack_once(self):
+        """-> (packed weight streams, placement table) of the persistent kernel, made at the first use"""
+        if self._packed is None:
+            low = self.lowered
+            self._packed = (torch.empty(max(low.packed_bytes, 512), dtype=torch.uint8, device=self.device),
+                            torch.from_numpy(np.ascontiguousarray(low.place)).to(self.device))
+            if self.keep is not None:
+                self.pack()
+        return self._packed
+
+    WP = property(lambda self: self._pack_once()[0])
+    PT = property(lambda self: self._pack_once()[1])
 
     def view(self, name):
         off, _, shape = self.lowered.scratch[name]
@@ -176,25 +204,39 @@ class Kernel:
         """fix the argument list once (launches then cost one call) and pack the weights"""
         L = lib()
         vals = []
-        if any(name == '_zeros' for name, _, _ in self.lowered.params) and '_zeros' not in residue:
+        zeros = residue.get('_zeros')
+        if 'zeros_len' in self.lowered.dims and zeros is None and any(name == '_zeros' for name, _, _ in self.lowered.params):
             # additive parameters the program does not have (lower.OPTIONAL_TERMS): the kernel reads zeros for them
-            residue = dict(residue, _zeros=torch.zeros(self.lowered.dims['zeros_len'], dtype=torch.float16, device=self.device))
+            zeros = torch.zeros(self.lowered.dims['zeros_len'], dtype=torch.float16, device=self.device)
+            residue = dict(residue, _zeros=zeros)
         for name, dt, _ in self.lowered.params:
             t = residue[name]
             assert t.is_cuda and t.dtype == TORCH_DT[dt] and t.is_contiguous(), (name, t.dtype, dt)
             assert t.device == self.device, (name, t.device)
             vals.append(t.data_ptr())
-        self.TM = self.tensor_maps(residue)
-        vals += [self.S.data_ptr(), self.bar.data_ptr(), self.TS.data_ptr(), self.WP.data_ptr(), self.PT.data_ptr(), self.TM.data_ptr(), 1]
-        self.args = (tuple(vals), tuple([ctypes.c_void_p] * len(vals)))
         self.keep = residue
         if self._bound:
             L.vesta_step_release(self._bound)
-        arr = (ctypes.c_ulonglong * len(vals))(*vals)
+            self._bound = None
         bound = ctypes.c_void_p()
-        ok(L.vesta_step_bind(self.fn, self.grid, self.block, self.smem, len(vals), arr, ctypes.byref(bound)))
-        self._bound = bound
-        self.pack(residue)
+        if self.chain:
+            from .passes import bind_step
+            vals += [self.S.data_ptr(), self.bar.data_ptr(), self.TS.data_ptr()]
+            with torch.cuda.device(self.device):
+                self._bound, self._work = bind_step(self, residue, zeros)
+            if self._packed is not None:
+                self.pack(residue)
+        else:
+            self.TM = self.tensor_maps(residue)
+            self.keep = None
+            wp, pt = self._pack_once()
+            self.keep = residue
+            vals += [self.S.data_ptr(), self.bar.data_ptr(), self.TS.data_ptr(), wp.data_ptr(), pt.data_ptr(), self.TM.data_ptr(), 1]
+            arr = (ctypes.c_ulonglong * len(vals))(*vals)
+            ok(L.vesta_step_bind(self.fn, self.grid, self.block, self.smem, len(vals), arr, ctypes.byref(bound)))
+            self._bound = bound
+            self.pack(residue)
+        self.args = (tuple(vals), tuple([ctypes.c_void_p] * len(vals)))
 
     def tensor_maps(self, residue):
         """the TMA descriptors of the step kernel, in device memory: the caches as the attention phase reads
@@ -213,7 +255,10 @@ class Kernel:
         return host.to(self.device)
 
     def pack(self, residue=None):
-        """(re)build the packed weight streams from the bound weights; call again after changing them"""
+        """(re)build the packed weight streams from the bound weights; call again after changing them (a chain reads the
+        weights where they are: nothing to do unless its persistent kernel has been asked for)"""
+        if self.chain and self._packed is None:
+            return
         residue = residue or self.keep
         L = lib()
         vals = [residue[n].data_ptr() for n in self.lowered.pack_params] + [self.WP.data_ptr(), self.PT.data_ptr()]

@@ -589,6 +589,13 @@ def lower(text, res, axis_max, batch=1, per_token=(), outputs=(), feedback=None,
             raise NotImplementedError(f'output {o}: only {env["$logit"]} and {env["$next"]} are kept for the host')
 
     tune = dict(tune or {})
+    # What a step as a chain of kernels (csrc/pass.cu) needs to know; Kernel runs that chain unless the caller asked for
+    # something that only the persistent kernels have (a placement option, timing sums, rows of prompts).
+    # Up to eight sequences the small persistent kernel is the faster one (one sequence 172 against 250 us per step, eight 243
+    # against 270, XL shape with one 1,164 against 1,290): its exchanges between a few CTAs cost less than kernel boundaries.
+    dims = dict(dims, chain=not (tune or timing or row_seq or slab_tiles or act_lo is not None) and B > 8 and D <= 4096,
+                step=dict(t_stride=int(t_per_token), tstep=int(fb.get(t_name, 0)), feedback=int(bool(fb)), prompt_len=int(prompt_len) if fb else 0,
+                          exact=int(B <= 8 or (B <= 16 and D <= 1024)), cpos=cpos))
     if B <= 8 and not tune.get('large_kernel') and act_lo is None and not slab_tiles and not row_seq:
         return _lower_small(env, dims, res, roles, fb, B, tmax, cpos, t_per_token, t_name, prompt_len, timing, grid, tune)
 

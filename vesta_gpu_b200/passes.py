@@ -47,6 +47,22 @@ def create(desc, device, graph=False):
     return h, ws
 
 
+def bind_step(kernel, residue, zeros):
+    """a decode step over the tensors of `residue` as a chain of kernels -> (handle for vesta_step_run, workspace)"""
+    low = kernel.lowered
+    d, st = low.dims, low.dims['step']
+    off = {n: kernel.S.data_ptr() + 4 * v[0] for n, v in low.scratch.items()}
+    logit, nxt = list(off.values())
+    desc = describe(low, residue, zeros, st['cpos'], rows=d['B'], logit_rows=d['B'], exact=st['exact'], t_stride=st['t_stride'],
+                    tstep=st['tstep'], feedback=st['feedback'], prompt_len=st['prompt_len'], x=residue[low.roles['x']], t=residue[low.roles['t']],
+                    prompt=residue['prompt'] if st['prompt_len'] else None, plen=residue['plen'] if st['prompt_len'] else None,
+                    logits=logit, next=nxt, bar=kernel.bar)
+    h, ws = create(desc, kernel.device, graph=True)
+    bound = ctypes.c_void_p()
+    ok(lib().vesta_pass_bind(h, ctypes.byref(bound)))
+    return bound, ws
+
+
 class PromptPass:
     """Whole prompts as dense passes over up to `rows` (sequence, position) rows that write a model's caches: every row's
     K and V are written before any row attends, so a row sees the rows of its own sequence before it. Only the last
