@@ -88,25 +88,24 @@ void vesta_step_release(void* bound);
 typedef struct vesta_pass_desc {
     int L, D, H, F, N, tmax, cpos;      /* sizes of the model, rows of a cache plane and of the position table */
     int rows, logit_rows;               /* most rows of a pass, most rows that want logits */
+    int prompts;                        /* 0: a decode step, a row per sequence; else the number of sequences whose prompts the pass reads */
     int exact;                          /* activations enter the products at fp32 accuracy (at most 16 rows), else rounded to fp16 */
     int t_stride, tstep, feedback, prompt_len;
     float eps, scale, gelu_a, gelu_b, gelu_c;
     const void *wte, *wpe, *ln1w, *ln1b, *qkvw, *qkvb, *ow, *ob, *ln2w, *ln2b, *fcw, *fcb, *pw, *pb, *lnfw, *lnfb;
     void *keys, *vals;
-    void *x, *t;                        /* tokens [row], positions [row * t_stride]; written back with feedback */
-    const void *seq;                    /* cache sequence of every row (NULL: its own number) */
+    void *x, *t;                        /* tokens [sequence], positions [sequence * t_stride]; written back with feedback, and after prompts */
     const void *prompt, *plen;          /* feedback: tokens fed while t + 1 < plen[row] (NULL: none) */
-    const void *tiles;                  /* prompts: int4 (first row, rows, sequence, first position) per run of at most 64 rows */
-    const void *want, *dst;             /* prompts: rows that want logits, and where in x_out the chosen token goes */
-    void *x_out;
     void *logits, *next;                /* fp32 [logit row][N]; fp32 [row] or NULL */
     void *bar;                          /* status words: [0] status, [2] abort flag */
 } vesta_pass_desc;
 int vesta_pass_workspace(const vesta_pass_desc* desc, size_t* bytes);
 /* workspace: that many bytes of device memory, zeroed. graph != 0: the pass is a decode step, kept as a CUDA graph. */
 int vesta_pass_create(const vesta_pass_desc* desc, void* workspace, int graph, void** pass);
-/* the launches of one pass over prompt rows (the metadata buffers of the descriptor hold them) */
-int vesta_pass_run(void* pass, void* stream, int rows, int logit_rows, int tiles);
+/* Whole prompts: tokens [prompts][ld] and lens [prompts] in host memory. Every prompt position goes into the caches (rows after a
+ * prompt are zeroed), x gets the token chosen after every prompt, t its position; in passes of at most desc.rows rows.
+ * Synchronises `stream`; *status as bar[0] (not zero: refused, a token outside the vocabulary). */
+int vesta_pass_prompts(void* pass, void* stream, const int* tokens, int ld, const int* lens, unsigned* status);
 /* a pass created with a graph as what vesta_step_run, vesta_step_run_fused and vesta_step_host take; owns the pass */
 int vesta_pass_bind(void* pass, void** bound);
 void vesta_pass_release(void* pass);

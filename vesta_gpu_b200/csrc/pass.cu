@@ -24,7 +24,18 @@ enum Kind { K_QKV = 0, K_PROJ = 1, K_FC = 2, K_P2 = 3, K_LOGITS = 4 };
 
 struct Tile { int bm, bn, stages, splits; };
 
-struct Layout { size_t z, q, act, att, gelu, part, fin, best, rowoff, pos, skip, total; };
+struct Layout {
+    size_t z, q, act, att, gelu, part, fin, best, rowoff, pos, skip;
+    size_t meta, total;                        // prompts: tokens, positions, sequences of the rows; attention runs; rows that want logits and where they go; lengths
+};
+// the metadata of a pass over prompts, as offsets in 32-bit words
+struct Meta {
+    int x, t, seq, tiles, want, dst, lens, words, max_tiles;
+    Meta(int rows, int lrows, int seqs) {
+        max_tiles = rows / 64 + std::min(rows, seqs) + 1;
+        tiles = 0; dst = tiles + 4 * max_tiles; x = dst + 2 * lrows; t = x + rows; seq = t + rows; want = seq + rows; lens = want + lrows; words = lens + seqs;
+    }
+};
 
 struct Pass {
     vesta_pass_desc d;
@@ -38,6 +49,8 @@ struct Pass {
     int max_parts;
     std::vector<cudaGraphExec_t> graphs;       // decode: one step
     int sms;
+    int* host;                                 // prompts: pinned metadata, one copy per pass of a call, then a status word
+    size_t host_words;
 };
 
 // rows of an operand: one product column per row; up to 16 rows at fp32 accuracy take two planes of 8 or 16
@@ -96,6 +109,7 @@ Layout layout(const Pass& p, int D, int F, int rows, int lrows) {
     o.rowoff = take((size_t)rows * 8);
     o.pos = take((size_t)rows * 4);
     o.skip = take(4);
+    o.meta = p.d.prompts ? take((size_t)Meta(rows, lrows, p.d.prompts).words * 4) : 0;
     o.total = at;
     return o;
 }
@@ -125,6 +139,18 @@ int plan(Pass& p, const vesta_pass_desc* d) {
     return 0;
 }
 
+// The kernels of a pass ask for the same split of an SM between shared memory and cache: an SM changes it only when it is idle,
+// and a block that waits for that cannot start under its predecessor (23 sequences: projection 3.0 -> 2.4 us, norm 4.5 -> 3.5).
+template <class F> cudaError_t all_shared(F* f) { return cudaFuncSetAttribute((const void*)f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared); }
+cudaError_t prepare_all() {
+    cudaError_t e = cudaSuccess;
+    auto one = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
+    one(all_shared(pass_norm<NORM_EMBED>)); one(all_shared(pass_norm<NORM_MID>)); one(all_shared(pass_norm<NORM_FINAL>));
+    one(all_shared(pass_norm_rows<6>)); one(all_shared(pass_norm_rows<13>)); one(all_shared(pass_norm_rows<16>));
+    one(all_shared(pass_attend<2>)); one(all_shared(pass_attend<4>)); one(all_shared(pass_attend_many));
+    one(cudaFuncSetAttribute((const void*)pass_attend<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * ATT_WARPS * 4096)); one(all_shared(pass_finish));
+    return e;
+}
 template <int BM, int EPI>
 cudaError_t launch_gemm(cudaLaunchConfig_t& c, const Tile& t, const CUtensorMap& w, const CUtensorMap& a, const GemmArgs& g) {
     c.dynamicSmemBytes = GemmShape<BM>::bytes(t.stages, t.bn);
@@ -133,7 +159,8 @@ cudaError_t launch_gemm(cudaLaunchConfig_t& c, const Tile& t, const CUtensorMap&
 }
 template <int BM, int EPI>
 cudaError_t prepare_gemm(const Tile& t) {
-    return cudaFuncSetAttribute(pass_gemm<BM, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    const cudaError_t e = all_shared(pass_gemm<BM, EPI>);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(pass_gemm<BM, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
 }
 // one case per tile shape and epilogue
 #define EACH(X) X(64, EPI_ADD) X(128, EPI_ADD) X(64, EPI_QKV) X(64, EPI_PART) X(64, EPI_GELU) X(64, EPI_LOGITS) X(128, EPI_QKV) X(128, EPI_PART) X(128, EPI_GELU) X(128, EPI_LOGITS)
@@ -163,12 +190,14 @@ struct Config {
 };
 
 // The launches of one pass over `rows` rows. Prompts: `tiles` runs of rows for the attention, `lrows` rows that want logits
-// (listed in d.want; none: the pass ends after the last layer's cache rows).
-int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles) {
+// (none: the pass ends with the last layer's cache rows); `clear`: zero the cache rows after the prompts.
+int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear = false) {
     const vesta_pass_desc& d = p.d;
     const int D = d.D, F = d.F, L = d.L, kbd = D / 64, kbf = (F + 63) / 64;
-    const bool many = d.tiles != 0;
+    const bool many = d.prompts != 0;
     auto u = [&](size_t off) { return p.ws + off; };
+    const Meta mt(d.rows, d.logit_rows, d.prompts);
+    const int* meta = (const int*)u(p.o.meta);
     float* z = (float*)u(p.o.z);
     u16 *act = (u16*)u(p.o.act), *att = (u16*)u(p.o.att), *fin = (u16*)u(p.o.fin);
     const int nthr = up(D / 4, 32);
@@ -177,15 +206,19 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles) {
         NormArgs n = {};
         n.D = D; n.nparts = nparts; n.rp = p.rp; n.eps = d.eps; n.z = z;
         n.part = (const float*)u(p.o.part); n.part_stride = (size_t)d.rows * D;
-        n.x = (const int*)d.x; n.t = (const int*)d.t; n.seq = (const int*)d.seq; n.t_stride = d.t_stride; n.N = d.N; n.cpos = d.cpos; n.tmax = d.tmax; n.L = L;
+        n.x = many ? meta + mt.x : (const int*)d.x; n.t = many ? meta + mt.t : (const int*)d.t; n.seq = many ? meta + mt.seq : 0; n.t_stride = many ? 1 : d.t_stride; n.N = d.N; n.cpos = d.cpos; n.tmax = d.tmax; n.L = L;
         n.wte = (const u16*)d.wte; n.wpe = (const u16*)d.wpe;
         n.rowoff = (long long*)u(p.o.rowoff); n.pos = (int*)u(p.o.pos); n.skip = (int*)u(p.o.skip); n.bar = (u32*)d.bar;
-        n.want = (const int*)d.want;
+        n.want = many ? meta + mt.want : 0;
         n.act = act;
         if (mode == 0) { n.gain = f16(d.ln1w, 0); n.shift = f16(d.ln1b, 0); }
         else if (mode == 1) { n.gain = f16(d.ln2w, (size_t)l * D); n.shift = f16(d.ln2b, (size_t)l * D); n.bias = f16(d.ob, (size_t)l * D); }
         else if (mode == 2) { n.gain = f16(d.ln1w, (size_t)(l + 1) * D); n.shift = f16(d.ln1b, (size_t)(l + 1) * D); n.bias = f16(d.pb, (size_t)l * D); }
         else { n.gain = f16(d.lnfw, 0); n.shift = f16(d.lnfb, 0); n.bias = f16(d.pb, (size_t)l * D); n.act = fin; }
+        if ((mode == 1 || mode == 2) && rows >= 2048 && D <= 2048 && !p.rp) {
+            Config c(dim3((rows + 7) / 8), 256, st, true);
+            return D <= 768 ? cudaLaunchKernelEx(&c.c, pass_norm_rows<6>, n, rows) : D <= 1664 ? cudaLaunchKernelEx(&c.c, pass_norm_rows<13>, n, rows) : cudaLaunchKernelEx(&c.c, pass_norm_rows<16>, n, rows);
+        }
         Config c(dim3(mode == 3 ? lrows : rows), nthr, st, mode != 0);
         return mode == 0 ? cudaLaunchKernelEx(&c.c, pass_norm<NORM_EMBED>, n) : mode == 3 ? cudaLaunchKernelEx(&c.c, pass_norm<NORM_FINAL>, n) : cudaLaunchKernelEx(&c.c, pass_norm<NORM_MID>, n);
     };
@@ -208,28 +241,33 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles) {
         Config c(dim3(t.bm == 64 && kind != K_LOGITS ? g.ntiles : std::min(g.ntiles, p.sms)), 192, st, true);
         return gemm(epi_of(kind, t), t, c.c, p.w[kind], p.a[kind], g);
     };
-    auto attend = [&](int l) {
+    auto attend = [&](int l, int tiles) {
         const float* q = (const float*)u(p.o.q);
         const u16 *kc = (const u16*)d.keys + (size_t)l * d.tmax * D, *vc = (const u16*)d.vals + (size_t)l * d.tmax * D;
         const long long ss = (long long)L * d.tmax * D;
         int e = 0;
         const int pow2 = frexpf(d.scale, &e) == 0.5f;
         if (many) {
-            AttManyArgs a = {q, kc, vc, ss, (const int4*)d.tiles, D, pow2, d.scale, att};
-            Config c(dim3(tiles, d.H), 128, st, true);
+            const int zb = clear ? (2 * p.sms + d.H - 1) / d.H : 0;
+            AttManyArgs a = {q, kc, vc, ss, (const int4*)(meta + mt.tiles), D, pow2, d.scale, att, zb, d.prompts, d.tmax, meta + mt.lens};
+            Config c(dim3(zb + tiles, d.H), 128, st, true);
             return cudaLaunchKernelEx(&c.c, pass_attend_many, a);
         }
-        AttArgs a = {q, kc, vc, ss, (const int*)d.t, (const int*)d.seq, d.t_stride, d.tmax, D, pow2, p.rp, d.scale, att};
+        AttArgs a = {q, kc, vc, ss, (const int*)d.t, (const int*)0, d.t_stride, d.tmax, D, pow2, p.rp, d.scale, att};
         int C = 1;
         while (C < 8 && rows * d.H * C * 2 <= 6 * p.sms && d.tmax > C * ATT_WARPS * ATT_RUN) C *= 2;
         Config c(dim3(d.H, rows, C), ATT_WARPS * 32, st, true, C);
-        return cudaLaunchKernelEx(&c.c, pass_attend, a);
+        // deep rings where few blocks share an SM, all blocks resident where they are many
+        const bool deep = rows * d.H * C <= 3 * p.sms;
+        c.c.dynamicSmemBytes = (deep ? 4 : 2) * ATT_WARPS * 4096;
+        return deep ? cudaLaunchKernelEx(&c.c, pass_attend<4>, a) : cudaLaunchKernelEx(&c.c, pass_attend<2>, a);
     };
     TRY(norm(0, 0, 0));
     for (int l = 0; l < L; l++) {
         TRY(mul(K_QKV, l));
-        if (l == L - 1 && lrows == 0) break;
-        TRY(attend(l));
+        const bool end = l == L - 1 && lrows == 0;
+        if (!end || clear) TRY(attend(l, end ? 0 : tiles));
+        if (end) break;
         TRY(mul(K_PROJ, l));
         TRY(norm(1, l, p.tile[K_PROJ].splits > 1 ? p.tile[K_PROJ].splits : 0));
         TRY(mul(K_FC, l));
@@ -239,8 +277,8 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles) {
     if (lrows) TRY(mul(K_LOGITS, 0));
     FinishArgs f = {};
     f.rows = lrows; f.best = (u64*)u(p.o.best); f.skip = (int*)u(p.o.skip); f.next = (float*)d.next; f.pos = (const int*)u(p.o.pos);
-    f.t_stride = d.t_stride; f.tstep = d.tstep; f.N = d.N; f.dst = (const int*)d.dst;
-    if (d.dst) f.x = (int*)d.x_out;
+    f.t_stride = d.t_stride; f.tstep = d.tstep; f.N = d.N;
+    if (many) { f.dst = (const int2*)(meta + mt.dst); f.x = (int*)d.x; f.t = (int*)d.t; }
     else if (d.feedback) { f.x = (int*)d.x; f.t = (int*)d.t; f.prompt = (const int*)d.prompt; f.plen = (const int*)d.plen; f.plen_cap = d.prompt_len; }
     Config c(dim3(1), 256, st, true);
     TRY(cudaLaunchKernelEx(&c.c, pass_finish, f));
@@ -281,6 +319,7 @@ int vesta_pass_create(const vesta_pass_desc* d, void* workspace, int graph, void
     const int D = d->D, F = d->F;
     const void* w[5] = {d->qkvw, d->ow, d->fcw, d->pw, d->wte};
     const int fold[5] = {D, D, D, F, D}, feat[5] = {3 * D, D, F, D, d->N};
+    if (!e) { const cudaError_t ce = prepare_all(); if (ce != cudaSuccess) e = cuda_fail(ce, "cudaFuncSetAttribute"); }
     unsigned char* op[5] = {p->ws + p->o.act, p->ws + p->o.att, p->ws + p->o.act, p->ws + p->o.gelu, p->ws + p->o.fin};
     for (int k = 0; k < 5 && !e; k++) {
         const Tile& t = p->tile[k];
@@ -312,17 +351,64 @@ int vesta_pass_create(const vesta_pass_desc* d, void* workspace, int graph, void
     return 0;
 }
 
-int vesta_pass_run(void* pass, void* stream, int rows, int logit_rows, int tiles) {
+int vesta_pass_prompts(void* pass, void* stream, const int* tokens, int ld, const int* lens, unsigned* status) {
     Pass* p = (Pass*)pass;
-    if (!p) return fail(-1, "vesta_pass_run: no pass");
-    if (rows < 1 || rows > p->d.rows || logit_rows < 0 || logit_rows > p->d.logit_rows || tiles < 0) return fail(-1, "vesta_pass_run: row counts outside what the pass was created for");
-    return enqueue(*p, (cudaStream_t)stream, rows, logit_rows, tiles);
+    if (!p || !p->d.prompts || !tokens || !lens || !status) return fail(-1, "vesta_pass_prompts: bad argument");
+    const vesta_pass_desc& d = p->d;
+    cudaStream_t st = (cudaStream_t)stream;
+    const int B = d.prompts;
+    const Meta mt(d.rows, d.logit_rows, B);
+    long long total = 0;
+    for (int s = 0; s < B; s++) {
+        if (lens[s] < 1 || lens[s] > ld || lens[s] > d.tmax) return fail(-1, "vesta_pass_prompts: a prompt length is outside 1 .. tmax");
+        total += lens[s];
+    }
+    // passes of equal size (whole tiles of 128 rows): two of 9,200 rows rather than one of 16,384 and a small one
+    const int passes = (int)((total + d.rows - 1) / d.rows);
+    const int per = std::min<long long>(d.rows, up((total + passes - 1) / passes, 128));
+    const size_t words = (size_t)passes * mt.words + 4;
+    if (p->host_words < words) {
+        if (p->host) cudaFreeHost(p->host);
+        p->host = nullptr; p->host_words = 0;
+        TRY(cudaMallocHost((void**)&p->host, words * 4));
+        p->host_words = words;
+    }
+    struct Run { int first, rows, seq, pos; };
+    std::vector<Run> runs;
+    int s = 0, pos = 0;                          // next position to read
+    for (int c = 0; c < passes; c++) {
+        int* m = p->host + (size_t)c * mt.words;
+        int n = 0, lrows = 0;
+        runs.clear();
+        while (n < per && s < B) {
+            const int take = std::min(per - n, lens[s] - pos);
+            for (int i = 0; i < take; i++) { m[mt.x + n + i] = tokens[(size_t)s * ld + pos + i]; m[mt.t + n + i] = pos + i; m[mt.seq + n + i] = s; }
+            for (int i = 0; i < take; i += 64) runs.push_back(Run{n + i, std::min(64, take - i), s, pos + i});
+            n += take; pos += take;
+            if (pos == lens[s]) {
+                m[mt.want + lrows] = n - 1; m[mt.dst + 2 * lrows] = s; m[mt.dst + 2 * lrows + 1] = lens[s];
+                lrows++; s++; pos = 0;
+            }
+        }
+        // the runs that see most positions first
+        std::stable_sort(runs.begin(), runs.end(), [](const Run& a, const Run& b) { return a.pos + a.rows > b.pos + b.rows; });
+        for (size_t i = 0; i < runs.size(); i++) { int* t = m + mt.tiles + 4 * i; t[0] = runs[i].first; t[1] = runs[i].rows; t[2] = runs[i].seq; t[3] = runs[i].pos; }
+        for (int i = 0; i < B; i++) m[mt.lens + i] = lens[i];
+        TRY(cudaMemcpyAsync(p->ws + p->o.meta, m, (size_t)mt.words * 4, cudaMemcpyHostToDevice, st));
+        if (int e = enqueue(*p, st, n, lrows, (int)runs.size(), c == 0)) return e;
+    }
+    unsigned* word = (unsigned*)(p->host + words - 4);
+    TRY(cudaMemcpyAsync(word, d.bar, 4, cudaMemcpyDeviceToHost, st));
+    TRY(cudaStreamSynchronize(st));
+    *status = *word;
+    return 0;
 }
 
 void vesta_pass_release(void* pass) {
     Pass* p = (Pass*)pass;
     if (!p) return;
     for (auto g : p->graphs) cudaGraphExecDestroy(g);
+    if (p->host) cudaFreeHost(p->host);
     delete p;
 }
 

@@ -105,6 +105,10 @@ __device__ __forceinline__ void tm_ld(float (&r)[16], u32 addr) {
                  : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]), "=f"(r[8]), "=f"(r[9]), "=f"(r[10]), "=f"(r[11]),
                    "=f"(r[12]), "=f"(r[13]), "=f"(r[14]), "=f"(r[15]) : "r"(addr) : "memory");
 }
+__device__ __forceinline__ void tm_ld(float (&r)[8], u32 addr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]) : "r"(addr) : "memory");
+}
 __device__ __forceinline__ void tm_ld(float (&r)[4], u32 addr) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]) : "r"(addr) : "memory");
 }
@@ -112,6 +116,9 @@ __device__ __forceinline__ void tm_ld(float (&r)[4], u32 addr) {
 __device__ __forceinline__ void tm_wait(float (&r)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" : "+f"(r[0]), "+f"(r[1]), "+f"(r[2]), "+f"(r[3]), "+f"(r[4]), "+f"(r[5]), "+f"(r[6]), "+f"(r[7]), "+f"(r[8]), "+f"(r[9]), "+f"(r[10]),
                  "+f"(r[11]), "+f"(r[12]), "+f"(r[13]), "+f"(r[14]), "+f"(r[15]) :: "memory");
+}
+__device__ __forceinline__ void tm_wait(float (&r)[8]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+f"(r[0]), "+f"(r[1]), "+f"(r[2]), "+f"(r[3]), "+f"(r[4]), "+f"(r[5]), "+f"(r[6]), "+f"(r[7]) :: "memory");
 }
 __device__ __forceinline__ void tm_wait(float (&r)[4]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" : "+f"(r[0]), "+f"(r[1]), "+f"(r[2]), "+f"(r[3]) :: "memory");
@@ -132,7 +139,7 @@ __device__ __forceinline__ u64 best_key(int ordered, u32 n) { return ((u64)((u32
 // tensor-memory address and the dead flag; per accumulator the row offsets (QKV) or the warps' best keys (LOGITS).
 template <int BM> struct GemmShape {
     static constexpr int KS = BM == 64 ? 4 : 1;          // blocks of 64 fold indices per stage
-    static constexpr int EW = BM == 64 ? 4 : 8;          // warps that read the accumulators
+    static constexpr int EW = 8;                         // warps that read the accumulators: two per quarter of the lanes
     static constexpr int THREADS = 64 + 32 * EW;
     static __host__ __device__ constexpr int stage(int bn) { return KS * (BM + bn) * 128; }
     static __host__ __device__ constexpr int tail(int stages, int bn) { return 2 * stages * 8 + 48 + bn * 8 * 4; }
@@ -281,26 +288,29 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS) pass_gemm(const __grid
                 for (int i = et; i < bn; i += EW * 32) side[b * bn + i] = (i < live && !skip) ? (u64)__ldcg(g.rowoff + row0 + i) : ~0ull;
                 asm volatile("bar.sync 1, %0;" :: "n"(EW * 32) : "memory");
             }
+            // the second warp of a quarter takes the upper half of the rows
+            const int half = live > 4 ? ((live + 15) / 16) * 8 : 4;
+            const int c_lo = ew >= 4 ? half : 0, c_hi = min(live, ew < 4 ? half : bn);
+            // ADD: what a chunk of rows is added to is requested one chunk ahead, the first before the products are done
+            float add[16];
+            auto fetch = [&](int c) {
+                const float* src = g.of + (size_t)(row0 + c) * g.nfeat + f;
+#pragma unroll
+                for (int i = 0; i < 16; i++) add[i] = own && c + i < c_hi ? __ldcg(src + (size_t)i * g.nfeat) : 0.f;
+            };
+            if (EPI == EPI_ADD) fetch(c_lo);
             const bool ok = mbar_wait(tmf + b * 8, (n >> 1) & 1, w, 0xB20u);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (__any_sync(0xffffffffu, !ok)) break;
             const u32 ta = tmem + ((u32)(quarter * 32) << 16) + (b ? bn : 0);
             const int part = EPI == EPI_QKV ? f / g.D : 0;                         // 0 query, 1 key, 2 value (a warp never straddles two)
             u16* cache = EPI == EPI_QKV ? (part == 1 ? g.kc : g.vc) + (f - part * g.D) : (u16*)0;
-            // eight warps: two per quarter of the lanes, the second takes the upper half of the rows
-            const int half = EW == 8 ? ((bn + 31) / 32) * 16 : bn;
-            const int c_lo = EW == 8 && ew >= 4 ? half : 0, c_hi = min(live, EW == 8 && ew < 4 ? half : bn);
             // CH rows at a time (no branch per row: their chains of arithmetic overlap, only the stores are predicated); the last
             // four or fewer on their own
             auto rows_of = [&](auto CHC, int c0) {
                 constexpr int CH = decltype(CHC)::n;
                 int m = min(CH, c_hi - c0);
-                float add[CH], v[CH];
-                if (EPI == EPI_ADD) {
-                    const float* src = g.of + (size_t)(row0 + c0) * g.nfeat + f;
-#pragma unroll
-                    for (int i = 0; i < CH; i++) add[i] = own && i < m ? __ldcg(src + (size_t)i * g.nfeat) : 0.f;
-                }
+                float v[CH];
                 tm_ld(v, ta + c0);
                 if (BM == 64 && g.rp) {
                     float q[CH];
@@ -314,8 +324,10 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS) pass_gemm(const __grid
 #pragma unroll
                 for (int i = 0; i < CH; i++) {
                     v[i] += bias;
+                    if (EPI == EPI_ADD) v[i] += add[i];
                     if (EPI == EPI_GELU) v[i] = gelu_tanh(v[i], g.a2, g.k1, g.k2);
                 }
+                if (EPI == EPI_ADD && CH == 16) fetch(c0 + 16);
                 if (!own) m = 0;
                 if (EPI == EPI_QKV) {
                     if (part == 0) {
@@ -332,7 +344,7 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS) pass_gemm(const __grid
                 } else if (EPI == EPI_PART || EPI == EPI_ADD) {
                     float* dst = g.of + (EPI == EPI_PART ? z * g.part_stride : 0) + (size_t)row * g.nfeat + f;
 #pragma unroll
-                    for (int i = 0; i < CH; i++) st_f32(dst + (size_t)i * g.nfeat, EPI == EPI_ADD ? v[i] + add[i] : v[i], i < m);
+                    for (int i = 0; i < CH; i++) st_f32(dst + (size_t)i * g.nfeat, v[i], i < m);
                 } else if (EPI == EPI_GELU) {
                     u16* dst = g.oh + (size_t)row * g.nfeat + f;
 #pragma unroll
@@ -359,8 +371,9 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS) pass_gemm(const __grid
             };
             int c0 = c_lo;
 #pragma unroll 1
-            for (; c0 + 4 < c_hi; c0 += 16) rows_of(Int<16>{}, c0);
-            if (c0 < c_hi) rows_of(Int<4>{}, c0);
+            for (; c0 + 8 < c_hi; c0 += 16) rows_of(Int<16>{}, c0);
+            if (c0 + 4 < c_hi) rows_of(Int<8>{}, c0);
+            else if (c0 < c_hi) rows_of(Int<4>{}, c0);
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(tme + b * 8) : "memory");
@@ -483,6 +496,59 @@ __global__ void __launch_bounds__(1024) pass_norm(const __grid_constant__ NormAr
     }
 }
 
+// The same for many rows: a warp per row, NV float4 per lane (8 rows of 768 floats per block; one row per block took 23 us for
+// 9,200 rows, 1.8 TB/s).
+template <int NV>
+__global__ void __launch_bounds__(256) pass_norm_rows(const __grid_constant__ NormArgs a, int rows) {
+    const int lane = threadIdx.x & 31, row = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (threadIdx.x == 0) dep_launch();
+    dep_wait();
+    if (row >= rows) return;
+    float* z = a.z + (size_t)row * a.D;
+    float4 v[NV];
+#pragma unroll
+    for (int i = 0; i < NV; i++) { const int d = i * 128 + lane * 4; v[i] = d < a.D ? __ldcg(reinterpret_cast<const float4*>(z + d)) : make_float4(0.f, 0.f, 0.f, 0.f); }
+    if (a.nparts) {
+#pragma unroll
+        for (int i = 0; i < NV; i++) {
+            const int d = i * 128 + lane * 4;
+            if (d < a.D) { const uint2 bw = __ldg(reinterpret_cast<const uint2*>(a.bias + d)); v[i].x += h_lo(bw.x); v[i].y += h_hi(bw.x); v[i].z += h_lo(bw.y); v[i].w += h_hi(bw.y); }
+        }
+#pragma unroll 1
+        for (int s = 0; s < a.nparts; s++) {
+            const float* p = a.part + s * a.part_stride + (size_t)row * a.D;
+#pragma unroll
+            for (int i = 0; i < NV; i++) {
+                const int d = i * 128 + lane * 4;
+                if (d < a.D) { const float4 q = __ldcg(reinterpret_cast<const float4*>(p + d)); v[i].x += q.x; v[i].y += q.y; v[i].z += q.z; v[i].w += q.w; }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < NV; i++) { const int d = i * 128 + lane * 4; if (d < a.D) *reinterpret_cast<float4*>(z + d) = v[i]; }
+    }
+    float s = 0.f, q = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; i++) s += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+#pragma unroll
+    for (int m = 16; m; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+    const float mean = s / a.D;
+#pragma unroll
+    for (int i = 0; i < NV; i++)
+        if (i * 128 + lane * 4 < a.D) { v[i].x -= mean; v[i].y -= mean; v[i].z -= mean; v[i].w -= mean; q += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w); }
+#pragma unroll
+    for (int m = 16; m; m >>= 1) q += __shfl_xor_sync(0xffffffffu, q, m);
+    const float rs = rsqrtf(q / a.D + a.eps);
+#pragma unroll
+    for (int i = 0; i < NV; i++) {
+        const int d = i * 128 + lane * 4;
+        if (d < a.D) {
+            const uint2 gw = __ldg(reinterpret_cast<const uint2*>(a.gain + d)), sw = __ldg(reinterpret_cast<const uint2*>(a.shift + d));
+            *reinterpret_cast<uint2*>(a.act + (size_t)row * a.D + d) = make_uint2(pack_h2(v[i].x * rs * h_lo(gw.x) + h_lo(sw.x), v[i].y * rs * h_hi(gw.x) + h_hi(sw.x)),
+                                                                                 pack_h2(v[i].z * rs * h_lo(gw.y) + h_lo(sw.y), v[i].w * rs * h_hi(gw.y) + h_hi(sw.y)));
+        }
+    }
+}
+
 // ---- attention of one position per row (decode) -----------------------------------------------------------------------
 struct AttArgs {
     const float* q;                  // [row][D] fp32
@@ -495,15 +561,25 @@ struct AttArgs {
 };
 #define ATT_WARPS 4
 // Block = one (row, head), or 1 / C of its positions where C blocks form a cluster; warps take runs of 16 positions in
-// turn. A group of eight lanes reads one position's 128 bytes (16 per lane), four positions per group are in flight for K
-// and for V, the next run's while one is computed. fp32 arithmetic on the ordinary cores: about 10 warp instructions per
-// position and head. The rows before the current position are there since earlier steps: a warp's first run is in its
-// registers, and the rest of its rows on the way to L2, before the block waits for the kernel that computes the query and the
-// current position's row. Six blocks per SM (64 sequences x 12 heads are resident at once; runs of 32 positions took 128
-// registers, four blocks per SM, and a second round).
+// turn. A group of eight lanes takes one position's 128 bytes (16 per lane), four positions per group and run, K and V. fp32
+// arithmetic on the ordinary cores: about 10 warp instructions per position and head. A lane's pieces of the next NS runs are
+// on their way into shared memory (its own slots: nobody else reads them), not through the L1 cache, which is small beside the
+// contractions' blocks: loads into registers then ran at 4.7 TB/s, and 5.8 with the cache at full size. The rows before the current
+// position are there since earlier steps: the first NS runs are requested before the block waits for the kernel that computes
+// the query and the current position's row.
 #define ATT_RUN 16
-__global__ void __launch_bounds__(ATT_WARPS * 32, 6) pass_attend(const __grid_constant__ AttArgs a) {
+__device__ __forceinline__ void cp16z(u32 dst, const void* src, bool yes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(dst), "l"(src), "r"(yes ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ uint4 lds128(u32 a) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+    return v;
+}
+template <int NS>
+__global__ void __launch_bounds__(ATT_WARPS * 32) pass_attend(const __grid_constant__ AttArgs a) {
     __shared__ float part[ATT_WARPS + 1][66];
+    extern __shared__ __align__(128) unsigned char ring_raw[];
     const int h = blockIdx.x, row = blockIdx.y, C = gridDim.z, cr = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, pl = lane >> 3, dl = lane & 7;
     if (threadIdx.x == 0) dep_launch();
@@ -512,45 +588,56 @@ __global__ void __launch_bounds__(ATT_WARPS * 32, 6) pass_attend(const __grid_co
     const u16* vp = a.vc + sq * a.seq_stride + h * 64 + dl * 8;
     const int step = C * ATT_WARPS * ATT_RUN;
     int p0 = (cr * ATT_WARPS + warp) * ATT_RUN;
-    uint4 k[4], v[4];
-    const uint4 zero = make_uint4(0, 0, 0, 0);
+    const u32 ring = smem_u32(ring_raw) + warp * (NS * 4096) + lane * 16;          // [stage][K, V][j][lane]
+    auto request = [&](int st, int p, int end) {
 #pragma unroll
-    for (int j = 0; j < 4; j++) { const int p = p0 + j * 4 + pl; k[j] = p < n - 1 ? __ldcg(reinterpret_cast<const uint4*>(kp + (size_t)p * a.D)) : zero; }
+        for (int j = 0; j < 4; j++) {
+            const int x = p + j * 4 + pl;
+            cp16z(ring + st * 4096 + j * 512, kp + (size_t)(x < end ? x : 0) * a.D, x < end);
+            cp16z(ring + st * 4096 + 2048 + j * 512, vp + (size_t)(x < end ? x : 0) * a.D, x < end);
+        }
+    };
 #pragma unroll
-    for (int j = 0; j < 4; j++) { const int p = p0 + j * 4 + pl; v[j] = p < n - 1 ? __ldcg(reinterpret_cast<const uint4*>(vp + (size_t)p * a.D)) : zero; }
-#pragma unroll 1
-    for (int p = p0 + step + (lane & 15); p < n - 1; p += step)
-        asm volatile("prefetch.global.L2 [%0];" :: "l"((lane < 16 ? kp : vp) - dl * 8 + (size_t)p * a.D));
+    for (int i = 0; i < NS; i++) {
+        if (p0 + i * step < n) request(i, p0 + i * step, n - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
     dep_wait();
     float q[8];
     {
         const float4* qp = reinterpret_cast<const float4*>(a.q + (size_t)row * a.D + h * 64 + dl * 8);
         const float4 q0 = __ldcg(qp), q1 = __ldcg(qp + 1);
-        const int at = n - 1 - p0;                                                 // the current position, if it is in this run
-        if (n > 0 && at >= 0 && at < ATT_RUN) {
-#pragma unroll
-            for (int j = 0; j < 4; j++)
-                if (at == j * 4 + pl) {
-                    k[j] = __ldcg(reinterpret_cast<const uint4*>(kp + (size_t)(n - 1) * a.D));
-                    v[j] = __ldcg(reinterpret_cast<const uint4*>(vp + (size_t)(n - 1) * a.D));
-                }
-        }
         const float sc = a.pow2 ? 1.0f / a.scale : 1.0f;
+        // the current position, if it is in one of the runs requested above: its pieces by the lanes that will read them
+        uint4 kc, vc;
+        u32 at = 0;
+#pragma unroll
+        for (int i = 0; i < NS; i++) {
+            const int x = n - 1 - (p0 + i * step);
+            if (x >= 0 && x < ATT_RUN && (x & 3) == pl) at = ring + i * 4096 + (x >> 2) * 512;
+        }
+        if (at) {
+            kc = __ldcg(reinterpret_cast<const uint4*>(kp + (size_t)(n - 1) * a.D)); vc = __ldcg(reinterpret_cast<const uint4*>(vp + (size_t)(n - 1) * a.D));
+            asm volatile("cp.async.wait_all;" ::: "memory");                       // (the zeros that were requested in its place)
+            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" :: "r"(at), "r"(kc.x), "r"(kc.y), "r"(kc.z), "r"(kc.w) : "memory");
+            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" :: "r"(at + 2048), "r"(vc.x), "r"(vc.y), "r"(vc.z), "r"(vc.w) : "memory");
+        }
         q[0] = q0.x * sc; q[1] = q0.y * sc; q[2] = q0.z * sc; q[3] = q0.w * sc; q[4] = q1.x * sc; q[5] = q1.y * sc; q[6] = q1.z * sc; q[7] = q1.w * sc;
     }
     float m = -3.0e38f, den = 0.f, o[8];
 #pragma unroll
     for (int e = 0; e < 8; e++) o[e] = 0.f;
+    int st = 0;
 #pragma unroll 1
     while (p0 < n) {
+        asm volatile("cp.async.wait_group %0;" :: "n"(NS - 1) : "memory");
+        const u32 slot = ring + st * 4096;
         float s[4];
 #pragma unroll
-        for (int j = 0; j < 4; j++)
-            s[j] = (q[0] * h_lo(k[j].x) + q[1] * h_hi(k[j].x)) + (q[2] * h_lo(k[j].y) + q[3] * h_hi(k[j].y)) +
-                   ((q[4] * h_lo(k[j].z) + q[5] * h_hi(k[j].z)) + (q[6] * h_lo(k[j].w) + q[7] * h_hi(k[j].w)));
-        const int p1 = p0 + step;
-#pragma unroll
-        for (int j = 0; j < 4; j++) { const int p = p1 + j * 4 + pl; if (p < n) k[j] = __ldcg(reinterpret_cast<const uint4*>(kp + (size_t)p * a.D)); }
+        for (int j = 0; j < 4; j++) {
+            const uint4 k = lds128(slot + j * 512);
+            s[j] = (q[0] * h_lo(k.x) + q[1] * h_hi(k.x)) + (q[2] * h_lo(k.y) + q[3] * h_hi(k.y)) + ((q[4] * h_lo(k.z) + q[5] * h_hi(k.z)) + (q[6] * h_lo(k.w) + q[7] * h_hi(k.w)));
+        }
         // sums over the eight lanes of a group, transposed: lane dl ends with the score of position p0 + 4 (dl / 2) + pl
 #pragma unroll
         for (int j = 0; j < 2; j++) { const float keep = (dl & 4) ? s[j + 2] : s[j], give = (dl & 4) ? s[j] : s[j + 2]; s[j] = keep + __shfl_xor_sync(0xffffffffu, give, 4); }
@@ -568,13 +655,15 @@ __global__ void __launch_bounds__(ATT_WARPS * 32, 6) pass_attend(const __grid_co
         for (int e = 0; e < 8; e++) o[e] *= corr;
 #pragma unroll
         for (int j = 0; j < 4; j++) {
+            const uint4 v = lds128(slot + 2048 + j * 512);
             const float pj = __shfl_sync(0xffffffffu, p, (lane & 24) | (2 * j));
-            o[0] += pj * h_lo(v[j].x); o[1] += pj * h_hi(v[j].x); o[2] += pj * h_lo(v[j].y); o[3] += pj * h_hi(v[j].y);
-            o[4] += pj * h_lo(v[j].z); o[5] += pj * h_hi(v[j].z); o[6] += pj * h_lo(v[j].w); o[7] += pj * h_hi(v[j].w);
+            o[0] += pj * h_lo(v.x); o[1] += pj * h_hi(v.x); o[2] += pj * h_lo(v.y); o[3] += pj * h_hi(v.y);
+            o[4] += pj * h_lo(v.z); o[5] += pj * h_hi(v.z); o[6] += pj * h_lo(v.w); o[7] += pj * h_hi(v.w);
         }
-        p0 = p1;
-#pragma unroll
-        for (int j = 0; j < 4; j++) { const int p = p0 + j * 4 + pl; if (p < n) v[j] = __ldcg(reinterpret_cast<const uint4*>(vp + (size_t)p * a.D)); }
+        if (p0 + NS * step < n) request(st, p0 + NS * step, n);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        p0 += step;
+        if (++st == NS) st = 0;
     }
 #pragma unroll
     for (int e = 0; e < 8; e++) { o[e] += __shfl_xor_sync(0xffffffffu, o[e], 8); o[e] += __shfl_xor_sync(0xffffffffu, o[e], 16); }
@@ -636,6 +725,8 @@ struct AttManyArgs {
     int D, pow2;
     float scale;
     u16* out;
+    int clear, seqs, tmax;           // the first `clear` blocks of a row of blocks zero the cache rows after the prompts
+    const int* lens;
 };
 __device__ __forceinline__ int kv_off(int row, int piece) { return row * 128 + ((piece ^ (row & 7)) << 4); }
 __device__ __forceinline__ void cp16(u32 dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory"); }
@@ -656,7 +747,20 @@ __global__ void __launch_bounds__(128) pass_attend_many(const __grid_constant__ 
     __shared__ __align__(128) unsigned char kv[2][2][64 * 128];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     if (threadIdx.x == 0) dep_launch();
-    const int4 tl = __ldg(a.tiles + blockIdx.x);
+    if ((int)blockIdx.x < a.clear) {
+        // The rows of the caches after the prompts, in pieces of 64 rows: nothing waits for them and they wait for nothing, so
+        // their blocks come first and write under the QKV contraction before this kernel. (On a stream of its own the clearing
+        // delayed the chain: no kernel of it started early until the clearing was done.)
+        const int per_row = a.D / 8, parts = (a.tmax + 63) / 64;
+        for (int j = blockIdx.x * gridDim.y + blockIdx.y; j < 2 * a.seqs * parts; j += a.clear * gridDim.y) {
+            const int sq = j / (2 * parts), r = j - sq * 2 * parts, part = r >> 1;
+            const int lo = max(part * 64, __ldg(a.lens + sq)), hi = min(part * 64 + 64, a.tmax);
+            uint4* p = reinterpret_cast<uint4*>(const_cast<u16*>((r & 1) ? a.vc : a.kc) + sq * a.seq_stride);
+            for (int i = lo * per_row + threadIdx.x; i < hi * per_row; i += 128) p[i] = make_uint4(0, 0, 0, 0);
+        }
+        return;
+    }
+    const int4 tl = __ldg(a.tiles + blockIdx.x - a.clear);
     const int h = blockIdx.y, row0 = tl.x, nrows = tl.y, pos0 = tl.w;
     dep_wait();
     const u16* kp = a.kc + tl.z * a.seq_stride + h * 64;
@@ -781,7 +885,7 @@ struct FinishArgs {
     int t_stride, tstep, N;
     const int *prompt, *plen;
     int plen_cap;
-    const int *dst;                  // prompts: where in x the row's token goes
+    const int2* dst;                 // prompts: sequence of the row, length of its prompt
 };
 __global__ void __launch_bounds__(256) pass_finish(const __grid_constant__ FinishArgs a) {
     dep_wait();
@@ -792,7 +896,12 @@ __global__ void __launch_bounds__(256) pass_finish(const __grid_constant__ Finis
         if (skip) continue;
         const u32 n = 0xFFFFFFFFu - (u32)(k & 0xFFFFFFFFull);
         if (a.next) a.next[b] = (float)n;
-        if (a.dst) { a.x[__ldg(a.dst + b)] = (n >= (u32)a.N) ? 0 : (int)n; continue; }
+        if (a.dst) {
+            const int2 e = __ldg(a.dst + b);
+            a.x[e.x] = (n >= (u32)a.N) ? 0 : (int)n;
+            a.t[e.x * a.t_stride] = e.y;
+            continue;
+        }
         if (a.x) {
             int nx = (int)n;
             const int tn = a.pos[b] + a.tstep;

@@ -126,7 +126,7 @@ class VestaGPT2:
         B, P = tokens.shape
         if B != self.B:
             raise ValueError('prefill needs one prompt per sequence of the batch')
-        lens = np.full(B, P, np.int32) if lengths is None else np.asarray(lengths, np.int32)
+        lens = np.full(B, P, np.int32) if lengths is None else np.ascontiguousarray(lengths, np.int32)
         if lens.min() < 1 or lens.max() > P or lens.max() > self.tmax:
             raise ValueError('prompt lengths must lie in 1..P and fit the cache')
         if self.t.numel() == 1 and lens.min() != lens.max():
@@ -136,10 +136,8 @@ class VestaGPT2:
         eng = self._prefill_engines.get(rows)
         if eng is None:
             eng = self._prefill_engines[rows] = PromptPass(self, rows)
-        self.reset()
-        first = eng.run(tokens, lens)
-        self.x.copy_(first)
-        self.t.copy_(torch.from_numpy(lens[:self.t.numel()].copy()))
+        with torch.cuda.device(self.device):
+            eng.run(tokens, lens)
         if hasattr(self, 'prompt'):
             buf = np.zeros(tuple(self.prompt.shape), np.int32)
             w = min(P, buf.shape[1])

@@ -58,7 +58,7 @@ def lib():
         L.vesta_step_release.restype = None
         L.vesta_pass_workspace.argtypes = [vp, ctypes.POINTER(sz)]
         L.vesta_pass_create.argtypes = [vp, vp, ci, ctypes.POINTER(vp)]
-        L.vesta_pass_run.argtypes = [vp, vp, ci, ci, ci]
+        L.vesta_pass_prompts.argtypes = [vp, vp, vp, ci, vp, ctypes.POINTER(cu)]
         L.vesta_pass_bind.argtypes = [vp, ctypes.POINTER(vp)]
         L.vesta_pass_release.argtypes = [vp]
         L.vesta_pass_release.restype = None
