@@ -44,9 +44,13 @@ struct Pass {
     int fplanes;                               // the same for the rows that want logits
     Layout o;
     unsigned char* ws;
-    Tile tile[5];
-    CUtensorMap w[5], a[5];                    // weights and operand of every contraction
-    int max_parts;
+    struct Plan {                              // tiles for a number of rows
+        int rows, lrows;
+        Tile tile[5];
+        CUtensorMap w[5], a[5];                // weights and operand of every contraction
+    };
+    std::vector<Plan> plans;                   // the last few
+    size_t part_rows;                          // rows of the parts buffer
     std::vector<cudaGraphExec_t> graphs;       // decode: one step
     int sms;
     int* host;                                 // prompts: pinned metadata, one copy per pass of a call, then a status word
@@ -59,40 +63,53 @@ int plane_rows(int rows, bool exact) { return !exact ? 0 : rows <= 8 ? 8 : 16; }
 // Tile sizes of a contraction of `feat` features over `kb` blocks of 64 for `rows` rows (columns of the product), from a
 // model of the kernel's time in microseconds, fitted to measurements on B200 (rows 16 to 16,384, folds of 768 to 6,400,
 // tiles of 16 to 256 rows; within 15 % of each):
-//   BM = 64 (one tile per block, whole share of the weights in flight): 1.75 + 0.22 per stage + the operand's rows;
-//   BM = 128: 2.2 + 0.0065 bn for the first fill and the last epilogue, then per block of the fold the larger of the products
-//     (2 bn cycles) and the loads (340 + 0.45 bn cycles), times the tiles a block takes in turn.
+//   BM = 64 (one tile per block, whole share of the weights in flight): 1.75, 0.22 per stage, 0.5 for every stage that has to
+//     wait for a free one, the operand's rows;
+//   BM = 128: 2.2 for the first fill, a term for the last epilogue, then per block of the fold the larger of the products and the loads
+//     (L2 into the SMs, the slower the more SMs take part); with several tiles per block, each but the last costs the larger
+//     of that and its epilogue;
+//   BM = 256 (two blocks): 3.0, and a third less for the loads: better for folds of more than about 1,000.
 // A cut fold (projections) costs its parts once more in the norm that adds them.
-Tile choose(int kind, int rows, int rp, int feat, int kb, int sms) {
+Tile choose(int kind, int rows, int rp, int feat, int kb, int sms, int max_parts = PARTS_MAX) {
     Tile best = {};
     double best_t = 1e30;
     const int cols = rp ? 2 * rp : rows;
     const bool cut = kind == K_PROJ || kind == K_P2;
-    for (int bm = 64; bm <= 128; bm += 64)
+    const double last = kind == K_FC ? 0.012 : kind == K_QKV ? 0.009 : 0.0065;
+    for (int bm = 64; bm <= 256; bm *= 2)
         for (int bn = 16; bn <= (bm == 64 ? 64 : 256); bn += 16) {
             if (rp && (bm != 64 || bn != cols)) continue;
-            if (bn > 16 && bn - 16 >= cols) continue;
-            const int ks = bm == 64 ? GemmShape<64>::KS : GemmShape<128>::KS;
-            const int stage = bm == 64 ? GemmShape<64>::stage(bn) : GemmShape<128>::stage(bn);
+            if ((bn > 16 && bn - 16 >= cols) || (bm == 256 && (bn < 64 || kind == K_LOGITS))) continue;
+            const int ks = bm == 64 ? GemmShape<64>::KS : 1;
+            const int stage = bm == 64 ? GemmShape<64>::stage(bn) : bm == 128 ? GemmShape<128>::stage(bn) : GemmShape<256>::stage(bn);
             const int room = 227 * 1024 - 1024 - 1024 - bn * 32;
             const int tiles = ((feat + bm - 1) / bm) * (rp ? 1 : (rows + bn - 1) / bn);
-            for (int sp = 1; sp <= (cut ? PARTS_MAX : 1); sp++) {
+            const int units = bm == 256 ? sms / 2 : sms;
+            const double epi = kind == K_FC || kind == K_LOGITS ? 0.016 * bn + 1.2 : kind == K_QKV ? 0.010 * bn + 2.0 : 0.0145 * bn + 1.7;
+            for (int sp = 1; sp <= (cut ? max_parts : 1); sp++) {
                 Tile t;
                 t.bm = bm; t.bn = bn;
                 const int per = (kb + sp - 1) / sp, nst = (per + ks - 1) / ks;
                 t.splits = (kb + per - 1) / per;
                 if (t.splits != sp) continue;
-                const int waves = (tiles * sp + sms - 1) / sms;
+                const int waves = (tiles * sp + units - 1) / units;
                 t.stages = std::max(1, std::min(bm == 64 || waves == 1 ? nst : 16, room / (stage + 16)));
                 double us;
-                if (bm == 64) us = (1.75 + 0.22 * nst + 0.0023 * (bn - 16) * per) * waves + 0.002 * tiles * sp;
-                else us = 2.2 + 0.0065 * bn + waves * per * std::max(2.0 * bn + 30, 340 + 0.45 * bn) / 1900;
+                if (bm == 64) us = (1.75 + 0.22 * nst + 0.5 * std::max(0, nst - t.stages) + 0.0023 * (bn - 16) * per) * waves + 0.002 * tiles * sp;
+                else {
+                    const double busy = std::min(1.0, (double)tiles * sp / (0.88 * units));
+                    const double kb_us = bm == 128 ? std::max(std::max(0.0011 * bn + 0.03, 0.19), busy * (0.0016 * bn + 0.02)) : 0.0010 * bn + 0.04 + 0.033 * busy;
+                    const double main = per * kb_us;
+                    us = (bm == 128 ? 2.2 : 3.0) + last * bn + main + (waves - 1) * std::max(main, epi);
+                }
                 if (cut && sp > 1) us += 0.1 * sp + (sp - 1) * (double)rows * feat * 4 / 4e6;
                 if (us < best_t) { best_t = us; best = t; }
             }
         }
     return best;
 }
+int k_blocks(int bm) { return bm == 64 ? GemmShape<64>::KS : 1; }
+int box_rows(const Tile& t) { return t.bm == 256 ? t.bn / 2 : t.bn; }
 
 Layout layout(const Pass& p, int D, int F, int rows, int lrows) {
     Layout o{};
@@ -103,7 +120,7 @@ Layout layout(const Pass& p, int D, int F, int rows, int lrows) {
     o.act = take((size_t)p.planes * D * 2);
     o.att = take((size_t)p.planes * D * 2);
     o.gelu = take((size_t)p.planes * F * 2 + 128);       // (the last block of the fold may reach past the last row)
-    o.part = take((size_t)p.max_parts * rows * D * 4);
+    o.part = take(p.part_rows * D * 4);
     o.fin = take((size_t)p.fplanes * D * 2);
     o.best = take((size_t)lrows * 8);
     o.rowoff = take((size_t)rows * 8);
@@ -124,17 +141,13 @@ int plan(Pass& p, const vesta_pass_desc* d) {
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&p.sms, cudaDevAttrMultiProcessorCount, dev);
     cudaGetLastError();                          // (sizes can be asked for without a device)
     p.rp = plane_rows(d->rows, d->exact != 0);
-    const int frp = plane_rows(d->logit_rows, d->exact != 0);
     p.planes = p.rp ? 2 * p.rp : up(d->rows, 128);
     p.fplanes = p.rp ? 2 * p.rp : up(d->logit_rows, 128);
-    (void)frp;
-    const int kbd = d->D / 64, kbf = (d->F + 63) / 64;
-    p.tile[K_QKV] = choose(K_QKV, d->rows, p.rp, 3 * d->D, kbd, p.sms);
-    p.tile[K_PROJ] = choose(K_PROJ, d->rows, p.rp, d->D, kbd, p.sms);
-    p.tile[K_FC] = choose(K_FC, d->rows, p.rp, d->F, kbd, p.sms);
-    p.tile[K_P2] = choose(K_P2, d->rows, p.rp, d->D, kbf, p.sms);
-    p.tile[K_LOGITS] = choose(K_LOGITS, d->logit_rows, p.rp, d->N, kbd, p.sms);
-    p.max_parts = std::max(p.tile[K_PROJ].splits, p.tile[K_P2].splits);
+    // parts of a cut fold: as many rows of them as the choice for some number of rows asks for (prompts: passes of any size)
+    size_t most = 1;
+    for (int r = d->prompts ? 1 : d->rows; r <= d->rows; r = r < 64 ? r + 1 : std::min(r + r / 16, d->rows) + (r == d->rows))
+        for (int k : {K_PROJ, K_P2}) { const Tile t = choose(k, r, p.rp, d->D, k == K_P2 ? (d->F + 63) / 64 : d->D / 64, p.sms); if (t.splits > 1) most = std::max(most, (size_t)t.splits * r); }
+    p.part_rows = most + most / 8;
     p.o = layout(p, d->D, d->F, d->rows, d->logit_rows);
     return 0;
 }
@@ -142,15 +155,6 @@ int plan(Pass& p, const vesta_pass_desc* d) {
 // The kernels of a pass ask for the same split of an SM between shared memory and cache: an SM changes it only when it is idle,
 // and a block that waits for that cannot start under its predecessor (23 sequences: projection 3.0 -> 2.4 us, norm 4.5 -> 3.5).
 template <class F> cudaError_t all_shared(F* f) { return cudaFuncSetAttribute((const void*)f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared); }
-cudaError_t prepare_all() {
-    cudaError_t e = cudaSuccess;
-    auto one = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
-    one(all_shared(pass_norm<NORM_EMBED>)); one(all_shared(pass_norm<NORM_MID>)); one(all_shared(pass_norm<NORM_FINAL>));
-    one(all_shared(pass_norm_rows<6>)); one(all_shared(pass_norm_rows<13>)); one(all_shared(pass_norm_rows<16>));
-    one(all_shared(pass_attend<2>)); one(all_shared(pass_attend<4>)); one(all_shared(pass_attend_many));
-    one(cudaFuncSetAttribute((const void*)pass_attend<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * ATT_WARPS * 4096)); one(all_shared(pass_finish));
-    return e;
-}
 template <int BM, int EPI>
 cudaError_t launch_gemm(cudaLaunchConfig_t& c, const Tile& t, const CUtensorMap& w, const CUtensorMap& a, const GemmArgs& g) {
     c.dynamicSmemBytes = GemmShape<BM>::bytes(t.stages, t.bn);
@@ -158,23 +162,34 @@ cudaError_t launch_gemm(cudaLaunchConfig_t& c, const Tile& t, const CUtensorMap&
     return cudaLaunchKernelEx(&c, pass_gemm<BM, EPI>, w, a, g);
 }
 template <int BM, int EPI>
-cudaError_t prepare_gemm(const Tile& t) {
+cudaError_t prepare_gemm() {
     const cudaError_t e = all_shared(pass_gemm<BM, EPI>);
     return e != cudaSuccess ? e : cudaFuncSetAttribute(pass_gemm<BM, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
 }
 // one case per tile shape and epilogue
-#define EACH(X) X(64, EPI_ADD) X(128, EPI_ADD) X(64, EPI_QKV) X(64, EPI_PART) X(64, EPI_GELU) X(64, EPI_LOGITS) X(128, EPI_QKV) X(128, EPI_PART) X(128, EPI_GELU) X(128, EPI_LOGITS)
+#define EACH(X) X(256, EPI_ADD) X(256, EPI_QKV) X(256, EPI_PART) X(256, EPI_GELU) X(64, EPI_ADD) X(128, EPI_ADD) X(64, EPI_QKV) X(64, EPI_PART) X(64, EPI_GELU) X(64, EPI_LOGITS) X(128, EPI_QKV) X(128, EPI_PART) X(128, EPI_GELU) X(128, EPI_LOGITS)
 cudaError_t gemm(int epi, const Tile& t, cudaLaunchConfig_t c, const CUtensorMap& w, const CUtensorMap& a, const GemmArgs& g) {
 #define ONE(M, E) if (epi == E && t.bm == M) return launch_gemm<M, E>(c, t, w, a, g);
     EACH(ONE)
 #undef ONE
     return cudaErrorInvalidValue;
 }
-cudaError_t gemm_prepare(int epi, const Tile& t) {
-#define ONE(M, E) if (epi == E && t.bm == M) return prepare_gemm<M, E>(t);
+cudaError_t gemm_prepare() {
+    cudaError_t e = cudaSuccess;
+#define ONE(M, E) if (e == cudaSuccess) e = prepare_gemm<M, E>();
     EACH(ONE)
 #undef ONE
-    return cudaErrorInvalidValue;
+    return e;
+}
+cudaError_t prepare_all() {
+    cudaError_t e = cudaSuccess;
+    auto one = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
+    one(all_shared(pass_norm<NORM_EMBED>)); one(all_shared(pass_norm<NORM_MID>)); one(all_shared(pass_norm<NORM_FINAL>));
+    one(all_shared(pass_norm_rows<6>)); one(all_shared(pass_norm_rows<13>)); one(all_shared(pass_norm_rows<16>));
+    one(all_shared(pass_attend<2>)); one(all_shared(pass_attend<4>)); one(all_shared(pass_attend_many));
+    one(gemm_prepare());
+    one(cudaFuncSetAttribute((const void*)pass_attend<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * ATT_WARPS * 4096)); one(all_shared(pass_finish));
+    return e;
 }
 int epi_of(int kind, const Tile& t) { return kind == K_QKV ? EPI_QKV : kind == K_FC ? EPI_GELU : kind == K_LOGITS ? EPI_LOGITS : t.splits > 1 ? EPI_PART : EPI_ADD; }
 
@@ -182,12 +197,36 @@ int epi_of(int kind, const Tile& t) { return kind == K_QKV ? EPI_QKV : kind == K
 struct Config {
     cudaLaunchConfig_t c = {};
     cudaLaunchAttribute at[2];
-    Config(dim3 grid, int block, cudaStream_t st, bool dependent, int cluster = 1) {
+    Config(dim3 grid, int block, cudaStream_t st, bool dependent, int cluster = 1, bool along_x = false) {
         c.gridDim = grid; c.blockDim = dim3(block); c.stream = st; c.attrs = at; c.numAttrs = 0;
         if (dependent) { at[c.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[c.numAttrs].val.programmaticStreamSerializationAllowed = 1; c.numAttrs++; }
-        if (cluster > 1) { at[c.numAttrs].id = cudaLaunchAttributeClusterDimension; at[c.numAttrs].val.clusterDim.x = 1; at[c.numAttrs].val.clusterDim.y = 1; at[c.numAttrs].val.clusterDim.z = cluster; c.numAttrs++; }
+        if (cluster > 1) { at[c.numAttrs].id = cudaLaunchAttributeClusterDimension; at[c.numAttrs].val.clusterDim.x = along_x ? cluster : 1; at[c.numAttrs].val.clusterDim.y = 1; at[c.numAttrs].val.clusterDim.z = along_x ? 1 : cluster; c.numAttrs++; }
     }
 };
+
+// The tiles and tensor maps for `rows` rows of which `lrows` want logits.
+int plan_for(Pass& p, int rows, int lrows, const Pass::Plan** out) {
+    for (auto& q : p.plans) if (q.rows == rows && q.lrows == lrows) { *out = &q; return 0; }
+    if (p.plans.size() >= 8) p.plans.erase(p.plans.begin());
+    const vesta_pass_desc& d = p.d;
+    const int D = d.D, F = d.F, kbd = D / 64, kbf = (F + 63) / 64;
+    Pass::Plan q;
+    q.rows = rows; q.lrows = lrows;
+    const void* w[5] = {d.qkvw, d.ow, d.fcw, d.pw, d.wte};
+    const int fold[5] = {D, D, D, F, D}, feat[5] = {3 * D, D, F, D, d.N}, kb[5] = {kbd, kbd, kbd, kbf, kbd};
+    const size_t op[5] = {p.o.act, p.o.att, p.o.act, p.o.gelu, p.o.fin};
+    for (int k = 0; k < 5; k++) {
+        const Tile t = q.tile[k] = choose(k, k == K_LOGITS ? std::max(lrows, 1) : rows, p.rp, feat[k], kb[k], p.sms, std::max<int>(1, std::min<size_t>(PARTS_MAX, p.part_rows / rows)));
+        int e;
+        if (k == K_LOGITS) e = vesta_rt::fold_map(&q.w[k], w[k], D, feat[k], t.bm, k_blocks(t.bm));
+        else e = vesta_rt::tensor_map(&q.w[k], w[k], feat[k], fold[k], d.L, (size_t)feat[k] * 2, (size_t)feat[k] * fold[k] * 2, 64 * k_blocks(t.bm), 1);
+        if (!e) e = vesta_rt::fold_map(&q.a[k], p.ws + op[k], fold[k], k == K_LOGITS ? p.fplanes : p.planes, box_rows(t), k_blocks(t.bm));
+        if (e) return e;
+    }
+    p.plans.push_back(q);
+    *out = &p.plans.back();
+    return 0;
+}
 
 // The launches of one pass over `rows` rows. Prompts: `tiles` runs of rows for the attention, `lrows` rows that want logits
 // (none: the pass ends with the last layer's cache rows); `clear`: zero the cache rows after the prompts.
@@ -201,11 +240,17 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
     float* z = (float*)u(p.o.z);
     u16 *act = (u16*)u(p.o.act), *att = (u16*)u(p.o.att), *fin = (u16*)u(p.o.fin);
     const int nthr = up(D / 4, 32);
+    // attention of a step: C blocks per (row, head) while the blocks of all stay resident; deep rings where few share an SM
+    int C = 1;
+    while (C < 8 && rows * d.H * C * 2 <= 6 * p.sms && d.tmax > C * ATT_WARPS * ATT_RUN) C *= 2;
+    const bool deep = rows * d.H * C <= 3 * p.sms;
+    const Pass::Plan* pl = nullptr;
+    if (int e = plan_for(p, rows, lrows, &pl)) return e;
     auto f16 = [](const void* q, size_t off) { return (const u16*)q + off; };
     auto norm = [&](int mode, int l, int nparts) {
         NormArgs n = {};
         n.D = D; n.nparts = nparts; n.rp = p.rp; n.eps = d.eps; n.z = z;
-        n.part = (const float*)u(p.o.part); n.part_stride = (size_t)d.rows * D;
+        n.part = (const float*)u(p.o.part); n.part_stride = (size_t)rows * D;
         n.x = many ? meta + mt.x : (const int*)d.x; n.t = many ? meta + mt.t : (const int*)d.t; n.seq = many ? meta + mt.seq : 0; n.t_stride = many ? 1 : d.t_stride; n.N = d.N; n.cpos = d.cpos; n.tmax = d.tmax; n.L = L;
         n.wte = (const u16*)d.wte; n.wpe = (const u16*)d.wpe;
         n.rowoff = (long long*)u(p.o.rowoff); n.pos = (int*)u(p.o.pos); n.skip = (int*)u(p.o.skip); n.bar = (u32*)d.bar;
@@ -223,7 +268,7 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
         return mode == 0 ? cudaLaunchKernelEx(&c.c, pass_norm<NORM_EMBED>, n) : mode == 3 ? cudaLaunchKernelEx(&c.c, pass_norm<NORM_FINAL>, n) : cudaLaunchKernelEx(&c.c, pass_norm<NORM_MID>, n);
     };
     auto mul = [&](int kind, int l) {
-        const Tile& t = p.tile[kind];
+        const Tile& t = pl->tile[kind];
         GemmArgs g = {};
         g.layer = l; g.D = D; g.rp = p.rp; g.stages = t.stages; g.status = (u32*)d.bar; g.skip = (const int*)u(p.o.skip);
         g.rows = kind == K_LOGITS ? lrows : rows;
@@ -235,11 +280,11 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
         } else if (kind == K_FC) {
             g.bias = f16(d.fcb, (size_t)l * F); g.oh = (u16*)u(p.o.gelu); g.a2 = 2 * d.gelu_a; g.k1 = d.gelu_b * 2.8853900817779268f; g.k2 = d.gelu_c * g.k1;
         } else if (kind == K_LOGITS) { g.of = (float*)d.logits; g.best = (u64*)u(p.o.best); }
-        else if (t.splits > 1) { g.of = (float*)u(p.o.part); g.part_stride = (size_t)d.rows * D; }
+        else if (t.splits > 1) { g.of = (float*)u(p.o.part); g.part_stride = (size_t)rows * D; }
         else { g.of = z; g.bias = kind == K_PROJ ? f16(d.ob, (size_t)l * D) : f16(d.pb, (size_t)l * D); }
         g.bn = t.bn; g.ftiles = (g.nfeat + t.bm - 1) / t.bm; g.rtiles = p.rp ? 1 : (g.rows + t.bn - 1) / t.bn; g.ntiles = g.ftiles * g.rtiles * t.splits;
-        Config c(dim3(t.bm == 64 && kind != K_LOGITS ? g.ntiles : std::min(g.ntiles, p.sms)), 192, st, true);
-        return gemm(epi_of(kind, t), t, c.c, p.w[kind], p.a[kind], g);
+        Config c(dim3(t.bm == 64 && kind != K_LOGITS ? g.ntiles : t.bm == 256 ? 2 * std::min(g.ntiles, p.sms / 2) : std::min(g.ntiles, p.sms)), 192, st, true, t.bm == 256 ? 2 : 1, true);
+        return gemm(epi_of(kind, t), t, c.c, pl->w[kind], pl->a[kind], g);
     };
     auto attend = [&](int l, int tiles) {
         const float* q = (const float*)u(p.o.q);
@@ -254,11 +299,7 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
             return cudaLaunchKernelEx(&c.c, pass_attend_many, a);
         }
         AttArgs a = {q, kc, vc, ss, (const int*)d.t, (const int*)0, d.t_stride, d.tmax, D, pow2, p.rp, d.scale, att};
-        int C = 1;
-        while (C < 8 && rows * d.H * C * 2 <= 6 * p.sms && d.tmax > C * ATT_WARPS * ATT_RUN) C *= 2;
         Config c(dim3(d.H, rows, C), ATT_WARPS * 32, st, true, C);
-        // deep rings where few blocks share an SM, all blocks resident where they are many
-        const bool deep = rows * d.H * C <= 3 * p.sms;
         c.c.dynamicSmemBytes = (deep ? 4 : 2) * ATT_WARPS * 4096;
         return deep ? cudaLaunchKernelEx(&c.c, pass_attend<4>, a) : cudaLaunchKernelEx(&c.c, pass_attend<2>, a);
     };
@@ -269,10 +310,10 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
         if (!end || clear) TRY(attend(l, end ? 0 : tiles));
         if (end) break;
         TRY(mul(K_PROJ, l));
-        TRY(norm(1, l, p.tile[K_PROJ].splits > 1 ? p.tile[K_PROJ].splits : 0));
+        TRY(norm(1, l, pl->tile[K_PROJ].splits > 1 ? pl->tile[K_PROJ].splits : 0));
         TRY(mul(K_FC, l));
         TRY(mul(K_P2, l));
-        TRY(norm(l + 1 < L ? 2 : 3, l, p.tile[K_P2].splits > 1 ? p.tile[K_P2].splits : 0));
+        TRY(norm(l + 1 < L ? 2 : 3, l, pl->tile[K_P2].splits > 1 ? pl->tile[K_P2].splits : 0));
     }
     if (lrows) TRY(mul(K_LOGITS, 0));
     FinishArgs f = {};
@@ -316,19 +357,7 @@ int vesta_pass_create(const vesta_pass_desc* d, void* workspace, int graph, void
     Pass* p = new Pass{};
     int e = plan(*p, d);
     p->ws = (unsigned char*)workspace;
-    const int D = d->D, F = d->F;
-    const void* w[5] = {d->qkvw, d->ow, d->fcw, d->pw, d->wte};
-    const int fold[5] = {D, D, D, F, D}, feat[5] = {3 * D, D, F, D, d->N};
     if (!e) { const cudaError_t ce = prepare_all(); if (ce != cudaSuccess) e = cuda_fail(ce, "cudaFuncSetAttribute"); }
-    unsigned char* op[5] = {p->ws + p->o.act, p->ws + p->o.att, p->ws + p->o.act, p->ws + p->o.gelu, p->ws + p->o.fin};
-    for (int k = 0; k < 5 && !e; k++) {
-        const Tile& t = p->tile[k];
-        const int ks = t.bm == 64 ? GemmShape<64>::KS : GemmShape<128>::KS;
-        if (k == K_LOGITS) e = vesta_rt::fold_map(&p->w[k], w[k], D, feat[k], t.bm, ks);
-        else e = vesta_rt::tensor_map(&p->w[k], w[k], feat[k], fold[k], d->L, (size_t)feat[k] * 2, (size_t)feat[k] * fold[k] * 2, 64 * ks, 1);
-        if (!e) e = vesta_rt::fold_map(&p->a[k], op[k], fold[k], k == K_LOGITS ? p->fplanes : p->planes, t.bn, ks);
-        if (!e) { const cudaError_t ce = gemm_prepare(epi_of(k, p->tile[k]), p->tile[k]); if (ce != cudaSuccess) e = cuda_fail(ce, "cudaFuncSetAttribute"); }
-    }
     if (!e && graph) {
         // a decode step as a graph, captured on a stream of its own
         cudaStream_t st = nullptr;

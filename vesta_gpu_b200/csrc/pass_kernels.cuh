@@ -48,6 +48,23 @@ __device__ __forceinline__ void tma3(u32 dst, const CUtensorMap* m, int x, int y
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                  :: "r"(dst), "l"(m), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
 }
+// the same into this block of a pair, counted on a barrier of the pair's first block (no multicast)
+__device__ __forceinline__ void tma3_pair(u32 dst, const CUtensorMap* m, int x, int y, int z, u32 bar) {
+    asm volatile("cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 :: "r"(dst), "l"(m), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
+}
+// a shared-memory address of this block as the same address of the first block of its cluster
+__device__ __forceinline__ u32 of_first(u32 a) {
+    u32 r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(a));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() { asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// arrives on `bar` (of a pair: at that address in both blocks) when the products issued so far are done
+template <bool PAIR> __device__ __forceinline__ void tc_commit(u32 bar) {
+    if (PAIR) asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" :: "r"(bar), "h"((u16)3) : "memory");
+    else asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar) : "memory");
+}
 __device__ __forceinline__ u32 elect_one() {
     u32 leader;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(leader));
@@ -138,10 +155,13 @@ __device__ __forceinline__ u64 best_key(int ordered, u32 n) { return ((u64)((u32
 // Shared memory of a block: the stages, then full and empty barriers, the accumulators' full and empty barriers, the
 // tensor-memory address and the dead flag; per accumulator the row offsets (QKV) or the warps' best keys (LOGITS).
 template <int BM> struct GemmShape {
+    static constexpr bool PAIR = BM == 256;              // two blocks of a cluster share the tile
+    static constexpr int AM = PAIR ? 128 : BM;           // features per block
     static constexpr int KS = BM == 64 ? 4 : 1;          // blocks of 64 fold indices per stage
     static constexpr int EW = 8;                         // warps that read the accumulators: two per quarter of the lanes
     static constexpr int THREADS = 64 + 32 * EW;
-    static __host__ __device__ constexpr int stage(int bn) { return KS * (BM + bn) * 128; }
+    static __host__ __device__ constexpr int box(int bn) { return PAIR ? bn / 2 : bn; }       // rows per block
+    static __host__ __device__ constexpr int stage(int bn) { return KS * (AM + box(bn)) * 128; }
     static __host__ __device__ constexpr int tail(int stages, int bn) { return 2 * stages * 8 + 48 + bn * 8 * 4; }
     static __host__ __device__ constexpr int bytes(int stages, int bn) { return stages * stage(bn) + tail(stages, bn) + 1024; }
     static __host__ __device__ constexpr int columns(int bn, bool two) { int c = 32; while (c < (two ? 2 * bn : bn)) c *= 2; return c; }
@@ -153,17 +173,25 @@ __device__ __forceinline__ void st_f32(float* p, float v, bool yes) {
     asm volatile("{.reg .pred p; setp.ne.s32 p, %2, 0; @p st.global.f32 [%0], %1;}" :: "l"(p), "f"(v), "r"((int)yes) : "memory");
 }
 
+__device__ __forceinline__ void add_f32(float* p, float v, bool yes) {
+    asm volatile("{.reg .pred p; setp.ne.s32 p, %2, 0; @p red.relaxed.gpu.global.add.f32 [%0], %1;}" :: "l"(p), "f"(v), "r"((int)yes) : "memory");
+}
+
 // Tiles of BM features x bn rows over kb_per blocks of 64 fold indices; a block takes the tiles blockIdx.x,
 // blockIdx.x + gridDim.x, ... Warp 0 loads (one lane), warp 1 issues the products, the others read the accumulators; with
 // more tiles than blocks two accumulators alternate, so that a tile's epilogue runs under the next one's products.
 //   BM = 64: few rows, one tile per block. What counts is the chain wait - operand - products - epilogue: the block's
 //     whole share of the weights is in flight before it waits for its predecessor, four blocks of the fold per stage (a
 //     stage costs the issuing warps 0.1 us whatever its size: 12 blocks of 64 x 16 took 2.0 us one by one, 1.0 in fours).
-//   BM = 128: many rows. 128 x 128 tiles run at 1,215 TFLOP/s without an epilogue, 1,119 with fp32 stores.
+//   BM = 128: many rows. What bounds it is the path from L2 into the SMs, 120 GB/s each whatever the tile: 128 x 192 tiles
+//     1,160 to 1,200 TFLOP/s.
+//   BM = 256: many rows, two blocks of a cluster with one product of 256 rows (cta_group::2): each loads its own 128 features and
+//     half the rows of the tile, so that a 256 x 256 tile costs an SM 32 KB per block of the fold instead of 48.
 template <int BM, int EPI>
 __global__ void __launch_bounds__(GemmShape<BM>::THREADS) pass_gemm(const __grid_constant__ CUtensorMap wm, const __grid_constant__ CUtensorMap am, const __grid_constant__ GemmArgs g) {
     using S = GemmShape<BM>;
-    constexpr int KS = S::KS, EW = S::EW;
+    constexpr int KS = S::KS, EW = S::EW, AM = S::AM;
+    constexpr bool PAIR = S::PAIR;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const int st = g.stages, bn = g.bn, stage = S::stage(bn);
@@ -173,22 +201,30 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS) pass_gemm(const __grid
     volatile u32* tmem_p = reinterpret_cast<volatile u32*>(tail);
     u64* side = reinterpret_cast<u64*>(tail + 16);
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-    const bool two = g.ntiles > (int)gridDim.x;
+    const int rank = PAIR ? (int)(blockIdx.x & 1) : 0;                             // block of the pair; the first one issues the products
+    const int t_first = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, t_step = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
+    const bool two = g.ntiles > t_step;
     const int cols = S::columns(bn, two);
     const Wait w{dead, g.status};
     if (threadIdx.x == 0) {
         *dead = 0;
         for (int i = 0; i < st; i++) { mbar_init(bars + i * 8, 1); mbar_init(bars + (st + i) * 8, 1); }
-        for (int i = 0; i < 2; i++) { mbar_init(tmf + i * 8, 1); mbar_init(tme + i * 8, EW); }
+        for (int i = 0; i < 2; i++) { mbar_init(tmf + i * 8, 1); mbar_init(tme + i * 8, PAIR ? 2 * EW : EW); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("prefetch.tensormap [%0];" :: "l"(&am) : "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(tail)), "r"(cols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(tail)), "r"(cols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(tail)), "r"(cols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     }
     __syncthreads();
+    if (PAIR) cluster_sync();                                                      // the other block's barriers are ready
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (threadIdx.x == 0) dep_launch();              // (after the allocation: the blocks of the next kernel queue behind it)
     const u32 tmem = *tmem_p;
@@ -198,19 +234,24 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS) pass_gemm(const __grid
         if (elect_one()) {
             int s = 0, ph = 1;
             bool first = true;
-            for (int t = blockIdx.x; t < g.ntiles; t += gridDim.x) {
-                const int z = t / per, r = t - z * per, rt = r / g.ftiles, f0 = (r - rt * g.ftiles) * BM, row0 = rt * bn;
+            for (int t = t_first; t < g.ntiles; t += t_step) {
+                const int z = t / per, r = t - z * per, rt = r / g.ftiles, f0 = (r - rt * g.ftiles) * BM + rank * AM, row0 = rt * bn + rank * S::box(bn);
                 const int kb0 = z * g.kb_per, nst = (min(g.kb_per, g.kblocks - kb0) + KS - 1) / KS;
+                auto load = [&](u32 dst, const CUtensorMap* m, int x, int y, int zz, u32 bar) {
+                    if (PAIR) tma3_pair(dst, m, x, y, zz, bar); else tma3(dst, m, x, y, zz, bar);
+                };
                 auto load_w = [&](int slot, int i) {
-                    const u32 dst = sbase + slot * stage, bar = bars + slot * 8;
-                    mbar_expect(bar, stage);
-                    if (EPI == EPI_LOGITS) tma3(dst, &wm, 0, f0, kb0 + i * KS, bar);
+                    const u32 dst = sbase + slot * stage, bar = PAIR ? of_first(bars + slot * 8) : bars + slot * 8;
+                    if (!PAIR || rank == 0) mbar_expect(bars + slot * 8, PAIR ? 2 * stage : stage);
+                    if (EPI == EPI_LOGITS) load(dst, &wm, 0, f0, kb0 + i * KS, bar);
                     else {
-                        tma3(dst, &wm, f0, (kb0 + i * KS) * 64, g.layer, bar);
-                        if (BM == 128) tma3(dst + KS * 8192, &wm, f0 + 64, (kb0 + i * KS) * 64, g.layer, bar);
+                        load(dst, &wm, f0, (kb0 + i * KS) * 64, g.layer, bar);
+                        if (AM == 128) load(dst + KS * 8192, &wm, f0 + 64, (kb0 + i * KS) * 64, g.layer, bar);
                     }
                 };
-                auto load_a = [&](int slot, int i) { tma3(sbase + slot * stage + KS * BM * 128, &am, 0, row0, kb0 + i * KS, bars + slot * 8); };
+                auto load_a = [&](int slot, int i) {
+                    load(sbase + slot * stage + KS * AM * 128, &am, 0, row0, kb0 + i * KS, PAIR ? of_first(bars + slot * 8) : bars + slot * 8);
+                };
                 int i = 0;
                 if (first) {
                     // the weights do not depend on the predecessor
@@ -233,10 +274,10 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS) pass_gemm(const __grid
     } else if (warp == 1) {
         // fp32 accumulators, fp16 operands; A M-major (bit 15) except for the table of the logits
         const u32 idesc = (1u << 4) | (EPI == EPI_LOGITS ? 0u : (1u << 15)) | ((u32)(bn >> 3) << 17) | ((u32)(BM >> 4) << 24);
-        constexpr int AKB = EPI == EPI_LOGITS ? BM * 128 : 8192, AK = EPI == EPI_LOGITS ? 32 : 2048;   // bytes to the next block, to the next 16 fold indices
+        constexpr int AKB = EPI == EPI_LOGITS ? AM * 128 : 8192, AK = EPI == EPI_LOGITS ? 32 : 2048;   // bytes to the next block, to the next 16 fold indices
         int s = 0, ph = 0, n = 0;
-        bool ok = true;
-        for (int t = blockIdx.x; t < g.ntiles && ok; t += gridDim.x, n++) {
+        bool ok = !PAIR || rank == 0;
+        for (int t = t_first; t < g.ntiles && ok; t += t_step, n++) {
             const int kb0 = (t / per) * g.kb_per, nkb = min(g.kb_per, g.kblocks - kb0), nst = (nkb + KS - 1) / KS, b = n & 1;
             if (n >= 2) ok = !__any_sync(0xffffffffu, !mbar_wait(tme + b * 8, ((n >> 1) & 1) ^ 1, w, 0xB30u));
             const u32 acc = tmem + (b ? bn : 0);
@@ -249,18 +290,23 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS) pass_gemm(const __grid
                 // registers one by one)
                 if (elect_one()) {
                     const u32 a = sbase + s * stage;
-                    const u64 ad = EPI == EPI_LOGITS ? desc_k(a) : desc_m(a, KS * 8192), bd = desc_k(a + KS * BM * 128);
+                    const u64 ad = EPI == EPI_LOGITS ? desc_k(a) : desc_m(a, KS * 8192), bd = desc_k(a + KS * AM * 128);
 #pragma unroll
                     for (int kb = 0; kb < KS; kb++)
                         if (KS == 1 || i * KS + kb < nkb) {
                             const u64 bk = bd + (u64)((kb * bn * 128) >> 4);
 #pragma unroll
-                            for (int k = 0; k < 4; k++)
-                                asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                                             :: "r"(acc), "l"(ad + (kb * AKB + k * AK) / 16), "l"(bk + 2 * k), "r"(idesc), "r"((i | kb | k) ? 1u : 0u) : "memory");
+                            for (int k = 0; k < 4; k++) {
+                                if (PAIR)
+                                    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                                                 :: "r"(acc), "l"(ad + (kb * AKB + k * AK) / 16), "l"(bk + 2 * k), "r"(idesc), "r"((i | kb | k) ? 1u : 0u) : "memory");
+                                else
+                                    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                                                 :: "r"(acc), "l"(ad + (kb * AKB + k * AK) / 16), "l"(bk + 2 * k), "r"(idesc), "r"((i | kb | k) ? 1u : 0u) : "memory");
+                            }
                         }
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bars + (st + s) * 8) : "memory");
-                    if (i == nst - 1) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(tmf + b * 8) : "memory");
+                    tc_commit<PAIR>(bars + (st + s) * 8);
+                    if (i == nst - 1) tc_commit<PAIR>(tmf + b * 8);
                 }
                 __syncwarp();
                 if (++s == st) { s = 0; ph ^= 1; }
@@ -268,37 +314,36 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS) pass_gemm(const __grid
         }
     } else {
         const int quarter = warp & 3, ew = warp - 2, et = threadIdx.x - 64;
-        const int fl = BM == 128 ? quarter * 32 + lane : quarter * 16 + lane;      // (a product of 64 rows leaves row m in lane 32 (m / 16) + m % 16)
+        const int fl = AM == 128 ? quarter * 32 + lane : quarter * 16 + lane;      // (a product of 64 rows leaves row m in lane 32 (m / 16) + m % 16)
         bool waited = false, skip = false;
         int n = 0;
-        for (int t = blockIdx.x; t < g.ntiles; t += gridDim.x, n++) {
-            const int z = t / per, r0 = t - z * per, rt = r0 / g.ftiles, f0 = (r0 - rt * g.ftiles) * BM, row0 = rt * bn, b = n & 1;
+        u64 off = ~0ull;                                                           // QKV: a row's offset in the caches, one tile ahead
+        auto row_offset = [&](int t) {
+            const int i = (t - t / per * per) / g.ftiles * bn + et;
+            return t < g.ntiles && et < bn && i < g.rows && !skip ? (u64)__ldcg(g.rowoff + i) : ~0ull;
+        };
+        for (int t = t_first; t < g.ntiles; t += t_step, n++) {
+            const int z = t / per, r0 = t - z * per, rt = r0 / g.ftiles, f0 = (r0 - rt * g.ftiles) * BM + rank * AM, row0 = rt * bn, b = n & 1;
             const int f = f0 + fl;
-            const bool own = (BM == 128 || lane < 16) && f < g.nfeat;
+            const bool own = (AM == 128 || lane < 16) && f < g.nfeat;
             float bias = 0.f;
             if ((EPI == EPI_QKV || EPI == EPI_GELU || EPI == EPI_ADD) && own) bias = h2f(__ldg(g.bias + f));
             if (!waited) {
                 dep_wait();
                 waited = true;
                 skip = (EPI == EPI_QKV || EPI == EPI_LOGITS) ? __ldcg(g.skip) != 0 : false;
+                if (EPI == EPI_QKV) off = row_offset(t);
             }
             const int live = min(g.rp ? g.rp : bn, g.rows - row0);                 // rows of this tile
             if (EPI == EPI_QKV) {
                 // (everyone is past the previous tile's offsets but one: two buffers)
-                for (int i = et; i < bn; i += EW * 32) side[b * bn + i] = (i < live && !skip) ? (u64)__ldcg(g.rowoff + row0 + i) : ~0ull;
+                if (et < bn) side[b * bn + et] = off;
+                off = row_offset(t + t_step);
                 asm volatile("bar.sync 1, %0;" :: "n"(EW * 32) : "memory");
             }
-            // the second warp of a quarter takes the upper half of the rows
-            const int half = live > 4 ? ((live + 15) / 16) * 8 : 4;
-            const int c_lo = ew >= 4 ? half : 0, c_hi = min(live, ew < 4 ? half : bn);
-            // ADD: what a chunk of rows is added to is requested one chunk ahead, the first before the products are done
-            float add[16];
-            auto fetch = [&](int c) {
-                const float* src = g.of + (size_t)(row0 + c) * g.nfeat + f;
-#pragma unroll
-                for (int i = 0; i < 16; i++) add[i] = own && c + i < c_hi ? __ldcg(src + (size_t)i * g.nfeat) : 0.f;
-            };
-            if (EPI == EPI_ADD) fetch(c_lo);
+            // the warps of a quarter share the rows
+            const int share = live > EW ? (live + 2 * EW - 1) / (2 * EW) * 8 : 4;
+            const int c_lo = (ew >> 2) * share, c_hi = min(live, c_lo + share);
             const bool ok = mbar_wait(tmf + b * 8, (n >> 1) & 1, w, 0xB20u);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (__any_sync(0xffffffffu, !ok)) break;
@@ -324,35 +369,49 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS) pass_gemm(const __grid
 #pragma unroll
                 for (int i = 0; i < CH; i++) {
                     v[i] += bias;
-                    if (EPI == EPI_ADD) v[i] += add[i];
                     if (EPI == EPI_GELU) v[i] = gelu_tanh(v[i], g.a2, g.k1, g.k2);
                 }
-                if (EPI == EPI_ADD && CH == 16) fetch(c0 + 16);
                 if (!own) m = 0;
                 if (EPI == EPI_QKV) {
                     if (part == 0) {
                         float* dst = g.of + (size_t)row * g.D + f;
 #pragma unroll
-                        for (int i = 0; i < CH; i++) st_f32(dst + (size_t)i * g.D, v[i], i < m);
+                        for (int i = 0; i < CH; i++, dst += g.D) st_f32(dst, v[i], i < m);
                     } else {
-                        long long o[CH];
 #pragma unroll
-                        for (int i = 0; i < CH; i++) o[i] = (long long)side[b * bn + c0 + i];
-#pragma unroll
-                        for (int i = 0; i < CH; i++) st_u16(cache + o[i], f2h(v[i]), i < m && o[i] >= 0);
+                        for (int i = 0; i < CH; i += 2) {
+                            const longlong2 o = *reinterpret_cast<const longlong2*>(side + b * bn + c0 + i);
+                            const u32 h = pack_h2(v[i], v[i + 1]);                 // (one conversion for two: alone each runs at a quarter of the rate)
+                            st_u16(cache + o.x, (u16)h, i < m && o.x >= 0);
+                            st_u16(cache + o.y, (u16)(h >> 16), i + 1 < m && o.y >= 0);
+                        }
                     }
-                } else if (EPI == EPI_PART || EPI == EPI_ADD) {
-                    float* dst = g.of + (EPI == EPI_PART ? z * g.part_stride : 0) + (size_t)row * g.nfeat + f;
+                } else if (EPI == EPI_PART) {
+                    float* dst = g.of + z * g.part_stride + (size_t)row * g.nfeat + f;
 #pragma unroll
-                    for (int i = 0; i < CH; i++) st_f32(dst + (size_t)i * g.nfeat, v[i], i < m);
+                    for (int i = 0; i < CH; i++, dst += g.nfeat) st_f32(dst, v[i], i < m);
+                } else if (EPI == EPI_ADD) {
+                    // (one addition per element: the order of blocks does not matter. Reading, adding and storing waited for L2
+                    // chunk by chunk: 15 us at 9,216 rows x 768 x 768)
+                    float* dst = g.of + (size_t)row * g.nfeat + f;
+#pragma unroll
+                    for (int i = 0; i < CH; i++, dst += g.nfeat) add_f32(dst, v[i], i < m);
                 } else if (EPI == EPI_GELU) {
                     u16* dst = g.oh + (size_t)row * g.nfeat + f;
-#pragma unroll
-                    for (int i = 0; i < CH; i++) st_u16(dst + (size_t)i * g.nfeat, f2h(v[i]), i < m);
                     if (BM == 64 && g.rp) {
-                        dst += (size_t)g.rp * g.nfeat;
+                        const size_t lo = (size_t)g.rp * g.nfeat;
 #pragma unroll
-                        for (int i = 0; i < CH; i++) st_u16(dst + (size_t)i * g.nfeat, f2h(v[i] - h2f(f2h(v[i]))), i < m);
+                        for (int i = 0; i < CH; i += 2, dst += 2 * g.nfeat) {
+                            const u32 h = pack_h2(v[i], v[i + 1]), r = pack_h2(v[i] - h_lo(h), v[i + 1] - h_hi(h));
+                            st_u16(dst, (u16)h, i < m); st_u16(dst + g.nfeat, (u16)(h >> 16), i + 1 < m);
+                            st_u16(dst + lo, (u16)r, i < m); st_u16(dst + lo + g.nfeat, (u16)(r >> 16), i + 1 < m);
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < CH; i += 2, dst += 2 * g.nfeat) {
+                            const u32 h = pack_h2(v[i], v[i + 1]);
+                            st_u16(dst, (u16)h, i < m); st_u16(dst + g.nfeat, (u16)(h >> 16), i + 1 < m);
+                        }
                     }
                 } else {
                     float* dst = g.of + (size_t)row * g.nfeat + f;
@@ -376,7 +435,10 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS) pass_gemm(const __grid
             else if (c0 < c_hi) rows_of(Int<4>{}, c0);
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(tme + b * 8) : "memory");
+            if (lane == 0) {
+                if (PAIR) asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" :: "r"(of_first(tme + b * 8)) : "memory");
+                else asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(tme + b * 8) : "memory");
+            }
             if (EPI == EPI_LOGITS) {
                 asm volatile("bar.sync 1, %0;" :: "n"(EW * 32) : "memory");
                 if (!skip)
@@ -392,7 +454,11 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS) pass_gemm(const __grid
         if (!waited) dep_wait();
     }
     __syncthreads();
-    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(cols) : "memory");
+    if (PAIR) cluster_sync();                                                      // (neither block leaves while the other may still reach into it)
+    if (warp == 1) {
+        if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(cols) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(cols) : "memory");
+    }
     if (*dead && threadIdx.x == 0) {
         // a wait ran out: let copies in flight land (bounded) before the block's shared memory goes to another
         const u64 t0 = now_ns();
@@ -560,41 +626,54 @@ struct AttArgs {
     u16* out;                        // [row][D] fp16 (and the remainder plane)
 };
 #define ATT_WARPS 4
+__device__ __forceinline__ int kv_off(int row, int piece) { return row * 128 + ((piece ^ (row & 7)) << 4); }
+__device__ __forceinline__ void cp16(u32 dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory"); }
+__device__ __forceinline__ void ldsm4(u32 (&r)[4], u32 p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(p) : "memory");
+}
+__device__ __forceinline__ void ldsm4t(u32 (&r)[4], u32 p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(p) : "memory");
+}
+__device__ __forceinline__ void mma16816(float (&c)[4], const u32 (&a)[4], u32 b0, u32 b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
 // Block = one (row, head), or 1 / C of its positions where C blocks form a cluster; warps take runs of 16 positions in
-// turn. A group of eight lanes takes one position's 128 bytes (16 per lane), four positions per group and run, K and V. fp32
-// arithmetic on the ordinary cores: about 10 warp instructions per position and head. A lane's pieces of the next NS runs are
-// on their way into shared memory (its own slots: nobody else reads them), not through the L1 cache, which is small beside the
-// contractions' blocks: loads into registers then ran at 4.7 TB/s, and 5.8 with the cache at full size. The rows before the current
-// position are there since earlier steps: the first NS runs are requested before the block waits for the kernel that computes
-// the query and the current position's row.
+// turn, on mma.sync: scores = K rows (16 positions x 16 dims per step) times the query, its fp16 head in column 0 and its fp16
+// remainder in column 1 (their sum is the fp32-accurate product); output = V transposed times the weights, head and remainder
+// again in two columns. The same in fp32 on the ordinary cores took 14 instructions per position and head, most of them
+// conversions of K and V, and was bound by them: 64 sequences of 512 positions 13.7 us per layer even with the cache in
+// L2. A warp's next NS runs are on their way into shared memory (the L1 cache is small beside the contractions'
+// blocks). The rows before the current position are there since earlier steps: the first NS runs are requested before the block
+// waits for the kernel that computes the query and the current position's row.
 #define ATT_RUN 16
 __device__ __forceinline__ void cp16z(u32 dst, const void* src, bool yes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(dst), "l"(src), "r"(yes ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ uint4 lds128(u32 a) {
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
-    return v;
 }
 template <int NS>
 __global__ void __launch_bounds__(ATT_WARPS * 32) pass_attend(const __grid_constant__ AttArgs a) {
     __shared__ float part[ATT_WARPS + 1][66];
     extern __shared__ __align__(128) unsigned char ring_raw[];
     const int h = blockIdx.x, row = blockIdx.y, C = gridDim.z, cr = blockIdx.z;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, pl = lane >> 3, dl = lane & 7;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, pl = lane >> 3, dl = lane & 7, g = lane >> 2, t4 = lane & 3;
     if (threadIdx.x == 0) dep_launch();
     const int n = min(__ldcg(a.t + row * a.t_stride) + 1, a.tmax), sq = a.seq ? __ldcg(a.seq + row) : row;
     const u16* kp = a.kc + sq * a.seq_stride + h * 64 + dl * 8;
     const u16* vp = a.vc + sq * a.seq_stride + h * 64 + dl * 8;
     const int step = C * ATT_WARPS * ATT_RUN;
     int p0 = (cr * ATT_WARPS + warp) * ATT_RUN;
-    const u32 ring = smem_u32(ring_raw) + warp * (NS * 4096) + lane * 16;          // [stage][K, V][j][lane]
+    // per stage 16 rows of K, then of V, 128 bytes each; the 16-byte pieces of a row swizzled (kv_off)
+    const u32 ring = smem_u32(ring_raw) + warp * (NS * 4096);
+    u32 put[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) put[j] = ring + kv_off(j * 4 + pl, dl);
     auto request = [&](int st, int p, int end) {
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const int x = p + j * 4 + pl;
-            cp16z(ring + st * 4096 + j * 512, kp + (size_t)(x < end ? x : 0) * a.D, x < end);
-            cp16z(ring + st * 4096 + 2048 + j * 512, vp + (size_t)(x < end ? x : 0) * a.D, x < end);
+            const size_t off = (size_t)(x < end ? x : 0) * a.D;
+            cp16z(put[j] + st * 4096, kp + off, x < end);
+            cp16z(put[j] + st * 4096 + 2048, vp + off, x < end);
         }
     };
 #pragma unroll
@@ -603,76 +682,96 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) pass_attend(const __grid_const
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
     dep_wait();
-    float q[8];
+    u32 bq[4][2];
     {
-        const float4* qp = reinterpret_cast<const float4*>(a.q + (size_t)row * a.D + h * 64 + dl * 8);
-        const float4 q0 = __ldcg(qp), q1 = __ldcg(qp + 1);
-        const float sc = a.pow2 ? 1.0f / a.scale : 1.0f;
-        // the current position, if it is in one of the runs requested above: its pieces by the lanes that will read them
-        uint4 kc, vc;
+        const float* qp = a.q + (size_t)row * a.D + h * 64;
+        float2 x[4][2];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            x[k][0] = g < 2 ? __ldcg(reinterpret_cast<const float2*>(qp + k * 16 + 2 * t4)) : make_float2(0.f, 0.f);
+            x[k][1] = g < 2 ? __ldcg(reinterpret_cast<const float2*>(qp + k * 16 + 2 * t4 + 8)) : make_float2(0.f, 0.f);
+        }
+        // the current position, if it is in one of the runs requested above
         u32 at = 0;
 #pragma unroll
         for (int i = 0; i < NS; i++) {
-            const int x = n - 1 - (p0 + i * step);
-            if (x >= 0 && x < ATT_RUN && (x & 3) == pl) at = ring + i * 4096 + (x >> 2) * 512;
+            const int y = n - 1 - (p0 + i * step);
+            if (y >= 0 && y < ATT_RUN && (y & 3) == pl) at = ring + i * 4096 + kv_off(y, dl);
         }
         if (at) {
-            kc = __ldcg(reinterpret_cast<const uint4*>(kp + (size_t)(n - 1) * a.D)); vc = __ldcg(reinterpret_cast<const uint4*>(vp + (size_t)(n - 1) * a.D));
+            const uint4 kc = __ldcg(reinterpret_cast<const uint4*>(kp + (size_t)(n - 1) * a.D)), vc = __ldcg(reinterpret_cast<const uint4*>(vp + (size_t)(n - 1) * a.D));
             asm volatile("cp.async.wait_all;" ::: "memory");                       // (the zeros that were requested in its place)
             asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" :: "r"(at), "r"(kc.x), "r"(kc.y), "r"(kc.z), "r"(kc.w) : "memory");
             asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" :: "r"(at + 2048), "r"(vc.x), "r"(vc.y), "r"(vc.z), "r"(vc.w) : "memory");
         }
-        q[0] = q0.x * sc; q[1] = q0.y * sc; q[2] = q0.z * sc; q[3] = q0.w * sc; q[4] = q1.x * sc; q[5] = q1.y * sc; q[6] = q1.z * sc; q[7] = q1.w * sc;
-    }
-    float m = -3.0e38f, den = 0.f, o[8];
+        const float sc = a.pow2 ? 1.0f / a.scale : 1.0f;
 #pragma unroll
-    for (int e = 0; e < 8; e++) o[e] = 0.f;
+        for (int k = 0; k < 4; k++)
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const float u = x[k][i].x * sc, v = x[k][i].y * sc;
+                const u32 hi = pack_h2(u, v);
+                bq[k][i] = g == 0 ? hi : g == 1 ? pack_h2(u - h_lo(hi), v - h_hi(hi)) : 0u;
+            }
+    }
+    float m = -3.0e38f, den = 0.f, o[4][4];              // o[mt]: dims mt*16 + g (regs 0 + 1) and mt*16 + g + 8 (regs 2 + 3), lanes with t4 == 0
+#pragma unroll
+    for (int i = 0; i < 4; i++) { o[i][0] = 0.f; o[i][1] = 0.f; o[i][2] = 0.f; o[i][3] = 0.f; }
     int st = 0;
+    const u32 ka = ring + kv_off(lane & 15, 0), va = ring + 2048 + ((lane & 7) + ((lane >> 4) ? 8 : 0)) * 128;
+    const int kx = lane >> 4, k7 = lane & 7, vx = (lane >> 3) & 1;
 #pragma unroll 1
     while (p0 < n) {
         asm volatile("cp.async.wait_group %0;" :: "n"(NS - 1) : "memory");
-        const u32 slot = ring + st * 4096;
-        float s[4];
+        __syncwarp();
+        const u32 so = st * 4096;
+        float s[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const uint4 k = lds128(slot + j * 512);
-            s[j] = (q[0] * h_lo(k.x) + q[1] * h_hi(k.x)) + (q[2] * h_lo(k.y) + q[3] * h_hi(k.y)) + ((q[4] * h_lo(k.z) + q[5] * h_hi(k.z)) + (q[6] * h_lo(k.w) + q[7] * h_hi(k.w)));
+        for (int k = 0; k < 4; k++) {
+            u32 r[4];
+            ldsm4(r, (ka & ~127u) + so + (((k * 2 + kx) ^ k7) << 4));
+            mma16816(s, r, bq[k][0], bq[k][1]);
         }
-        // sums over the eight lanes of a group, transposed: lane dl ends with the score of position p0 + 4 (dl / 2) + pl
-#pragma unroll
-        for (int j = 0; j < 2; j++) { const float keep = (dl & 4) ? s[j + 2] : s[j], give = (dl & 4) ? s[j] : s[j + 2]; s[j] = keep + __shfl_xor_sync(0xffffffffu, give, 4); }
-        { const float keep = (dl & 2) ? s[1] : s[0], give = (dl & 2) ? s[0] : s[1]; s[0] = keep + __shfl_xor_sync(0xffffffffu, give, 2); }
-        s[0] += __shfl_xor_sync(0xffffffffu, s[0], 1);
-        const float sc = a.pow2 ? s[0] : s[0] / a.scale;
-        const bool live = p0 + (dl >> 1) * 4 + pl < n;
-        int km = __float_as_int(live ? sc : -3.0e38f);
+        float s0 = s[0] + s[1], s1 = s[2] + s[3];        // positions p0 + g and p0 + g + 8, in the lanes with t4 == 0
+        if (!a.pow2) { s0 /= a.scale; s1 /= a.scale; }
+        if (t4 != 0 || p0 + g >= n) s0 = -3.0e38f;
+        if (t4 != 0 || p0 + g + 8 >= n) s1 = -3.0e38f;
+        int km = __float_as_int(fmaxf(s0, s1));
         km = __reduce_max_sync(0xffffffffu, km >= 0 ? km : km ^ 0x7fffffff);
-        const float mn = fmaxf(m, __int_as_float(km >= 0 ? km : km ^ 0x7fffffff));
-        const float corr = fast_exp(m - mn), p = live ? fast_exp(sc - mn) : 0.f;
-        m = mn;
-        den = den * corr + ((dl & 1) ? 0.f : p);
+        const float mx = __int_as_float(km >= 0 ? km : km ^ 0x7fffffff);
+        if (mx > m) {                                    // (the same in the whole warp)
+            const float corr = fast_exp(m - mx);
+            m = mx;
+            den *= corr;
 #pragma unroll
-        for (int e = 0; e < 8; e++) o[e] *= corr;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const uint4 v = lds128(slot + 2048 + j * 512);
-            const float pj = __shfl_sync(0xffffffffu, p, (lane & 24) | (2 * j));
-            o[0] += pj * h_lo(v.x); o[1] += pj * h_hi(v.x); o[2] += pj * h_lo(v.y); o[3] += pj * h_hi(v.y);
-            o[4] += pj * h_lo(v.z); o[5] += pj * h_hi(v.z); o[6] += pj * h_lo(v.w); o[7] += pj * h_hi(v.w);
+            for (int i = 0; i < 4; i++) { o[i][0] *= corr; o[i][1] *= corr; o[i][2] *= corr; o[i][3] *= corr; }
         }
+        const float pa = s0 > -1.0e38f ? fast_exp(s0 - m) : 0.f, pb = s1 > -1.0e38f ? fast_exp(s1 - m) : 0.f;
+        den += pa + pb;
+        // the weights as operand: lane (g, t4) holds positions 2 t4, 2 t4 + 1 (and + 8); that of position r < 8 is `pa` of lane 4 r
+        const float w00 = __shfl_sync(0xffffffffu, pa, 8 * t4), w01 = __shfl_sync(0xffffffffu, pa, 8 * t4 + 4);
+        const float w10 = __shfl_sync(0xffffffffu, pb, 8 * t4), w11 = __shfl_sync(0xffffffffu, pb, 8 * t4 + 4);
+        u32 b0 = pack_h2(w00, w01), b1 = pack_h2(w10, w11);
+        if (g == 1) { b0 = pack_h2(w00 - h_lo(b0), w01 - h_hi(b0)); b1 = pack_h2(w10 - h_lo(b1), w11 - h_hi(b1)); }
+        if (g > 1) { b0 = 0; b1 = 0; }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            u32 r[4];
+            ldsm4t(r, va + so + (((i * 2 + vx) ^ k7) << 4));
+            mma16816(o[i], r, b0, b1);
+        }
+        __syncwarp();                                    // every lane has read the stage
         if (p0 + NS * step < n) request(st, p0 + NS * step, n);
         asm volatile("cp.async.commit_group;" ::: "memory");
         p0 += step;
         if (++st == NS) st = 0;
     }
 #pragma unroll
-    for (int e = 0; e < 8; e++) { o[e] += __shfl_xor_sync(0xffffffffu, o[e], 8); o[e] += __shfl_xor_sync(0xffffffffu, o[e], 16); }
-#pragma unroll
     for (int x = 16; x; x >>= 1) den += __shfl_xor_sync(0xffffffffu, den, x);
-    if (lane == 0) { part[warp][64] = m; part[warp][65] = den; }
-    if (lane < 8)
+    if (t4 == 0)
 #pragma unroll
-        for (int e = 0; e < 8; e++) part[warp][dl * 8 + e] = o[e];
+        for (int i = 0; i < 4; i++) { part[warp][i * 16 + g] = o[i][0] + o[i][1]; part[warp][i * 16 + g + 8] = o[i][2] + o[i][3]; }
+    if (lane == 0) { part[warp][64] = m; part[warp][65] = den; }
     __syncthreads();
     float M = -3.0e38f, dd = 0.f, num = 0.f;
     if (threadIdx.x < 64) {
@@ -728,18 +827,6 @@ struct AttManyArgs {
     int clear, seqs, tmax;           // the first `clear` blocks of a row of blocks zero the cache rows after the prompts
     const int* lens;
 };
-__device__ __forceinline__ int kv_off(int row, int piece) { return row * 128 + ((piece ^ (row & 7)) << 4); }
-__device__ __forceinline__ void cp16(u32 dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory"); }
-__device__ __forceinline__ void ldsm4(u32 (&r)[4], u32 p) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(p) : "memory");
-}
-__device__ __forceinline__ void ldsm4t(u32 (&r)[4], u32 p) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(p) : "memory");
-}
-__device__ __forceinline__ void mma16816(float (&c)[4], const u32 (&a)[4], u32 b0, u32 b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 // Block = up to 64 consecutive positions of one sequence x one head, sixteen per warp; the cache in tiles of 64 positions,
 // double buffered; causal. Queries and weights enter the products as fp16 head and fp16 remainder (two products each),
 // as in the decode kernels: scores and output at fp32 accuracy over the fp16 cache.
