@@ -32,7 +32,7 @@ struct Layout {
 struct Meta {
     int x, t, seq, tiles, want, dst, lens, words, max_tiles;
     Meta(int rows, int lrows, int seqs) {
-        max_tiles = rows / 64 + std::min(rows, seqs) + 1;
+        max_tiles = rows / 128 + std::min(rows, seqs) + 1;
         tiles = 0; dst = tiles + 4 * max_tiles; x = dst + 2 * lrows; t = x + rows; seq = t + rows; want = seq + rows; lens = want + lrows; words = lens + seqs;
     }
 };
@@ -50,6 +50,7 @@ struct Pass {
         CUtensorMap w[5], a[5];                // weights and operand of every contraction
     };
     std::vector<Plan> plans;                   // the last few
+    CUtensorMap kmap, vmap;                    // prompts: the caches, 128 rows of one head per box
     size_t part_rows;                          // rows of the parts buffer
     std::vector<cudaGraphExec_t> graphs;       // decode: one step
     int sms;
@@ -158,7 +159,7 @@ template <class F> cudaError_t all_shared(F* f) { return cudaFuncSetAttribute((c
 template <int BM, int EPI>
 cudaError_t launch_gemm(cudaLaunchConfig_t& c, const Tile& t, const CUtensorMap& w, const CUtensorMap& a, const GemmArgs& g) {
     c.dynamicSmemBytes = GemmShape<BM>::bytes(t.stages, t.bn);
-    c.blockDim = dim3(GemmShape<BM>::THREADS);
+    c.blockDim = dim3(GemmShape<BM>::THREADS + (EPI == EPI_QKV && g.seqs ? 32 : 0));
     return cudaLaunchKernelEx(&c, pass_gemm<BM, EPI>, w, a, g);
 }
 template <int BM, int EPI>
@@ -186,8 +187,10 @@ cudaError_t prepare_all() {
     auto one = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
     one(all_shared(pass_norm<NORM_EMBED>)); one(all_shared(pass_norm<NORM_MID>)); one(all_shared(pass_norm<NORM_FINAL>));
     one(all_shared(pass_norm_rows<6>)); one(all_shared(pass_norm_rows<13>)); one(all_shared(pass_norm_rows<16>));
-    one(all_shared(pass_attend<2>)); one(all_shared(pass_attend<4>)); one(all_shared(pass_attend_many));
+    one(all_shared(pass_attend<2>)); one(all_shared(pass_attend<4>)); one(all_shared(pass_attend_many<true>)); one(all_shared(pass_attend_many<false>));
     one(gemm_prepare());
+    one(cudaFuncSetAttribute((const void*)pass_attend_many<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, AM_SMEM));
+    one(cudaFuncSetAttribute((const void*)pass_attend_many<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AM_SMEM));
     one(cudaFuncSetAttribute((const void*)pass_attend<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * ATT_WARPS * 4096)); one(all_shared(pass_finish));
     return e;
 }
@@ -229,7 +232,7 @@ int plan_for(Pass& p, int rows, int lrows, const Pass::Plan** out) {
 }
 
 // The launches of one pass over `rows` rows. Prompts: `tiles` runs of rows for the attention, `lrows` rows that want logits
-// (none: the pass ends with the last layer's cache rows); `clear`: zero the cache rows after the prompts.
+// (none: the pass ends with the last layer's cache rows); `clear`: zero the cache rows behind the ones that the pass writes.
 int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear = false) {
     const vesta_pass_desc& d = p.d;
     const int D = d.D, F = d.F, L = d.L, kbd = D / 64, kbf = (F + 63) / 64;
@@ -277,6 +280,7 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
         if (kind == K_QKV) {
             g.bias = f16(d.qkvb, (size_t)l * 3 * D); g.of = (float*)u(p.o.q); g.rowoff = (const long long*)u(p.o.rowoff);
             g.kc = (u16*)d.keys + (size_t)l * d.tmax * D; g.vc = (u16*)d.vals + (size_t)l * d.tmax * D;
+            if (clear) { g.lens = meta + mt.lens; g.seqs = d.prompts; g.seq_stride = (long long)L * d.tmax * D; g.tmax = d.tmax; }
         } else if (kind == K_FC) {
             g.bias = f16(d.fcb, (size_t)l * F); g.oh = (u16*)u(p.o.gelu); g.a2 = 2 * d.gelu_a; g.k1 = d.gelu_b * 2.8853900817779268f; g.k2 = d.gelu_c * g.k1;
         } else if (kind == K_LOGITS) { g.of = (float*)d.logits; g.best = (u64*)u(p.o.best); }
@@ -286,17 +290,17 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
         Config c(dim3(t.bm == 64 && kind != K_LOGITS ? g.ntiles : t.bm == 256 ? 2 * std::min(g.ntiles, p.sms / 2) : std::min(g.ntiles, p.sms)), 192, st, true, t.bm == 256 ? 2 : 1, true);
         return gemm(epi_of(kind, t), t, c.c, pl->w[kind], pl->a[kind], g);
     };
-    auto attend = [&](int l, int tiles) {
+    auto attend = [&](int l) {
         const float* q = (const float*)u(p.o.q);
         const u16 *kc = (const u16*)d.keys + (size_t)l * d.tmax * D, *vc = (const u16*)d.vals + (size_t)l * d.tmax * D;
         const long long ss = (long long)L * d.tmax * D;
         int e = 0;
         const int pow2 = frexpf(d.scale, &e) == 0.5f;
         if (many) {
-            const int zb = clear ? (2 * p.sms + d.H - 1) / d.H : 0;
-            AttManyArgs a = {q, kc, vc, ss, (const int4*)(meta + mt.tiles), D, pow2, d.scale, att, zb, d.prompts, d.tmax, meta + mt.lens};
-            Config c(dim3(zb + tiles, d.H), 128, st, true);
-            return cudaLaunchKernelEx(&c.c, pass_attend_many, a);
+            AttManyArgs a = {q, (const int4*)(meta + mt.tiles), l, L, D, pow2, d.scale, att, (u32*)d.bar};
+            Config c(dim3(tiles, d.H), 192, st, true);
+            c.c.dynamicSmemBytes = AM_SMEM;
+            return pow2 ? cudaLaunchKernelEx(&c.c, pass_attend_many<true>, p.kmap, p.vmap, a) : cudaLaunchKernelEx(&c.c, pass_attend_many<false>, p.kmap, p.vmap, a);
         }
         AttArgs a = {q, kc, vc, ss, (const int*)d.t, (const int*)0, d.t_stride, d.tmax, D, pow2, p.rp, d.scale, att};
         Config c(dim3(d.H, rows, C), ATT_WARPS * 32, st, true, C);
@@ -306,9 +310,8 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
     TRY(norm(0, 0, 0));
     for (int l = 0; l < L; l++) {
         TRY(mul(K_QKV, l));
-        const bool end = l == L - 1 && lrows == 0;
-        if (!end || clear) TRY(attend(l, end ? 0 : tiles));
-        if (end) break;
+        if (l == L - 1 && lrows == 0) break;
+        TRY(attend(l));
         TRY(mul(K_PROJ, l));
         TRY(norm(1, l, pl->tile[K_PROJ].splits > 1 ? pl->tile[K_PROJ].splits : 0));
         TRY(mul(K_FC, l));
@@ -358,6 +361,11 @@ int vesta_pass_create(const vesta_pass_desc* d, void* workspace, int graph, void
     int e = plan(*p, d);
     p->ws = (unsigned char*)workspace;
     if (!e) { const cudaError_t ce = prepare_all(); if (ce != cudaSuccess) e = cuda_fail(ce, "cudaFuncSetAttribute"); }
+    if (!e && d->prompts) {
+        const unsigned long long D = d->D, planes = (unsigned long long)d->prompts * d->L;
+        e = vesta_rt::tensor_map(&p->kmap, d->keys, D, d->tmax, planes, D * 2, D * 2 * d->tmax, 128, 1);
+        if (!e) e = vesta_rt::tensor_map(&p->vmap, d->vals, D, d->tmax, planes, D * 2, D * 2 * d->tmax, 128, 1);
+    }
     if (!e && graph) {
         // a decode step as a graph, captured on a stream of its own
         cudaStream_t st = nullptr;
@@ -404,6 +412,7 @@ int vesta_pass_prompts(void* pass, void* stream, const int* tokens, int ld, cons
     }
     struct Run { int first, rows, seq, pos; };
     std::vector<Run> runs;
+    std::vector<int> written(B);
     int s = 0, pos = 0;                          // next position to read
     for (int c = 0; c < passes; c++) {
         int* m = p->host + (size_t)c * mt.words;
@@ -412,7 +421,7 @@ int vesta_pass_prompts(void* pass, void* stream, const int* tokens, int ld, cons
         while (n < per && s < B) {
             const int take = std::min(per - n, lens[s] - pos);
             for (int i = 0; i < take; i++) { m[mt.x + n + i] = tokens[(size_t)s * ld + pos + i]; m[mt.t + n + i] = pos + i; m[mt.seq + n + i] = s; }
-            for (int i = 0; i < take; i += 64) runs.push_back(Run{n + i, std::min(64, take - i), s, pos + i});
+            for (int i = 0; i < take; i += 128) runs.push_back(Run{n + i, std::min(128, take - i), s, pos + i});
             n += take; pos += take;
             if (pos == lens[s]) {
                 m[mt.want + lrows] = n - 1; m[mt.dst + 2 * lrows] = s; m[mt.dst + 2 * lrows + 1] = lens[s];
@@ -422,7 +431,9 @@ int vesta_pass_prompts(void* pass, void* stream, const int* tokens, int ld, cons
         // the runs that see most positions first
         std::stable_sort(runs.begin(), runs.end(), [](const Run& a, const Run& b) { return a.pos + a.rows > b.pos + b.rows; });
         for (size_t i = 0; i < runs.size(); i++) { int* t = m + mt.tiles + 4 * i; t[0] = runs[i].first; t[1] = runs[i].rows; t[2] = runs[i].seq; t[3] = runs[i].pos; }
-        for (int i = 0; i < B; i++) m[mt.lens + i] = lens[i];
+        // rows written by the first pass: everything behind them is cleared there, what later passes will write included
+        if (c == 0) for (int i = 0; i < B; i++) written[i] = i < s ? lens[i] : i == s ? pos : 0;
+        for (int i = 0; i < B; i++) m[mt.lens + i] = written[i];
         TRY(cudaMemcpyAsync(p->ws + p->o.meta, m, (size_t)mt.words * 4, cudaMemcpyHostToDevice, st));
         if (int e = enqueue(*p, st, n, lrows, (int)runs.size(), c == 0)) return e;
     }

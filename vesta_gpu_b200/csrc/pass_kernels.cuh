@@ -107,6 +107,10 @@ struct GemmArgs {
     u64* best;                       // LOGITS: packed (value, ~index) maximum of every row
     u32* status;
     float a2, k1, k2;                // GELU: see gelu_tanh
+    // QKV, prompts: one more warp zeroes this layer's cache rows behind the first lens[sequence], which this pass writes
+    const int* lens;
+    long long seq_stride;
+    int seqs, tmax;
 };
 
 // shared-memory operand descriptors, 128-byte swizzle. K-major: rows of 128 bytes (64 fold indices), groups of eight rows
@@ -187,8 +191,9 @@ __device__ __forceinline__ void add_f32(float* p, float v, bool yes) {
 //     1,160 to 1,200 TFLOP/s.
 //   BM = 256: many rows, two blocks of a cluster with one product of 256 rows (cta_group::2): each loads its own 128 features and
 //     half the rows of the tile, so that a 256 x 256 tile costs an SM 32 KB per block of the fold instead of 48.
+#define CLEAR_ROWS 16
 template <int BM, int EPI>
-__global__ void __launch_bounds__(GemmShape<BM>::THREADS) pass_gemm(const __grid_constant__ CUtensorMap wm, const __grid_constant__ CUtensorMap am, const __grid_constant__ GemmArgs g) {
+__global__ void __launch_bounds__(GemmShape<BM>::THREADS + (EPI == EPI_QKV ? 32 : 0)) pass_gemm(const __grid_constant__ CUtensorMap wm, const __grid_constant__ CUtensorMap am, const __grid_constant__ GemmArgs g) {
     using S = GemmShape<BM>;
     constexpr int KS = S::KS, EW = S::EW, AM = S::AM;
     constexpr bool PAIR = S::PAIR;
@@ -311,6 +316,17 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS) pass_gemm(const __grid
                 __syncwarp();
                 if (++s == st) { s = 0; ph ^= 1; }
             }
+        }
+    } else if (EPI == EPI_QKV && warp == EW + 2) {
+        // Nothing waits for these rows before the attention and they wait for nothing: they leave in the shadow of the
+        // products, which need little of the memory. (As a kernel of its own on another stream the clearing delayed the chain:
+        // none of its kernels started early until it was done; as blocks of the attention it was that kernel's tail.)
+        const int per_row = g.D / 8, parts = (g.tmax + CLEAR_ROWS - 1) / CLEAR_ROWS;
+        for (int j = blockIdx.x; j < 2 * g.seqs * parts; j += gridDim.x) {
+            const int sq = j / (2 * parts), r = j - sq * 2 * parts, part = r >> 1;
+            const int lo = max(part * CLEAR_ROWS, __ldg(g.lens + sq)) * per_row, hi = min((part + 1) * CLEAR_ROWS, g.tmax) * per_row;
+            uint4* p = reinterpret_cast<uint4*>(((r & 1) ? g.vc : g.kc) + sq * g.seq_stride);
+            for (int i = lo + lane; i < hi; i += 32) p[i] = make_uint4(0, 0, 0, 0);
         }
     } else {
         const int quarter = warp & 3, ew = warp - 2, et = threadIdx.x - 64;
@@ -817,147 +833,248 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) pass_attend(const __grid_const
 
 // ---- attention of many positions (prompts) ----------------------------------------------------------------------------
 struct AttManyArgs {
-    const float* q;
-    const u16 *kc, *vc;
-    long long seq_stride;
-    const int4* tiles;               // (first row, rows, sequence, first position) of every run of at most 64 rows of one sequence
-    int D, pow2;
+    const float* q;                  // [row][D] fp32
+    const int4* tiles;               // (first row, rows, sequence, first position) of every run of at most 128 rows of one sequence
+    int layer, L, D, pow2;
     float scale;
-    u16* out;
-    int clear, seqs, tmax;           // the first `clear` blocks of a row of blocks zero the cache rows after the prompts
-    const int* lens;
+    u16* out;                        // [row][D] fp16
+    u32* status;
 };
-// Block = up to 64 consecutive positions of one sequence x one head, sixteen per warp; the cache in tiles of 64 positions,
-// double buffered; causal. Queries and weights enter the products as fp16 head and fp16 remainder (two products each),
-// as in the decode kernels: scores and output at fp32 accuracy over the fp16 cache.
-__global__ void __launch_bounds__(128) pass_attend_many(const __grid_constant__ AttManyArgs a) {
-    __shared__ __align__(128) unsigned char kv[2][2][64 * 128];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+__device__ __forceinline__ void tm_ld32(u32 (&r)[32], u32 addr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
+                   "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]),
+                   "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]) : "r"(addr) : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]),
+                   "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]),
+                   "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]) : : "memory");
+    asm volatile("" : "+r"(r[30]), "+r"(r[31]));
+}
+__device__ __forceinline__ void tm_st32(u32 addr, const u32 (&r)[32]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31};"
+                 :: "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
+                    "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]),
+                    "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]), "r"(addr) : "memory");
+}
+#define AM_STAGES 2
+#define AM_SMEM (32768 + AM_STAGES * 32768 + 128 + 1024)
+// Block = up to 128 consecutive positions of one sequence x one head; the cache in tiles of 128 positions; causal. On tcgen05:
+// scores = queries (fp16 head and remainder, two products: fp32 accuracy over the fp16 cache) x K rows, 128 x 128 in tensor
+// memory; a thread owns a row: maximum, exponentials and sum without exchange; the weights go back into the columns of the
+// scores as fp16 head and remainder (operand A of the second product, in tensor memory) x V rows (N-major as they lie in the
+// cache). The output is rescaled only when a row's maximum has grown by more than 5.5 (the weights stay below 2^8, and the
+// same maximum normalises them at the end). Two blocks per SM: one's exponentials run under the other's products.
+// With mma.sync (64 rows per block, the same two-part operands) the products set the time: 58 us per layer at 9,200 rows of 32
+// prompts of 64 to 512.
+template <bool POW2>                                    // the divisor of the scores is a power of two: applied to the queries
+__global__ void __launch_bounds__(192, 2) pass_attend_many(const __grid_constant__ CUtensorMap km, const __grid_constant__ CUtensorMap vm, const __grid_constant__ AttManyArgs a) {
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    const u32 sq = smem_u32(smem), skv = sq + 32768, bars = skv + AM_STAGES * 32768;
+    const u32 qf = bars, sf = bars + 8, pf = bars + 16, of = bars + 24, kvf = bars + 32, kve = kvf + AM_STAGES * 8;
+    unsigned char* tail = smem + 32768 + AM_STAGES * 32768 + 32 + AM_STAGES * 16;
+    volatile u32* tmem_p = reinterpret_cast<volatile u32*>(tail);
+    volatile int* dead = reinterpret_cast<volatile int*>(tail + 4);
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const Wait w{dead, a.status};
+    if (threadIdx.x == 0) {
+        *dead = 0;
+        mbar_init(qf, 4); mbar_init(sf, 1); mbar_init(pf, 4); mbar_init(of, 1);
+        for (int i = 0; i < AM_STAGES; i++) { mbar_init(kvf + i * 8, 1); mbar_init(kve + i * 8, 1); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("prefetch.tensormap [%0];" :: "l"(&km) : "memory");
+        asm volatile("prefetch.tensormap [%0];" :: "l"(&vm) : "memory");
+    }
+    if (warp == 5) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(tail)), "n"(256) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    }
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (threadIdx.x == 0) dep_launch();
-    if ((int)blockIdx.x < a.clear) {
-        // The rows of the caches after the prompts, in pieces of 64 rows: nothing waits for them and they wait for nothing, so
-        // their blocks come first and write under the QKV contraction before this kernel. (On a stream of its own the clearing
-        // delayed the chain: no kernel of it started early until the clearing was done.)
-        const int per_row = a.D / 8, parts = (a.tmax + 63) / 64;
-        for (int j = blockIdx.x * gridDim.y + blockIdx.y; j < 2 * a.seqs * parts; j += a.clear * gridDim.y) {
-            const int sq = j / (2 * parts), r = j - sq * 2 * parts, part = r >> 1;
-            const int lo = max(part * 64, __ldg(a.lens + sq)), hi = min(part * 64 + 64, a.tmax);
-            uint4* p = reinterpret_cast<uint4*>(const_cast<u16*>((r & 1) ? a.vc : a.kc) + sq * a.seq_stride);
-            for (int i = lo * per_row + threadIdx.x; i < hi * per_row; i += 128) p[i] = make_uint4(0, 0, 0, 0);
-        }
-        return;
-    }
-    const int4 tl = __ldg(a.tiles + blockIdx.x - a.clear);
-    const int h = blockIdx.y, row0 = tl.x, nrows = tl.y, pos0 = tl.w;
-    dep_wait();
-    const u16* kp = a.kc + tl.z * a.seq_stride + h * 64;
-    const u16* vp = a.vc + tl.z * a.seq_stride + h * 64;
-    const int total = pos0 + nrows, ntiles = (total + 63) / 64;
-    auto fetch = [&](int j) {
-        const u32 ks = smem_u32(kv[j & 1][0]), vs = smem_u32(kv[j & 1][1]);
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int e = threadIdx.x + i * 128, r = e >> 3, c = e & 7;
-            const size_t off = (size_t)min(j * 64 + r, total - 1) * a.D + c * 8;
-            cp16(ks + kv_off(r, c), kp + off);
-            cp16(vs + kv_off(r, c), vp + off);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    fetch(0);
-    u32 qh[4][4], ql[4][4];
-    const int rA = warp * 16 + g, rB = rA + 8;
-    {
-        const float sc = a.pow2 ? 1.0f / a.scale : 1.0f;
-        const float* qa = a.q + (size_t)(row0 + min(rA, nrows - 1)) * a.D + h * 64 + 2 * t;
-        const float* qb = a.q + (size_t)(row0 + min(rB, nrows - 1)) * a.D + h * 64 + 2 * t;
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            float2 x[4];
-            x[0] = __ldcg(reinterpret_cast<const float2*>(qa + k * 16)); x[1] = __ldcg(reinterpret_cast<const float2*>(qb + k * 16));
-            x[2] = __ldcg(reinterpret_cast<const float2*>(qa + k * 16 + 8)); x[3] = __ldcg(reinterpret_cast<const float2*>(qb + k * 16 + 8));
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const float u = x[i].x * sc, v = x[i].y * sc;
-                qh[k][i] = pack_h2(u, v);
-                ql[k][i] = pack_h2(u - h_lo(qh[k][i]), v - h_hi(qh[k][i]));
+    const u32 tmem = *tmem_p, tO = tmem + 128;                                     // scores / weights: columns 0..127, output: 128..191
+    const int4 tl = __ldg(a.tiles + blockIdx.x);
+    const int h = blockIdx.y, row0 = tl.x, nrows = tl.y, pos0 = tl.w, total = pos0 + nrows, nt = (total + 127) / 128;
+    if (warp == 4) {
+        if (elect_one()) {
+            dep_wait();
+            for (int j = 0; j < nt; j++) {
+                const int s = j % AM_STAGES;
+                if (j >= AM_STAGES && !mbar_wait(kve + s * 8, (j / AM_STAGES - 1) & 1, w, 0xC00u)) break;
+                const u32 dst = skv + s * 32768;
+                mbar_expect(kvf + s * 8, 32768);
+                tma3(dst, &km, h * 64, j * 128, tl.z * a.L + a.layer, kvf + s * 8);
+                tma3(dst + 16384, &vm, h * 64, j * 128, tl.z * a.L + a.layer, kvf + s * 8);
             }
         }
-    }
-    float mA = -3.0e38f, mB = -3.0e38f, dA = 0.f, dB = 0.f, o[8][4];
+    } else if (warp == 5) {
+        constexpr u32 i_s = (1u << 4) | ((128u >> 3) << 17) | ((128u >> 4) << 24), i_o = (1u << 4) | (1u << 16) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
+        bool ok = !__any_sync(0xffffffffu, !mbar_wait(qf, 0, w, 0xC10u));
+        for (int j = 0; j < nt && ok; j++) {
+            const int s = j % AM_STAGES;
+            ok = !__any_sync(0xffffffffu, !mbar_wait(kvf + s * 8, (j / AM_STAGES) & 1, w, 0xC20u));
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (elect_one()) {
+                const u64 q = desc_k(sq), k = desc_k(skv + s * 32768);
 #pragma unroll
-    for (int n = 0; n < 8; n++)
+                for (int i = 0; i < 8; i++)
+                    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                                 :: "r"(tmem), "l"(q + (i >> 2) * 1024 + 2 * (i & 3)), "l"(k + 2 * (i & 3)), "r"(i_s), "r"(i ? 1u : 0u) : "memory");
+                tc_commit<false>(sf);
+            }
+            __syncwarp();
+            ok = !__any_sync(0xffffffffu, !mbar_wait(pf, j & 1, w, 0xC30u));
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (elect_one()) {
+                const u64 v = desc_m(skv + s * 32768 + 16384, 8192);
+                const int nk = min(8, (total - j * 128 + 15) / 16);                // steps of 16 positions that some row sees
 #pragma unroll
-        for (int i = 0; i < 4; i++) o[n][i] = 0.f;
+                for (int k = 0; k < 8; k++)
+                    if (k < nk) {
+#pragma unroll
+                        for (int x = 0; x < 2; x++)
+                            asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                                         :: "r"(tO), "r"(tmem + (k >> 1) * 32 + (k & 1) * 8 + x * 16), "l"(v + 128 * k), "r"(i_o), "r"((j | k | x) ? 1u : 0u) : "memory");
+                    }
+                tc_commit<false>(kve + s * 8);
+                if (j == nt - 1) tc_commit<false>(of);
+            }
+            __syncwarp();
+        }
+    } else {
+        const int row = warp * 32 + lane, p = pos0 + row;                          // this thread's row of the tile, its position
+        const u32 mine = (u32)(warp * 32) << 16;
+        dep_wait();
+        {
+            // sixteen lanes read a row's 256 bytes, a warp two rows at a time
+            const float sc = POW2 ? 1.0f / a.scale : 1.0f;
+            const int piece = lane & 15;
+            float4 x[16];
+#pragma unroll
+            for (int i = 0; i < 16; i++) x[i] = __ldcg(reinterpret_cast<const float4*>(a.q + (size_t)(row0 + min(warp * 32 + i * 2 + (lane >> 4), nrows - 1)) * a.D + h * 64) + piece);
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                const float4 u = make_float4(x[i].x * sc, x[i].y * sc, x[i].z * sc, x[i].w * sc);
+                const u32 h0 = pack_h2(u.x, u.y), h1 = pack_h2(u.z, u.w), l0 = pack_h2(u.x - h_lo(h0), u.y - h_hi(h0)), l1 = pack_h2(u.z - h_lo(h1), u.w - h_hi(h1));
+                const u32 at = sq + kv_off(warp * 32 + i * 2 + (lane >> 4), piece >> 1) + (piece & 1) * 8;
+                asm volatile("st.shared.v2.u32 [%0], {%1,%2};" :: "r"(at), "r"(h0), "r"(h1) : "memory");
+                asm volatile("st.shared.v2.u32 [%0], {%1,%2};" :: "r"(at + 16384), "r"(l0), "r"(l1) : "memory");
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(qf) : "memory");
+        }
+        constexpr float LOG2E = 1.4426950408889634f;
+        float m = -3.0e38f, den = 0.f;
+        bool ok = true;
 #pragma unroll 1
-    for (int j = 0; j < ntiles; j++) {
-        if (j + 1 < ntiles) { fetch(j + 1); asm volatile("cp.async.wait_group 1;" ::: "memory"); }
-        else asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();
-        const u32 ks = smem_u32(kv[j & 1][0]), vs = smem_u32(kv[j & 1][1]);
-        float s[8][4];
+        for (int j = 0; j < nt; j++) {
+            ok = !__any_sync(0xffffffffu, !mbar_wait(sf, j & 1, w, 0xC40u));
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int lim = p - j * 128;                                           // last column of the tile that this row sees
+            const int chunks = min(4, (total - j * 128 + 31) / 32);                // chunks of 32 columns that the second product reads,
+            const int seen = max(0, min(chunks, (lim - lane + 31) / 32 + (lim - lane + 31 >= 0 ? 1 : 0)));   // and that some row of this warp sees
+            u32 r[32];
+            // (chunks that all rows of the warp see whole carry no mask: 7 instead of 11 instructions per score)
+            const int whole = min(seen, (lim - lane + 1) >> 5);
+            float top[4] = {-3.0e38f, -3.0e38f, -3.0e38f, -3.0e38f};
+            auto maxima = [&](auto MASK, int c) {
+                tm_ld32(r, tmem + mine + c * 32);
 #pragma unroll
-        for (int n = 0; n < 8; n++)
+                for (int i = 0; i < 32; i++) {
+                    float s = __uint_as_float(r[i]);
+                    if (!POW2) s /= a.scale;
+                    if (decltype(MASK)::n) s = c * 32 + i <= lim ? s : -3.0e38f;
+                    top[i & 3] = fmaxf(top[i & 3], s);
+                }
+            };
+            int c = 0;
+#pragma unroll 1
+            for (; c < whole; c++) maxima(Int<0>{}, c);
+#pragma unroll 1
+            for (; c < seen; c++) maxima(Int<1>{}, c);
+            const float mx = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3]));
+            const bool grow = mx > m + 5.5f;
+            if (__any_sync(0xffffffffu, grow)) {
+                const float corr = grow ? fast_exp(m - mx) : 1.0f;
+                if (grow) m = mx;
+                den *= corr;
+                if (j > 0) {                                                       // (the products into the output have completed: the scores' came after them)
+#pragma unroll 1
+                    for (c = 0; c < 2; c++) {
+                        tm_ld32(r, tO + mine + c * 32);
 #pragma unroll
-            for (int i = 0; i < 4; i++) s[n][i] = 0.f;
-#pragma unroll
-        for (int k = 0; k < 4; k++)
-#pragma unroll
-            for (int n = 0; n < 8; n += 2) {
-                u32 b[4];
-                ldsm4(b, ks + kv_off(n * 8 + (lane & 7) + ((lane >> 4) << 3), k * 2 + ((lane >> 3) & 1)));
-                mma16816(s[n], qh[k], b[0], b[1]); mma16816(s[n + 1], qh[k], b[2], b[3]);
-                mma16816(s[n], ql[k], b[0], b[1]); mma16816(s[n + 1], ql[k], b[2], b[3]);
+                        for (int i = 0; i < 32; i++) r[i] = __float_as_uint(__uint_as_float(r[i]) * corr);
+                        tm_st32(tO + mine + c * 32, r);
+                    }
+                }
             }
-        const int pA = pos0 + rA - j * 64, pB = pA + 8;                            // last position of the tile that the rows see
-        float xA = -3.0e38f, xB = -3.0e38f;
+            const float m2 = m * LOG2E;
+            auto weights = [&](auto MASK, int c) {
+                u32 o[32];
+                float sum[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+                tm_ld32(r, tmem + mine + c * 32);
 #pragma unroll
-        for (int n = 0; n < 8; n++)
+                for (int i = 0; i < 32; i += 2) {
+                    float e[2];
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                if (!a.pow2) s[n][i] /= a.scale;
-                if (n * 8 + 2 * t + (i & 1) > ((i & 2) ? pB : pA)) s[n][i] = -3.0e38f;
-                if (i & 2) xB = fmaxf(xB, s[n][i]); else xA = fmaxf(xA, s[n][i]);
+                    for (int x = 0; x < 2; x++) {
+                        float s = __uint_as_float(r[i + x]);
+                        if (!POW2) s /= a.scale;
+                        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e[x]) : "f"(fmaf(s, LOG2E, -m2)));
+                        if (decltype(MASK)::n) e[x] = c * 32 + i + x <= lim ? e[x] : 0.f;
+                        sum[(i / 2) & 1][x] += e[x];
+                    }
+                    o[i / 2] = pack_h2(e[0], e[1]);
+                    o[16 + i / 2] = pack_h2(e[0] - h_lo(o[i / 2]), e[1] - h_hi(o[i / 2]));
+                }
+                den += (sum[0][0] + sum[0][1]) + (sum[1][0] + sum[1][1]);
+                tm_st32(tmem + mine + c * 32, o);
+            };
+#pragma unroll 1
+            for (c = 0; c < whole; c++) weights(Int<0>{}, c);
+#pragma unroll 1
+            for (; c < seen; c++) weights(Int<1>{}, c);
+#pragma unroll 1
+            for (; c < chunks; c++) {
+#pragma unroll
+                for (int i = 0; i < 32; i++) r[i] = 0u;
+                tm_st32(tmem + mine + c * 32, r);
             }
-        xA = fmaxf(xA, __shfl_xor_sync(0xffffffffu, xA, 1)); xA = fmaxf(xA, __shfl_xor_sync(0xffffffffu, xA, 2));
-        xB = fmaxf(xB, __shfl_xor_sync(0xffffffffu, xB, 1)); xB = fmaxf(xB, __shfl_xor_sync(0xffffffffu, xB, 2));
-        const float nA = fmaxf(mA, xA), nB = fmaxf(mB, xB), cA = fast_exp(mA - nA), cB = fast_exp(mB - nB);
-        mA = nA; mB = nB; dA *= cA; dB *= cB;
-#pragma unroll
-        for (int n = 0; n < 8; n++) {
-            o[n][0] *= cA; o[n][1] *= cA; o[n][2] *= cB; o[n][3] *= cB;
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                s[n][i] = s[n][i] > -1.0e38f ? fast_exp(s[n][i] - ((i & 2) ? nB : nA)) : 0.f;
-                if (i & 2) dB += s[n][i]; else dA += s[n][i];
-            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(pf) : "memory");
         }
+        if (ok) ok = !__any_sync(0xffffffffu, !mbar_wait(of, 0, w, 0xC50u));
+        if (ok) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const float inv = den > 0.f ? __fdividef(1.0f, den) : 0.f;
+            uint4* out = reinterpret_cast<uint4*>(a.out + (size_t)(row0 + row) * a.D + h * 64);
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            u32 ph[4], pr[4];
+            for (int c = 0; c < 2; c++) {
+                u32 r[32];
+                tm_ld32(r, tO + mine + c * 32);
+                if (row < nrows)
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const float u = s[2 * k + (i >> 1)][(i & 1) * 2], v = s[2 * k + (i >> 1)][(i & 1) * 2 + 1];
-                ph[i] = pack_h2(u, v);
-                pr[i] = pack_h2(u - h_lo(ph[i]), v - h_hi(ph[i]));
+                    for (int i = 0; i < 4; i++) {
+                        const float* v = reinterpret_cast<const float*>(r) + i * 8;
+                        out[c * 4 + i] = make_uint4(pack_h2(v[0] * inv, v[1] * inv), pack_h2(v[2] * inv, v[3] * inv), pack_h2(v[4] * inv, v[5] * inv), pack_h2(v[6] * inv, v[7] * inv));
+                    }
             }
-#pragma unroll
-            for (int n = 0; n < 8; n += 2) {
-                u32 b[4];
-                ldsm4t(b, vs + kv_off(k * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, n + (lane >> 4)));
-                mma16816(o[n], ph, b[0], b[1]); mma16816(o[n + 1], ph, b[2], b[3]);
-                mma16816(o[n], pr, b[0], b[1]); mma16816(o[n + 1], pr, b[2], b[3]);
-            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         }
-        __syncthreads();
     }
-    dA += __shfl_xor_sync(0xffffffffu, dA, 1); dA += __shfl_xor_sync(0xffffffffu, dA, 2);
-    dB += __shfl_xor_sync(0xffffffffu, dB, 1); dB += __shfl_xor_sync(0xffffffffu, dB, 2);
-    const float iA = dA > 0.f ? __fdividef(1.0f, dA) : 0.f, iB = dB > 0.f ? __fdividef(1.0f, dB) : 0.f;
-#pragma unroll
-    for (int n = 0; n < 8; n++) {
-        if (rA < nrows) *reinterpret_cast<u32*>(a.out + (size_t)(row0 + rA) * a.D + h * 64 + n * 8 + 2 * t) = pack_h2(o[n][0] * iA, o[n][1] * iA);
-        if (rB < nrows) *reinterpret_cast<u32*>(a.out + (size_t)(row0 + rB) * a.D + h * 64 + n * 8 + 2 * t) = pack_h2(o[n][2] * iB, o[n][3] * iB);
+    __syncthreads();
+    if (warp == 5) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "n"(256) : "memory");
+    if (*dead && threadIdx.x == 0) {
+        const u64 t0 = now_ns();
+        while (now_ns() - t0 < 2000000ull) { }
     }
 }
 
