@@ -243,9 +243,11 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
     float* z = (float*)u(p.o.z);
     u16 *act = (u16*)u(p.o.act), *att = (u16*)u(p.o.att), *fin = (u16*)u(p.o.fin);
     const int nthr = up(D / 4, 32);
-    // attention of a step: C blocks per (row, head) while the blocks of all stay resident; deep rings where few share an SM
-    int C = 1;
-    while (C < 8 && rows * d.H * C * 2 <= 6 * p.sms && d.tmax > C * ATT_WARPS * ATT_RUN) C *= 2;
+    // attention of a step: two blocks per (row, head) where that is at most three blocks per SM and the cache has two runs of
+    // positions. Clusters of four and eight lost everywhere (XL shape, 6 sequences at 128 positions: 1,342 -> 1,337 us per
+    // step with two blocks instead of four; 9 sequences, small shape, two instead of eight: 298 -> 270 us, at 1,000 positions
+    // 340 -> 321), and so did two beyond that line (23 sequences at 128 positions with one block: 294 -> 277 us).
+    const int C = rows * d.H * 2 <= 3 * p.sms && d.tmax > ATT_WARPS * ATT_RUN ? 2 : 1;
     const bool deep = rows * d.H * C <= 3 * p.sms;
     const Pass::Plan* pl = nullptr;
     if (int e = plan_for(p, rows, lrows, &pl)) return e;

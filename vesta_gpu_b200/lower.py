@@ -401,9 +401,11 @@ def _lower_small(env, dims, res, roles, fb, B, tmax, cpos, t_per_token, t_name, 
 
     # position chunks per (sequence, head), from the measured costs of the attention phase (cycles): an item costs a fixed
     # 1,500 plus 1,300 per tile of 128 positions, a CTA runs its items one after the other, and the projection that
-    # follows merges the chunks of a pair at about 80 per chunk; sized for a full cache
+    # follows merges the chunks of a pair at about 80 per chunk; sized for a full cache. More items than CTAs cost the two or
+    # three exchanges below, with a grid barrier each (eight sequences of the small shape, three chunks instead of one: 249
+    # against 211 us per step at 128 positions, 282 against 267 at 1,000)
     def att_cost(k):
-        return math.ceil(B * H * k / grid) * (1500 + 1300 * math.ceil(math.ceil(tmax / k) / 128)) + 80 * k
+        return math.ceil(B * H * k / grid) * (1500 + 1300 * math.ceil(math.ceil(tmax / k) / 128)) + 80 * k + 5000 * (B * H * k > grid)
     nch = int(tune.get('nch', min(range(1, 17), key=lambda k: (att_cost(k), k))))
     # One chunk per (sequence, head): the CTA that finishes an item also applies the head's 64 rows of the attention
     # projection (streamed behind the item's K/V tiles) and adds the result into z1; the projection phase and its grid
@@ -591,9 +593,13 @@ def lower(text, res, axis_max, batch=1, per_token=(), outputs=(), feedback=None,
     tune = dict(tune or {})
     # What a step as a chain of kernels (csrc/pass.cu) needs to know; Kernel runs that chain unless the caller asked for
     # something that only the persistent kernels have (a placement option, timing sums, rows of prompts).
-    # Up to eight sequences the small persistent kernel is the faster one (one sequence 172 against 250 us per step, eight 243
-    # against 270, XL shape with one 1,164 against 1,290): its exchanges between a few CTAs cost less than kernel boundaries.
-    dims = dict(dims, chain=not (tune or timing or row_seq or slab_tiles or act_lo is not None) and B > 8 and D <= 4096,
+    # Up to eight sequences the small persistent kernel is the faster one (one sequence 172 against 250 us per step, eight 211
+    # against 263, XL shape with four 1,243 against 1,415): its exchanges between a few CTAs cost less than kernel boundaries.
+    # With more (sequence, head) pairs than CTAs it has to fall back on grid barriers (XL shape, eight: 1,679 against 1,275 us;
+    # twenty heads, eight: 688 against 611), and where rows of more than 1,280 are normalised in every CTA, one warp per row, it
+    # loses from five sequences on (XL shape, five: 1,394 against 1,311).
+    persistent = B <= 8 and B * H <= grid and (B <= 4 or D <= 1280)
+    dims = dict(dims, chain=not (tune or timing or row_seq or slab_tiles or act_lo is not None) and not persistent and D <= 4096,
                 step=dict(t_stride=int(t_per_token), tstep=int(fb.get(t_name, 0)), feedback=int(bool(fb)), prompt_len=int(prompt_len) if fb else 0,
                           exact=int(B <= 8 or (B <= 16 and D <= 1024)), cpos=cpos))
     if B <= 8 and not tune.get('large_kernel') and act_lo is None and not slab_tiles and not row_seq:
