@@ -50,7 +50,7 @@ struct Pass {
         CUtensorMap w[5], a[5];                // weights and operand of every contraction
     };
     std::vector<Plan> plans;                   // the last few
-    CUtensorMap kmap, vmap;                    // prompts: the caches, 128 rows of one head per box
+    CUtensorMap qmap, kmap, vmap;              // prompts: queries (two planes) and the caches, 128 rows of one head per box
     size_t part_rows;                          // rows of the parts buffer
     std::vector<cudaGraphExec_t> graphs;       // decode: one step
     int sms;
@@ -272,6 +272,8 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
         Config c(dim3(mode == 3 ? lrows : rows), nthr, st, mode != 0);
         return mode == 0 ? cudaLaunchKernelEx(&c.c, pass_norm<NORM_EMBED>, n) : mode == 3 ? cudaLaunchKernelEx(&c.c, pass_norm<NORM_FINAL>, n) : cudaLaunchKernelEx(&c.c, pass_norm<NORM_MID>, n);
     };
+    int expo = 0;
+    const int pow2 = frexpf(d.scale, &expo) == 0.5f;
     auto mul = [&](int kind, int l) {
         const Tile& t = pl->tile[kind];
         GemmArgs g = {};
@@ -282,6 +284,7 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
         if (kind == K_QKV) {
             g.bias = f16(d.qkvb, (size_t)l * 3 * D); g.of = (float*)u(p.o.q); g.rowoff = (const long long*)u(p.o.rowoff);
             g.kc = (u16*)d.keys + (size_t)l * d.tmax * D; g.vc = (u16*)d.vals + (size_t)l * d.tmax * D;
+            if (many) { g.oh = (u16*)u(p.o.q); g.part_stride = (size_t)d.rows * D; g.a2 = pow2 ? 1.0f / d.scale : 1.0f; }
             if (clear) { g.lens = meta + mt.lens; g.seqs = d.prompts; g.seq_stride = (long long)L * d.tmax * D; g.tmax = d.tmax; }
         } else if (kind == K_FC) {
             g.bias = f16(d.fcb, (size_t)l * F); g.oh = (u16*)u(p.o.gelu); g.a2 = 2 * d.gelu_a; g.k1 = d.gelu_b * 2.8853900817779268f; g.k2 = d.gelu_c * g.k1;
@@ -296,13 +299,11 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
         const float* q = (const float*)u(p.o.q);
         const u16 *kc = (const u16*)d.keys + (size_t)l * d.tmax * D, *vc = (const u16*)d.vals + (size_t)l * d.tmax * D;
         const long long ss = (long long)L * d.tmax * D;
-        int e = 0;
-        const int pow2 = frexpf(d.scale, &e) == 0.5f;
         if (many) {
-            AttManyArgs a = {q, (const int4*)(meta + mt.tiles), l, L, D, pow2, d.scale, att, (u32*)d.bar};
-            Config c(dim3(tiles, d.H), 192, st, true);
+            AttManyArgs a = {(const int4*)(meta + mt.tiles), l, L, D, d.scale, att, (u32*)d.bar};
+            Config c(dim3(d.H, tiles), AM_THREADS, st, true);
             c.c.dynamicSmemBytes = AM_SMEM;
-            return pow2 ? cudaLaunchKernelEx(&c.c, pass_attend_many<true>, p.kmap, p.vmap, a) : cudaLaunchKernelEx(&c.c, pass_attend_many<false>, p.kmap, p.vmap, a);
+            return pow2 ? cudaLaunchKernelEx(&c.c, pass_attend_many<true>, p.qmap, p.kmap, p.vmap, a) : cudaLaunchKernelEx(&c.c, pass_attend_many<false>, p.qmap, p.kmap, p.vmap, a);
         }
         AttArgs a = {q, kc, vc, ss, (const int*)d.t, (const int*)0, d.t_stride, d.tmax, D, pow2, p.rp, d.scale, att};
         Config c(dim3(d.H, rows, C), ATT_WARPS * 32, st, true, C);
@@ -366,6 +367,7 @@ int vesta_pass_create(const vesta_pass_desc* d, void* workspace, int graph, void
     if (!e && d->prompts) {
         const unsigned long long D = d->D, planes = (unsigned long long)d->prompts * d->L;
         e = vesta_rt::tensor_map(&p->kmap, d->keys, D, d->tmax, planes, D * 2, D * 2 * d->tmax, 128, 1);
+        if (!e) e = vesta_rt::tensor_map(&p->qmap, p->ws + p->o.q, D, d->rows, 2, D * 2, D * 2 * d->rows, 128, 1);
         if (!e) e = vesta_rt::tensor_map(&p->vmap, d->vals, D, d->tmax, planes, D * 2, D * 2 * d->tmax, 128, 1);
     }
     if (!e && graph) {

@@ -98,15 +98,15 @@ struct GemmArgs {
     int bn, ftiles, rtiles, ntiles;  // rows per tile (a multiple of 16); tiles of features, of rows, in all (with the parts of the fold)
     int D;
     const u16* bias;                 // QKV, FC: of the layer
-    float* of;                       // QKV: queries [row][D]; PART: sums [part][row][nfeat]; ADD: vector added to [row][nfeat]; LOGITS: logits [row][nfeat]
-    size_t part_stride;              // floats between two parts
-    u16* oh;                         // GELU: [row][nfeat], the remainder plane rp rows further
+    float* of;                       // QKV: queries [row][D] (prompts: `oh`); PART: sums [part][row][nfeat]; ADD: vector added to [row][nfeat]; LOGITS: logits [row][nfeat]
+    size_t part_stride;              // floats between two parts; QKV, prompts: from a query's heads to its remainders
+    u16* oh;                         // GELU: [row][nfeat], the remainder plane rp rows further; QKV, prompts: queries times a2, [fp16 head, remainder][row][D]
     u16 *kc, *vc;                    // QKV: the caches at this layer
     const long long* rowoff;         // QKV: element offset of every row's position in the caches (-1: none)
     const int* skip;                 // not zero: the pass was refused, nothing may be written that outlives it
     u64* best;                       // LOGITS: packed (value, ~index) maximum of every row
     u32* status;
-    float a2, k1, k2;                // GELU: see gelu_tanh
+    float a2, k1, k2;                // GELU: see gelu_tanh; QKV, prompts: a2 = 1 / scale where that is a power of two
     // QKV, prompts: one more warp zeroes this layer's cache rows behind the first lens[sequence], which this pass writes
     const int* lens;
     long long seq_stride;
@@ -389,7 +389,16 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS + (EPI == EPI_QKV ? 32 
                 }
                 if (!own) m = 0;
                 if (EPI == EPI_QKV) {
-                    if (part == 0) {
+                    if (part == 0 && g.oh) {
+                        u16* dst = g.oh + (size_t)row * g.D + f;
+#pragma unroll
+                        for (int i = 0; i < CH; i += 2, dst += 2 * g.D) {
+                            const float a = v[i] * g.a2, c = v[i + 1] * g.a2;
+                            const u32 h = pack_h2(a, c), r = pack_h2(a - h_lo(h), c - h_hi(h));
+                            st_u16(dst, (u16)h, i < m); st_u16(dst + g.D, (u16)(h >> 16), i + 1 < m);
+                            st_u16(dst + g.part_stride, (u16)r, i < m); st_u16(dst + g.part_stride + g.D, (u16)(r >> 16), i + 1 < m);
+                        }
+                    } else if (part == 0) {
                         float* dst = g.of + (size_t)row * g.D + f;
 #pragma unroll
                         for (int i = 0; i < CH; i++, dst += g.D) st_f32(dst, v[i], i < m);
@@ -833,9 +842,8 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) pass_attend(const __grid_const
 
 // ---- attention of many positions (prompts) ----------------------------------------------------------------------------
 struct AttManyArgs {
-    const float* q;                  // [row][D] fp32
     const int4* tiles;               // (first row, rows, sequence, first position) of every run of at most 128 rows of one sequence
-    int layer, L, D, pow2;
+    int layer, L, D;
     float scale;
     u16* out;                        // [row][D] fp16
     u32* status;
@@ -858,17 +866,19 @@ __device__ __forceinline__ void tm_st32(u32 addr, const u32 (&r)[32]) {
                     "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]), "r"(addr) : "memory");
 }
 #define AM_STAGES 2
-#define AM_SMEM (32768 + AM_STAGES * 32768 + 128 + 1024)
+#define AM_SMEM (32768 + AM_STAGES * 32768 + 128 + 2048 + 1024)
+#define AM_THREADS 320
 // Block = up to 128 consecutive positions of one sequence x one head; the cache in tiles of 128 positions; causal. On tcgen05:
-// scores = queries (fp16 head and remainder, two products: fp32 accuracy over the fp16 cache) x K rows, 128 x 128 in tensor
-// memory; a thread owns a row: maximum, exponentials and sum without exchange; the weights go back into the columns of the
+// scores = queries (fp16 head and remainder from the QKV contraction, two products: fp32 accuracy over the fp16 cache) x K rows, 128 x 128 in tensor
+// memory; two threads own a row, 32 columns in turn, and exchange its maximum; the weights go back into the columns of the
 // scores as fp16 head and remainder (operand A of the second product, in tensor memory) x V rows (N-major as they lie in the
 // cache). The output is rescaled only when a row's maximum has grown by more than 5.5 (the weights stay below 2^8, and the
 // same maximum normalises them at the end). Two blocks per SM: one's exponentials run under the other's products.
-// With mma.sync (64 rows per block, the same two-part operands) the products set the time: 58 us per layer at 9,200 rows of 32
-// prompts of 64 to 512.
+// At 9,200 rows of 32 prompts of 64 to 512 a layer took 58 us with mma.sync (64 rows per block, the same two-part operands;
+// bound by the products), 39 with one thread per row and queries read as fp32, 35 now, of which the products are 9: a block
+// is a chain of load, products, exponentials, products, and two fit an SM. 77 positions: 5.7 -> 4.6 us.
 template <bool POW2>                                    // the divisor of the scores is a power of two: applied to the queries
-__global__ void __launch_bounds__(192, 2) pass_attend_many(const __grid_constant__ CUtensorMap km, const __grid_constant__ CUtensorMap vm, const __grid_constant__ AttManyArgs a) {
+__global__ void __launch_bounds__(AM_THREADS, 2) pass_attend_many(const __grid_constant__ CUtensorMap qm, const __grid_constant__ CUtensorMap km, const __grid_constant__ CUtensorMap vm, const __grid_constant__ AttManyArgs a) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const u32 sq = smem_u32(smem), skv = sq + 32768, bars = skv + AM_STAGES * 32768;
@@ -876,17 +886,19 @@ __global__ void __launch_bounds__(192, 2) pass_attend_many(const __grid_constant
     unsigned char* tail = smem + 32768 + AM_STAGES * 32768 + 32 + AM_STAGES * 16;
     volatile u32* tmem_p = reinterpret_cast<volatile u32*>(tail);
     volatile int* dead = reinterpret_cast<volatile int*>(tail + 4);
+    float* pair = reinterpret_cast<float*>(tail + 16);                             // [tile & 1][half][row]: maxima, at the end sums
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const Wait w{dead, a.status};
     if (threadIdx.x == 0) {
         *dead = 0;
-        mbar_init(qf, 4); mbar_init(sf, 1); mbar_init(pf, 4); mbar_init(of, 1);
+        mbar_init(qf, 1); mbar_init(sf, 1); mbar_init(pf, 8); mbar_init(of, 1);
         for (int i = 0; i < AM_STAGES; i++) { mbar_init(kvf + i * 8, 1); mbar_init(kve + i * 8, 1); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("prefetch.tensormap [%0];" :: "l"(&qm) : "memory");
         asm volatile("prefetch.tensormap [%0];" :: "l"(&km) : "memory");
         asm volatile("prefetch.tensormap [%0];" :: "l"(&vm) : "memory");
     }
-    if (warp == 5) {
+    if (warp == 9) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(tail)), "n"(256) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -895,11 +907,14 @@ __global__ void __launch_bounds__(192, 2) pass_attend_many(const __grid_constant
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (threadIdx.x == 0) dep_launch();
     const u32 tmem = *tmem_p, tO = tmem + 128;                                     // scores / weights: columns 0..127, output: 128..191
-    const int4 tl = __ldg(a.tiles + blockIdx.x);
-    const int h = blockIdx.y, row0 = tl.x, nrows = tl.y, pos0 = tl.w, total = pos0 + nrows, nt = (total + 127) / 128;
-    if (warp == 4) {
+    const int4 tl = __ldg(a.tiles + blockIdx.y);                                   // (runs in the order of their work, all heads of one before the next)
+    const int h = blockIdx.x, row0 = tl.x, nrows = tl.y, pos0 = tl.w, total = pos0 + nrows, nt = (total + 127) / 128;
+    if (warp == 8) {
         if (elect_one()) {
             dep_wait();
+            mbar_expect(qf, 32768);
+            tma3(sq, &qm, h * 64, row0, 0, qf);
+            tma3(sq + 16384, &qm, h * 64, row0, 1, qf);
             for (int j = 0; j < nt; j++) {
                 const int s = j % AM_STAGES;
                 if (j >= AM_STAGES && !mbar_wait(kve + s * 8, (j / AM_STAGES - 1) & 1, w, 0xC00u)) break;
@@ -909,7 +924,7 @@ __global__ void __launch_bounds__(192, 2) pass_attend_many(const __grid_constant
                 tma3(dst + 16384, &vm, h * 64, j * 128, tl.z * a.L + a.layer, kvf + s * 8);
             }
         }
-    } else if (warp == 5) {
+    } else if (warp == 9) {
         constexpr u32 i_s = (1u << 4) | ((128u >> 3) << 17) | ((128u >> 4) << 24), i_o = (1u << 4) | (1u << 16) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
         bool ok = !__any_sync(0xffffffffu, !mbar_wait(qf, 0, w, 0xC10u));
         for (int j = 0; j < nt && ok; j++) {
@@ -946,35 +961,19 @@ __global__ void __launch_bounds__(192, 2) pass_attend_many(const __grid_constant
             __syncwarp();
         }
     } else {
-        const int row = warp * 32 + lane, p = pos0 + row;                          // this thread's row of the tile, its position
-        const u32 mine = (u32)(warp * 32) << 16;
-        dep_wait();
-        {
-            // sixteen lanes read a row's 256 bytes, a warp two rows at a time
-            const float sc = POW2 ? 1.0f / a.scale : 1.0f;
-            const int piece = lane & 15;
-            float4 x[16];
-#pragma unroll
-            for (int i = 0; i < 16; i++) x[i] = __ldcg(reinterpret_cast<const float4*>(a.q + (size_t)(row0 + min(warp * 32 + i * 2 + (lane >> 4), nrows - 1)) * a.D + h * 64) + piece);
-#pragma unroll
-            for (int i = 0; i < 16; i++) {
-                const float4 u = make_float4(x[i].x * sc, x[i].y * sc, x[i].z * sc, x[i].w * sc);
-                const u32 h0 = pack_h2(u.x, u.y), h1 = pack_h2(u.z, u.w), l0 = pack_h2(u.x - h_lo(h0), u.y - h_hi(h0)), l1 = pack_h2(u.z - h_lo(h1), u.w - h_hi(h1));
-                const u32 at = sq + kv_off(warp * 32 + i * 2 + (lane >> 4), piece >> 1) + (piece & 1) * 8;
-                asm volatile("st.shared.v2.u32 [%0], {%1,%2};" :: "r"(at), "r"(h0), "r"(h1) : "memory");
-                asm volatile("st.shared.v2.u32 [%0], {%1,%2};" :: "r"(at + 16384), "r"(l0), "r"(l1) : "memory");
-            }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(qf) : "memory");
-        }
+        const int quad = warp & 3, half = warp >> 2;                               // two threads per row: 32 columns of the scores in turn
+        const int row = quad * 32 + lane, p = pos0 + row;                          // this thread's row of the tile, its position
+        const u32 mine = (u32)(quad * 32) << 16;
         constexpr float LOG2E = 1.4426950408889634f;
         float m = -3.0e38f, den = 0.f;
         bool ok = true;
 #pragma unroll 1
         for (int j = 0; j < nt; j++) {
-            ok = !__any_sync(0xffffffffu, !mbar_wait(sf, j & 1, w, 0xC40u));
-            if (!ok) break;
+            if (ok) ok = !__any_sync(0xffffffffu, !mbar_wait(sf, j & 1, w, 0xC40u));
+            if (!ok) {                                                             // (the other warp of these rows may not have given up)
+                asm volatile("bar.sync %0, 64;" :: "r"(1 + quad) : "memory");
+                continue;
+            }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int lim = p - j * 128;                                           // last column of the tile that this row sees
             const int chunks = min(4, (total - j * 128 + 31) / 32);                // chunks of 32 columns that the second product reads,
@@ -993,25 +992,25 @@ __global__ void __launch_bounds__(192, 2) pass_attend_many(const __grid_constant
                     top[i & 3] = fmaxf(top[i & 3], s);
                 }
             };
-            int c = 0;
+            int c = half;
 #pragma unroll 1
-            for (; c < whole; c++) maxima(Int<0>{}, c);
+            for (; c < whole; c += 2) maxima(Int<0>{}, c);
 #pragma unroll 1
-            for (; c < seen; c++) maxima(Int<1>{}, c);
-            const float mx = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3]));
+            for (; c < seen; c += 2) maxima(Int<1>{}, c);
+            float mx = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3]));
+            pair[(j & 1) * 256 + half * 128 + row] = mx;
+            asm volatile("bar.sync %0, 64;" :: "r"(1 + quad) : "memory");
+            mx = fmaxf(mx, pair[(j & 1) * 256 + (half ^ 1) * 128 + row]);
             const bool grow = mx > m + 5.5f;
             if (__any_sync(0xffffffffu, grow)) {
                 const float corr = grow ? fast_exp(m - mx) : 1.0f;
                 if (grow) m = mx;
                 den *= corr;
                 if (j > 0) {                                                       // (the products into the output have completed: the scores' came after them)
-#pragma unroll 1
-                    for (c = 0; c < 2; c++) {
-                        tm_ld32(r, tO + mine + c * 32);
+                    tm_ld32(r, tO + mine + half * 32);
 #pragma unroll
-                        for (int i = 0; i < 32; i++) r[i] = __float_as_uint(__uint_as_float(r[i]) * corr);
-                        tm_st32(tO + mine + c * 32, r);
-                    }
+                    for (int i = 0; i < 32; i++) r[i] = __float_as_uint(__uint_as_float(r[i]) * corr);
+                    tm_st32(tO + mine + half * 32, r);
                 }
             }
             const float m2 = m * LOG2E;
@@ -1037,11 +1036,11 @@ __global__ void __launch_bounds__(192, 2) pass_attend_many(const __grid_constant
                 tm_st32(tmem + mine + c * 32, o);
             };
 #pragma unroll 1
-            for (c = 0; c < whole; c++) weights(Int<0>{}, c);
+            for (c = half; c < whole; c += 2) weights(Int<0>{}, c);
 #pragma unroll 1
-            for (; c < seen; c++) weights(Int<1>{}, c);
+            for (; c < seen; c += 2) weights(Int<1>{}, c);
 #pragma unroll 1
-            for (; c < chunks; c++) {
+            for (; c < chunks; c += 2) {
 #pragma unroll
                 for (int i = 0; i < 32; i++) r[i] = 0u;
                 tm_st32(tmem + mine + c * 32, r);
@@ -1052,26 +1051,28 @@ __global__ void __launch_bounds__(192, 2) pass_attend_many(const __grid_constant
             if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(pf) : "memory");
         }
         if (ok) ok = !__any_sync(0xffffffffu, !mbar_wait(of, 0, w, 0xC50u));
-        if (ok) {
+        if (!ok) asm volatile("bar.sync %0, 64;" :: "r"(1 + quad) : "memory");
+        else {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            // (every row has waited for the last products, which came after all reads of the maxima)
+            pair[half * 128 + row] = den;
+            asm volatile("bar.sync %0, 64;" :: "r"(1 + quad) : "memory");
+            den += pair[(half ^ 1) * 128 + row];
             const float inv = den > 0.f ? __fdividef(1.0f, den) : 0.f;
-            uint4* out = reinterpret_cast<uint4*>(a.out + (size_t)(row0 + row) * a.D + h * 64);
+            uint4* out = reinterpret_cast<uint4*>(a.out + (size_t)(row0 + row) * a.D + h * 64 + half * 32);
+            u32 r[32];
+            tm_ld32(r, tO + mine + half * 32);
+            if (row < nrows)
 #pragma unroll
-            for (int c = 0; c < 2; c++) {
-                u32 r[32];
-                tm_ld32(r, tO + mine + c * 32);
-                if (row < nrows)
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        const float* v = reinterpret_cast<const float*>(r) + i * 8;
-                        out[c * 4 + i] = make_uint4(pack_h2(v[0] * inv, v[1] * inv), pack_h2(v[2] * inv, v[3] * inv), pack_h2(v[4] * inv, v[5] * inv), pack_h2(v[6] * inv, v[7] * inv));
-                    }
-            }
+                for (int i = 0; i < 4; i++) {
+                    const float* v = reinterpret_cast<const float*>(r) + i * 8;
+                    out[i] = make_uint4(pack_h2(v[0] * inv, v[1] * inv), pack_h2(v[2] * inv, v[3] * inv), pack_h2(v[4] * inv, v[5] * inv), pack_h2(v[6] * inv, v[7] * inv));
+                }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         }
     }
     __syncthreads();
-    if (warp == 5) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "n"(256) : "memory");
+    if (warp == 9) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "n"(256) : "memory");
     if (*dead && threadIdx.x == 0) {
         const u64 t0 = now_ns();
         while (now_ns() - t0 < 2000000ull) { }

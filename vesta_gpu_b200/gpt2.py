@@ -126,18 +126,22 @@ class VestaGPT2:
         B, P = tokens.shape
         if B != self.B:
             raise ValueError('prefill needs one prompt per sequence of the batch')
-        lens = np.full(B, P, np.int32) if lengths is None else np.ascontiguousarray(lengths, np.int32)
-        if lens.min() < 1 or lens.max() > P or lens.max() > self.tmax:
+        if lengths is None:
+            lens, low, high, total = np.full(B, P, np.int32), P, P, B * P
+        else:
+            lens = np.ascontiguousarray(lengths, np.int32)
+            if lens.shape != (B,):
+                raise ValueError('one prompt length per sequence')
+            low, high, total = int(lens.min()), int(lens.max()), int(lens.sum())
+        if low < 1 or high > P or high > self.tmax:
             raise ValueError('prompt lengths must lie in 1..P and fit the cache')
-        if self.t.numel() == 1 and lens.min() != lens.max():
+        if self.t.numel() == 1 and low != high:
             raise ValueError('prompts of different lengths need per_sequence_t=True')
-        total = int(lens.sum())
         rows = int(rows or next((r for r in PREFILL_ROWS if total <= r), PREFILL_ROWS[-1]))
         eng = self._prefill_engines.get(rows)
         if eng is None:
             eng = self._prefill_engines[rows] = PromptPass(self, rows)
-        with torch.cuda.device(self.device):
-            eng.run(tokens, lens)
+        eng.run(tokens, lens)
         if hasattr(self, 'prompt'):
             buf = np.zeros(tuple(self.prompt.shape), np.int32)
             w = min(P, buf.shape[1])

@@ -80,6 +80,7 @@ class PromptPass:
                         t_stride=int(model.t.numel() > 1), x=model.x, t=model.t, logits=self.logits, bar=self.bar)
         with torch.cuda.device(dev):
             self.h, self.ws = create(desc, dev)
+        self._prompts = lib().vesta_pass_prompts
         self.low = Lowered(src='', params=[], scratch={}, scratch_floats=0, shared_bytes=0, barriers_per_launch=0, grid=low.grid,
                            plan=[('prompt rows', 'one kernel per norm, contraction and attention of a layer, tcgen05 contractions')],
                            dims=dict(low.dims, B=rows, kernel='pass', tc=True, tcl=True), roles=low.roles)
@@ -87,9 +88,13 @@ class PromptPass:
     def run(self, tokens, lens):
         """tokens (B, P), lens (B,) int32 numpy: the caches, x and t of the model after the prompts"""
         tokens = np.ascontiguousarray(tokens, np.int32)
-        stream = torch.cuda.current_stream(self.model.device).cuda_stream
-        status = ctypes.c_uint()
-        ok(lib().vesta_pass_prompts(self.h, stream, tokens.ctypes.data, tokens.shape[1], lens.ctypes.data, ctypes.byref(status)))
+        dev, status = self.model.device, ctypes.c_uint()
+        at = tokens.__array_interface__['data'][0], tokens.shape[1], lens.__array_interface__['data'][0], ctypes.byref(status)
+        if torch.cuda.current_device() == dev.index:
+            ok(self._prompts(self.h, torch.cuda.current_stream(dev).cuda_stream, *at))
+        else:
+            with torch.cuda.device(dev):
+                ok(self._prompts(self.h, torch.cuda.current_stream(dev).cuda_stream, *at))
         v = status.value
         if v:
             self.bar.zero_()
