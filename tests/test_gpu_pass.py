@@ -1,0 +1,135 @@
+"""Passes as chains of kernels (csrc/pass.cu) at the edges of their tiles and dispatch rules, against the oracle."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import TIGHT, MARGIN
+from test_gpu_parity import model
+
+pytestmark = pytest.mark.gpu
+
+
+def shape(name, **kw):
+    """two or three narrow layers with room for 400 positions"""
+    from vesta_gpu_b200.shapes import Shape
+    return Shape(name, **dict(dict(L=2, D=192, H=3, E=64, F=320, N=333, C=400), **kw))
+
+
+def seeded(m, sh, ctx, seed):
+    """caches of `ctx[b]` positions per sequence -> the oracle's copies"""
+    from vesta_gpu_b200.synth import make_cache
+    out = []
+    m.reset()
+    for b, c in enumerate(ctx):
+        k0, v0 = make_cache(sh, seed + b, int(c))
+        ck, cv = np.zeros((sh.L, m.tmax, sh.H, sh.E), np.float16), np.zeros((sh.L, m.tmax, sh.H, sh.E), np.float16)
+        ck[:, :c] = k0
+        cv[:, :c] = v0
+        out.append((ck, cv))
+        m.keys[b, :, :c].copy_(torch.from_numpy(k0))
+        m.vals[b, :, :c].copy_(torch.from_numpy(v0))
+    return out
+
+
+@pytest.mark.parametrize('batch,kw', [
+    (9, {}), (16, {}), (17, {}),                      # operands at fp32 accuracy up to 16 rows; two blocks per (row, head) in the attention
+    (64, {}), (65, {}),                               # edges of a tile of rows
+    (130, {}),                                        # more (row, head) pairs than blocks in flight: one block each
+    (200, {}),                                        # ... and shallow rings
+    (9, dict(D=320, H=5, F=1296)),                    # folds of five blocks, the last block of the second one ragged
+    (16, dict(D=1216, H=19, F=64)),                   # a fold of 19 blocks, fp16 operands at 16 rows
+    (8, dict(L=1, D=1280, H=20)),                     # 160 (sequence, head) pairs at eight sequences: a chain, not the persistent kernel
+    (5, dict(L=1, D=1344, H=21)),                     # five sequences of a wide shape: the same
+])
+def test_step_as_a_chain(batch, kw):
+    """ragged decode steps over seeded caches, contexts from none to nearly all of the cache"""
+    from oracle import gpt2_numpy as O
+    sh, steps = shape('chain', **kw), 2
+    m, hf = model(sh, 17, 'rich', batch, sh.C, per_sequence_t=True)
+    assert m.low.dims['chain']
+    W = O.upcast(hf.weights)
+    ctx = np.array([(37 * b) % 390 for b in range(batch)], np.int32)
+    ctx[:4] = (389, 0, 63, 64)
+    caches = seeded(m, sh, ctx, 900)
+    x = np.array([(b * 31 + 5) % sh.N for b in range(batch)], np.int32)
+    m.t.copy_(torch.from_numpy(ctx))
+    m.x.copy_(torch.from_numpy(x))
+    some = sorted(set(range(5)) | set(range(5, batch, max(1, batch // 12))) | {batch - 1})
+    for s in range(steps):
+        m.step()
+        lg, nx = m.logits().cpu().numpy(), m.x.cpu().numpy()
+        for b in some:
+            ref, rn = O.step(sh, W, *caches[b], int(x[b]), int(ctx[b]) + s)
+            assert np.abs(lg[b] - ref).max() < TIGHT * (1 if batch <= 16 and sh.D <= 1024 or batch <= 8 else 2), (s, b)
+            if O.margin(ref) > MARGIN:
+                assert int(nx[b]) == rn
+        x = nx
+    for b in some:
+        c = int(ctx[b])
+        assert np.abs(m.keys[b, :, c:c + steps].float().cpu().numpy() - caches[b][0][:, c:c + steps].astype(np.float32)).max() <= 4e-3
+    m.k.check()
+
+
+def test_refused_step_stays_refused():
+    """a position outside the cache, then the abort flag alone: nothing is published, later steps are refused until the status is cleared"""
+    sh = shape('refused')
+    m, _ = model(sh, 3, 'rich', 12, 100, per_sequence_t=True)
+    for spoil in (lambda: m.t.fill_(100), lambda: m.k.bar[2].fill_(1)):
+        m.reset()
+        m.t.fill_(7)
+        spoil()
+        m.step(2)
+        m.t.fill_(7)
+        m.x.fill_(1)
+        keys = m.keys.clone()
+        m.step(2)
+        assert (m.t == 7).all() and (m.x == 1).all() and torch.equal(keys, m.keys)
+        with pytest.raises(RuntimeError):
+            m.k.check()
+        m.k.clear_status()
+        m.step(2)
+        m.k.check()
+        assert (m.t == 9).all()
+
+
+@pytest.mark.parametrize('lens,rows,kw,divisor', [
+    ((127, 128, 129, 1, 255, 257, 16, 384), None, {}, 8),       # edges of the attention's runs
+    ((127, 128, 129, 1, 255, 257, 16, 384), 256, {}, 8),        # prompts that several passes read
+    ((77,), None, dict(D=320, H=5, F=1296), 8),                 # one prompt, folds of five blocks, a ragged one behind
+    ((200, 131), None, {}, 7),                                  # scores divided by what is not a power of two
+    (tuple(range(60, 380, 10)), None, dict(D=768, H=12, F=832), 8),   # 6,880 rows: norms by warps, pairs of blocks, several tiles per block
+])
+def test_prompts_as_a_pass(lens, rows, kw, divisor, tmp_path):
+    """first token, keys and values of every prompt position and zeros behind them"""
+    from oracle import gpt2_numpy as O
+    from vesta_gpu_b200.program_text import decode_program
+    sh, batch, lens = shape('prompts', **kw), len(lens), np.array(lens, np.int32)
+    more = {}
+    if divisor != 8:
+        text = decode_program(sh)
+        assert text.count('/ 8\n') == 1
+        (tmp_path / 'p.vst').write_text(text.replace('/ 8\n', f'/ {divisor}\n'))
+        more = dict(program=str(tmp_path / 'p.vst'))
+    m, hf = model(sh, 23, 'rich', batch, sh.C, per_sequence_t=True, **more)
+    W = O.upcast(hf.weights)
+    toks = np.random.RandomState(5).randint(0, sh.N, (batch, int(lens.max()))).astype(np.int32)
+    m.keys.fill_(1.0)
+    m.vals.fill_(1.0)
+    m.prefill(toks, lens, rows=rows)
+    assert m.t.cpu().numpy().tolist() == lens.tolist()
+    for i in range(batch):
+        assert not m.keys[i, :, lens[i]:].any() and not m.vals[i, :, lens[i]:].any()
+    first = m.x.cpu().numpy()
+    ref_w = dict(W)
+    if divisor != 8:                                            # the oracle divides by 8
+        ref_w['qkvw'], ref_w['qkvb'] = W['qkvw'].copy(), W['qkvb'].copy()
+        ref_w['qkvw'][:, :, :sh.D] *= np.float32(8 / divisor)
+        ref_w['qkvb'][:, :sh.D] *= np.float32(8 / divisor)
+    for i in range(batch) if batch <= 8 else (0, 17, batch - 1):
+        ck, cv = O.new_cache(sh, int(lens[i]))
+        for p in range(int(lens[i])):
+            lg, nx = O.step(sh, ref_w, ck, cv, int(toks[i, p]), p)
+        for got, ref in ((m.keys, ck), (m.vals, cv)):
+            assert np.abs(got[i, :, :lens[i]].float().cpu().numpy() - ref.astype(np.float32)).max() <= 4e-3, i
+        if O.margin(lg) > MARGIN:
+            assert int(first[i]) == nx

@@ -53,7 +53,7 @@ struct Pass {
     CUtensorMap qmap, kmap, vmap;              // prompts: queries (two planes) and the caches, 128 rows of one head per box
     size_t part_rows;                          // rows of the parts buffer
     std::vector<cudaGraphExec_t> graphs;       // decode: one step
-    int sms;
+    int sms, dev;
     int* host;                                 // prompts: pinned metadata, one copy per pass of a call, then a status word
     size_t host_words;
 };
@@ -137,9 +137,9 @@ int plan(Pass& p, const vesta_pass_desc* d) {
     if (d->L < 1 || d->D % 64 || d->D > 4096 || d->H * 64 != d->D || d->F % 16 || d->N < 1) return fail(-1, "vesta_pass: sizes outside the supported family");
     if (d->exact && d->rows > 16) return fail(-1, "vesta_pass: fp32-accurate operands are kept for at most 16 rows");
     p.d = *d;
-    int dev = 0;
+    p.dev = 0;
     p.sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&p.sms, cudaDevAttrMultiProcessorCount, dev);
+    if (cudaGetDevice(&p.dev) == cudaSuccess) cudaDeviceGetAttribute(&p.sms, cudaDevAttrMultiProcessorCount, p.dev);
     cudaGetLastError();                          // (sizes can be asked for without a device)
     p.rp = plane_rows(d->rows, d->exact != 0);
     p.planes = p.rp ? 2 * p.rp : up(d->rows, 128);
@@ -323,7 +323,7 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
     }
     if (lrows) TRY(mul(K_LOGITS, 0));
     FinishArgs f = {};
-    f.rows = lrows; f.best = (u64*)u(p.o.best); f.skip = (int*)u(p.o.skip); f.next = (float*)d.next; f.pos = (const int*)u(p.o.pos);
+    f.rows = lrows; f.best = (u64*)u(p.o.best); f.skip = (int*)u(p.o.skip); f.bar = (const u32*)d.bar; f.next = (float*)d.next; f.pos = (const int*)u(p.o.pos);
     f.t_stride = d.t_stride; f.tstep = d.tstep; f.N = d.N;
     if (many) { f.dst = (const int2*)(meta + mt.dst); f.x = (int*)d.x; f.t = (int*)d.t; }
     else if (d.feedback) { f.x = (int*)d.x; f.t = (int*)d.t; f.prompt = (const int*)d.prompt; f.plen = (const int*)d.plen; f.plen_cap = d.prompt_len; }
@@ -335,8 +335,17 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
 }  // namespace
 
 namespace vesta_rt {
+namespace {
+// the device of a pass for the calls of a scope (launches go to a stream of the current device)
+struct OnDevice {
+    int was = 0, dev;
+    explicit OnDevice(int d) : dev(d) { if (cudaGetDevice(&was) == cudaSuccess && was != dev) cudaSetDevice(dev); }
+    ~OnDevice() { if (was != dev) cudaSetDevice(was); }
+};
+}
 int pass_steps(void* pass, void* stream, int steps) {
     Pass* p = (Pass*)pass;
+    const OnDevice on(p->dev);
     cudaStream_t st = (cudaStream_t)stream;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     TRY(cudaStreamIsCapturing(st, &cap));

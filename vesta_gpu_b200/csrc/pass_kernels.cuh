@@ -71,8 +71,8 @@ __device__ __forceinline__ u32 elect_one() {
     return leader;
 }
 
-// Every wait gives up after half a second: it leaves a code in the status word and a flag that ends the block's other
-// waits, and the block runs to its end.
+// Every wait gives up after half a second: it leaves a code in the status word, a flag that ends the block's other waits (the
+// block runs to its end) and the abort flag: this pass publishes no token or position, and every later one is refused.
 #define PASS_WAIT_NS 500000000ull
 struct Wait { volatile int* dead; u32* status; };
 __device__ __noinline__ bool mbar_wait_slow(u32 bar, u32 parity, const Wait& w, u32 code) {
@@ -82,6 +82,7 @@ __device__ __noinline__ bool mbar_wait_slow(u32 bar, u32 parity, const Wait& w, 
         if (*w.dead) return false;
         if ((++spins & 63u) == 0 && now_ns() - t0 > PASS_WAIT_NS) {
             atomicCAS(w.status, 0u, code | (blockIdx.x << 16));
+            atomicExch(w.status + 2, 1u);
             *w.dead = 1;
             return false;
         }
@@ -539,7 +540,7 @@ __global__ void __launch_bounds__(1024) pass_norm(const __grid_constant__ NormAr
         const bool aborted = __ldcg(a.bar + 2) != 0u;
         const bool bad = t >= a.tmax || t >= a.cpos || x < 0 || x >= a.N || aborted;
         if (tid == 0) {
-            if (bad) { atomicExch(a.skip, 1); atomicCAS(a.bar, 0u, 0x900u); }
+            if (bad) { atomicExch(a.skip, 1); atomicCAS(a.bar, 0u, 0x900u); atomicExch(a.bar + 2, 1u); }
             a.rowoff[row] = (bad || t < 0) ? -1ll : ((long long)sq * a.L * a.tmax + t) * a.D;
             a.pos[row] = bad ? -1 : t;
         }
@@ -1084,6 +1085,7 @@ struct FinishArgs {
     int rows;
     u64* best;
     int* skip;
+    const u32* bar;                  // [2] abort flag
     float* next;                     // decode: the chosen tokens as float (0: none)
     const int* pos;
     int *x, *t;                      // fed back (0: no feedback)
@@ -1094,7 +1096,7 @@ struct FinishArgs {
 };
 __global__ void __launch_bounds__(256) pass_finish(const __grid_constant__ FinishArgs a) {
     dep_wait();
-    const bool skip = __ldcg(a.skip) != 0;
+    const bool skip = __ldcg(a.skip) != 0 || __ldcg(a.bar + 2) != 0u;
     for (int b = threadIdx.x; b < a.rows; b += blockDim.x) {
         const u64 k = __ldcg(a.best + b);
         a.best[b] = 0ull;
