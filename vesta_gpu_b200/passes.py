@@ -1,6 +1,7 @@
 """Forward passes as chains of kernels (csrc/pass.cu, csrc/pass_kernels.cuh): the descriptor of a pass and the dense prompt
 pass behind VestaGPT2.prefill."""
 import ctypes
+import weakref
 
 import numpy as np
 import torch
@@ -71,7 +72,7 @@ class PromptPass:
     def __init__(self, model, rows):
         dev, low = model.device, model.low
         lrows = min(rows, model.B)
-        self.model, self.R = model, rows
+        self.model, self.R = weakref.proxy(model), rows          # (the model owns the pass: no cycle, its memory is free when it goes)
         self.logits = torch.empty(lrows, low.dims['N'], dtype=torch.float32, device=dev)
         self.bar = torch.zeros(32, dtype=torch.int32, device=dev)
         self.zeros = torch.zeros(low.dims['zeros_len'], dtype=torch.float16, device=dev)
