@@ -730,8 +730,8 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) pass_attend(const __grid_const
         float2 x[4][2];
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            x[k][0] = g < 2 ? __ldcg(reinterpret_cast<const float2*>(qp + k * 16 + 2 * t4)) : make_float2(0.f, 0.f);
-            x[k][1] = g < 2 ? __ldcg(reinterpret_cast<const float2*>(qp + k * 16 + 2 * t4 + 8)) : make_float2(0.f, 0.f);
+            x[k][0] = __ldcg(reinterpret_cast<const float2*>(qp + k * 16 + 2 * t4));
+            x[k][1] = __ldcg(reinterpret_cast<const float2*>(qp + k * 16 + 2 * t4 + 8));
         }
         // the current position, if it is in one of the runs requested above
         u32 at = 0;
@@ -753,7 +753,7 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) pass_attend(const __grid_const
             for (int i = 0; i < 2; i++) {
                 const float u = x[k][i].x * sc, v = x[k][i].y * sc;
                 const u32 hi = pack_h2(u, v);
-                bq[k][i] = g == 0 ? hi : g == 1 ? pack_h2(u - h_lo(hi), v - h_hi(hi)) : 0u;
+                bq[k][i] = g & 1 ? pack_h2(u - h_lo(hi), v - h_hi(hi)) : hi;   // (every pair of columns alike: all lanes get scores)
             }
     }
     float m = -3.0e38f, den = 0.f, o[4][4];              // o[mt]: dims mt*16 + g (regs 0 + 1) and mt*16 + g + 8 (regs 2 + 3), lanes with t4 == 0
@@ -774,13 +774,14 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) pass_attend(const __grid_const
             ldsm4(r, (ka & ~127u) + so + (((k * 2 + kx) ^ k7) << 4));
             mma16816(s, r, bq[k][0], bq[k][1]);
         }
-        float s0 = s[0] + s[1], s1 = s[2] + s[3];        // positions p0 + g and p0 + g + 8, in the lanes with t4 == 0
+        float s0 = s[0] + s[1], s1 = s[2] + s[3];        // positions p0 + g and p0 + g + 8
         if (!a.pow2) { s0 /= a.scale; s1 /= a.scale; }
-        if (t4 != 0 || p0 + g >= n) s0 = -3.0e38f;
-        if (t4 != 0 || p0 + g + 8 >= n) s1 = -3.0e38f;
-        int km = __float_as_int(fmaxf(s0, s1));
-        km = __reduce_max_sync(0xffffffffu, km >= 0 ? km : km ^ 0x7fffffff);
-        const float mx = __int_as_float(km >= 0 ? km : km ^ 0x7fffffff);
+        if (p0 + g >= n) s0 = -3.0e38f;
+        if (p0 + g + 8 >= n) s1 = -3.0e38f;
+        // (shuffles over the eight groups: redux took longer, 16 sequences of the XL shape 1,359 -> 1,344 us per step)
+        float mx = fmaxf(s0, s1);
+#pragma unroll
+        for (int x = 4; x < 32; x <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, x));
         if (mx > m) {                                    // (the same in the whole warp)
             const float corr = fast_exp(m - mx);
             m = mx;
@@ -809,7 +810,7 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) pass_attend(const __grid_const
         if (++st == NS) st = 0;
     }
 #pragma unroll
-    for (int x = 16; x; x >>= 1) den += __shfl_xor_sync(0xffffffffu, den, x);
+    for (int x = 16; x > 2; x >>= 1) den += __shfl_xor_sync(0xffffffffu, den, x);
     if (t4 == 0)
 #pragma unroll
         for (int i = 0; i < 4; i++) { part[warp][i * 16 + g] = o[i][0] + o[i][1]; part[warp][i * 16 + g + 8] = o[i][2] + o[i][3]; }
