@@ -680,7 +680,7 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const u32 (&a)[4], u32 b
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// Block = one (row, head), or 1 / C of its positions where C blocks form a cluster; warps take runs of 16 positions in
+// Block = one (row, head), or half its positions where two blocks form a cluster (C = 2); warps take runs of 16 positions in
 // turn, on mma.sync: scores = K rows (16 positions x 16 dims per step) times the query, its fp16 head in column 0 and its fp16
 // remainder in column 1 (their sum is the fp32-accurate product); output = V transposed times the weights, head and remainder
 // again in two columns. The same in fp32 on the ordinary cores took 14 instructions per position and head, most of them
@@ -699,6 +699,7 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) pass_attend(const __grid_const
     const int h = blockIdx.x, row = blockIdx.y, C = gridDim.z, cr = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, pl = lane >> 3, dl = lane & 7, g = lane >> 2, t4 = lane & 3;
     if (threadIdx.x == 0) dep_launch();
+    if (C == 2) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // (waited for before the other block's memory is written)
     const int n = min(__ldcg(a.t + row * a.t_stride) + 1, a.tmax), sq = a.seq ? __ldcg(a.seq + row) : row;
     const u16* kp = a.kc + sq * a.seq_stride + h * 64 + dl * 8;
     const u16* vp = a.vc + sq * a.seq_stride + h * 64 + dl * 8;
@@ -823,32 +824,21 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) pass_attend(const __grid_const
 #pragma unroll
         for (int i = 0; i < ATT_WARPS; i++) { const float c = fast_exp(part[i][64] - M); dd += part[i][65] * c; num += part[i][threadIdx.x] * c; }
     }
-    if (C > 1) {
-        // the blocks of a cluster: their results meet in the first one
-        if (threadIdx.x < 64) { part[ATT_WARPS][threadIdx.x] = num; if (threadIdx.x == 0) { part[ATT_WARPS][64] = M; part[ATT_WARPS][65] = dd; } }
-        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-        if (cr == 0 && threadIdx.x < 64) {
-            float mm[8], de[8], nu[8];
-            const u32 mine = smem_u32(&part[ATT_WARPS][0]);
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                mm[i] = -3.0e38f; de[i] = 0.f; nu[i] = 0.f;
-                if (i < C) {
-                    u32 r;
-                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(mine), "r"(i));
-                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(mm[i]) : "r"(r + 64 * 4) : "memory");
-                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(de[i]) : "r"(r + 65 * 4) : "memory");
-                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(nu[i]) : "r"(r + threadIdx.x * 4) : "memory");
-                }
-            }
-            M = -3.0e38f; dd = 0.f; num = 0.f;
-#pragma unroll
-            for (int i = 0; i < 8; i++) M = fmaxf(M, mm[i]);
-#pragma unroll
-            for (int i = 0; i < 8; i++) { const float c = fast_exp(mm[i] - M); dd += de[i] * c; num += nu[i] * c; }
+    if (C == 2) {
+        // the second block's result goes into the first one's shared memory
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (cr == 1 && threadIdx.x < 64) {
+            const u32 to = of_first(smem_u32(&part[ATT_WARPS][0]));
+            asm volatile("st.shared::cluster.f32 [%0], %1;" :: "r"(to + threadIdx.x * 4), "f"(num) : "memory");
+            if (threadIdx.x == 0) asm volatile("st.shared::cluster.f32 [%0], %1;\n\tst.shared::cluster.f32 [%0+4], %2;" :: "r"(to + 64 * 4), "f"(M), "f"(dd) : "memory");
         }
-        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-        if (cr != 0) return;
+        cluster_sync();
+        if (cr == 1) return;
+        if (threadIdx.x < 64) {
+            const float m1 = part[ATT_WARPS][64], top = fmaxf(M, m1), c0 = fast_exp(M - top), c1 = fast_exp(m1 - top);
+            dd = dd * c0 + part[ATT_WARPS][65] * c1;
+            num = num * c0 + part[ATT_WARPS][threadIdx.x] * c1;
+        }
     }
     if (threadIdx.x < 64) {
         const float r = dd > 0.f ? __fdividef(num, dd) : 0.f;                      // a sequence that has not started attends to nothing
