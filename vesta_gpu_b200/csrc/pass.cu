@@ -25,7 +25,7 @@ enum Kind { K_QKV = 0, K_PROJ = 1, K_FC = 2, K_P2 = 3, K_LOGITS = 4 };
 struct Tile { int bm, bn, stages, splits; };
 
 struct Layout {
-    size_t z, q, act, att, gelu, part, fin, best, rowoff, pos, skip;
+    size_t z, q, act, att, gelu, fin, best, rowoff, pos, skip;
     size_t meta, total;                        // prompts: tokens, positions, sequences of the rows; attention runs; rows that want logits and where they go; lengths
 };
 // the metadata of a pass over prompts, as offsets in 32-bit words
@@ -51,7 +51,6 @@ struct Pass {
     };
     std::vector<Plan> plans;                   // the last few
     CUtensorMap qmap, kmap, vmap;              // prompts: queries (two planes) and the caches, 128 rows of one head per box
-    size_t part_rows;                          // rows of the parts buffer
     std::vector<cudaGraphExec_t> graphs;       // decode: one step
     int sms, dev;
     int* host;                                 // prompts: pinned metadata, one copy per pass of a call, then a status word
@@ -70,8 +69,8 @@ int plane_rows(int rows, bool exact) { return !exact ? 0 : rows <= 8 ? 8 : 16; }
 //     (L2 into the SMs, the slower the more SMs take part); with several tiles per block, each but the last costs the larger
 //     of that and its epilogue;
 //   BM = 256 (two blocks): 3.0, and a third less for the loads: better for folds of more than about 1,000.
-// A cut fold (projections) costs its parts once more in the norm that adds them.
-Tile choose(int kind, int rows, int rp, int feat, int kb, int sms, int max_parts = PARTS_MAX) {
+// A cut fold (projections) costs one more reduction per element and part: hidden by the chain up to about 0.5 MB of sums.
+Tile choose(int kind, int rows, int rp, int feat, int kb, int sms) {
     Tile best = {};
     double best_t = 1e30;
     const int cols = rp ? 2 * rp : rows;
@@ -87,7 +86,7 @@ Tile choose(int kind, int rows, int rp, int feat, int kb, int sms, int max_parts
             const int tiles = ((feat + bm - 1) / bm) * (rp ? 1 : (rows + bn - 1) / bn);
             const int units = bm == 256 ? sms / 2 : sms;
             const double epi = kind == K_FC || kind == K_LOGITS ? 0.016 * bn + 1.2 : kind == K_QKV ? 0.010 * bn + 2.0 : 0.0145 * bn + 1.7;
-            for (int sp = 1; sp <= (cut ? max_parts : 1); sp++) {
+            for (int sp = 1; sp <= (cut ? PARTS_MAX : 1); sp++) {
                 Tile t;
                 t.bm = bm; t.bn = bn;
                 const int per = (kb + sp - 1) / sp, nst = (per + ks - 1) / ks;
@@ -103,7 +102,10 @@ Tile choose(int kind, int rows, int rp, int feat, int kb, int sms, int max_parts
                     const double main = per * kb_us;
                     us = (bm == 128 ? 2.2 : 3.0) + last * bn + main + (waves - 1) * std::max(main, epi);
                 }
-                if (cut && sp > 1) us += 0.1 * sp + (sp - 1) * (double)rows * feat * 4 / 4e6;
+                if (cut) {
+                    const double mb = rows * (double)feat * 4e-6;
+                    us += (sp - 1) * (mb < 0.5 ? 0.125 * mb : 0.13 + 0.1 * mb);
+                }
                 if (us < best_t) { best_t = us; best = t; }
             }
         }
@@ -121,7 +123,6 @@ Layout layout(const Pass& p, int D, int F, int rows, int lrows) {
     o.act = take((size_t)p.planes * D * 2);
     o.att = take((size_t)p.planes * D * 2);
     o.gelu = take((size_t)p.planes * F * 2 + 128);       // (the last block of the fold may reach past the last row)
-    o.part = take(p.part_rows * D * 4);
     o.fin = take((size_t)p.fplanes * D * 2);
     o.best = take((size_t)lrows * 8);
     o.rowoff = take((size_t)rows * 8);
@@ -144,11 +145,6 @@ int plan(Pass& p, const vesta_pass_desc* d) {
     p.rp = plane_rows(d->rows, d->exact != 0);
     p.planes = p.rp ? 2 * p.rp : up(d->rows, 128);
     p.fplanes = p.rp ? 2 * p.rp : up(d->logit_rows, 128);
-    // parts of a cut fold: as many rows of them as the choice for some number of rows asks for (prompts: passes of any size)
-    size_t most = 1;
-    for (int r = d->prompts ? 1 : d->rows; r <= d->rows; r = r < 64 ? r + 1 : std::min(r + r / 16, d->rows) + (r == d->rows))
-        for (int k : {K_PROJ, K_P2}) { const Tile t = choose(k, r, p.rp, d->D, k == K_P2 ? (d->F + 63) / 64 : d->D / 64, p.sms); if (t.splits > 1) most = std::max(most, (size_t)t.splits * r); }
-    p.part_rows = most + most / 8;
     p.o = layout(p, d->D, d->F, d->rows, d->logit_rows);
     return 0;
 }
@@ -168,7 +164,7 @@ cudaError_t prepare_gemm() {
     return e != cudaSuccess ? e : cudaFuncSetAttribute(pass_gemm<BM, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
 }
 // one case per tile shape and epilogue
-#define EACH(X) X(256, EPI_ADD) X(256, EPI_QKV) X(256, EPI_PART) X(256, EPI_GELU) X(64, EPI_ADD) X(128, EPI_ADD) X(64, EPI_QKV) X(64, EPI_PART) X(64, EPI_GELU) X(64, EPI_LOGITS) X(128, EPI_QKV) X(128, EPI_PART) X(128, EPI_GELU) X(128, EPI_LOGITS)
+#define EACH(X) X(256, EPI_ADD) X(256, EPI_QKV) X(256, EPI_GELU) X(64, EPI_ADD) X(128, EPI_ADD) X(64, EPI_QKV) X(64, EPI_GELU) X(64, EPI_LOGITS) X(128, EPI_QKV) X(128, EPI_GELU) X(128, EPI_LOGITS)
 cudaError_t gemm(int epi, const Tile& t, cudaLaunchConfig_t c, const CUtensorMap& w, const CUtensorMap& a, const GemmArgs& g) {
 #define ONE(M, E) if (epi == E && t.bm == M) return launch_gemm<M, E>(c, t, w, a, g);
     EACH(ONE)
@@ -194,7 +190,7 @@ cudaError_t prepare_all() {
     one(cudaFuncSetAttribute((const void*)pass_attend<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * ATT_WARPS * 4096)); one(all_shared(pass_finish));
     return e;
 }
-int epi_of(int kind, const Tile& t) { return kind == K_QKV ? EPI_QKV : kind == K_FC ? EPI_GELU : kind == K_LOGITS ? EPI_LOGITS : t.splits > 1 ? EPI_PART : EPI_ADD; }
+int epi_of(int kind) { return kind == K_QKV ? EPI_QKV : kind == K_FC ? EPI_GELU : kind == K_LOGITS ? EPI_LOGITS : EPI_ADD; }
 
 // launch attributes: `dependent` = may start while the kernel before it runs
 struct Config {
@@ -219,7 +215,7 @@ int plan_for(Pass& p, int rows, int lrows, const Pass::Plan** out) {
     const int fold[5] = {D, D, D, F, D}, feat[5] = {3 * D, D, F, D, d.N}, kb[5] = {kbd, kbd, kbd, kbf, kbd};
     const size_t op[5] = {p.o.act, p.o.att, p.o.act, p.o.gelu, p.o.fin};
     for (int k = 0; k < 5; k++) {
-        const Tile t = q.tile[k] = choose(k, k == K_LOGITS ? std::max(lrows, 1) : rows, p.rp, feat[k], kb[k], p.sms, std::max<int>(1, std::min<size_t>(PARTS_MAX, p.part_rows / rows)));
+        const Tile t = q.tile[k] = choose(k, k == K_LOGITS ? std::max(lrows, 1) : rows, p.rp, feat[k], kb[k], p.sms);
         int e;
         if (k == K_LOGITS) e = vesta_rt::fold_map(&q.w[k], w[k], D, feat[k], t.bm, k_blocks(t.bm));
         else e = vesta_rt::tensor_map(&q.w[k], w[k], feat[k], fold[k], d.L, (size_t)feat[k] * 2, (size_t)feat[k] * fold[k] * 2, 64 * k_blocks(t.bm), 1);
@@ -252,19 +248,18 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
     const Pass::Plan* pl = nullptr;
     if (int e = plan_for(p, rows, lrows, &pl)) return e;
     auto f16 = [](const void* q, size_t off) { return (const u16*)q + off; };
-    auto norm = [&](int mode, int l, int nparts) {
+    auto norm = [&](int mode, int l) {
         NormArgs n = {};
-        n.D = D; n.nparts = nparts; n.rp = p.rp; n.eps = d.eps; n.z = z;
-        n.part = (const float*)u(p.o.part); n.part_stride = (size_t)rows * D;
+        n.D = D; n.rp = p.rp; n.eps = d.eps; n.z = z;
         n.x = many ? meta + mt.x : (const int*)d.x; n.t = many ? meta + mt.t : (const int*)d.t; n.seq = many ? meta + mt.seq : 0; n.t_stride = many ? 1 : d.t_stride; n.N = d.N; n.cpos = d.cpos; n.tmax = d.tmax; n.L = L;
         n.wte = (const u16*)d.wte; n.wpe = (const u16*)d.wpe;
         n.rowoff = (long long*)u(p.o.rowoff); n.pos = (int*)u(p.o.pos); n.skip = (int*)u(p.o.skip); n.bar = (u32*)d.bar;
         n.want = many ? meta + mt.want : 0;
         n.act = act;
         if (mode == 0) { n.gain = f16(d.ln1w, 0); n.shift = f16(d.ln1b, 0); }
-        else if (mode == 1) { n.gain = f16(d.ln2w, (size_t)l * D); n.shift = f16(d.ln2b, (size_t)l * D); n.bias = f16(d.ob, (size_t)l * D); }
-        else if (mode == 2) { n.gain = f16(d.ln1w, (size_t)(l + 1) * D); n.shift = f16(d.ln1b, (size_t)(l + 1) * D); n.bias = f16(d.pb, (size_t)l * D); }
-        else { n.gain = f16(d.lnfw, 0); n.shift = f16(d.lnfb, 0); n.bias = f16(d.pb, (size_t)l * D); n.act = fin; }
+        else if (mode == 1) { n.gain = f16(d.ln2w, (size_t)l * D); n.shift = f16(d.ln2b, (size_t)l * D); }
+        else if (mode == 2) { n.gain = f16(d.ln1w, (size_t)(l + 1) * D); n.shift = f16(d.ln1b, (size_t)(l + 1) * D); }
+        else { n.gain = f16(d.lnfw, 0); n.shift = f16(d.lnfb, 0); n.act = fin; }
         if ((mode == 1 || mode == 2) && rows >= 2048 && D <= 2048 && !p.rp) {
             Config c(dim3((rows + 7) / 8), 256, st, true);
             return D <= 768 ? cudaLaunchKernelEx(&c.c, pass_norm_rows<6>, n, rows) : D <= 1664 ? cudaLaunchKernelEx(&c.c, pass_norm_rows<13>, n, rows) : cudaLaunchKernelEx(&c.c, pass_norm_rows<16>, n, rows);
@@ -284,16 +279,15 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
         if (kind == K_QKV) {
             g.bias = f16(d.qkvb, (size_t)l * 3 * D); g.of = (float*)u(p.o.q); g.rowoff = (const long long*)u(p.o.rowoff);
             g.kc = (u16*)d.keys + (size_t)l * d.tmax * D; g.vc = (u16*)d.vals + (size_t)l * d.tmax * D;
-            if (many) { g.oh = (u16*)u(p.o.q); g.part_stride = (size_t)d.rows * D; g.a2 = pow2 ? 1.0f / d.scale : 1.0f; }
+            if (many) { g.oh = (u16*)u(p.o.q); g.low = (size_t)d.rows * D; g.a2 = pow2 ? 1.0f / d.scale : 1.0f; }
             if (clear) { g.lens = meta + mt.lens; g.seqs = d.prompts; g.seq_stride = (long long)L * d.tmax * D; g.tmax = d.tmax; }
         } else if (kind == K_FC) {
             g.bias = f16(d.fcb, (size_t)l * F); g.oh = (u16*)u(p.o.gelu); g.a2 = 2 * d.gelu_a; g.k1 = d.gelu_b * 2.8853900817779268f; g.k2 = d.gelu_c * g.k1;
         } else if (kind == K_LOGITS) { g.of = (float*)d.logits; g.best = (u64*)u(p.o.best); }
-        else if (t.splits > 1) { g.of = (float*)u(p.o.part); g.part_stride = (size_t)rows * D; }
         else { g.of = z; g.bias = kind == K_PROJ ? f16(d.ob, (size_t)l * D) : f16(d.pb, (size_t)l * D); }
         g.bn = t.bn; g.ftiles = (g.nfeat + t.bm - 1) / t.bm; g.rtiles = p.rp ? 1 : (g.rows + t.bn - 1) / t.bn; g.ntiles = g.ftiles * g.rtiles * t.splits;
         Config c(dim3(t.bm == 64 && kind != K_LOGITS ? g.ntiles : t.bm == 256 ? 2 * std::min(g.ntiles, p.sms / 2) : std::min(g.ntiles, p.sms)), 192, st, true, t.bm == 256 ? 2 : 1, true);
-        return gemm(epi_of(kind, t), t, c.c, pl->w[kind], pl->a[kind], g);
+        return gemm(epi_of(kind), t, c.c, pl->w[kind], pl->a[kind], g);
     };
     auto attend = [&](int l) {
         const float* q = (const float*)u(p.o.q);
@@ -310,16 +304,16 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
         c.c.dynamicSmemBytes = (deep ? 4 : 2) * ATT_WARPS * 4096;
         return deep ? cudaLaunchKernelEx(&c.c, pass_attend<4>, a) : cudaLaunchKernelEx(&c.c, pass_attend<2>, a);
     };
-    TRY(norm(0, 0, 0));
+    TRY(norm(0, 0));
     for (int l = 0; l < L; l++) {
         TRY(mul(K_QKV, l));
         if (l == L - 1 && lrows == 0) break;
         TRY(attend(l));
         TRY(mul(K_PROJ, l));
-        TRY(norm(1, l, pl->tile[K_PROJ].splits > 1 ? pl->tile[K_PROJ].splits : 0));
+        TRY(norm(1, l));
         TRY(mul(K_FC, l));
         TRY(mul(K_P2, l));
-        TRY(norm(l + 1 < L ? 2 : 3, l, pl->tile[K_P2].splits > 1 ? pl->tile[K_P2].splits : 0));
+        TRY(norm(l + 1 < L ? 2 : 3, l));
     }
     if (lrows) TRY(mul(K_LOGITS, 0));
     FinishArgs f = {};

@@ -92,15 +92,15 @@ __device__ __noinline__ bool mbar_wait_slow(u32 bar, u32 parity, const Wait& w, 
 __device__ __forceinline__ bool mbar_wait(u32 bar, u32 parity, const Wait& w, u32 code) { return mbar_try(bar, parity) || mbar_wait_slow(bar, parity, w, code); }
 
 // ---- contractions ---------------------------------------------------------------------------------------------------
-enum { EPI_QKV = 0, EPI_PART = 1, EPI_GELU = 2, EPI_LOGITS = 3, EPI_ADD = 4 };
+enum { EPI_QKV = 0, EPI_ADD = 1, EPI_GELU = 2, EPI_LOGITS = 3 };
 
 struct GemmArgs {
     int layer, nfeat, kblocks, kb_per, rows, rp, stages;
     int bn, ftiles, rtiles, ntiles;  // rows per tile (a multiple of 16); tiles of features, of rows, in all (with the parts of the fold)
     int D;
-    const u16* bias;                 // QKV, FC: of the layer
-    float* of;                       // QKV: queries [row][D] (prompts: `oh`); PART: sums [part][row][nfeat]; ADD: vector added to [row][nfeat]; LOGITS: logits [row][nfeat]
-    size_t part_stride;              // floats between two parts; QKV, prompts: from a query's heads to its remainders
+    const u16* bias;                 // of the layer
+    float* of;                       // QKV: queries [row][D] (prompts: `oh`); ADD: vector added to [row][nfeat]; LOGITS: logits [row][nfeat]
+    size_t low;                      // QKV, prompts: from a query's heads to its remainders
     u16* oh;                         // GELU: [row][nfeat], the remainder plane rp rows further; QKV, prompts: queries times a2, [fp16 head, remainder][row][D]
     u16 *kc, *vc;                    // QKV: the caches at this layer
     const long long* rowoff;         // QKV: element offset of every row's position in the caches (-1: none)
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS + (EPI == EPI_QKV ? 32 
             const int f = f0 + fl;
             const bool own = (AM == 128 || lane < 16) && f < g.nfeat;
             float bias = 0.f;
-            if ((EPI == EPI_QKV || EPI == EPI_GELU || EPI == EPI_ADD) && own) bias = h2f(__ldg(g.bias + f));
+            if ((EPI == EPI_QKV || EPI == EPI_GELU || (EPI == EPI_ADD && z == 0)) && own) bias = h2f(__ldg(g.bias + f));
             if (!waited) {
                 dep_wait();
                 waited = true;
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS + (EPI == EPI_QKV ? 32 
                             const float a = v[i] * g.a2, c = v[i + 1] * g.a2;
                             const u32 h = pack_h2(a, c), r = pack_h2(a - h_lo(h), c - h_hi(h));
                             st_u16(dst, (u16)h, i < m); st_u16(dst + g.D, (u16)(h >> 16), i + 1 < m);
-                            st_u16(dst + g.part_stride, (u16)r, i < m); st_u16(dst + g.part_stride + g.D, (u16)(r >> 16), i + 1 < m);
+                            st_u16(dst + g.low, (u16)r, i < m); st_u16(dst + g.low + g.D, (u16)(r >> 16), i + 1 < m);
                         }
                     } else if (part == 0) {
                         float* dst = g.of + (size_t)row * g.D + f;
@@ -412,13 +412,10 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS + (EPI == EPI_QKV ? 32 
                             st_u16(cache + o.y, (u16)(h >> 16), i + 1 < m && o.y >= 0);
                         }
                     }
-                } else if (EPI == EPI_PART) {
-                    float* dst = g.of + z * g.part_stride + (size_t)row * g.nfeat + f;
-#pragma unroll
-                    for (int i = 0; i < CH; i++, dst += g.nfeat) st_f32(dst, v[i], i < m);
                 } else if (EPI == EPI_ADD) {
-                    // (one addition per element: the order of blocks does not matter. Reading, adding and storing waited for L2
-                    // chunk by chunk: 15 us at 9,216 rows x 768 x 768)
+                    // (Reading, adding and storing waited for L2 chunk by chunk: 15 us at 9,216 rows x 768 x 768. Parts of a cut fold
+                    // add here too: stored one by one and added by the norm behind they cost every pass more, 256 sequences
+                    // 801 -> 762 us per step, 16 of the XL shape 1,344 -> 1,268, 8 x 128 prompts 618 -> 587)
                     float* dst = g.of + (size_t)row * g.nfeat + f;
 #pragma unroll
                     for (int i = 0; i < CH; i++, dst += g.nfeat) add_f32(dst, v[i], i < m);
@@ -509,15 +506,13 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS + (EPI == EPI_QKV ? 32 
 }
 
 // ---- norm: residual sums, LayerNorm, operand ---------------------------------------------------------------------------
-#define PARTS_MAX 8
+#define PARTS_MAX 12                  // most parts of a cut fold
 enum { NORM_EMBED = 0, NORM_MID = 1, NORM_FINAL = 2 };
 struct NormArgs {
-    int D, nparts, rp;
+    int D, rp;
     float eps;
     float* z;                        // residual stream [row][D], updated in place
-    const float* part;               // [part][row][D]: sums of the projection before this norm (nparts = 0: already in z)
-    size_t part_stride;
-    const u16 *bias, *gain, *shift;
+    const u16 *gain, *shift;
     u16* act;                        // [row][D] fp16 (and the remainder plane rp rows further)
     // EMBED: tokens and positions
     const int *x, *t, *seq;
@@ -529,8 +524,8 @@ struct NormArgs {
     const int* want;                 // FINAL: rows that want logits (0: all)
 };
 
-// One row per block, four elements per thread (the row stays in registers: one read, one write). Latency bound for few rows:
-// all parts of the sum are requested together, and mean and variance cost one exchange through shared memory: every warp
+// One row per block, four elements per thread (the row stays in registers). Latency bound for few rows:
+// mean and variance cost one exchange through shared memory: every warp
 // takes the mean and the squared deviations of its own elements, the block combines them (Chan's formula).
 template <int MODE>
 __global__ void __launch_bounds__(1024) pass_norm(const __grid_constant__ NormArgs a) {
@@ -538,10 +533,9 @@ __global__ void __launch_bounds__(1024) pass_norm(const __grid_constant__ NormAr
     const int tid = threadIdx.x, d = tid * 4, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
     const bool own = d < a.D;
     if (tid == 0) dep_launch();
-    uint2 gw = make_uint2(0, 0), sw = make_uint2(0, 0), bw = make_uint2(0, 0);
+    uint2 gw = make_uint2(0, 0), sw = make_uint2(0, 0);
     if (own) {
         gw = __ldg(reinterpret_cast<const uint2*>(a.gain + d)); sw = __ldg(reinterpret_cast<const uint2*>(a.shift + d));
-        if (MODE != NORM_EMBED && a.nparts) bw = __ldg(reinterpret_cast<const uint2*>(a.bias + d));
     }
     const float rd = 1.0f / (float)a.D, rl = 1.0f / (float)(a.D - (nw - 1) * 128);   // one over the elements of the row, of the last warp
     if (MODE != NORM_EMBED) dep_wait();
@@ -565,15 +559,9 @@ __global__ void __launch_bounds__(1024) pass_norm(const __grid_constant__ NormAr
             v = make_float4(h_lo(e.x) + h_lo(p.x), h_hi(e.x) + h_hi(p.x), h_lo(e.y) + h_lo(p.y), h_hi(e.y) + h_hi(p.y));
         }
     } else if (own) {
-        float4 p[PARTS_MAX];
         v = __ldcg(reinterpret_cast<const float4*>(a.z + (size_t)row * a.D + d));
-#pragma unroll
-        for (int s = 0; s < PARTS_MAX; s++) p[s] = s < a.nparts ? __ldcg(reinterpret_cast<const float4*>(a.part + s * a.part_stride + (size_t)row * a.D + d)) : make_float4(0.f, 0.f, 0.f, 0.f);
-        v.x += h_lo(bw.x); v.y += h_hi(bw.x); v.z += h_lo(bw.y); v.w += h_hi(bw.y);
-#pragma unroll
-        for (int s = 0; s < PARTS_MAX; s++) { v.x += p[s].x; v.y += p[s].y; v.z += p[s].z; v.w += p[s].w; }
     }
-    if (own && (MODE == NORM_EMBED || (MODE == NORM_MID && a.nparts))) *reinterpret_cast<float4*>(a.z + (size_t)row * a.D + d) = v;
+    if (own && MODE == NORM_EMBED) *reinterpret_cast<float4*>(a.z + (size_t)row * a.D + d) = v;
     float s = (v.x + v.y) + (v.z + v.w);
 #pragma unroll
     for (int m = 16; m; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
@@ -616,24 +604,6 @@ __global__ void __launch_bounds__(256) pass_norm_rows(const __grid_constant__ No
     float4 v[NV];
 #pragma unroll
     for (int i = 0; i < NV; i++) { const int d = i * 128 + lane * 4; v[i] = d < a.D ? __ldcg(reinterpret_cast<const float4*>(z + d)) : make_float4(0.f, 0.f, 0.f, 0.f); }
-    if (a.nparts) {
-#pragma unroll
-        for (int i = 0; i < NV; i++) {
-            const int d = i * 128 + lane * 4;
-            if (d < a.D) { const uint2 bw = __ldg(reinterpret_cast<const uint2*>(a.bias + d)); v[i].x += h_lo(bw.x); v[i].y += h_hi(bw.x); v[i].z += h_lo(bw.y); v[i].w += h_hi(bw.y); }
-        }
-#pragma unroll 1
-        for (int s = 0; s < a.nparts; s++) {
-            const float* p = a.part + s * a.part_stride + (size_t)row * a.D;
-#pragma unroll
-            for (int i = 0; i < NV; i++) {
-                const int d = i * 128 + lane * 4;
-                if (d < a.D) { const float4 q = __ldcg(reinterpret_cast<const float4*>(p + d)); v[i].x += q.x; v[i].y += q.y; v[i].z += q.z; v[i].w += q.w; }
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < NV; i++) { const int d = i * 128 + lane * 4; if (d < a.D) *reinterpret_cast<float4*>(z + d) = v[i]; }
-    }
     float s = 0.f, q = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; i++) s += (v[i].x + v[i].y) + (v[i].z + v[i].w);
