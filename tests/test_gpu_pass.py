@@ -39,7 +39,7 @@ def seeded(m, sh, ctx, seed):
     (9, dict(D=320, H=5, F=1296)),                    # folds of five blocks, the last block of the second one ragged
     (16, dict(D=1216, H=19, F=64)),                   # a fold of 19 blocks, fp16 operands at 16 rows
     (8, dict(L=1, D=1280, H=20)),                     # 160 (sequence, head) pairs at eight sequences: a chain, not the persistent kernel
-    (5, dict(L=1, D=1344, H=21)),                     # five sequences of a wide shape: the same
+    (3, dict(L=1, D=1344, H=21)),                     # three sequences of a wide shape: the same
 ])
 def test_step_as_a_chain(batch, kw):
     """ragged decode steps over seeded caches, contexts from none to nearly all of the cache"""
@@ -49,12 +49,12 @@ def test_step_as_a_chain(batch, kw):
     assert m.low.dims['chain']
     W = O.upcast(hf.weights)
     ctx = np.array([(37 * b) % 390 for b in range(batch)], np.int32)
-    ctx[:4] = (389, 0, 63, 64)
+    ctx[:4] = (389, 0, 63, 64)[:batch]
     caches = seeded(m, sh, ctx, 900)
     x = np.array([(b * 31 + 5) % sh.N for b in range(batch)], np.int32)
     m.t.copy_(torch.from_numpy(ctx))
     m.x.copy_(torch.from_numpy(x))
-    some = sorted(set(range(5)) | set(range(5, batch, max(1, batch // 12))) | {batch - 1})
+    some = sorted(set(range(min(5, batch))) | set(range(5, batch, max(1, batch // 12))) | {batch - 1})
     for s in range(steps):
         m.step()
         lg, nx = m.logits().cpu().numpy(), m.x.cpu().numpy()

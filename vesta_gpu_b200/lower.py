@@ -593,12 +593,12 @@ def lower(text, res, axis_max, batch=1, per_token=(), outputs=(), feedback=None,
     tune = dict(tune or {})
     # What a step as a chain of kernels (csrc/pass.cu) needs to know; Kernel runs that chain unless the caller asked for
     # something that only the persistent kernels have (a placement option, timing sums, rows of prompts).
-    # Up to eight sequences the small persistent kernel is the faster one (one sequence 172 against 250 us per step, eight 211
-    # against 263, XL shape with four 1,243 against 1,415): its exchanges between a few CTAs cost less than kernel boundaries.
-    # With more (sequence, head) pairs than CTAs it has to fall back on grid barriers (XL shape, eight: 1,679 against 1,275 us;
-    # twenty heads, eight: 688 against 611), and where rows of more than 1,280 are normalised in every CTA, one warp per row, it
-    # loses from five sequences on (XL shape, five: 1,394 against 1,311).
-    persistent = B <= 8 and B * H <= grid and (B <= 4 or D <= 1280)
+    # Up to eight sequences the small persistent kernel is the faster one at widths up to 1,024 (one sequence of the small shape 175
+    # against 219 us per step, eight 215 against 244 at 200 positions): its exchanges between a few CTAs cost less than kernel
+    # boundaries. The wider the rows, the less a boundary weighs and the more every CTA's norms do: five sequences of width 1,280
+    # 547 against 540, three of the XL shape 1,246 against 1,164, two 1,224 against 1,170 (left where results repeat bit for bit);
+    # and with more (sequence, head) pairs than CTAs the kernel falls back on grid barriers (XL shape, eight: 1,679 against 1,245).
+    persistent = B <= (8 if D <= 1024 else 4 if D <= 1280 else 2) and B * H <= grid
     dims = dict(dims, chain=not (tune or timing or row_seq or slab_tiles or act_lo is not None) and not persistent and D <= 4096,
                 step=dict(t_stride=int(t_per_token), tstep=int(fb.get(t_name, 0)), feedback=int(bool(fb)), prompt_len=int(prompt_len) if fb else 0,
                           exact=int(B <= 8 or (B <= 16 and D <= 1024)), cpos=cpos))
