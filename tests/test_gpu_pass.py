@@ -133,3 +133,41 @@ def test_prompts_as_a_pass(lens, rows, kw, divisor, tmp_path):
             assert np.abs(got[i, :, :lens[i]].float().cpu().numpy() - ref.astype(np.float32)).max() <= 4e-3, i
         if O.margin(lg) > MARGIN:
             assert int(first[i]) == nx
+
+
+def overflowing(sh, seed):
+    """weights of a one-layer model in which token 1 drives one GELU output past fp16 and no other token does: the first FC
+    column points where token 1's normalised embedding does, and its row of the MLP projection is zero -> (model, its weights)"""
+    from vesta_gpu_b200.synth import SynthGPT2, make_weights
+    w = make_weights(sh, seed, 'rich')
+    w['wte'][1] *= 20
+    w['fcw'][0, :, 0] = np.sign(w['wte'][1].astype(np.float32)) * 700
+    w['pw'][0, 0] = 0
+    return SynthGPT2(sh, seed, weights=w), w
+
+
+@pytest.mark.parametrize('batch', [12, 20])
+def test_a_row_that_overflows_leaves_its_neighbours_alone(batch):
+    """an MLP width that is no multiple of 64: the last fold block of the MLP projection ends inside a row's padding, so an
+    infinity (or, as head and remainder, a NaN) in one sequence stays in that sequence; steps and prompts"""
+    from oracle import gpt2_numpy as O
+    from vesta_gpu_b200.gpt2 import VestaGPT2
+    sh = shape('ragged', L=1, F=80)
+    hf, w = overflowing(sh, 29)
+    W = O.upcast(w)
+    m = VestaGPT2(hf, batch=batch, tmax=8, per_sequence_t=True)
+    x = np.array([1 if b % 3 == 1 else 2 + b for b in range(batch)], np.int32)
+    ref = [O.step(sh, W, *O.new_cache(sh, 1), int(x[b]), 0)[0] for b in range(batch)]
+    m.x.copy_(torch.from_numpy(x))
+    m.step()
+    got = m.logits().cpu().numpy()
+    assert not np.isfinite(got[x == 1]).all()                    # (the rows of token 1 did overflow)
+    bound = np.full(sh.N, TIGHT * (1 if batch <= 16 else 2))
+    bound[1] *= 20                                               # (token 1's embedding is 20 times the others', and so is what rounding leaves of its logit)
+    for b in np.flatnonzero(x != 1):
+        assert (np.abs(got[b] - ref[b]) < bound).all(), b
+    m.prefill(x[:, None])
+    first = m.x.cpu().numpy()
+    for b in np.flatnonzero(x != 1):
+        if O.margin(ref[b]) > MARGIN:
+            assert int(first[b]) == int(ref[b].argmax()), b

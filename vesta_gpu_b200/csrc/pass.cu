@@ -122,7 +122,7 @@ Layout layout(const Pass& p, int D, int F, int rows, int lrows) {
     o.q = take((size_t)rows * D * 4);
     o.act = take((size_t)p.planes * D * 2);
     o.att = take((size_t)p.planes * D * 2);
-    o.gelu = take((size_t)p.planes * F * 2 + 128);       // (the last block of the fold may reach past the last row)
+    o.gelu = take((size_t)p.planes * up(F, 64) * 2);     // (whole blocks of the fold per row: no product meets another row's values)
     o.fin = take((size_t)p.fplanes * D * 2);
     o.best = take((size_t)lrows * 8);
     o.rowoff = take((size_t)rows * 8);
@@ -212,14 +212,14 @@ int plan_for(Pass& p, int rows, int lrows, const Pass::Plan** out) {
     Pass::Plan q;
     q.rows = rows; q.lrows = lrows;
     const void* w[5] = {d.qkvw, d.ow, d.fcw, d.pw, d.wte};
-    const int fold[5] = {D, D, D, F, D}, feat[5] = {3 * D, D, F, D, d.N}, kb[5] = {kbd, kbd, kbd, kbf, kbd};
+    const int fold[5] = {D, D, D, F, D}, pitch[5] = {D, D, D, up(F, 64), D}, feat[5] = {3 * D, D, F, D, d.N}, kb[5] = {kbd, kbd, kbd, kbf, kbd};
     const size_t op[5] = {p.o.act, p.o.att, p.o.act, p.o.gelu, p.o.fin};
     for (int k = 0; k < 5; k++) {
         const Tile t = q.tile[k] = choose(k, k == K_LOGITS ? std::max(lrows, 1) : rows, p.rp, feat[k], kb[k], p.sms);
         int e;
         if (k == K_LOGITS) e = vesta_rt::fold_map(&q.w[k], w[k], D, feat[k], t.bm, k_blocks(t.bm));
         else e = vesta_rt::tensor_map(&q.w[k], w[k], feat[k], fold[k], d.L, (size_t)feat[k] * 2, (size_t)feat[k] * fold[k] * 2, 64 * k_blocks(t.bm), 1);
-        if (!e) e = vesta_rt::fold_map(&q.a[k], p.ws + op[k], fold[k], k == K_LOGITS ? p.fplanes : p.planes, box_rows(t), k_blocks(t.bm));
+        if (!e) e = vesta_rt::fold_map(&q.a[k], p.ws + op[k], pitch[k], k == K_LOGITS ? p.fplanes : p.planes, box_rows(t), k_blocks(t.bm));
         if (e) return e;
     }
     p.plans.push_back(q);
@@ -282,7 +282,7 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
             if (many) { g.oh = (u16*)u(p.o.q); g.low = (size_t)d.rows * D; g.a2 = pow2 ? 1.0f / d.scale : 1.0f; }
             if (clear) { g.lens = meta + mt.lens; g.seqs = d.prompts; g.seq_stride = (long long)L * d.tmax * D; g.tmax = d.tmax; }
         } else if (kind == K_FC) {
-            g.bias = f16(d.fcb, (size_t)l * F); g.oh = (u16*)u(p.o.gelu); g.a2 = 2 * d.gelu_a; g.k1 = d.gelu_b * 2.8853900817779268f; g.k2 = d.gelu_c * g.k1;
+            g.bias = f16(d.fcb, (size_t)l * F); g.oh = (u16*)u(p.o.gelu); g.pitch = up(F, 64); g.a2 = 2 * d.gelu_a; g.k1 = d.gelu_b * 2.8853900817779268f; g.k2 = d.gelu_c * g.k1;
         } else if (kind == K_LOGITS) { g.of = (float*)d.logits; g.best = (u64*)u(p.o.best); }
         else { g.of = z; g.bias = kind == K_PROJ ? f16(d.ob, (size_t)l * D) : f16(d.pb, (size_t)l * D); }
         g.bn = t.bn; g.ftiles = (g.nfeat + t.bm - 1) / t.bm; g.rtiles = p.rp ? 1 : (g.rows + t.bn - 1) / t.bn; g.ntiles = g.ftiles * g.rtiles * t.splits;

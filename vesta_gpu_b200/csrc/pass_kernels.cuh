@@ -97,11 +97,11 @@ enum { EPI_QKV = 0, EPI_ADD = 1, EPI_GELU = 2, EPI_LOGITS = 3 };
 struct GemmArgs {
     int layer, nfeat, kblocks, kb_per, rows, rp, stages;
     int bn, ftiles, rtiles, ntiles;  // rows per tile (a multiple of 16); tiles of features, of rows, in all (with the parts of the fold)
-    int D;
+    int D, pitch;                    // GELU: elements from a row to the next, nfeat rounded up to 64: the padding stays zero
     const u16* bias;                 // of the layer
     float* of;                       // QKV: queries [row][D] (prompts: `oh`); ADD: vector added to [row][nfeat]; LOGITS: logits [row][nfeat]
     size_t low;                      // QKV, prompts: from a query's heads to its remainders
-    u16* oh;                         // GELU: [row][nfeat], the remainder plane rp rows further; QKV, prompts: queries times a2, [fp16 head, remainder][row][D]
+    u16* oh;                         // GELU: [row][pitch], the remainder plane rp rows further; QKV, prompts: queries times a2, [fp16 head, remainder][row][D]
     u16 *kc, *vc;                    // QKV: the caches at this layer
     const long long* rowoff;         // QKV: element offset of every row's position in the caches (-1: none)
     const int* skip;                 // not zero: the pass was refused, nothing may be written that outlives it
@@ -420,20 +420,20 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS + (EPI == EPI_QKV ? 32 
 #pragma unroll
                     for (int i = 0; i < CH; i++, dst += g.nfeat) add_f32(dst, v[i], i < m);
                 } else if (EPI == EPI_GELU) {
-                    u16* dst = g.oh + (size_t)row * g.nfeat + f;
+                    u16* dst = g.oh + (size_t)row * g.pitch + f;
                     if (BM == 64 && g.rp) {
-                        const size_t lo = (size_t)g.rp * g.nfeat;
+                        const size_t lo = (size_t)g.rp * g.pitch;
 #pragma unroll
-                        for (int i = 0; i < CH; i += 2, dst += 2 * g.nfeat) {
+                        for (int i = 0; i < CH; i += 2, dst += 2 * g.pitch) {
                             const u32 h = pack_h2(v[i], v[i + 1]), r = pack_h2(v[i] - h_lo(h), v[i + 1] - h_hi(h));
-                            st_u16(dst, (u16)h, i < m); st_u16(dst + g.nfeat, (u16)(h >> 16), i + 1 < m);
-                            st_u16(dst + lo, (u16)r, i < m); st_u16(dst + lo + g.nfeat, (u16)(r >> 16), i + 1 < m);
+                            st_u16(dst, (u16)h, i < m); st_u16(dst + g.pitch, (u16)(h >> 16), i + 1 < m);
+                            st_u16(dst + lo, (u16)r, i < m); st_u16(dst + lo + g.pitch, (u16)(r >> 16), i + 1 < m);
                         }
                     } else {
 #pragma unroll
-                        for (int i = 0; i < CH; i += 2, dst += 2 * g.nfeat) {
+                        for (int i = 0; i < CH; i += 2, dst += 2 * g.pitch) {
                             const u32 h = pack_h2(v[i], v[i + 1]);
-                            st_u16(dst, (u16)h, i < m); st_u16(dst + g.nfeat, (u16)(h >> 16), i + 1 < m);
+                            st_u16(dst, (u16)h, i < m); st_u16(dst + g.pitch, (u16)(h >> 16), i + 1 < m);
                         }
                     }
                 } else {
