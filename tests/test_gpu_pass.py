@@ -171,3 +171,21 @@ def test_a_row_that_overflows_leaves_its_neighbours_alone(batch):
     for b in np.flatnonzero(x != 1):
         if O.margin(ref[b]) > MARGIN:
             assert int(first[b]) == int(ref[b].argmax()), b
+
+
+@pytest.mark.parametrize('batch', [20, 70])
+def test_best_of_logits_that_are_all_minus_infinity(batch):
+    """an output norm that overflows fp16 makes every logit minus infinity: all equal, so the lowest token, as the order of
+    (value, lowest index) has it; tiles of 64 features (half of whose lanes hold none) and of 128"""
+    from vesta_gpu_b200.gpt2 import VestaGPT2
+    from vesta_gpu_b200.synth import SynthGPT2, make_weights
+    sh = shape('low', L=1)
+    w = make_weights(sh, 31, 'rich')
+    w['wte'][:, 0] = 4                      # every state is large and positive there,
+    w['lnfw'][0], w['lnfb'][0] = -10000, -65504      # the norm's output minus infinity as fp16, and so is its product with the table
+    m = VestaGPT2(SynthGPT2(sh, 31, weights=w), batch=batch, tmax=8)
+    m.x.copy_(torch.arange(batch, dtype=torch.int32) + 2)
+    m.step()
+    assert torch.isneginf(m.logits()).all()
+    assert (m.next() == 0).all() and (m.x == 0).all()
+    m.k.check()

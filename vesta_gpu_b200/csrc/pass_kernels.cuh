@@ -445,8 +445,8 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS + (EPI == EPI_QKV ? 32 
                     int best[CH], at[CH];
 #pragma unroll
                     for (int i = 0; i < CH; i++) {
-                        best[i] = own ? __float_as_int(v[i]) : __float_as_int(-3.0e38f);
-                        best[i] = best[i] >= 0 ? best[i] : best[i] ^ 0x7fffffff;
+                        best[i] = __float_as_int(v[i]);
+                        best[i] = !own ? (int)0x80000000 : best[i] >= 0 ? best[i] : best[i] ^ 0x7fffffff;   // (below every logit, minus infinity included)
                         at[i] = lane;
                     }
                     int mine = 0;
