@@ -189,3 +189,43 @@ def test_best_of_logits_that_are_all_minus_infinity(batch):
     assert torch.isneginf(m.logits()).all()
     assert (m.next() == 0).all() and (m.x == 0).all()
     m.k.check()
+
+
+def test_waits_of_a_chain_that_run_out():
+    """with the limit of a wait at a nanosecond every wait that is not over within one try gives up, at different times in the
+    warps of a block and in the blocks of a pair: a step of 256 rows (several tiles per block in every contraction) and prompts
+    of 4,096 positions (pairs of blocks, attention on tensor memory) end with a status, publish nothing, and run again as
+    before once the limit is back"""
+    from vesta_gpu_b200.launch import lib, ok
+    sh, batch, P = shape('wide', L=2, D=1600, H=25, F=1600, N=20000, C=64), 256, 16
+    m, _ = model(sh, 41, 'rich', batch, sh.C)
+    toks = np.random.RandomState(3).randint(0, sh.N, (batch, P)).astype(np.int32)
+    m.prefill(toks)
+    keys, vals, x = m.keys.clone(), m.vals.clone(), m.x.clone()
+    m.step()
+    logits, after, new = m.logits().clone(), m.x.clone(), m.keys[:, :, P].clone()
+    state = dict(keys=keys, vals=vals, x=x, t=torch.tensor([P], dtype=torch.int32).cuda())
+    m.load_state(state)
+    nxt = m.next().clone()
+    ok(lib().vesta_pass_wait_limit(m.k._pass, 1))
+    m.step(2)
+    assert 'operands of a contraction' in str(m.k.status())
+    assert int(m.k.bar[2]) == 1 and int(m.t[0]) == P and torch.equal(m.x, x) and torch.equal(m.next(), nxt)
+    ok(lib().vesta_pass_wait_limit(m.k._pass, 0))
+    m.step()                                                     # (refused until the status is cleared)
+    assert int(m.t[0]) == P and torch.equal(m.x, x)
+    m.k.clear_status()
+    m.load_state(state)
+    m.step()
+    m.k.check()
+    assert int(m.t[0]) == P + 1 and (m.logits() - logits).abs().max() < 2 * TIGHT
+    assert (m.keys[:, :, P].float() - new.float()).abs().max() <= 4e-3
+    eng, = m._prefill_engines.values()
+    ok(lib().vesta_pass_wait_limit(eng.h, 1))
+    with pytest.raises(RuntimeError, match='gave up'):
+        m.prefill(toks)
+    ok(lib().vesta_pass_wait_limit(eng.h, 0))
+    m.prefill(toks)
+    assert int(m.t[0]) == P
+    for got, ref in ((m.keys, keys), (m.vals, vals)):
+        assert (got[:, :, :P].float() - ref[:, :, :P].float()).abs().max() <= 4e-3 and not got[:, :, P:].any()

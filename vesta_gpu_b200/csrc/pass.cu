@@ -25,7 +25,7 @@ enum Kind { K_QKV = 0, K_PROJ = 1, K_FC = 2, K_P2 = 3, K_LOGITS = 4 };
 struct Tile { int bm, bn, stages, splits; };
 
 struct Layout {
-    size_t z, q, act, att, gelu, fin, best, rowoff, pos, skip;
+    size_t z, q, act, att, gelu, fin, best, rowoff, pos, skip, limit;
     size_t meta, total;                        // prompts: tokens, positions, sequences of the rows; attention runs; rows that want logits and where they go; lengths
 };
 // the metadata of a pass over prompts, as offsets in 32-bit words
@@ -128,6 +128,7 @@ Layout layout(const Pass& p, int D, int F, int rows, int lrows) {
     o.rowoff = take((size_t)rows * 8);
     o.pos = take((size_t)rows * 4);
     o.skip = take(4);
+    o.limit = take(8);
     o.meta = p.d.prompts ? take((size_t)Meta(rows, lrows, p.d.prompts).words * 4) : 0;
     o.total = at;
     return o;
@@ -272,7 +273,7 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
     auto mul = [&](int kind, int l) {
         const Tile& t = pl->tile[kind];
         GemmArgs g = {};
-        g.layer = l; g.D = D; g.rp = p.rp; g.stages = t.stages; g.status = (u32*)d.bar; g.skip = (const int*)u(p.o.skip);
+        g.layer = l; g.D = D; g.rp = p.rp; g.stages = t.stages; g.status = (u32*)d.bar; g.limit = (const u64*)u(p.o.limit); g.skip = (const int*)u(p.o.skip);
         g.rows = kind == K_LOGITS ? lrows : rows;
         g.kblocks = kind == K_P2 ? kbf : kbd; g.kb_per = (g.kblocks + t.splits - 1) / t.splits;
         g.nfeat = kind == K_QKV ? 3 * D : kind == K_FC ? F : kind == K_LOGITS ? d.N : D;
@@ -294,7 +295,7 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
         const u16 *kc = (const u16*)d.keys + (size_t)l * d.tmax * D, *vc = (const u16*)d.vals + (size_t)l * d.tmax * D;
         const long long ss = (long long)L * d.tmax * D;
         if (many) {
-            AttManyArgs a = {(const int4*)(meta + mt.tiles), l, L, D, d.scale, att, (u32*)d.bar};
+            AttManyArgs a = {(const int4*)(meta + mt.tiles), l, L, D, d.scale, att, (u32*)d.bar, (const u64*)u(p.o.limit)};
             Config c(dim3(d.H, tiles), AM_THREADS, st, true);
             c.c.dynamicSmemBytes = AM_SMEM;
             return pow2 ? cudaLaunchKernelEx(&c.c, pass_attend_many<true>, p.qmap, p.kmap, p.vmap, a) : cudaLaunchKernelEx(&c.c, pass_attend_many<false>, p.qmap, p.kmap, p.vmap, a);
@@ -448,6 +449,14 @@ int vesta_pass_prompts(void* pass, void* stream, const int* tokens, int ld, cons
     TRY(cudaMemcpyAsync(word, d.bar, 4, cudaMemcpyDeviceToHost, st));
     TRY(cudaStreamSynchronize(st));
     *status = *word;
+    return 0;
+}
+
+int vesta_pass_wait_limit(void* pass, unsigned long long ns) {
+    Pass* p = (Pass*)pass;
+    if (!p) return fail(-1, "vesta_pass_wait_limit: null argument");
+    const vesta_rt::OnDevice on(p->dev);
+    TRY(cudaMemcpy(p->ws + p->o.limit, &ns, 8, cudaMemcpyHostToDevice));
     return 0;
 }
 

@@ -53,12 +53,13 @@ __device__ __forceinline__ void tma3_pair(u32 dst, const CUtensorMap* m, int x, 
     asm volatile("cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                  :: "r"(dst), "l"(m), "r"(x), "r"(y), "r"(z), "r"(bar) : "memory");
 }
-// a shared-memory address of this block as the same address of the first block of its cluster
-__device__ __forceinline__ u32 of_first(u32 a) {
+// a shared-memory address of this block as the same address of block `rank` of its cluster
+__device__ __forceinline__ u32 of_block(u32 a, u32 rank) {
     u32 r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(a));
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
     return r;
 }
+__device__ __forceinline__ u32 of_first(u32 a) { return of_block(a, 0); }
 __device__ __forceinline__ void cluster_sync() { asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // arrives on `bar` (of a pair: at that address in both blocks) when the products issued so far are done
 template <bool PAIR> __device__ __forceinline__ void tc_commit(u32 bar) {
@@ -71,23 +72,31 @@ __device__ __forceinline__ u32 elect_one() {
     return leader;
 }
 
-// Every wait gives up after half a second: it leaves a code in the status word, a flag that ends the block's other waits (the
-// block runs to its end) and the abort flag: this pass publishes no token or position, and every later one is refused.
+// Every wait gives up after half a second (or `*limit` nanoseconds, where that is not zero): it leaves a code in the status word,
+// a flag that ends the other waits of the block (of the pair: `peer` is the flag of the other block) and the abort flag: this pass
+// publishes no token or position, and every later one is refused. The block runs to its end: a warp whose wait gave up goes on
+// through the barriers that other warps of the block wait at, and does nothing between them.
 #define PASS_WAIT_NS 500000000ull
-struct Wait { volatile int* dead; u32* status; };
+struct Wait { volatile int* dead; u32* status; const u64* limit; u32 peer; };
 __device__ __noinline__ bool mbar_wait_slow(u32 bar, u32 parity, const Wait& w, u32 code) {
-    const u64 t0 = now_ns();
-    u32 spins = 0;
-    while (!mbar_try(bar, parity)) {
+    const u64 t0 = now_ns(), set = __ldcg(w.limit), limit = set ? set : PASS_WAIT_NS;
+    while (!mbar_try(bar, parity)) {                     // (a try holds the thread for up to 4 us)
         if (*w.dead) return false;
-        if ((++spins & 63u) == 0 && now_ns() - t0 > PASS_WAIT_NS) {
+        if (now_ns() - t0 > limit) {
             atomicCAS(w.status, 0u, code | (blockIdx.x << 16));
             atomicExch(w.status + 2, 1u);
             *w.dead = 1;
+            if (w.peer) asm volatile("st.shared::cluster.u32 [%0], %1;" :: "r"(w.peer), "r"(1u) : "memory");
             return false;
         }
     }
     return true;
+}
+// After a wait that gave up: copies and products in flight land (in a few microseconds) before the block's shared memory and
+// tensor memory go to another.
+__device__ __noinline__ void settle() {
+    const u64 t0 = now_ns();
+    while (now_ns() - t0 < 2000000ull) { }
 }
 __device__ __forceinline__ bool mbar_wait(u32 bar, u32 parity, const Wait& w, u32 code) { return mbar_try(bar, parity) || mbar_wait_slow(bar, parity, w, code); }
 
@@ -107,6 +116,7 @@ struct GemmArgs {
     const int* skip;                 // not zero: the pass was refused, nothing may be written that outlives it
     u64* best;                       // LOGITS: packed (value, ~index) maximum of every row
     u32* status;
+    const u64* limit;                // of a wait
     float a2, k1, k2;                // GELU: see gelu_tanh; QKV, prompts: a2 = 1 / scale where that is a power of two
     // QKV, prompts: one more warp zeroes this layer's cache rows behind the first lens[sequence], which this pass writes
     const int* lens;
@@ -211,7 +221,7 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS + (EPI == EPI_QKV ? 32 
     const int t_first = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, t_step = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
     const bool two = g.ntiles > t_step;
     const int cols = S::columns(bn, two);
-    const Wait w{dead, g.status};
+    const Wait w{dead, g.status, g.limit, PAIR ? of_block(smem_u32(tail + 4), rank ^ 1) : 0u};
     if (threadIdx.x == 0) {
         *dead = 0;
         for (int i = 0; i < st; i++) { mbar_init(bars + i * 8, 1); mbar_init(bars + (st + i) * 8, 1); }
@@ -332,7 +342,7 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS + (EPI == EPI_QKV ? 32 
     } else {
         const int quarter = warp & 3, ew = warp - 2, et = threadIdx.x - 64;
         const int fl = AM == 128 ? quarter * 32 + lane : quarter * 16 + lane;      // (a product of 64 rows leaves row m in lane 32 (m / 16) + m % 16)
-        bool waited = false, skip = false;
+        bool waited = false, skip = false, ok = true;
         int n = 0;
         u64 off = ~0ull;                                                           // QKV: a row's offset in the caches, one tile ahead
         auto row_offset = [&](int t) {
@@ -361,9 +371,15 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS + (EPI == EPI_QKV ? 32 
             // the warps of a quarter share the rows
             const int share = live > EW ? (live + 2 * EW - 1) / (2 * EW) * 8 : 4;
             const int c_lo = (ew >> 2) * share, c_hi = min(live, c_lo + share);
-            const bool ok = mbar_wait(tmf + b * 8, (n >> 1) & 1, w, 0xB20u);
+            if (ok) ok = !__any_sync(0xffffffffu, !mbar_wait(tmf + b * 8, (n >> 1) & 1, w, 0xB20u));
+            if (!ok) {                                                             // (another warp may have seen the same tile complete: it waits at these)
+                if (EPI == EPI_LOGITS) {
+                    asm volatile("bar.sync 1, %0;" :: "n"(EW * 32) : "memory");
+                    if (two) asm volatile("bar.sync 1, %0;" :: "n"(EW * 32) : "memory");
+                }
+                continue;
+            }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (__any_sync(0xffffffffu, !ok)) break;
             const u32 ta = tmem + ((u32)(quarter * 32) << 16) + (b ? bn : 0);
             const int part = EPI == EPI_QKV ? f / g.D : 0;                         // 0 query, 1 key, 2 value (a warp never straddles two)
             u16* cache = EPI == EPI_QKV ? (part == 1 ? g.kc : g.vc) + (f - part * g.D) : (u16*)0;
@@ -495,13 +511,9 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS + (EPI == EPI_QKV ? 32 
     __syncthreads();
     if (PAIR) cluster_sync();                                                      // (neither block leaves while the other may still reach into it)
     if (warp == 1) {
+        if (*dead) settle();                                                       // (of a pair: both or none)
         if (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(cols) : "memory");
         else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(cols) : "memory");
-    }
-    if (*dead && threadIdx.x == 0) {
-        // a wait ran out: let copies in flight land (bounded) before the block's shared memory goes to another
-        const u64 t0 = now_ns();
-        while (now_ns() - t0 < 2000000ull) { }
     }
 }
 
@@ -825,6 +837,7 @@ struct AttManyArgs {
     float scale;
     u16* out;                        // [row][D] fp16
     u32* status;
+    const u64* limit;                // of a wait
 };
 __device__ __forceinline__ void tm_ld32(u32 (&r)[32], u32 addr) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
@@ -866,7 +879,7 @@ __global__ void __launch_bounds__(AM_THREADS, 2) pass_attend_many(const __grid_c
     volatile int* dead = reinterpret_cast<volatile int*>(tail + 4);
     float* pair = reinterpret_cast<float*>(tail + 16);                             // [tile & 1][half][row]: maxima, at the end sums
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-    const Wait w{dead, a.status};
+    const Wait w{dead, a.status, a.limit, 0u};
     if (threadIdx.x == 0) {
         *dead = 0;
         mbar_init(qf, 1); mbar_init(sf, 1); mbar_init(pf, 8); mbar_init(of, 1);
@@ -1050,10 +1063,9 @@ __global__ void __launch_bounds__(AM_THREADS, 2) pass_attend_many(const __grid_c
         }
     }
     __syncthreads();
-    if (warp == 9) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "n"(256) : "memory");
-    if (*dead && threadIdx.x == 0) {
-        const u64 t0 = now_ns();
-        while (now_ns() - t0 < 2000000ull) { }
+    if (warp == 9) {
+        if (*dead) settle();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "n"(256) : "memory");
     }
 }
 

@@ -59,6 +59,7 @@ def lib():
         L.vesta_pass_workspace.argtypes = [vp, ctypes.POINTER(sz)]
         L.vesta_pass_create.argtypes = [vp, vp, ci, ctypes.POINTER(vp)]
         L.vesta_pass_prompts.argtypes = [vp, vp, vp, ci, vp, ctypes.POINTER(cu)]
+        L.vesta_pass_wait_limit.argtypes = [vp, ctypes.c_ulonglong]
         L.vesta_pass_bind.argtypes = [vp, ctypes.POINTER(vp)]
         L.vesta_pass_release.argtypes = [vp]
         L.vesta_pass_release.restype = None
@@ -223,7 +224,7 @@ class Kernel:
             from .passes import bind_step
             vals += [self.S.data_ptr(), self.bar.data_ptr(), self.TS.data_ptr()]
             with torch.cuda.device(self.device):
-                self._bound, self._work = bind_step(self, residue, zeros)
+                self._bound, self._pass, self._work = bind_step(self, residue, zeros)
             if self._packed is not None:
                 self.pack(residue)
         else:

@@ -49,7 +49,7 @@ def create(desc, device, graph=False):
 
 
 def bind_step(kernel, residue, zeros):
-    """a decode step over the tensors of `residue` as a chain of kernels -> (handle for vesta_step_run, workspace)"""
+    """a decode step over the tensors of `residue` as a chain of kernels -> (handle for vesta_step_run, the pass that it owns, workspace)"""
     low = kernel.lowered
     d, st = low.dims, low.dims['step']
     off = {n: kernel.S.data_ptr() + 4 * v[0] for n, v in low.scratch.items()}
@@ -61,7 +61,7 @@ def bind_step(kernel, residue, zeros):
     h, ws = create(desc, kernel.device, graph=True)
     bound = ctypes.c_void_p()
     ok(lib().vesta_pass_bind(h, ctypes.byref(bound)))
-    return bound, ws
+    return bound, h, ws
 
 
 class PromptPass:
