@@ -100,7 +100,8 @@ typedef struct vesta_pass_desc {
     void *bar;                          /* status words: [0] status, [2] abort flag */
 } vesta_pass_desc;
 int vesta_pass_workspace(const vesta_pass_desc* desc, size_t* bytes);
-/* workspace: that many bytes of device memory, zeroed. graph != 0: the pass is a decode step, kept as a CUDA graph. */
+/* workspace: that many bytes of device memory, zeroed, on a 256-byte boundary (matrices, table and caches: 16 bytes, norm
+ * parameters and wpe: 8 bytes; anything else is refused). graph != 0: the pass is a decode step, kept as a CUDA graph. */
 int vesta_pass_create(const vesta_pass_desc* desc, void* workspace, int graph, void** pass);
 /* Whole prompts: tokens [prompts][ld] and lens [prompts] in host memory. Every prompt position goes into the caches (rows after a
  * prompt are zeroed), x gets the token chosen after every prompt, t its position; in passes of at most desc.rows rows.

@@ -101,3 +101,32 @@ def test_static_step_refuses_oversized_requests_before_touching_the_gpu(built_li
     assert call(counters=1 << 20) != 0 and b'counter' in lib.vesta_static_last_error()
     assert call(lo=(1 << 64) - 8, ln=16) != 0 and b'output range' in lib.vesta_static_last_error()
     assert call(no=1000, nn=100) != 0 and b'output range' in lib.vesta_static_last_error()
+
+
+def pass_desc(**kw):
+    """a descriptor of a pass that would be accepted, over addresses that nobody follows"""
+    from vesta_gpu_b200.passes import Desc, _PTRS
+    d = Desc(L=2, D=128, H=2, F=256, N=211, tmax=64, cpos=64, rows=16, logit_rows=16, eps=1e-5, scale=8.0)
+    for n in _PTRS:
+        setattr(d, n, 0x10000)
+    for n, v in kw.items():
+        setattr(d, n, v)
+    return d
+
+
+def create_pass(d, workspace=0x10000):
+    """-> the message with which vesta_pass_create refuses (without a GPU every descriptor is refused in the end)"""
+    from vesta_gpu_b200 import launch
+    L, out = launch.lib(), ctypes.c_void_p()
+    assert L.vesta_pass_create(ctypes.byref(d), ctypes.c_void_p(workspace), 0, ctypes.byref(out)) != 0 and not out.value
+    return L.vesta_last_error().decode()
+
+
+def test_a_pass_refuses_tensors_that_its_loads_cannot_reach(built_library):
+    for name in ('keys', 'vals', 'wte', 'qkvw', 'ow', 'fcw', 'pw'):
+        assert '16-byte boundary' in create_pass(pass_desc(**{name: 0x10008})), name
+    for name in ('wpe', 'ln1w', 'ln1b', 'ln2w', 'ln2b', 'lnfw', 'lnfb'):
+        assert '8-byte boundary' in create_pass(pass_desc(**{name: 0x10002})), name
+    for name in ('x', 't', 'logits', 'bar', 'qkvb', 'ob', 'fcb', 'pb'):
+        assert 'missing' in create_pass(pass_desc(**{name: None})), name
+    assert '256-byte boundary' in create_pass(pass_desc(), workspace=0x10010)

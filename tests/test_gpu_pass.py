@@ -229,3 +229,63 @@ def test_waits_of_a_chain_that_run_out():
     assert int(m.t[0]) == P
     for got, ref in ((m.keys, keys), (m.vals, vals)):
         assert (got[:, :, :P].float() - ref[:, :, :P].float()).abs().max() <= 4e-3 and not got[:, :, P:].any()
+
+
+def moved(t):
+    """the same values two bytes behind a 16-byte boundary"""
+    v = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)[1:].view(t.shape)
+    assert v.data_ptr() % 16 == 2
+    return v.copy_(t)
+
+
+@pytest.mark.parametrize('batch', [3, 12])
+def test_weights_off_a_16_byte_boundary(batch):
+    """weights that are views into a larger buffer, in the persistent kernel and in a chain: read through aligned copies that
+    pack() renews; the caches are refused"""
+    from vesta_gpu_b200.launch import Kernel
+    sh = shape('moved')
+    m, _ = model(sh, 3, 'rich', batch, 20)
+    k = Kernel(m.low, device=m.device.index)
+    R = dict(m.k.keep)
+    for role in ('ln1w', 'ln1b', 'qkvw', 'qkvb', 'ow', 'ob', 'ln2w', 'ln2b', 'fcw', 'fcb', 'pw', 'pb', 'lnfw', 'lnfb', 'wpe'):
+        R[role] = moved(R[role])
+    for name in ('x', 't', 'keys', 'vals'):
+        R[name] = R[name].clone()
+    m.x.fill_(7)
+    R['x'].fill_(7)
+    k.bind(R)
+    m.step()
+    k.launch()
+    assert (m.logits() - k.view('logit')).abs().max() < TIGHT and torch.equal(m.t, R['t'])
+    for W in (m.k.keep, R):                                      # changed in place
+        W['lnfw'].mul_(0.5)
+        W['fcw'].mul_(2)
+    m.k.pack()
+    k.pack()
+    m.step()
+    k.launch()
+    assert (m.logits() - k.view('logit')).abs().max() < TIGHT
+    k.check()
+    with pytest.raises(RuntimeError):
+        k.bind(dict(R, keys=moved(R['keys'])))
+
+
+def test_prompts_with_weights_off_a_16_byte_boundary():
+    """a state dict of views (position table, output norm): prefill reads what the weights are when it is called"""
+    from vesta_gpu_b200.gpt2 import VestaGPT2
+    sh = shape('moved')
+    m, hf = model(sh, 3, 'rich', 2, 20)
+
+    class Views:
+        def state_dict(self):
+            return {n: moved(t.cuda()) if n in ('transformer.wpe.weight', 'transformer.ln_f.weight', 'transformer.ln_f.bias') else t
+                    for n, t in hf.state_dict().items()}
+    v = VestaGPT2(Views(), batch=2, tmax=20)
+    assert v.W['wpe'].data_ptr() % 16 == 2
+    toks = np.arange(24, dtype=np.int32).reshape(2, 12)
+    for _ in range(2):
+        m.prefill(toks)
+        v.prefill(toks)
+        assert (m.keys.float() - v.keys.float()).abs().max() <= 4e-3 and m.keys.any()
+        for w in (m, v):
+            w.W['wpe'].mul_(-1)

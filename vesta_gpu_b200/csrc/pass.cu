@@ -150,6 +150,18 @@ int plan(Pass& p, const vesta_pass_desc* d) {
     return 0;
 }
 
+// The weights and caches are there and start where the kernels' loads want them: 16 bytes for tensor copies and 16-byte pieces, 8 for
+// the norms' parameters and the position table
+int check(const vesta_pass_desc& d) {
+    const void* wide[] = {d.wte, d.qkvw, d.ow, d.fcw, d.pw, d.keys, d.vals};
+    const void* four[] = {d.wpe, d.ln1w, d.ln1b, d.ln2w, d.ln2b, d.lnfw, d.lnfb};
+    for (const void* q : {(const void*)d.qkvb, (const void*)d.ob, (const void*)d.fcb, (const void*)d.pb, (const void*)d.x, (const void*)d.t, (const void*)d.logits, (const void*)d.bar})
+        if (!q) return fail(-1, "vesta_pass: a tensor is missing");
+    for (const void* q : wide) if (!q || (size_t)q % 16) return fail(-1, "vesta_pass: matrices, table and caches start on a 16-byte boundary");
+    for (const void* q : four) if (!q || (size_t)q % 8) return fail(-1, "vesta_pass: norm parameters and position table start on an 8-byte boundary");
+    return 0;
+}
+
 // The kernels of a pass ask for the same split of an SM between shared memory and cache: an SM changes it only when it is idle,
 // and a block that waits for that cannot start under its predecessor (23 sequences: projection 3.0 -> 2.4 us, norm 4.5 -> 3.5).
 template <class F> cudaError_t all_shared(F* f) { return cudaFuncSetAttribute((const void*)f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared); }
@@ -366,6 +378,8 @@ int vesta_pass_create(const vesta_pass_desc* d, void* workspace, int graph, void
     if (!out || !workspace) return fail(-1, "vesta_pass_create: null argument");
     Pass* p = new Pass{};
     int e = plan(*p, d);
+    if (!e) e = check(*d);
+    if (!e && (size_t)workspace % 256) e = fail(-1, "vesta_pass: the workspace starts on a 256-byte boundary");
     p->ws = (unsigned char*)workspace;
     if (!e) { const cudaError_t ce = prepare_all(); if (ce != cudaSuccess) e = cuda_fail(ce, "cudaFuncSetAttribute"); }
     if (!e && d->prompts) {

@@ -148,6 +148,7 @@ class Kernel:
             self.bar = torch.zeros(lowered.counters, dtype=torch.int32, device=self.device)
             self.TS = torch.zeros(2048, dtype=torch.int64, device=self.device)
             self._module = self._packed = None
+            self._copies = []                                    # (copy, original) of weights bound off a 16-byte boundary
             self.args, self.keep, self._bound = None, None, None
             self.fuse = 16                                       # decode steps per launch in launch(steps > 1)
             self.feeds_back = '#define V_FEEDBACK 1' in lowered.src
@@ -214,8 +215,11 @@ class Kernel:
             t = residue[name]
             assert t.is_cuda and t.dtype == TORCH_DT[dt] and t.is_contiguous(), (name, t.dtype, dt)
             assert t.device == self.device, (name, t.device)
-            vals.append(t.data_ptr())
-        self.keep = residue
+        from .passes import VECTORS, WEIGHTS, aligned
+        # (the persistent kernels read the matrices and the position table element by element)
+        here, copies = aligned(self.lowered, residue, WEIGHTS[1:] if self.chain else VECTORS)
+        vals += [here[name].data_ptr() for name, _, _ in self.lowered.params]
+        self.keep, self._copies = residue, copies
         if self._bound:
             L.vesta_step_release(self._bound)
             self._bound = None
@@ -224,7 +228,7 @@ class Kernel:
             from .passes import bind_step
             vals += [self.S.data_ptr(), self.bar.data_ptr(), self.TS.data_ptr()]
             with torch.cuda.device(self.device):
-                self._bound, self._pass, self._work = bind_step(self, residue, zeros)
+                self._bound, self._pass, self._work = bind_step(self, here, zeros)
             if self._packed is not None:
                 self.pack(residue)
         else:
@@ -257,7 +261,10 @@ class Kernel:
 
     def pack(self, residue=None):
         """(re)build the packed weight streams from the bound weights; call again after changing them (a chain reads the
-        weights where they are: nothing to do unless its persistent kernel has been asked for)"""
+        weights where they are: nothing to do but for weights that do not start on a 16-byte boundary, of which it reads a
+        copy, unless its persistent kernel has been asked for)"""
+        for copy, original in self._copies:
+            copy.copy_(original)
         if self.chain and self._packed is None:
             return
         residue = residue or self.keep

@@ -12,6 +12,7 @@ from .lower import Lowered, ZEROS
 _PTRS = ('wte', 'wpe', 'ln1w', 'ln1b', 'qkvw', 'qkvb', 'ow', 'ob', 'ln2w', 'ln2b', 'fcw', 'fcb', 'pw', 'pb', 'lnfw', 'lnfb',
          'keys', 'vals', 'x', 't', 'prompt', 'plen', 'logits', 'next', 'bar')
 WEIGHTS = _PTRS[:16]
+VECTORS = ('ln1w', 'ln1b', 'qkvb', 'ob', 'ln2w', 'ln2b', 'fcb', 'pb', 'lnfw', 'lnfb')
 
 
 class Desc(ctypes.Structure):
@@ -20,6 +21,22 @@ class Desc(ctypes.Structure):
                                             't_stride', 'tstep', 'feedback', 'prompt_len')] + \
                [(n, ctypes.c_float) for n in ('eps', 'scale', 'gelu_a', 'gelu_b', 'gelu_c')] + \
                [(n, ctypes.c_void_p) for n in _PTRS]
+
+
+def aligned(low, residue, roles):
+    """-> (`residue` as kernels that load 16 bytes at a time can read it, [(copy, original)]): the weights named by `roles` that do
+    not start on a 16-byte boundary (views into a larger buffer) are copied. The table and the caches are read and written
+    where they are: refused."""
+    out, copies = dict(residue), []
+    for role in ('wte', 'keys', 'vals'):
+        if residue[low.roles[role]].data_ptr() % 16:
+            raise RuntimeError(f'{low.roles[role]} must start on a 16-byte boundary')
+    for role in roles:
+        name = low.roles[role]
+        if name != ZEROS and residue[name].data_ptr() % 16:
+            out[name] = residue[name].clone()
+            copies.append((out[name], residue[name]))
+    return out, copies
 
 
 def describe(low, residue, zeros, cpos, **kw):
@@ -76,7 +93,7 @@ class PromptPass:
         self.logits = torch.empty(lrows, low.dims['N'], dtype=torch.float32, device=dev)
         self.bar = torch.zeros(32, dtype=torch.int32, device=dev)
         self.zeros = torch.zeros(low.dims['zeros_len'], dtype=torch.float16, device=dev)
-        R = {**model.W, 'keys': model.keys, 'vals': model.vals}
+        R, self.copies = aligned(low, {**model.W, 'keys': model.keys, 'vals': model.vals}, WEIGHTS[1:])
         desc = describe(low, R, self.zeros, low.dims['step']['cpos'], rows=rows, logit_rows=lrows, prompts=model.B,
                         t_stride=int(model.t.numel() > 1), x=model.x, t=model.t, logits=self.logits, bar=self.bar)
         with torch.cuda.device(dev):
@@ -89,6 +106,8 @@ class PromptPass:
     def run(self, tokens, lens):
         """tokens (B, P), lens (B,) int32 numpy: the caches, x and t of the model after the prompts"""
         tokens = np.ascontiguousarray(tokens, np.int32)
+        for copy, original in self.copies:
+            copy.copy_(original)
         dev, status = self.model.device, ctypes.c_uint()
         at = tokens.__array_interface__['data'][0], tokens.shape[1], lens.__array_interface__['data'][0], ctypes.byref(status)
         if torch.cuda.current_device() == dev.index:
