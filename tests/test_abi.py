@@ -130,3 +130,18 @@ def test_a_pass_refuses_tensors_that_its_loads_cannot_reach(built_library):
     for name in ('x', 't', 'logits', 'bar', 'qkvb', 'ob', 'fcb', 'pb'):
         assert 'missing' in create_pass(pass_desc(**{name: None})), name
     assert '256-byte boundary' in create_pass(pass_desc(), workspace=0x10010)
+
+
+def test_a_pass_refuses_sizes_that_would_leave_its_buffers(built_library):
+    """fewer logit rows than prompts that can end in a pass (metadata and logits would be written past their ends), counts below
+    zero or beyond what 32-bit indices hold, empty dimensions"""
+    from vesta_gpu_b200 import launch
+    L, n = launch.lib(), ctypes.c_size_t()
+
+    def sizes(**kw):
+        d = pass_desc(**kw)
+        return L.vesta_pass_workspace(ctypes.byref(d), ctypes.byref(n))
+    assert sizes() == 0 and sizes(prompts=4, rows=64, logit_rows=4) == 0 and sizes(prompts=40, rows=16, logit_rows=16) == 0
+    for bad in (dict(prompts=4, rows=64, logit_rows=3), dict(prompts=40, rows=16, logit_rows=15), dict(prompts=-1), dict(logit_rows=17), dict(rows=0),
+                dict(rows=2 ** 31 - 1), dict(D=0, H=0), dict(F=0), dict(F=-16), dict(tmax=0), dict(cpos=0), dict(exact=1, rows=17, logit_rows=17)):
+        assert sizes(**bad) != 0 and L.vesta_last_error().startswith(b'vesta_pass'), bad

@@ -3,6 +3,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <algorithm>
+#include <exception>
 #include <string>
 #include <vector>
 
@@ -135,8 +136,9 @@ Layout layout(const Pass& p, int D, int F, int rows, int lrows) {
 }
 
 int plan(Pass& p, const vesta_pass_desc* d) {
-    if (!d || d->rows < 1 || d->logit_rows < 1 || d->logit_rows > d->rows) return fail(-1, "vesta_pass: bad row counts");
-    if (d->L < 1 || d->D % 64 || d->D > 4096 || d->H * 64 != d->D || d->F % 16 || d->N < 1) return fail(-1, "vesta_pass: sizes outside the supported family");
+    if (!d || d->rows < 1 || d->rows > 1 << 28 || d->logit_rows < 1 || d->logit_rows > d->rows) return fail(-1, "vesta_pass: bad row counts");
+    if (d->prompts < 0 || (d->prompts && d->logit_rows < std::min(d->rows, d->prompts))) return fail(-1, "vesta_pass: a pass over prompts needs a logit row for every prompt that can end in it");
+    if (d->L < 1 || d->D < 64 || d->D % 64 || d->D > 4096 || d->H * 64 != d->D || d->F < 16 || d->F % 16 || d->N < 1 || d->tmax < 1 || d->cpos < 1) return fail(-1, "vesta_pass: sizes outside the supported family");
     if (d->exact && d->rows > 16) return fail(-1, "vesta_pass: fp32-accurate operands are kept for at most 16 rows");
     p.d = *d;
     p.dev = 0;
@@ -339,48 +341,18 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
     return 0;
 }
 
-}  // namespace
-
-namespace vesta_rt {
-namespace {
-// the device of a pass for the calls of a scope (launches go to a stream of the current device)
-struct OnDevice {
-    int was = 0, dev;
-    explicit OnDevice(int d) : dev(d) { if (cudaGetDevice(&was) == cudaSuccess && was != dev) cudaSetDevice(dev); }
-    ~OnDevice() { if (was != dev) cudaSetDevice(was); }
-};
-}
-int pass_steps(void* pass, void* stream, int steps) {
-    Pass* p = (Pass*)pass;
-    const OnDevice on(p->dev);
-    cudaStream_t st = (cudaStream_t)stream;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    TRY(cudaStreamIsCapturing(st, &cap));
-    for (int i = 0; i < steps; i++) {
-        if (cap != cudaStreamCaptureStatusNone || p->graphs.empty()) { if (int e = enqueue(*p, st, p->d.rows, p->d.logit_rows, 0)) return e; }
-        else TRY(cudaGraphLaunch(p->graphs[0], st));
-    }
-    return 0;
-}
-}  // namespace vesta_rt
-
-extern "C" {
-
-int vesta_pass_workspace(const vesta_pass_desc* d, size_t* bytes) {
-    Pass p{};
-    if (!bytes) return fail(-1, "vesta_pass_workspace: null argument");
-    if (int e = plan(p, d)) return e;
-    *bytes = p.o.total;
-    return 0;
+// No exception leaves an entry of the library.
+template <class F> int guarded(F f) {
+    try { return f(); }
+    catch (const std::exception& e) { return fail(-1, e.what()); }
 }
 
-int vesta_pass_create(const vesta_pass_desc* d, void* workspace, int graph, void** out) {
-    if (!out || !workspace) return fail(-1, "vesta_pass_create: null argument");
-    Pass* p = new Pass{};
+// sizes, tensor maps and, for decode steps, the graph of a pass
+int make(Pass* p, const vesta_pass_desc* d, unsigned char* workspace, bool graph) {
     int e = plan(*p, d);
     if (!e) e = check(*d);
     if (!e && (size_t)workspace % 256) e = fail(-1, "vesta_pass: the workspace starts on a 256-byte boundary");
-    p->ws = (unsigned char*)workspace;
+    p->ws = workspace;
     if (!e) { const cudaError_t ce = prepare_all(); if (ce != cudaSuccess) e = cuda_fail(ce, "cudaFuncSetAttribute"); }
     if (!e && d->prompts) {
         const unsigned long long D = d->D, planes = (unsigned long long)d->prompts * d->L;
@@ -396,7 +368,7 @@ int vesta_pass_create(const vesta_pass_desc* d, void* workspace, int graph, void
         cudaError_t ce = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
         if (ce == cudaSuccess) ce = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
         if (ce == cudaSuccess) {
-            e = enqueue(*p, st, d->rows, d->logit_rows, 0);
+            e = guarded([&] { return enqueue(*p, st, d->rows, d->logit_rows, 0); });      // (the capture ends whatever happens in it)
             ce = cudaStreamEndCapture(st, &g);
         }
         if (ce == cudaSuccess && !e) ce = cudaGraphInstantiate(&ge, g, 0);
@@ -405,16 +377,12 @@ int vesta_pass_create(const vesta_pass_desc* d, void* workspace, int graph, void
         if (st) cudaStreamDestroy(st);
         if (ce != cudaSuccess && !e) e = cuda_fail(ce, "vesta_pass_create: graph of a step");
     }
-    if (e) { vesta_pass_release(p); return e; }
-    *out = p;
-    return 0;
+    return e;
 }
 
-int vesta_pass_prompts(void* pass, void* stream, const int* tokens, int ld, const int* lens, unsigned* status) {
-    Pass* p = (Pass*)pass;
-    if (!p || !p->d.prompts || !tokens || !lens || !status) return fail(-1, "vesta_pass_prompts: bad argument");
+// whole prompts: the passes of a call, their metadata and the status word
+int read_prompts(Pass* p, cudaStream_t st, const int* tokens, int ld, const int* lens, unsigned* status) {
     const vesta_pass_desc& d = p->d;
-    cudaStream_t st = (cudaStream_t)stream;
     const int B = d.prompts;
     const Meta mt(d.rows, d.logit_rows, B);
     long long total = 0;
@@ -464,6 +432,59 @@ int vesta_pass_prompts(void* pass, void* stream, const int* tokens, int ld, cons
     TRY(cudaStreamSynchronize(st));
     *status = *word;
     return 0;
+}
+
+}  // namespace
+
+namespace vesta_rt {
+namespace {
+// the device of a pass for the calls of a scope (launches go to a stream of the current device)
+struct OnDevice {
+    int was = 0, dev;
+    explicit OnDevice(int d) : dev(d) { if (cudaGetDevice(&was) == cudaSuccess && was != dev) cudaSetDevice(dev); }
+    ~OnDevice() { if (was != dev) cudaSetDevice(was); }
+};
+}
+int pass_steps(void* pass, void* stream, int steps) {
+    Pass* p = (Pass*)pass;
+    const OnDevice on(p->dev);
+    cudaStream_t st = (cudaStream_t)stream;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    TRY(cudaStreamIsCapturing(st, &cap));
+    return guarded([&]() -> int {
+        for (int i = 0; i < steps; i++) {
+            if (cap != cudaStreamCaptureStatusNone || p->graphs.empty()) { if (int e = enqueue(*p, st, p->d.rows, p->d.logit_rows, 0)) return e; }
+            else TRY(cudaGraphLaunch(p->graphs[0], st));
+        }
+        return 0;
+    });
+}
+}  // namespace vesta_rt
+
+extern "C" {
+
+int vesta_pass_workspace(const vesta_pass_desc* d, size_t* bytes) {
+    Pass p{};
+    if (!bytes) return fail(-1, "vesta_pass_workspace: null argument");
+    if (int e = plan(p, d)) return e;
+    *bytes = p.o.total;
+    return 0;
+}
+
+int vesta_pass_create(const vesta_pass_desc* d, void* workspace, int graph, void** out) {
+    if (!out || !workspace) return fail(-1, "vesta_pass_create: null argument");
+    Pass* p = nullptr;
+    if (const int e = guarded([&] { p = new Pass{}; return make(p, d, (unsigned char*)workspace, graph != 0); })) { vesta_pass_release(p); return e; }
+    *out = p;
+    return 0;
+}
+
+int vesta_pass_prompts(void* pass, void* stream, const int* tokens, int ld, const int* lens, unsigned* status) {
+    Pass* p = (Pass*)pass;
+    if (!p || !p->d.prompts || !tokens || !lens || !status) return fail(-1, "vesta_pass_prompts: bad argument");
+    const int e = guarded([&] { return read_prompts(p, (cudaStream_t)stream, tokens, ld, lens, status); });
+    if (e) cudaStreamSynchronize((cudaStream_t)stream);                  // (the next call writes the pinned metadata that copies may still read)
+    return e;
 }
 
 int vesta_pass_wait_limit(void* pass, unsigned long long ns) {

@@ -7,6 +7,7 @@
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -353,7 +354,8 @@ int vesta_step_run_fused(void* bound, void* stream, int steps, int per_launch) {
 
 int vesta_pass_bind(void* pass, void** bound) {
     if (!pass || !bound) return fail(-1, "vesta_pass_bind: null argument");
-    Bound* b = new Bound;
+    Bound* b = new (std::nothrow) Bound;
+    if (!b) return fail(-1, "out of host memory");
     b->pass = pass;
     *bound = b;
     return 0;
