@@ -289,3 +289,28 @@ def test_prompts_with_weights_off_a_16_byte_boundary():
         assert (m.keys.float() - v.keys.float()).abs().max() <= 4e-3 and m.keys.any()
         for w in (m, v):
             w.W['wpe'].mul_(-1)
+
+
+@pytest.mark.parametrize('batch', [12, 70])
+def test_the_persistent_kernel_of_a_chain_by_its_argument_list(batch):
+    """Kernel.fn and Kernel.args belong together also where steps run as a chain: launched by hand they do the same step"""
+    import ctypes
+    from vesta_gpu_b200.launch import lib, ok
+    sh = shape('by hand')
+    m, _ = model(sh, 3, 'rich', batch, 20)
+    k, x = m.k, torch.arange(batch, dtype=torch.int32).cuda()
+    vals, kinds = k.args
+    assert k.chain and len(vals) == len(kinds) == len(m.low.params) + 7
+    m.x.copy_(x)
+    m.step()
+    logits, after = m.logits().clone(), m.x.clone()
+    m.reset()
+    m.x.copy_(x)
+    store = (ctypes.c_ulonglong * len(vals))(*vals)
+    at = (ctypes.c_void_p * len(vals))(*[ctypes.addressof(store) + 8 * i for i in range(len(vals))])
+    ok(lib().vesta_launch_cooperative(k.fn, k.grid, k.block, k.smem, torch.cuda.current_stream().cuda_stream, at))
+    assert (m.logits() - logits).abs().max() < 2 * TIGHT and int(m.t[0]) == 1
+    top = logits.topk(2, dim=1).values
+    sure = top[:, 0] - top[:, 1] > MARGIN
+    assert torch.equal(m.x[sure], after[sure])
+    k.check()

@@ -149,7 +149,7 @@ class Kernel:
             self.TS = torch.zeros(2048, dtype=torch.int64, device=self.device)
             self._module = self._packed = None
             self._copies = []                                    # (copy, original) of weights bound off a 16-byte boundary
-            self.args, self.keep, self._bound = None, None, None
+            self._vals = self._args = self._tm = self.keep = self._bound = None
             self.fuse = 16                                       # decode steps per launch in launch(steps > 1)
             self.feeds_back = '#define V_FEEDBACK 1' in lowered.src
             self.launches = 0
@@ -193,6 +193,21 @@ class Kernel:
     WP = property(lambda self: self._pack_once()[0])
     PT = property(lambda self: self._pack_once()[1])
 
+    @property
+    def TM(self):
+        """the TMA descriptors of the persistent kernel for the bound tensors, made at the first use"""
+        if self._tm is None and self.keep is not None:
+            self._tm = self.tensor_maps(self.keep)
+        return self._tm
+
+    @property
+    def args(self):
+        """the argument list of `fn` for the bound tensors, (values, types); None before bind()"""
+        if self._args is None and self._vals is not None:
+            vals = self._vals + [self.WP.data_ptr(), self.PT.data_ptr(), self.TM.data_ptr(), 1]
+            self._args = (tuple(vals), tuple([ctypes.c_void_p] * len(vals)))
+        return self._args
+
     def view(self, name):
         off, _, shape = self.lowered.scratch[name]
         n = 1
@@ -205,7 +220,6 @@ class Kernel:
     def bind(self, residue):
         """fix the argument list once (launches then cost one call) and pack the weights"""
         L = lib()
-        vals = []
         zeros = residue.get('_zeros')
         if 'zeros_len' in self.lowered.dims and zeros is None and any(name == '_zeros' for name, _, _ in self.lowered.params):
             # additive parameters the program does not have (lower.OPTIONAL_TERMS): the kernel reads zeros for them
@@ -218,30 +232,25 @@ class Kernel:
         from .passes import VECTORS, WEIGHTS, aligned
         # (the persistent kernels read the matrices and the position table element by element)
         here, copies = aligned(self.lowered, residue, WEIGHTS[1:] if self.chain else VECTORS)
-        vals += [here[name].data_ptr() for name, _, _ in self.lowered.params]
-        self.keep, self._copies = residue, copies
         if self._bound:
             L.vesta_step_release(self._bound)
             self._bound = None
-        bound = ctypes.c_void_p()
+        self._vals = [here[name].data_ptr() for name, _, _ in self.lowered.params] + [self.S.data_ptr(), self.bar.data_ptr(), self.TS.data_ptr()]
+        self.keep, self._copies, self._args, self._tm = residue, copies, None, None
         if self.chain:
             from .passes import bind_step
-            vals += [self.S.data_ptr(), self.bar.data_ptr(), self.TS.data_ptr()]
             with torch.cuda.device(self.device):
                 self._bound, self._pass, self._work = bind_step(self, here, zeros)
             if self._packed is not None:
                 self.pack(residue)
         else:
-            self.TM = self.tensor_maps(residue)
-            self.keep = None
-            wp, pt = self._pack_once()
-            self.keep = residue
-            vals += [self.S.data_ptr(), self.bar.data_ptr(), self.TS.data_ptr(), wp.data_ptr(), pt.data_ptr(), self.TM.data_ptr(), 1]
+            if self._packed is not None:
+                self.pack(residue)
+            vals = self.args[0]                                  # (packs, the first time)
             arr = (ctypes.c_ulonglong * len(vals))(*vals)
+            bound = ctypes.c_void_p()
             ok(L.vesta_step_bind(self.fn, self.grid, self.block, self.smem, len(vals), arr, ctypes.byref(bound)))
             self._bound = bound
-            self.pack(residue)
-        self.args = (tuple(vals), tuple([ctypes.c_void_p] * len(vals)))
 
     def tensor_maps(self, residue):
         """the TMA descriptors of the step kernel, in device memory: the caches as the attention phase reads
