@@ -314,3 +314,28 @@ def test_the_persistent_kernel_of_a_chain_by_its_argument_list(batch):
     sure = top[:, 0] - top[:, 1] > MARGIN
     assert torch.equal(m.x[sure], after[sure])
     k.check()
+
+
+def test_binding_a_chain_again():
+    """other tensors, one call per step as the reference has it, then launches again: the same workspace throughout (a step that
+    runs on another stream keeps its memory), the same steps as a model's"""
+    from vesta_gpu_b200.launch import Kernel
+    sh = shape('again')
+    m, _ = model(sh, 3, 'rich', 12, 20)
+    k = Kernel(m.low, device=m.device.index)
+    own = lambda: dict(m.k.keep, **{n: torch.zeros_like(m.k.keep[n]) for n in ('x', 't', 'keys', 'vals')})
+    R, S = own(), own()
+    k.bind(R)
+    work = k._work.data_ptr()
+    k.launch()
+    k(S)
+    k(S)
+    k.launch(2)
+    k.bind(R)
+    k.launch(3)
+    assert k._work.data_ptr() == work
+    m.step(4)
+    assert int(R['t'][0]) == int(S['t'][0]) == int(m.t[0]) == 4
+    for T in (R, S):
+        assert (T['keys'].float() - m.keys.float()).abs().max() <= 4e-3 and torch.equal(T['x'], m.x)
+    k.check()

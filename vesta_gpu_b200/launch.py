@@ -148,7 +148,8 @@ class Kernel:
             self.bar = torch.zeros(lowered.counters, dtype=torch.int32, device=self.device)
             self.TS = torch.zeros(2048, dtype=torch.int64, device=self.device)
             self._module = self._packed = None
-            self._copies = []                                    # (copy, original) of weights bound off a 16-byte boundary
+            self._copies = {}                                    # (copy, original) of weights bound off a 16-byte boundary
+            self._work, self._direct = None, False               # a chain's workspace; its steps are launched kernel by kernel, no graph yet
             self._vals = self._args = self._tm = self.keep = self._bound = None
             self.fuse = 16                                       # decode steps per launch in launch(steps > 1)
             self.feeds_back = '#define V_FEEDBACK 1' in lowered.src
@@ -219,6 +220,9 @@ class Kernel:
 
     def bind(self, residue):
         """fix the argument list once (launches then cost one call) and pack the weights"""
+        self._bind(residue, graph=True)
+
+    def _bind(self, residue, graph):
         L = lib()
         zeros = residue.get('_zeros')
         if 'zeros_len' in self.lowered.dims and zeros is None and any(name == '_zeros' for name, _, _ in self.lowered.params):
@@ -231,16 +235,15 @@ class Kernel:
             assert t.device == self.device, (name, t.device)
         from .passes import VECTORS, WEIGHTS, aligned
         # (the persistent kernels read the matrices and the position table element by element)
-        here, copies = aligned(self.lowered, residue, WEIGHTS[1:] if self.chain else VECTORS)
+        here, copies = aligned(self.lowered, residue, WEIGHTS[1:] if self.chain else VECTORS, self._copies)
         if self._bound:
             L.vesta_step_release(self._bound)
             self._bound = None
         self._vals = [here[name].data_ptr() for name, _, _ in self.lowered.params] + [self.S.data_ptr(), self.bar.data_ptr(), self.TS.data_ptr()]
         self.keep, self._copies, self._args, self._tm = residue, copies, None, None
         if self.chain:
-            from .passes import bind_step
-            with torch.cuda.device(self.device):
-                self._bound, self._pass, self._work = bind_step(self, here, zeros)
+            self._here = here, zeros
+            self._bind_chain(graph)
             if self._packed is not None:
                 self.pack(residue)
         else:
@@ -251,6 +254,15 @@ class Kernel:
             bound = ctypes.c_void_p()
             ok(L.vesta_step_bind(self.fn, self.grid, self.block, self.smem, len(vals), arr, ctypes.byref(bound)))
             self._bound = bound
+
+    def _bind_chain(self, graph):
+        from .passes import bind_step
+        if self._bound:
+            lib().vesta_step_release(self._bound)
+            self._bound = None
+        with torch.cuda.device(self.device):
+            self._bound, self._pass, self._work = bind_step(self, *self._here, graph)
+        self._direct = not graph
 
     def tensor_maps(self, residue):
         """the TMA descriptors of the step kernel, in device memory: the caches as the attention phase reads
@@ -272,7 +284,7 @@ class Kernel:
         """(re)build the packed weight streams from the bound weights; call again after changing them (a chain reads the
         weights where they are: nothing to do but for weights that do not start on a 16-byte boundary, of which it reads a
         copy, unless its persistent kernel has been asked for)"""
-        for copy, original in self._copies:
+        for copy, original in self._copies.values():
             copy.copy_(original)
         if self.chain and self._packed is None:
             return
@@ -289,6 +301,11 @@ class Kernel:
         """`steps` decode steps on the current stream. With feedback on, up to `per_launch` steps (default
         Kernel.fuse) run inside one launch: the kernel feeds its own token and position between them, which saves
         the gap between launches; without feedback every step is its own launch."""
+        if self._direct and not torch.cuda.is_current_stream_capturing():
+            self._bind_chain(graph=True)
+        self._launch(steps, per_launch)
+
+    def _launch(self, steps, per_launch=None):
         stream = ctypes.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
         per = per_launch or self.fuse
         if steps > 1 and per > 1 and self.feeds_back:
@@ -303,6 +320,8 @@ class Kernel:
         (pinned), stream synchronised on return: a single call into the library (vesta_step_host)"""
         # (a host loop calls this once per step: the argument list is kept for the buffers of the last call, the stream
         # handle comes from torch's raw accessor)
+        if self._direct:
+            self._bind_chain(graph=True)
         key = (x_dev.data_ptr(), tokens_host.data_ptr(), result_dev.data_ptr(), result_host.data_ptr(), tokens_host.numel(), result_host.numel())
         if self._host_key != key:
             self._host_key = key
@@ -317,8 +336,11 @@ class Kernel:
         self.launches += 1
 
     def __call__(self, residue):
-        self.bind(residue)
-        self.launch()
+        # (a graph is made for more than one step: its capture and instantiation take longer than the launches of one. Nine sequences
+        # of the small shape: 788 -> 354 us per call,
+        # 64: 886 -> 410)
+        self._bind(residue, graph=False)
+        self._launch(1)
 
     def status(self):
         """0 if every launch so far ran to its end; otherwise a description of the first failure

@@ -23,19 +23,19 @@ class Desc(ctypes.Structure):
                [(n, ctypes.c_void_p) for n in _PTRS]
 
 
-def aligned(low, residue, roles):
-    """-> (`residue` as kernels that load 16 bytes at a time can read it, [(copy, original)]): the weights named by `roles` that do
-    not start on a 16-byte boundary (views into a larger buffer) are copied. The table and the caches are read and written
-    where they are: refused."""
-    out, copies = dict(residue), []
+def aligned(low, residue, roles, kept=()):
+    """-> (`residue` as kernels that load 16 bytes at a time can read it, {name: (copy, original)}): the weights named by `roles`
+    that do not start on a 16-byte boundary (views into a larger buffer) are copied, into the copies of `kept` where it has
+    them. The table and the caches are read and written where they are: refused."""
+    out, copies = dict(residue), {}
     for role in ('wte', 'keys', 'vals'):
         if residue[low.roles[role]].data_ptr() % 16:
             raise RuntimeError(f'{low.roles[role]} must start on a 16-byte boundary')
     for role in roles:
         name = low.roles[role]
         if name != ZEROS and residue[name].data_ptr() % 16:
-            out[name] = residue[name].clone()
-            copies.append((out[name], residue[name]))
+            out[name] = kept[name][0].copy_(residue[name]) if name in kept else residue[name].clone()
+            copies[name] = out[name], residue[name]
     return out, copies
 
 
@@ -54,18 +54,20 @@ def describe(low, residue, zeros, cpos, **kw):
     return desc
 
 
-def create(desc, device, graph=False):
-    """-> (handle, workspace tensor)"""
-    n = ctypes.c_size_t()
-    ok(lib().vesta_pass_workspace(ctypes.byref(desc), ctypes.byref(n)))
-    ws = torch.zeros(n.value, dtype=torch.uint8, device=device)
+def create(desc, device, graph=False, ws=None):
+    """-> (handle, workspace tensor). `ws`: the workspace of an earlier pass of the same sizes (every pass leaves it as it
+    found it): a step that still runs on another stream then keeps its memory, and nothing has to be cleared or awaited"""
+    if ws is None:
+        n = ctypes.c_size_t()
+        ok(lib().vesta_pass_workspace(ctypes.byref(desc), ctypes.byref(n)))
+        ws = torch.zeros(n.value, dtype=torch.uint8, device=device)
+        torch.cuda.current_stream(device).synchronize()
     h = ctypes.c_void_p()
-    torch.cuda.current_stream(device).synchronize() if graph else None
     ok(lib().vesta_pass_create(ctypes.byref(desc), ctypes.c_void_p(ws.data_ptr()), int(graph), ctypes.byref(h)))
     return h, ws
 
 
-def bind_step(kernel, residue, zeros):
+def bind_step(kernel, residue, zeros, graph):
     """a decode step over the tensors of `residue` as a chain of kernels -> (handle for vesta_step_run, the pass that it owns, workspace)"""
     low = kernel.lowered
     d, st = low.dims, low.dims['step']
@@ -75,7 +77,7 @@ def bind_step(kernel, residue, zeros):
                     tstep=st['tstep'], feedback=st['feedback'], prompt_len=st['prompt_len'], x=residue[low.roles['x']], t=residue[low.roles['t']],
                     prompt=residue['prompt'] if st['prompt_len'] else None, plen=residue['plen'] if st['prompt_len'] else None,
                     logits=logit, next=nxt, bar=kernel.bar)
-    h, ws = create(desc, kernel.device, graph=True)
+    h, ws = create(desc, kernel.device, graph, kernel._work)
     bound = ctypes.c_void_p()
     ok(lib().vesta_pass_bind(h, ctypes.byref(bound)))
     return bound, h, ws
@@ -106,7 +108,7 @@ class PromptPass:
     def run(self, tokens, lens):
         """tokens (B, P), lens (B,) int32 numpy: the caches, x and t of the model after the prompts"""
         tokens = np.ascontiguousarray(tokens, np.int32)
-        for copy, original in self.copies:
+        for copy, original in self.copies.values():
             copy.copy_(original)
         dev, status = self.model.device, ctypes.c_uint()
         at = tokens.__array_interface__['data'][0], tokens.shape[1], lens.__array_interface__['data'][0], ctypes.byref(status)
