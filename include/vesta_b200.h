@@ -107,7 +107,8 @@ int vesta_pass_create(const vesta_pass_desc* desc, void* workspace, int graph, v
  * prompt are zeroed), x gets the token chosen after every prompt, t its position; in passes of at most desc.rows rows.
  * Synchronises `stream`; *status as bar[0] (not zero: refused, a token outside the vocabulary). */
 int vesta_pass_prompts(void* pass, void* stream, const int* tokens, int ld, const int* lens, unsigned* status);
-/* A wait inside the kernels of a pass gives up after `ns` nanoseconds (0: half a second, the limit of a new pass); waits for the device. */
+/* A wait inside the kernels of a pass gives up after `ns` nanoseconds (0: half a second, the limit of a new pass), from the next step or
+ * prompts on. */
 int vesta_pass_wait_limit(void* pass, unsigned long long ns);
 /* a pass created with a graph as what vesta_step_run, vesta_step_run_fused and vesta_step_host take; owns the pass */
 int vesta_pass_bind(void* pass, void** bound);

@@ -21,12 +21,14 @@ int cuda_fail(cudaError_t e, const char* what) { return fail((int)e, std::string
 
 int up(long long v, int a) { return (int)((v + a - 1) / a * a); }
 
+const u64 WAIT_NS = 500000000ull;              // waits of a new pass give up after half a second
+
 enum Kind { K_QKV = 0, K_PROJ = 1, K_FC = 2, K_P2 = 3, K_LOGITS = 4 };
 
 struct Tile { int bm, bn, stages, splits; };
 
 struct Layout {
-    size_t z, q, act, att, gelu, fin, best, rowoff, pos, skip, limit;
+    size_t z, q, act, att, gelu, fin, best, rowoff, pos, skip;
     size_t meta, total;                        // prompts: tokens, positions, sequences of the rows; attention runs; rows that want logits and where they go; lengths
 };
 // the metadata of a pass over prompts, as offsets in 32-bit words
@@ -52,8 +54,9 @@ struct Pass {
     };
     std::vector<Plan> plans;                   // the last few
     CUtensorMap qmap, kmap, vmap;              // prompts: queries (two planes) and the caches, 128 rows of one head per box
-    std::vector<cudaGraphExec_t> graphs;       // decode: one step
+    cudaGraphExec_t graph;                     // decode: one step, or null
     int sms, dev;
+    u64 wait_ns;                               // limit of a wait
     int* host;                                 // prompts: pinned metadata, one copy per pass of a call, then a status word
     size_t host_words;
 };
@@ -129,7 +132,6 @@ Layout layout(const Pass& p, int D, int F, int rows, int lrows) {
     o.rowoff = take((size_t)rows * 8);
     o.pos = take((size_t)rows * 4);
     o.skip = take(4);
-    o.limit = take(8);
     o.meta = p.d.prompts ? take((size_t)Meta(rows, lrows, p.d.prompts).words * 4) : 0;
     o.total = at;
     return o;
@@ -142,6 +144,7 @@ int plan(Pass& p, const vesta_pass_desc* d) {
     if (d->exact && d->rows > 16) return fail(-1, "vesta_pass: fp32-accurate operands are kept for at most 16 rows");
     p.d = *d;
     p.dev = 0;
+    p.wait_ns = WAIT_NS;
     p.sms = 148;
     if (cudaGetDevice(&p.dev) == cudaSuccess) cudaDeviceGetAttribute(&p.sms, cudaDevAttrMultiProcessorCount, p.dev);
     cudaGetLastError();                          // (sizes can be asked for without a device)
@@ -287,7 +290,7 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
     auto mul = [&](int kind, int l) {
         const Tile& t = pl->tile[kind];
         GemmArgs g = {};
-        g.layer = l; g.D = D; g.rp = p.rp; g.stages = t.stages; g.status = (u32*)d.bar; g.limit = (const u64*)u(p.o.limit); g.skip = (const int*)u(p.o.skip);
+        g.layer = l; g.D = D; g.rp = p.rp; g.stages = t.stages; g.status = (u32*)d.bar; g.limit = p.wait_ns; g.skip = (const int*)u(p.o.skip);
         g.rows = kind == K_LOGITS ? lrows : rows;
         g.kblocks = kind == K_P2 ? kbf : kbd; g.kb_per = (g.kblocks + t.splits - 1) / t.splits;
         g.nfeat = kind == K_QKV ? 3 * D : kind == K_FC ? F : kind == K_LOGITS ? d.N : D;
@@ -309,7 +312,7 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
         const u16 *kc = (const u16*)d.keys + (size_t)l * d.tmax * D, *vc = (const u16*)d.vals + (size_t)l * d.tmax * D;
         const long long ss = (long long)L * d.tmax * D;
         if (many) {
-            AttManyArgs a = {(const int4*)(meta + mt.tiles), l, L, D, d.scale, att, (u32*)d.bar, (const u64*)u(p.o.limit)};
+            AttManyArgs a = {(const int4*)(meta + mt.tiles), l, L, D, d.scale, att, (u32*)d.bar, p.wait_ns};
             Config c(dim3(d.H, tiles), AM_THREADS, st, true);
             c.c.dynamicSmemBytes = AM_SMEM;
             return pow2 ? cudaLaunchKernelEx(&c.c, pass_attend_many<true>, p.qmap, p.kmap, p.vmap, a) : cudaLaunchKernelEx(&c.c, pass_attend_many<false>, p.qmap, p.kmap, p.vmap, a);
@@ -347,6 +350,28 @@ template <class F> int guarded(F f) {
     catch (const std::exception& e) { return fail(-1, e.what()); }
 }
 
+// a decode step as a graph, captured on a stream of its own, in place of the one that the pass has
+int capture(Pass* p) {
+    cudaStream_t st = nullptr;
+    cudaGraph_t g = nullptr;
+    cudaGraphExec_t ge = nullptr;
+    int e = 0;
+    cudaError_t ce = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+    if (ce == cudaSuccess) ce = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
+    if (ce == cudaSuccess) {
+        e = guarded([&] { return enqueue(*p, st, p->d.rows, p->d.logit_rows, 0); });      // (the capture ends whatever happens in it)
+        ce = cudaStreamEndCapture(st, &g);
+    }
+    if (ce == cudaSuccess && !e) ce = cudaGraphInstantiate(&ge, g, 0);
+    if (ge) {
+        if (p->graph) cudaGraphExecDestroy(p->graph);
+        p->graph = ge;
+    }
+    if (g) cudaGraphDestroy(g);
+    if (st) cudaStreamDestroy(st);
+    return ce != cudaSuccess && !e ? cuda_fail(ce, "vesta_pass: graph of a step") : e;
+}
+
 // sizes, tensor maps and, for decode steps, the graph of a pass
 int make(Pass* p, const vesta_pass_desc* d, unsigned char* workspace, bool graph) {
     int e = plan(*p, d);
@@ -360,23 +385,7 @@ int make(Pass* p, const vesta_pass_desc* d, unsigned char* workspace, bool graph
         if (!e) e = vesta_rt::tensor_map(&p->qmap, p->ws + p->o.q, D, d->rows, 2, D * 2, D * 2 * d->rows, 128, 1);
         if (!e) e = vesta_rt::tensor_map(&p->vmap, d->vals, D, d->tmax, planes, D * 2, D * 2 * d->tmax, 128, 1);
     }
-    if (!e && graph) {
-        // a decode step as a graph, captured on a stream of its own
-        cudaStream_t st = nullptr;
-        cudaGraph_t g = nullptr;
-        cudaGraphExec_t ge = nullptr;
-        cudaError_t ce = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-        if (ce == cudaSuccess) ce = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
-        if (ce == cudaSuccess) {
-            e = guarded([&] { return enqueue(*p, st, d->rows, d->logit_rows, 0); });      // (the capture ends whatever happens in it)
-            ce = cudaStreamEndCapture(st, &g);
-        }
-        if (ce == cudaSuccess && !e) ce = cudaGraphInstantiate(&ge, g, 0);
-        if (ge) p->graphs.push_back(ge);
-        if (g) cudaGraphDestroy(g);
-        if (st) cudaStreamDestroy(st);
-        if (ce != cudaSuccess && !e) e = cuda_fail(ce, "vesta_pass_create: graph of a step");
-    }
+    if (!e && graph) e = capture(p);
     return e;
 }
 
@@ -453,8 +462,8 @@ int pass_steps(void* pass, void* stream, int steps) {
     TRY(cudaStreamIsCapturing(st, &cap));
     return guarded([&]() -> int {
         for (int i = 0; i < steps; i++) {
-            if (cap != cudaStreamCaptureStatusNone || p->graphs.empty()) { if (int e = enqueue(*p, st, p->d.rows, p->d.logit_rows, 0)) return e; }
-            else TRY(cudaGraphLaunch(p->graphs[0], st));
+            if (cap != cudaStreamCaptureStatusNone || !p->graph) { if (int e = enqueue(*p, st, p->d.rows, p->d.logit_rows, 0)) return e; }
+            else TRY(cudaGraphLaunch(p->graph, st));
         }
         return 0;
     });
@@ -491,14 +500,14 @@ int vesta_pass_wait_limit(void* pass, unsigned long long ns) {
     Pass* p = (Pass*)pass;
     if (!p) return fail(-1, "vesta_pass_wait_limit: null argument");
     const vesta_rt::OnDevice on(p->dev);
-    TRY(cudaMemcpy(p->ws + p->o.limit, &ns, 8, cudaMemcpyHostToDevice));
-    return 0;
+    p->wait_ns = ns ? ns : WAIT_NS;
+    return p->graph ? capture(p) : 0;
 }
 
 void vesta_pass_release(void* pass) {
     Pass* p = (Pass*)pass;
     if (!p) return;
-    for (auto g : p->graphs) cudaGraphExecDestroy(g);
+    if (p->graph) cudaGraphExecDestroy(p->graph);
     if (p->host) cudaFreeHost(p->host);
     delete p;
 }

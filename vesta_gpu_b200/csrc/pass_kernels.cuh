@@ -72,21 +72,25 @@ __device__ __forceinline__ u32 elect_one() {
     return leader;
 }
 
-// Every wait gives up after half a second (or `*limit` nanoseconds, where that is not zero): it leaves a code in the status word,
-// a flag that ends the other waits of the block (of the pair: `peer` is the flag of the other block) and the abort flag: this pass
-// publishes no token or position, and every later one is refused. The block runs to its end: a warp whose wait gave up goes on
-// through the barriers that other warps of the block wait at, and does nothing between them.
-#define PASS_WAIT_NS 500000000ull
-struct Wait { volatile int* dead; u32* status; const u64* limit; u32 peer; };
-__device__ __noinline__ bool mbar_wait_slow(u32 bar, u32 parity, const Wait& w, u32 code) {
-    const u64 t0 = now_ns(), set = __ldcg(w.limit), limit = set ? set : PASS_WAIT_NS;
+// Every wait gives up after `limit` nanoseconds (half a second): it leaves a code in the status word, a flag that ends the other
+// waits of the block (of the pair: `peer` is the flag of the other block) and the abort flag: this pass publishes no token or
+// position, and every later one is refused. The block runs to its end: a warp whose wait gave up goes on through the
+// barriers that other warps of the block wait at, and does nothing between them.
+struct Wait { u32 dead, peer; u32* status; u64 limit; };
+// (All by value, and the limit a parameter of the kernel: a structure passed by reference gave every kernel a stack frame, and a
+// limit read from memory here held up the next try: together 0.2 to 0.6 us per contraction, 16 sequences of the XL shape
+// 5,064 -> 5,257 us per four steps, 8 x 128 prompts 576 -> 600.)
+__device__ __noinline__ bool mbar_wait_slow(u32 bar, u32 parity, u32 code, u32 dead, u32 peer, u32* status, u64 limit) {
+    const u64 t0 = now_ns();
     while (!mbar_try(bar, parity)) {                     // (a try holds the thread for up to 4 us)
-        if (*w.dead) return false;
+        u32 over;
+        asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(over) : "r"(dead) : "memory");
+        if (over) return false;
         if (now_ns() - t0 > limit) {
-            atomicCAS(w.status, 0u, code | (blockIdx.x << 16));
-            atomicExch(w.status + 2, 1u);
-            *w.dead = 1;
-            if (w.peer) asm volatile("st.shared::cluster.u32 [%0], %1;" :: "r"(w.peer), "r"(1u) : "memory");
+            atomicCAS(status, 0u, code | (blockIdx.x << 16));
+            atomicExch(status + 2, 1u);
+            asm volatile("st.volatile.shared.u32 [%0], %1;" :: "r"(dead), "r"(1u) : "memory");
+            if (peer) asm volatile("st.shared::cluster.u32 [%0], %1;" :: "r"(peer), "r"(1u) : "memory");
             return false;
         }
     }
@@ -98,7 +102,7 @@ __device__ __noinline__ void settle() {
     const u64 t0 = now_ns();
     while (now_ns() - t0 < 2000000ull) { }
 }
-__device__ __forceinline__ bool mbar_wait(u32 bar, u32 parity, const Wait& w, u32 code) { return mbar_try(bar, parity) || mbar_wait_slow(bar, parity, w, code); }
+__device__ __forceinline__ bool mbar_wait(u32 bar, u32 parity, const Wait& w, u32 code) { return mbar_try(bar, parity) || mbar_wait_slow(bar, parity, code, w.dead, w.peer, w.status, w.limit); }
 
 // ---- contractions ---------------------------------------------------------------------------------------------------
 enum { EPI_QKV = 0, EPI_ADD = 1, EPI_GELU = 2, EPI_LOGITS = 3 };
@@ -116,7 +120,7 @@ struct GemmArgs {
     const int* skip;                 // not zero: the pass was refused, nothing may be written that outlives it
     u64* best;                       // LOGITS: packed (value, ~index) maximum of every row
     u32* status;
-    const u64* limit;                // of a wait
+    u64 limit;                       // of a wait, ns
     float a2, k1, k2;                // GELU: see gelu_tanh; QKV, prompts: a2 = 1 / scale where that is a power of two
     // QKV, prompts: one more warp zeroes this layer's cache rows behind the first lens[sequence], which this pass writes
     const int* lens;
@@ -221,7 +225,7 @@ __global__ void __launch_bounds__(GemmShape<BM>::THREADS + (EPI == EPI_QKV ? 32 
     const int t_first = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, t_step = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
     const bool two = g.ntiles > t_step;
     const int cols = S::columns(bn, two);
-    const Wait w{dead, g.status, g.limit, PAIR ? of_block(smem_u32(tail + 4), rank ^ 1) : 0u};
+    const Wait w{smem_u32(tail + 4), PAIR ? of_block(smem_u32(tail + 4), rank ^ 1) : 0u, g.status, g.limit};
     if (threadIdx.x == 0) {
         *dead = 0;
         for (int i = 0; i < st; i++) { mbar_init(bars + i * 8, 1); mbar_init(bars + (st + i) * 8, 1); }
@@ -837,7 +841,7 @@ struct AttManyArgs {
     float scale;
     u16* out;                        // [row][D] fp16
     u32* status;
-    const u64* limit;                // of a wait
+    u64 limit;                       // of a wait, ns
 };
 __device__ __forceinline__ void tm_ld32(u32 (&r)[32], u32 addr) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
@@ -879,7 +883,7 @@ __global__ void __launch_bounds__(AM_THREADS, 2) pass_attend_many(const __grid_c
     volatile int* dead = reinterpret_cast<volatile int*>(tail + 4);
     float* pair = reinterpret_cast<float*>(tail + 16);                             // [tile & 1][half][row]: maxima, at the end sums
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-    const Wait w{dead, a.status, a.limit, 0u};
+    const Wait w{smem_u32(tail + 4), 0u, a.status, a.limit};
     if (threadIdx.x == 0) {
         *dead = 0;
         mbar_init(qf, 1); mbar_init(sf, 1); mbar_init(pf, 8); mbar_init(of, 1);
