@@ -407,6 +407,7 @@ class Run:
         the reference's protocol of one position per step; -> dict or None (ragged workloads feed prompts on the device)"""
         if self.ragged:
             return None
+        from vesta_gpu_b200.passes import tiles
         torch, m = self.torch, self.m
         prompts = self.pd.cpu().numpy()
 
@@ -419,13 +420,13 @@ class Run:
                 torch.cuda.synchronize()
                 out.append(e0.elapsed_time(e1))
             return statistics.median(out)
-        m.prefill(prompts); torch.cuda.synchronize()              # builds the second lowering and its weight image, untimed
+        m.prefill(prompts); torch.cuda.synchronize()              # makes the pass and its workspace, untimed
         dense = timed(lambda: m.prefill(prompts))
         first_dense = m.x.clone()
         step = timed(self.prefill)
         rows = max(m._prefill_engines)
         return dict(positions=int(prompts.size), dense_ms=dense, one_position_per_step_ms=step, rows_per_launch=rows,
-                    tensor_core_contractions=bool(m._prefill_engines[rows].low.dims['tcl']),
+                    contraction_tiles=tiles(m._prefill_engines[rows].desc, min(rows, int(prompts.size)), m.B),
                     first_tokens_equal=round(float((first_dense == m.x).float().mean()), 4))
 
     def bytes_per_step(self):

@@ -100,6 +100,9 @@ typedef struct vesta_pass_desc {
     void *bar;                          /* status words: [0] status, [2] abort flag */
 } vesta_pass_desc;
 int vesta_pass_workspace(const vesta_pass_desc* desc, size_t* bytes);
+/* The tiles that a pass takes for `rows` rows of which `logit_rows` want logits: for QKV, projection, FC, MLP projection and logits
+ * the features and rows of a tile, stages, parts of the fold and shared memory of a block: out[25]. No device needed. */
+int vesta_pass_tiles(const vesta_pass_desc* desc, int rows, int logit_rows, int* out);
 /* workspace: that many bytes of device memory, zeroed, on a 256-byte boundary (matrices, table and caches: 16 bytes, norm
  * parameters and wpe: 8 bytes; anything else is refused). graph != 0: the pass is a decode step, kept as a CUDA graph. */
 int vesta_pass_create(const vesta_pass_desc* desc, void* workspace, int graph, void** pass);

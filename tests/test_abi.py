@@ -145,3 +145,23 @@ def test_a_pass_refuses_sizes_that_would_leave_its_buffers(built_library):
     for bad in (dict(prompts=4, rows=64, logit_rows=3), dict(prompts=40, rows=16, logit_rows=15), dict(prompts=-1), dict(logit_rows=17), dict(rows=0),
                 dict(rows=2 ** 31 - 1), dict(D=0, H=0), dict(F=0), dict(F=-16), dict(tmax=0), dict(cpos=0), dict(exact=1, rows=17, logit_rows=17)):
         assert sizes(**bad) != 0 and L.vesta_last_error().startswith(b'vesta_pass'), bad
+
+
+@pytest.mark.parametrize('name,exact', [('gpt2', 0), ('gpt2_xl', 0), ('tiny3', 0), ('heads20', 0), ('gpt2', 1), ('tiny', 1)])
+def test_tiles_of_a_pass_fit_a_block(built_library, name, exact):
+    """every tile that is chosen is one the kernels are written for: the rows of one product, the columns of tensor memory (two
+    accumulators), shared memory, no empty part of a fold; rows at fp32 accuracy in one tile of head and remainder"""
+    from vesta_gpu_b200.passes import tiles
+    from vesta_gpu_b200.shapes import SHAPES
+    sh = SHAPES[name]
+    for rows in ([1, 3, 8, 9, 16] if exact else [1, 15, 16, 17, 23, 64, 65, 100, 128, 129, 256, 1000, 1024, 4097, 9200, 16384]):
+        lrows = min(rows, 256)
+        d = pass_desc(L=sh.L, D=sh.D, H=sh.H, F=sh.F, N=sh.N, rows=rows, logit_rows=lrows, exact=exact, prompts=0 if exact else lrows)
+        for kind, (bm, bn, stages, parts, smem) in tiles(d, rows, lrows).items():
+            at, blocks = (name, rows, kind), (-(-sh.F // 64) if kind == 'p2' else sh.D // 64)
+            assert bm in (64, 128, 256) and bn % 16 == 0 and 16 <= bn <= (64 if bm == 64 else 256), at
+            assert stages >= 1 and smem <= 227 * 1024, at
+            assert 1 <= parts <= (12 if kind in ('proj', 'p2') else 1) and -(-blocks // -(-blocks // parts)) == parts, at
+            assert bm != 256 or (bn >= 64 and kind != 'logits'), at
+            if exact:
+                assert (bm, bn) == (64, 2 * (8 if rows <= 8 else 16)), at

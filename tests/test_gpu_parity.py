@@ -548,8 +548,7 @@ def test_dense_prefill_equals_the_oracle(shape_name, batch, rows):
     m.prefill(toks[:, :pmax], lens, rows=rows)
     m.k.check()
     assert m.t.cpu().numpy().tolist() == lens.tolist()
-    if shape_name == 'tiny':
-        assert m._prefill_engines[rows].low.dims['tcl']               # tensor-core contractions at widths of 128
+    assert list(m._prefill_engines) == [rows]                         # one pass object of so many rows read them all
     W = O.upcast(hf.weights)
     first = m.x.cpu().numpy()
     keys = m.keys.float().cpu().numpy()
@@ -582,7 +581,11 @@ def test_dense_prefill_at_full_size_against_the_reference(rows):
     B, P = prompts.shape
     m, _ = model(sh, seed, init, B, P + 16)
     m.prefill(prompts, rows=rows)
-    assert m._prefill_engines[rows or 1024].low.dims['tcl']
+    eng, = m._prefill_engines.values()
+    assert eng.R == (rows or 1024)
+    from vesta_gpu_b200.passes import tiles
+    full = [t[0] for k, t in tiles(eng.desc, eng.R, B).items() if k != 'logits']
+    assert rows or min(full) >= 128, full                             # 1,024 rows: products of 128 features and more in every layer contraction
     toks = [m.x.clone()]
     for _ in range(11):
         m.step(); toks.append(m.x.clone())

@@ -221,19 +221,26 @@ struct Config {
     }
 };
 
+// the tile of contraction `k` for `rows` rows of which `lrows` want logits
+Tile tile_of(const Pass& p, int k, int rows, int lrows) {
+    const vesta_pass_desc& d = p.d;
+    const int feat[5] = {3 * d.D, d.D, d.F, d.D, d.N};
+    return choose(k, k == K_LOGITS ? std::max(lrows, 1) : rows, p.rp, feat[k], k == K_P2 ? (d.F + 63) / 64 : d.D / 64, p.sms);
+}
+
 // The tiles and tensor maps for `rows` rows of which `lrows` want logits.
 int plan_for(Pass& p, int rows, int lrows, const Pass::Plan** out) {
     for (auto& q : p.plans) if (q.rows == rows && q.lrows == lrows) { *out = &q; return 0; }
     if (p.plans.size() >= 8) p.plans.erase(p.plans.begin());
     const vesta_pass_desc& d = p.d;
-    const int D = d.D, F = d.F, kbd = D / 64, kbf = (F + 63) / 64;
+    const int D = d.D, F = d.F;
     Pass::Plan q;
     q.rows = rows; q.lrows = lrows;
     const void* w[5] = {d.qkvw, d.ow, d.fcw, d.pw, d.wte};
-    const int fold[5] = {D, D, D, F, D}, pitch[5] = {D, D, D, up(F, 64), D}, feat[5] = {3 * D, D, F, D, d.N}, kb[5] = {kbd, kbd, kbd, kbf, kbd};
+    const int fold[5] = {D, D, D, F, D}, pitch[5] = {D, D, D, up(F, 64), D}, feat[5] = {3 * D, D, F, D, d.N};
     const size_t op[5] = {p.o.act, p.o.att, p.o.act, p.o.gelu, p.o.fin};
     for (int k = 0; k < 5; k++) {
-        const Tile t = q.tile[k] = choose(k, k == K_LOGITS ? std::max(lrows, 1) : rows, p.rp, feat[k], kb[k], p.sms);
+        const Tile t = q.tile[k] = tile_of(p, k, rows, lrows);
         int e;
         if (k == K_LOGITS) e = vesta_rt::fold_map(&q.w[k], w[k], D, feat[k], t.bm, k_blocks(t.bm));
         else e = vesta_rt::tensor_map(&q.w[k], w[k], feat[k], fold[k], d.L, (size_t)feat[k] * 2, (size_t)feat[k] * fold[k] * 2, 64 * k_blocks(t.bm), 1);
@@ -477,6 +484,18 @@ int vesta_pass_workspace(const vesta_pass_desc* d, size_t* bytes) {
     if (!bytes) return fail(-1, "vesta_pass_workspace: null argument");
     if (int e = plan(p, d)) return e;
     *bytes = p.o.total;
+    return 0;
+}
+
+int vesta_pass_tiles(const vesta_pass_desc* d, int rows, int logit_rows, int* out) {
+    Pass p{};
+    if (!out || !d || rows < 1 || rows > d->rows || logit_rows < 0 || logit_rows > d->logit_rows) return fail(-1, "vesta_pass_tiles: bad argument");
+    if (int e = plan(p, d)) return e;
+    for (int k = 0; k < 5; k++) {
+        const Tile t = tile_of(p, k, rows, logit_rows);
+        const int v[5] = {t.bm, t.bn, t.stages, t.splits, t.bm == 64 ? GemmShape<64>::bytes(t.stages, t.bn) : t.bm == 128 ? GemmShape<128>::bytes(t.stages, t.bn) : GemmShape<256>::bytes(t.stages, t.bn)};
+        std::copy(v, v + 5, out + 5 * k);
+    }
     return 0;
 }
 

@@ -57,6 +57,7 @@ def lib():
         L.vesta_step_release.argtypes = [vp]
         L.vesta_step_release.restype = None
         L.vesta_pass_workspace.argtypes = [vp, ctypes.POINTER(sz)]
+        L.vesta_pass_tiles.argtypes = [vp, ci, ci, ctypes.POINTER(ci)]
         L.vesta_pass_create.argtypes = [vp, vp, ci, ctypes.POINTER(vp)]
         L.vesta_pass_prompts.argtypes = [vp, vp, vp, ci, vp, ctypes.POINTER(cu)]
         L.vesta_pass_wait_limit.argtypes = [vp, ctypes.c_ulonglong]

@@ -7,7 +7,7 @@ import numpy as np
 import torch
 
 from .launch import STATUS_WHERE, lib, ok
-from .lower import Lowered, ZEROS
+from .lower import ZEROS
 
 _PTRS = ('wte', 'wpe', 'ln1w', 'ln1b', 'qkvw', 'qkvb', 'ow', 'ob', 'ln2w', 'ln2b', 'fcw', 'fcb', 'pw', 'pb', 'lnfw', 'lnfb',
          'keys', 'vals', 'x', 't', 'prompt', 'plen', 'logits', 'next', 'bar')
@@ -52,6 +52,14 @@ def describe(low, residue, zeros, cpos, **kw):
         if v is not None:
             setattr(desc, k, v.data_ptr() if isinstance(v, torch.Tensor) else v)
     return desc
+
+
+def tiles(desc, rows, logit_rows):
+    """the tiles of the contractions of a pass over `rows` rows of which `logit_rows` want logits: for 'qkv', 'proj', 'fc', 'p2' and
+    'logits' (features, rows, stages, parts of the fold, bytes of shared memory)"""
+    out = (ctypes.c_int * 25)()
+    ok(lib().vesta_pass_tiles(ctypes.byref(desc), rows, logit_rows, out))
+    return {k: tuple(out[5 * i:5 * i + 5]) for i, k in enumerate(('qkv', 'proj', 'fc', 'p2', 'logits'))}
 
 
 def create(desc, device, graph=False, ws=None):
@@ -101,9 +109,7 @@ class PromptPass:
         with torch.cuda.device(dev):
             self.h, self.ws = create(desc, dev)
         self._prompts = lib().vesta_pass_prompts
-        self.low = Lowered(src='', params=[], scratch={}, scratch_floats=0, shared_bytes=0, barriers_per_launch=0, grid=low.grid,
-                           plan=[('prompt rows', 'one kernel per norm, contraction and attention of a layer, tcgen05 contractions')],
-                           dims=dict(low.dims, B=rows, kernel='pass', tc=True, tcl=True), roles=low.roles)
+        self.desc = desc
 
     def run(self, tokens, lens):
         """tokens (B, P), lens (B,) int32 numpy: the caches, x and t of the model after the prompts"""
