@@ -210,7 +210,7 @@ cudaError_t prepare_all() {
 }
 int epi_of(int kind) { return kind == K_QKV ? EPI_QKV : kind == K_FC ? EPI_GELU : kind == K_LOGITS ? EPI_LOGITS : EPI_ADD; }
 
-// launch attributes: `dependent` = may start while the kernel before it runs
+// launch attributes: `dependent` = may start while the kernel before it runs (a contraction's launch sets its threads by itself)
 struct Config {
     cudaLaunchConfig_t c = {};
     cudaLaunchAttribute at[2];
@@ -311,7 +311,7 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
         } else if (kind == K_LOGITS) { g.of = (float*)d.logits; g.best = (u64*)u(p.o.best); }
         else { g.of = z; g.bias = kind == K_PROJ ? f16(d.ob, (size_t)l * D) : f16(d.pb, (size_t)l * D); }
         g.bn = t.bn; g.ftiles = (g.nfeat + t.bm - 1) / t.bm; g.rtiles = p.rp ? 1 : (g.rows + t.bn - 1) / t.bn; g.ntiles = g.ftiles * g.rtiles * t.splits;
-        Config c(dim3(t.bm == 64 && kind != K_LOGITS ? g.ntiles : t.bm == 256 ? 2 * std::min(g.ntiles, p.sms / 2) : std::min(g.ntiles, p.sms)), 192, st, true, t.bm == 256 ? 2 : 1, true);
+        Config c(dim3(t.bm == 64 && kind != K_LOGITS ? g.ntiles : t.bm == 256 ? 2 * std::min(g.ntiles, p.sms / 2) : std::min(g.ntiles, p.sms)), 0, st, true, t.bm == 256 ? 2 : 1, true);
         return gemm(epi_of(kind), t, c.c, pl->w[kind], pl->a[kind], g);
     };
     auto attend = [&](int l) {
@@ -324,7 +324,7 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
             c.c.dynamicSmemBytes = AM_SMEM;
             return pow2 ? cudaLaunchKernelEx(&c.c, pass_attend_many<true>, p.qmap, p.kmap, p.vmap, a) : cudaLaunchKernelEx(&c.c, pass_attend_many<false>, p.qmap, p.kmap, p.vmap, a);
         }
-        AttArgs a = {q, kc, vc, ss, (const int*)d.t, (const int*)0, d.t_stride, d.tmax, D, pow2, p.rp, d.scale, att};
+        AttArgs a = {q, kc, vc, ss, (const int*)d.t, d.t_stride, d.tmax, D, pow2, p.rp, d.scale, att};
         Config c(dim3(d.H, rows, C), ATT_WARPS * 32, st, true, C);
         c.c.dynamicSmemBytes = (deep ? 4 : 2) * ATT_WARPS * 4096;
         return deep ? cudaLaunchKernelEx(&c.c, pass_attend<4>, a) : cudaLaunchKernelEx(&c.c, pass_attend<2>, a);

@@ -648,7 +648,7 @@ struct AttArgs {
     const float* q;                  // [row][D] fp32
     const u16 *kc, *vc;              // the caches at this layer
     long long seq_stride;            // elements between two sequences
-    const int *t, *seq;              // positions as the step began (they change only after it)
+    const int* t;                    // positions as the step began (they change only after it)
     int t_stride, tmax, D, pow2, rp;
     float scale;
     u16* out;                        // [row][D] fp16 (and the remainder plane)
@@ -686,9 +686,9 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) pass_attend(const __grid_const
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, pl = lane >> 3, dl = lane & 7, g = lane >> 2, t4 = lane & 3;
     if (threadIdx.x == 0) dep_launch();
     if (C == 2) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // (waited for before the other block's memory is written)
-    const int n = min(__ldcg(a.t + row * a.t_stride) + 1, a.tmax), sq = a.seq ? __ldcg(a.seq + row) : row;
-    const u16* kp = a.kc + sq * a.seq_stride + h * 64 + dl * 8;
-    const u16* vp = a.vc + sq * a.seq_stride + h * 64 + dl * 8;
+    const int n = min(__ldcg(a.t + row * a.t_stride) + 1, a.tmax);
+    const u16* kp = a.kc + row * a.seq_stride + h * 64 + dl * 8;
+    const u16* vp = a.vc + row * a.seq_stride + h * 64 + dl * 8;
     const int step = C * ATT_WARPS * ATT_RUN;
     int p0 = (cr * ATT_WARPS + warp) * ATT_RUN;
     // per stage 16 rows of K, then of V, 128 bytes each; the 16-byte pieces of a row swizzled (kv_off)

@@ -90,7 +90,7 @@ class VestaGPT2:
         self.low = lower(text, spec, axis_max={'s': tmax}, batch=batch, per_token=per_token,
                          outputs=('logit', 'next'), feedback={'x': 'next', 't': 1} if feedback else None,
                          timing=timing, grid=sms, prompt_len=prompt_len if feedback else 0, slab_tiles=slab_tiles, tune=tune)
-        self._text, self._tune, self._prefill_engines = text, tune, {}
+        self._prefill_engines = {}
         self.k = Kernel(self.low, device=dev.index, blocks_per_sm=blocks_per_sm)
         if prompt_len and feedback:
             R = dict(R, prompt=self.prompt, plen=self.plen)
