@@ -106,12 +106,14 @@ def test_gpt2_xl_shape():
     run_fixture('gpt2_xl_b1')
 
 
-@pytest.mark.parametrize('name', ['gpt2_cfg3_sample', 'gpt2_cfg5_sample', 'gpt2_xl16_sample', 'gpt2_cfg5_b64_sample', 'gpt2_cfg5_b256_sample',
-                                  'gpt2_cfg3_tail_sample', 'gpt2_xl1_sample'])
-def test_deep_context_samples_against_the_reference(name):
-    """the large-batch paths at full model size against the reference interpreter: (cfg3) 64 sequences with 600
-    positions in every cache: slabs, distributed LayerNorm, fold-slice MLP projection, several attention items of
-    five tiles per CTA, tcgen05 logits; (cfg5) ragged batches of 32, 64 and 256 (what the batch-sharded benchmark runs per
+@pytest.mark.parametrize('name,tune', [(n, None) for n in ('gpt2_cfg3_sample', 'gpt2_cfg5_sample', 'gpt2_xl16_sample', 'gpt2_cfg5_b64_sample', 'gpt2_cfg5_b256_sample',
+                                                          'gpt2_cfg3_tail_sample', 'gpt2_xl1_sample')]
+                         + [(n, dict(ln_dist=True)) for n in ('gpt2_cfg3_sample', 'gpt2_cfg5_b64_sample', 'gpt2_cfg3_tail_sample')])
+def test_deep_context_samples_against_the_reference(name, tune):
+    """the large-batch paths at full model size against the reference interpreter, as a chain of kernels and, where `tune` names
+    the option that the persistent kernel takes by itself there, in that kernel: (cfg3) 64 sequences with 600
+    positions in every cache (the persistent kernel: distributed LayerNorm, fold-slice MLP projection, several attention items
+    of five tiles per CTA, tcgen05 contractions); (cfg5) ragged batches of 32, 64 and 256 (what the batch-sharded benchmark runs per
     GPU on 8, 4 and 1 GPUs) with 64..512 positions per sequence and per-sequence positions; (cfg3 tail) 64 sequences at
     positions 1021..1023 of a 1024-row cache: the last K/V tile and the last position the cache holds; (xl16, xl1) the XL
     shape at batch 16 and batch 1, context 300. Caches are seeded (synth.make_cache); the sampled sequences are compared over two
@@ -122,9 +124,10 @@ def test_deep_context_samples_against_the_reference(name):
     sh, steps, stride, B = SHAPES[str(g['shape'])], int(g['steps']), int(g['stride']), int(g['batch'])
     ctxs = g['ctxs'].astype(np.int32)
     ragged = int(ctxs.min()) != int(ctxs.max())
-    m, _ = model(sh, int(g['seed']), str(g['init']), B, int(ctxs.max()) + steps, per_sequence_t=ragged)
-    if B >= 64:
-        assert m.low.dims['tc'] and m.low.dims['ksplit']
+    m, _ = model(sh, int(g['seed']), str(g['init']), B, int(ctxs.max()) + steps, per_sequence_t=ragged, tune=tune)
+    assert m.k.chain == (B > 8 and not tune)
+    if not m.k.chain and B >= 64:
+        assert m.low.dims['tc'] and m.low.dims['ksplit'] and m.low.dims['tcl']
     m.reset()
     for b in range(B):
         k0, v0 = make_cache(sh, int(g['cache_seed_base']) + b, int(ctxs[b]))
@@ -313,13 +316,14 @@ def test_tensor_core_layer_contractions(batch, tune):
     m.k.check()
 
 
-def test_ragged_prompts_fed_on_the_device():
-    """per-sequence prompt lengths, consumed by the kernel's own feedback (no host write between steps),
+@pytest.mark.parametrize('B', [6, 12])
+def test_ragged_prompts_fed_on_the_device(B):
+    """in the persistent kernel and in a chain: per-sequence prompt lengths, consumed by the kernel's own feedback (no host write between steps),
     late starts so that every prompt ends at the same step; the greedy streams equal the oracle's"""
     from oracle import gpt2_numpy as O
     from vesta_gpu_b200.shapes import TINY3
     from vesta_gpu_b200.synth import make_ragged_prompts
-    B, gen = 6, 8
+    gen = 8
     lens, toks = make_ragged_prompts(TINY3, B, 1, 9, seed=3)
     pmax = int(lens.max()); steps = pmax + gen
     m, hf = model(TINY3, 11, 'rich', B, steps, per_sequence_t=True, prompt_len=pmax)
@@ -601,17 +605,18 @@ def test_dense_prefill_at_full_size_against_the_reference(rows):
     assert compared >= 4 * B
 
 
-@pytest.mark.parametrize('batch', [3, 70])
+@pytest.mark.parametrize('batch,tune', [(3, None), (70, dict(ln_dist=True)), (70, None), (12, None)])
 @pytest.mark.parametrize('without', [('qkvb', 'fcb'), ('ln1b', 'qkvb', 'ob', 'ln2b', 'fcb', 'pb', 'lnfb')])
-def test_program_without_shifts_or_biases(batch, without):
-    """a program that leaves out additive parameters (both kernel texts; at 70 sequences the tensor-core contractions):
-    the kernel reads zeros in their place; against the oracle with those parameters set to zero, which is the same
-    arithmetic as the shorter statements"""
+def test_program_without_shifts_or_biases(batch, tune, without):
+    """a program that leaves out additive parameters (both kernel texts, at 70 sequences the tensor-core contractions, and the
+    chain) and the same tokens as prompts: the kernel reads zeros in their place; against the oracle with those parameters set
+    to zero, which is the same arithmetic as the shorter statements"""
     from oracle import gpt2_numpy as O
     from vesta_gpu_b200.shapes import TINY
     from vesta_gpu_b200.synth import make_prompts
     steps = 5
-    m, hf = model(TINY, 5, 'rich', batch, steps, without=without, tune=dict(ln_dist=True) if batch > 8 else None)
+    m, hf = model(TINY, 5, 'rich', batch, steps, without=without, tune=tune)
+    assert m.k.chain == (batch > 8 and not tune)
     assert m.low.dims['absent'] == sorted(without) and not set(without) & set(m.W)
     weights = dict(hf.weights)
     for n in without:
@@ -628,6 +633,9 @@ def test_program_without_shifts_or_biases(batch, without):
             assert np.abs(lg[i] - ref).max() < TIGHT, (t, i)
             if O.margin(ref) > MARGIN:
                 assert int(nx[i]) == rn
+    keys, vals = m.keys.float(), m.vals.float()
+    m.prefill(feed)
+    assert (m.keys.float() - keys).abs().max() <= 4e-3 and (m.vals.float() - vals).abs().max() <= 4e-3
     m.k.check()
 
 
@@ -706,3 +714,39 @@ def test_kernel_api_mirrors_reference():
     with pytest.raises(AssertionError):
         k.bind(R)
     assert m.weight_bytes == TINY.weight_bytes() and m.kv_bytes(5) == 2 * TINY.L * 2 * 5 * TINY.D * 2
+
+
+def test_rows_of_prompts_in_the_persistent_kernel():
+    """lower(row_seq=True): rows are (cache sequence, position) pairs, every row attends to the rows of its sequence that the same
+    step writes; rows with a negative position are idle, rows marked with bit 30 want no logits (those that do come first)"""
+    from oracle import gpt2_numpy as O
+    from vesta_gpu_b200.launch import Kernel, TORCH_DT
+    from vesta_gpu_b200.lower import lower
+    from vesta_gpu_b200.program_text import decode_program
+    from vesta_gpu_b200.shapes import TINY3 as sh
+    rows, lens, tmax = 20, (5, 1, 11), 16
+    toks = np.random.RandomState(1).randint(0, sh.N, (3, 11)).astype(np.int32)
+    m, hf = model(sh, 11, 'rich', 3, tmax)
+    pairs = sorted(((s, p) for s in range(3) for p in range(lens[s])), key=lambda e: e[1] != lens[e[0]] - 1)
+    x, t, seq = np.zeros(rows, np.int32), np.full(rows, -1, np.int32), np.full(rows, 1 << 30, np.int32)
+    for r, (s, p) in enumerate(pairs):
+        x[r], t[r], seq[r] = toks[s, p], p, s | (0 if p == lens[s] - 1 else 1 << 30)
+    up = lambda a: torch.from_numpy(a).cuda()
+    R = {'x': up(x), 't': up(t), **m.W, 'keys': m.keys, 'vals': m.vals}
+    names = {v: k for k, v in TORCH_DT.items()}
+    low = lower(decode_program(sh), {n: (tuple(v.shape), names[v.dtype]) for n, v in R.items()}, {'s': tmax}, batch=rows, per_token=('x', 'keys', 'vals', 't'),
+                outputs=('logit', 'next'), grid=m.k.sms, row_seq=True)
+    k = Kernel(low)
+    assert not k.chain
+    k.bind(dict(R, row_seq=up(seq)))
+    k.launch()
+    k.check()
+    W = O.upcast(hf.weights)
+    for r, (s, _) in enumerate(pairs[:3]):
+        ck, cv = O.new_cache(sh, tmax)
+        for p in range(lens[s]):
+            ref, nx = O.step(sh, W, ck, cv, int(toks[s, p]), p)
+        assert np.abs(k.view('logit')[r].cpu().numpy() - ref).max() < 2 * TIGHT, s
+        assert O.margin(ref) <= MARGIN or int(k.view('next')[r]) == nx
+        for got, want in ((m.keys, ck), (m.vals, cv)):
+            assert np.abs(got[s].float().cpu().numpy() - want.astype(np.float32)).max() <= 4e-3, s

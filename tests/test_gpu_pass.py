@@ -93,6 +93,7 @@ def test_refused_step_stays_refused():
 
 
 @pytest.mark.parametrize('lens,rows,kw,divisor', [
+    ((9, 3, 1), 5, {}, 8),                                      # passes of five rows: less than one product of 16
     ((127, 128, 129, 1, 255, 257, 16, 384), None, {}, 8),       # edges of the attention's runs
     ((127, 128, 129, 1, 255, 257, 16, 384), 256, {}, 8),        # prompts that several passes read
     ((77,), None, dict(D=320, H=5, F=1296), 8),                 # one prompt, folds of five blocks, a ragged one behind
@@ -339,3 +340,22 @@ def test_binding_a_chain_again():
     for T in (R, S):
         assert (T['keys'].float() - m.keys.float()).abs().max() <= 4e-3 and torch.equal(T['x'], m.x)
     k.check()
+
+
+def test_steps_of_a_chain_inside_a_captured_graph():
+    """a caller's own CUDA graph of steps: the kernels of the chain one by one instead of the chain's graph"""
+    sh = shape('captured')
+    m, _ = model(sh, 3, 'rich', 12, 20)
+    m.x.fill_(5)
+    m.step(6)
+    x, logits = m.x.clone(), m.logits().clone()
+    g = torch.cuda.CUDAGraph()
+    m.reset()
+    m.x.fill_(5)
+    with torch.cuda.graph(g):
+        m.step(3)
+    assert int(m.t[0]) == 0
+    g.replay()
+    g.replay()
+    assert int(m.t[0]) == 6 and (m.logits() - logits).abs().max() < TIGHT and torch.equal(m.x, x)
+    m.k.check()
