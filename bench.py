@@ -61,9 +61,8 @@ REF_DIR = os.path.join(ROOT, 'oracle', '_ref')          # an installed copy of t
 NCU_CAPTURE = {
     'cfg2': dict(bytes=291.0e6, positions=131.5, source='scaled from the ncu capture in profiles/vesta_step_gpt2_small_b1_b8.md (two steps at contexts 131 and 132) by the K/V bytes of this run\'s contexts'),
     'cfg1': dict(bytes=256.3e6, positions=131.5, source='scaled from the ncu capture in profiles/vesta_step_gpt2_small_b1_b8.md (two steps at contexts 131 and 132) by the K/V bytes of this run\'s contexts'),
-    'cfg3': dict(bytes=1484.9e6, positions=513.5, source='scaled from the ncu capture in profiles/vesta_step_gpt2_small_b64.md (two steps at contexts 513 and 514) by the K/V bytes of this run\'s contexts'),
 }
-NCU_SOURCE = 'no capture of this workload for the current kernel: see profiles/'
+NCU_SOURCE = 'no capture of a whole step of this workload (a chain of kernels, profiles/pass_chain.md, or another persistent kernel): see profiles/'
 
 
 def peaks():
@@ -433,6 +432,10 @@ class Run:
         """algorithmic bytes of one step on one GPU: every weight once + the attended K/V of its sequences"""
         return sum(self.sh.weight_bytes() + self.sh.kv_bytes_per_pos() * sum(c) / self.world for c in self.ctx_lens) / self.K
 
+    def steps_per_launch(self):
+        """decode steps of one launch: a persistent kernel runs several, a chain is one graph per step"""
+        return 1 if self.m.k.chain else min(self.args.per_launch, self.K)
+
     def reduce_max(self, *vals):
         if self.world == 1:
             return vals
@@ -443,6 +446,7 @@ class Run:
 
     def measure(self, repeats, with_e2e=True):
         """-> (dict of the measured figures, token stream on the device)"""
+        from vesta_gpu_b200.passes import kernels_of_a_step
         times = self.device_loop(repeats)
         stream = self.token_stream()
         med = statistics.median(times)
@@ -456,7 +460,7 @@ class Run:
         peak, peak_src = peaks()
         bps = self.bytes_per_step()
         achieved = bps / (med / K) / 1e9
-        spl = min(self.args.per_launch, K)
+        spl = self.steps_per_launch()
         cap = NCU_CAPTURE.get(self.name) if world == 1 else None
         traffic = None
         if cap:
@@ -466,9 +470,9 @@ class Run:
                    contexts=[min(self.ctx_lens[0]), max(self.ctx_lens[-1])],
                    roofline=dict(bound='hbm', achieved=achieved, peak=peak, unit='GB/s', frac=achieved / peak, traffic=traffic,
                                  traffic_source=(cap['source'] if cap else NCU_SOURCE),
-                                 peak_source=peak_src, bytes_per_step=bps, bytes_per_launch=bps * spl, kernel='vesta_step',
+                                 peak_source=peak_src, bytes_per_step=bps, bytes_per_launch=bps * spl, kernel='pass_* (a chain of kernels per step)' if self.m.k.chain else 'vesta_step',
                                  frac_of_8tbs=achieved / 8000.0),
-                   gpu_launches=-(-K // self.args.per_launch))
+                   steps_per_launch=spl, gpu_launches=-(-K // spl) * (kernels_of_a_step(self.sh.L) if self.m.k.chain else 1))
         if with_e2e:
             out['e2e'] = dict(value=B * world * K / e2e_med, unit=UNIT, h2d_bytes_per_step=B * 4, d2h_bytes_per_step=B * 4,
                               tokens_match_device_loop=same)
@@ -556,10 +560,10 @@ def main():
 
     line = dict(metric=METRIC, value=res['value'], unit=UNIT, n_gpus=world, steps=K, warmup=max(args.warmup, 3),
                 ms_per_step=res['ms_per_step'], higher_is_better=True, scaling='strong' if total else 'weak', vs_baseline=None,
-                dtype='f16 weights and KV, f32 accumulate' + ('' if wl['batch'] // (world if total else 1) <= 16 else ' (activations rounded to f16 before the products above 16 sequences)'),
+                dtype='f16 weights and KV, f32 accumulate' + ('' if B <= (16 if sh.D <= 1024 else 8) else ' (activations rounded to f16 before the products)'),
                 data='synthetic',
                 config=dict(workload=args.workload, **{k: v for k, v in wl.items() if k != 'total'}, batch_per_gpu=B, repeats=args.repeats,
-                            steps_per_launch=min(args.per_launch, K), contexts=res['contexts'],
+                            steps_per_launch=res['steps_per_launch'], contexts=res['contexts'],
                             l2='weights + KV read per step (%.0f MB) exceed the 126 MB L2' % (res['roofline']['bytes_per_step'] / 1e6), cv=res['cv']),
                 clocks=clocks, gpu_launches=res['gpu_launches'], e2e=res['e2e'], roofline=res['roofline'])
     if prefill:

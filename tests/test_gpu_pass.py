@@ -334,7 +334,7 @@ def test_binding_a_chain_again():
     k.launch(2)
     k.bind(R)
     k.launch(3)
-    assert k._work.data_ptr() == work
+    assert k._work.data_ptr() == work and k.launches == 8
     m.step(4)
     assert int(R['t'][0]) == int(S['t'][0]) == int(m.t[0]) == 4
     for T in (R, S):

@@ -1,6 +1,7 @@
-"""Run a Lowered program through the C ABI of libvesta_b200.so (include/vesta_b200.h) bound with ctypes: a decode step as a
-chain of kernels of the library (passes.py), or, where the lowering asks for it (tune options, timing), as one persistent
-kernel compiled with NVRTC for sm_100a and launched cooperatively.
+"""Run a Lowered program through the C ABI of libvesta_b200.so (include/vesta_b200.h) bound with ctypes: a decode step as one
+persistent kernel, compiled with NVRTC for sm_100a and launched cooperatively (few sequences, and wherever the lowering asks
+for what only it has: tune options, timing, rows of prompts), or as a chain of kernels of the library (passes.py); which of
+the two, Lowered.dims['chain'] says.
 
 Mirrors the reference run-time (vesta/launch.py:10-73): `TORCH_DT`, `ok`, `compile_cubin`,
 and `Kernel` with `view`, `bind`, `launch`, `__call__` and the attributes `mod, fn, smem, sms,
@@ -154,7 +155,7 @@ class Kernel:
             self._vals = self._args = self._tm = self.keep = self._bound = None
             self.fuse = 16                                       # decode steps per launch in launch(steps > 1)
             self.feeds_back = '#define V_FEEDBACK 1' in lowered.src
-            self.launches = 0
+            self.launches = 0                                    # of the persistent kernel, or of a chain's graph
             if not self.chain:
                 self._load()
 
@@ -300,8 +301,8 @@ class Kernel:
 
     def launch(self, steps=1, per_launch=None):
         """`steps` decode steps on the current stream. With feedback on, up to `per_launch` steps (default
-        Kernel.fuse) run inside one launch: the kernel feeds its own token and position between them, which saves
-        the gap between launches; without feedback every step is its own launch."""
+        Kernel.fuse) run inside one launch of the persistent kernel: it feeds its own token and position between them, which
+        saves the gap between launches; without feedback, and as a chain (a graph per step), every step is its own launch."""
         if self._direct and not torch.cuda.is_current_stream_capturing():
             self._bind_chain(graph=True)
         self._launch(steps, per_launch)
@@ -311,7 +312,7 @@ class Kernel:
         per = per_launch or self.fuse
         if steps > 1 and per > 1 and self.feeds_back:
             ok(lib().vesta_step_run_fused(self._bound, stream, steps, per))
-            self.launches += -(-steps // per)
+            self.launches += steps if self.chain else -(-steps // per)
         else:
             ok(lib().vesta_step_run(self._bound, stream, steps))
             self.launches += steps

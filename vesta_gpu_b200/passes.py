@@ -54,6 +54,11 @@ def describe(low, residue, zeros, cpos, **kw):
     return desc
 
 
+def kernels_of_a_step(layers):
+    """kernels that a decode step launches as a chain: seven per layer, the embedding with its norm, the logits, the end"""
+    return 7 * layers + 3
+
+
 def tiles(desc, rows, logit_rows):
     """the tiles of the contractions of a pass over `rows` rows of which `logit_rows` want logits: for 'qkv', 'proj', 'fc', 'p2' and
     'logits' (features, rows, stages, parts of the fold, bytes of shared memory)"""
