@@ -66,7 +66,9 @@ int plane_rows(int rows, bool exact) { return !exact ? 0 : rows <= 8 ? 8 : 16; }
 
 // Tile sizes of a contraction of `feat` features over `kb` blocks of 64 for `rows` rows (columns of the product), from a
 // model of the kernel's time in microseconds, fitted to measurements on B200 (rows 16 to 16,384, folds of 768 to 6,400,
-// tiles of 16 to 256 rows; within 15 % of each):
+// tiles of 16 to 256 rows) of a kernel by itself, its weights in L2: within 15 % of each. It ranks tiles; it is not the time of a
+// kernel in a pass, where its boundary and weights that come from memory are added (9,200 rows of the small shape, FC: 36.5
+// and 38.3 seen, QKV 26.5 and 31.7; 77 rows, QKV 3.1 and 4.5; 16 of the XL shape, QKV 4.4 and 4.5, MLP projection 3.2 and 6.1):
 //   BM = 64 (one tile per block, whole share of the weights in flight): 1.75, 0.22 per stage, 0.5 for every stage that has to
 //     wait for a free one, the operand's rows;
 //   BM = 128: 2.2 for the first fill, a term for the last epilogue, then per block of the fold the larger of the products and the loads

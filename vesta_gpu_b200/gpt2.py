@@ -1,5 +1,5 @@
-"""The decode-step program on the GPU: Hugging Face style weights as residue, lowered to one
-persistent kernel per step.
+"""The decode-step program on the GPU: Hugging Face style weights as residue, a step as one persistent kernel (few
+sequences) or as a chain of kernels, prompts as dense passes of the same chain.
 
     m = VestaGPT2(hf, dtype='f16', batch=8, tmax=1024)
     m.reset(); m.x.copy_(tok); m.t.fill_(p); m.step()     # one decode step

@@ -359,9 +359,10 @@ class Kernel:
 
     def clear_status(self):
         """forget a refused step or an abandoned wait: status word, abort flag and the barrier counters back to zero.
-        Both are sticky: until this is called every further launch returns at once without touching x, t or the cache
-        (a refused step never wrote anything; a launch in which a wait ran out may have written part of a step, so
-        reset or reload the decode state before going on)."""
+        The status stays until this is called. After an abandoned wait, and in a chain after a refused step too, every
+        further launch returns without touching x, t or the cache; the persistent kernels run a good step after a refused
+        one. (A refused step never wrote anything; a launch in which a wait ran out may have written part of a step, so
+        reset or reload the decode state before going on.)"""
         self.bar.zero_()
 
     def __del__(self):

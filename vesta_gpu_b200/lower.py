@@ -1,5 +1,7 @@
 """Placement of a decode-step program on the 148 SMs of a B200 and assembly of the CUDA source
-of ONE persistent cooperative kernel (plus a one-time weight-packing kernel).
+of ONE persistent cooperative kernel (plus a one-time weight-packing kernel). With more than a few
+sequences a step runs as a chain of the library's own kernels instead (csrc/pass.cu; dims['chain']
+says so): the source is then compiled only for callers that ask for the persistent kernel.
 
     lower(text, res, axis_max, batch=1, per_token=(), outputs=(), feedback=None, timing=False) -> Lowered
 
@@ -18,8 +20,8 @@ different by design: instead of deriving scalar CUDA C statement by statement, t
      balancing the bytes every CTA streams per step, and lays each CTA's share of the fp16 weights
      out as one contiguous stream of mma-ordered 16x16 tiles (Lowered.place, consumed by the
      packing kernel and the step kernel);
-  3. prepends the sizes, placement constants and the kernel signatures to the hand-written
-     sm_100a kernel text in csrc/step_kernel.cuh.
+  3. prepends the sizes, placement constants and the kernel signatures to one of two hand-written
+     sm_100a kernel texts, csrc/step_small.cuh (at most eight sequences) or csrc/step_kernel.cuh.
 """
 import math
 from dataclasses import dataclass, field, fields, is_dataclass
@@ -46,6 +48,9 @@ DEFAULT_SMS = 148      # B200
 
 @dataclass
 class Lowered:
+    """What lower() makes of a program. `src`, `shared_bytes`, `barriers_per_launch`, `plan`, `sites`, `block`, `place`, `packed_bytes`
+    and the placement entries of `dims` (tc, tcl, ksplit, nch, ...) describe the persistent kernel, also where dims['chain'] is
+    set and Kernel runs steps as a chain; the tiles of a chain are the library's choice (passes.tiles)."""
     src: str
     params: list             # (name, dtype, emitted) in kernel argument order
     scratch: dict            # host-visible name -> (offset, axes, static shape)
@@ -593,10 +598,11 @@ def lower(text, res, axis_max, batch=1, per_token=(), outputs=(), feedback=None,
     tune = dict(tune or {})
     # What a step as a chain of kernels (csrc/pass.cu) needs to know; Kernel runs that chain unless the caller asked for
     # something that only the persistent kernels have (a placement option, timing sums, rows of prompts).
-    # Up to eight sequences the small persistent kernel is the faster one at widths up to 1,024 (one sequence of the small shape 175
-    # against 219 us per step, eight 215 against 244 at 200 positions): its exchanges between a few CTAs cost less than kernel
-    # boundaries. The wider the rows, the less a boundary weighs and the more every CTA's norms do: five sequences of width 1,280
-    # 547 against 540, three of the XL shape 1,246 against 1,164, two 1,224 against 1,170 (left where results repeat bit for bit);
+    # Up to eight sequences the small persistent kernel is the faster one at widths up to 1,024 (small shape at 200 positions: one
+    # sequence 174 against 227 us per step, four 189 against 232, eight 213 against 247, at 1,000 positions 268 against 282): its
+    # exchanges between a few CTAs cost less than kernel boundaries. The wider the rows, the less a boundary weighs and the more
+    # every CTA's norms do: width 1,280 (twelve layers) with four sequences 280 against 279, with five 293 against 286; XL shape
+    # with three 1,253 against 1,168, two 1,224 against 1,165 and one 1,155 against 1,157 (left where results repeat bit for bit);
     # and with more (sequence, head) pairs than CTAs the kernel falls back on grid barriers (XL shape, eight: 1,679 against 1,245).
     persistent = B <= (8 if D <= 1024 else 4 if D <= 1280 else 2) and B * H <= grid
     dims = dict(dims, chain=not (tune or timing or row_seq or slab_tiles or act_lo is not None) and not persistent and D <= 4096,
