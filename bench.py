@@ -434,7 +434,7 @@ class Run:
 
     def steps_per_launch(self):
         """decode steps of one launch: a persistent kernel runs several, a chain is one graph per step"""
-        return 1 if self.m.k.chain else min(self.args.per_launch, self.K)
+        return 1 if self.m.k.graphs else min(self.args.per_launch, self.K)
 
     def reduce_max(self, *vals):
         if self.world == 1:
@@ -461,7 +461,7 @@ class Run:
         bps = self.bytes_per_step()
         achieved = bps / (med / K) / 1e9
         spl = self.steps_per_launch()
-        cap = NCU_CAPTURE.get(self.name) if world == 1 else None
+        cap = NCU_CAPTURE.get(self.name) if world == 1 and not self.m.k.graphs else None
         traffic = None
         if cap:
             mean_pos = sum(sum(c) for c in self.ctx_lens) / K / (B * world)
@@ -470,9 +470,9 @@ class Run:
                    contexts=[min(self.ctx_lens[0]), max(self.ctx_lens[-1])],
                    roofline=dict(bound='hbm', achieved=achieved, peak=peak, unit='GB/s', frac=achieved / peak, traffic=traffic,
                                  traffic_source=(cap['source'] if cap else NCU_SOURCE),
-                                 peak_source=peak_src, bytes_per_step=bps, bytes_per_launch=bps * spl, kernel='pass_* (a chain of kernels per step)' if self.m.k.chain else 'vesta_step',
+                                 peak_source=peak_src, bytes_per_step=bps, bytes_per_launch=bps * spl, kernel='few_* (a chain of kernels per step)' if self.m.k.few else 'pass_* (a chain of kernels per step)' if self.m.k.chain else 'vesta_step',
                                  frac_of_8tbs=achieved / 8000.0),
-                   steps_per_launch=spl, gpu_launches=-(-K // spl) * (kernels_of_a_step(self.sh.L) if self.m.k.chain else 1))
+                   steps_per_launch=spl, gpu_launches=-(-K // spl) * (kernels_of_a_step(self.sh.L, self.m.k.few) if self.m.k.graphs else 1))
         if with_e2e:
             out['e2e'] = dict(value=B * world * K / e2e_med, unit=UNIT, h2d_bytes_per_step=B * 4, d2h_bytes_per_step=B * 4,
                               tokens_match_device_loop=same)

@@ -84,12 +84,14 @@ void vesta_step_release(void* bound);
 
 /* A forward pass over rows as a chain of kernels (no counterpart in the reference, which has one generated kernel): the rows
  * are the sequences of a decode step or the (sequence, position) pairs of prompts. All pointers are device memory; weights
- * as the residues hold them (fp16, stacked on the layer, [fold][feature]); nothing is packed. */
+ * as the residues hold them (fp16, stacked on the layer, [fold][feature]); nothing is packed but with exact == 2. */
 typedef struct vesta_pass_desc {
     int L, D, H, F, N, tmax, cpos;      /* sizes of the model, rows of a cache plane and of the position table */
     int rows, logit_rows;               /* most rows of a pass, most rows that want logits */
     int prompts;                        /* 0: a decode step, a row per sequence; else the number of sequences whose prompts the pass reads */
-    int exact;                          /* activations enter the products at fp32 accuracy (at most 16 rows), else rounded to fp16 */
+    int exact;                          /* activations enter the products at fp32 accuracy (at most 16 rows), else rounded to fp16;
+                                           2: the same for a decode step of at most eight rows from a packed copy of the weights in the
+                                           workspace, which vesta_pass_pack makes; sizes that do not suit it are refused */
     int t_stride, tstep, feedback, prompt_len;
     float eps, scale, gelu_a, gelu_b, gelu_c;
     const void *wte, *wpe, *ln1w, *ln1b, *qkvw, *qkvb, *ow, *ob, *ln2w, *ln2b, *fcw, *fcb, *pw, *pb, *lnfw, *lnfb;
@@ -106,6 +108,9 @@ int vesta_pass_tiles(const vesta_pass_desc* desc, int rows, int logit_rows, int*
 /* workspace: that many bytes of device memory, zeroed, on a 256-byte boundary (matrices, table and caches: 16 bytes, norm
  * parameters and wpe: 8 bytes; anything else is refused). graph != 0: the pass is a decode step, kept as a CUDA graph. */
 int vesta_pass_create(const vesta_pass_desc* desc, void* workspace, int graph, void** pass);
+/* exact == 2: (re)makes the packed copy of the weights on `stream`; to be called before the first step and whenever the weights have
+ * changed. Nothing to do for any other pass. */
+int vesta_pass_pack(void* pass, void* stream);
 /* Whole prompts: tokens [prompts][ld] and lens [prompts] in host memory. Every prompt position goes into the caches (rows after a
  * prompt are zeroed), x gets the token chosen after every prompt, t its position; in passes of at most desc.rows rows.
  * Synchronises `stream`; *status as bar[0] (not zero: refused, a token outside the vocabulary). */

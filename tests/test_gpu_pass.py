@@ -70,6 +70,70 @@ def test_step_as_a_chain(batch, kw):
     m.k.check()
 
 
+@pytest.mark.parametrize('batch,kw', [
+    (1, {}), (2, {}), (3, {}), (4, {}),               # heads and remainders side by side; 8, 4 and 2 blocks per sequence in the attention
+    (5, {}), (8, {}),                                 # all heads, then all remainders; one block per sequence, contexts deeper than its rings
+    (1, dict(D=64, H=1, F=16)),                       # fewer units of the fold, and of the outputs, than warps
+    (8, dict(D=320, H=5, F=1296)),                    # ten pairs of units for eight warps
+    (2, dict(L=1, D=1024, H=16, F=4096)), (6, dict(L=1, D=1024, H=16, F=2384)),   # two tiles per block; 149 tiles, the last block has one
+    (3, dict(L=1, D=832, H=13, F=2384)),
+])
+def test_step_of_few_sequences(batch, kw):
+    """three kernels per layer from packed weights: ragged steps over seeded caches against the oracle; up to two sequences the same
+    bits twice; the persistent kernel takes the same step"""
+    from oracle import gpt2_numpy as O
+    sh, steps = shape('few', **kw), 2
+    m, hf = model(sh, 17, 'rich', batch, sh.C, per_sequence_t=True)
+    assert m.k.few and not m.k.chain
+    W = O.upcast(hf.weights)
+    ctx = np.array((389, 0, 63, 64, 255, 256, 257, 18)[:batch], np.int32)
+    first = np.array([(b * 31 + 5) % sh.N for b in range(batch)], np.int32)
+    runs = []
+    for _ in range(2):
+        caches, x = seeded(m, sh, ctx, 900), first
+        m.t.copy_(torch.from_numpy(ctx))
+        m.x.copy_(torch.from_numpy(x))
+        for s in range(steps):
+            m.step()
+            lg, nx = m.logits().cpu().numpy(), m.x.cpu().numpy()
+            for b in range(batch):
+                ref, rn = O.step(sh, W, *caches[b], int(x[b]), int(ctx[b]) + s)
+                assert np.abs(lg[b] - ref).max() < TIGHT, (s, b)
+                assert O.margin(ref) <= MARGIN or int(nx[b]) == rn
+            x = nx
+        for b in range(batch):
+            c = int(ctx[b])
+            assert np.abs(m.keys[b, :, c:c + steps].float().cpu().numpy() - caches[b][0][:, c:c + steps].astype(np.float32)).max() <= 4e-3
+        runs.append((m.logits().clone(), m.keys.clone(), m.vals.clone()))
+    assert batch > 2 or all(torch.equal(a, b) for a, b in zip(*runs))
+    m.k.check()
+
+
+def test_a_good_step_of_few_sequences_runs_after_a_refused_one():
+    """a position outside the cache: nothing is published; the status stays, the next step runs; after an abort flag none does"""
+    sh = shape('refused few')
+    m, _ = model(sh, 3, 'rich', 3, 100, per_sequence_t=True)
+    m.reset()
+    m.t.fill_(7)
+    m.step()
+    logits, keys = m.logits().clone(), m.keys.clone()
+    m.t[1] = 100
+    x, t = m.x.clone(), m.t.clone()
+    m.step(2)
+    assert torch.equal(m.logits(), logits) and torch.equal(m.keys, keys) and torch.equal(m.x, x) and torch.equal(m.t, t)
+    assert 'out of range' in str(m.k.status())
+    m.t.fill_(8)
+    m.step()
+    assert (m.t == 9).all() and not torch.equal(m.keys, keys)
+    m.k.bar[2].fill_(1)
+    m.step()
+    assert (m.t == 9).all()
+    m.k.clear_status()
+    m.step()
+    assert (m.t == 10).all()
+    m.k.check()
+
+
 def test_refused_step_stays_refused():
     """a position outside the cache, then the abort flag alone: nothing is published, later steps are refused until the status is cleared"""
     sh = shape('refused')

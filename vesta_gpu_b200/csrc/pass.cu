@@ -7,6 +7,7 @@
 #include <string>
 #include <vector>
 
+#include "pass_few.cuh"
 #include "pass_kernels.cuh"
 #include "rt_internal.h"
 #include "vesta_b200.h"
@@ -29,6 +30,7 @@ struct Tile { int bm, bn, stages, splits; };
 
 struct Layout {
     size_t z, q, act, att, gelu, fin, best, rowoff, pos, skip;
+    size_t sums[2], packed;                    // few sequences: the vectors after the MLP, in turn; the packed weights
     size_t meta, total;                        // prompts: tokens, positions, sequences of the rows; attention runs; rows that want logits and where they go; lengths
 };
 // the metadata of a pass over prompts, as offsets in 32-bit words
@@ -40,8 +42,16 @@ struct Meta {
     }
 };
 
+// A decode step of few sequences (pass_few.cuh): tiles per block of the two kernels that cut features
+struct Few {
+    bool on, fixed;                            // fixed: the state as State<true>
+    int qkv_per, mlp_per;
+};
+const int SMEM_MAX = 227 * 1024;
+
 struct Pass {
     vesta_pass_desc d;
+    Few few;
     int rp;                                    // rows of an operand plane when head and remainder are kept, else 0
     int planes;                                // operand rows: rp * 2, or the rows rounded up to whole tiles
     int fplanes;                               // the same for the rows that want logits
@@ -124,6 +134,18 @@ Layout layout(const Pass& p, int D, int F, int rows, int lrows) {
     Layout o{};
     size_t at = 0;
     auto take = [&](size_t bytes) { const size_t r = at; at += (bytes + 255) / 256 * 256; return r; };
+    if (p.few.on) {
+        const size_t state = (size_t)rows * D * (p.few.fixed ? 8 : 4);
+        o.z = take(state); o.sums[0] = take(state); o.sums[1] = take(state);
+        o.q = take((size_t)rows * D * 4);
+        o.fin = take((size_t)p.fplanes * D * 2);
+        o.best = take((size_t)lrows * 8);
+        o.pos = take((size_t)rows * 4);
+        o.skip = take(4);
+        o.packed = take(FewPack(D, F).layer * p.d.L);
+        o.total = at;
+        return o;
+    }
     o.z = take((size_t)rows * D * 4);
     o.q = take((size_t)rows * D * 4);
     o.act = take((size_t)p.planes * D * 2);
@@ -139,10 +161,26 @@ Layout layout(const Pass& p, int D, int F, int rows, int lrows) {
     return o;
 }
 
+// The tiles of a step of few sequences: about a block per SM, as far as the blocks' weights fit shared memory; false: they do not.
+bool few_plan(Pass& p, const vesta_pass_desc& d) {
+    if (d.rows > FEW_ROWS || d.prompts || d.D > 1024) return false;
+    Few f{};
+    f.on = true;
+    f.fixed = d.rows <= 2;
+    const int sms = 148;
+    f.qkv_per = (3 * d.D / 16 + sms - 1) / sms;
+    f.mlp_per = (d.F / 16 + sms - 1) / sms;
+    if (std::max(f.qkv_per, f.mlp_per) > FEW_TILES || FewMlp::bytes(d.D, d.rows, f.mlp_per) > SMEM_MAX - 1024) return false;
+    p.few = f;
+    return true;
+}
+
 int plan(Pass& p, const vesta_pass_desc* d) {
     if (!d || d->rows < 1 || d->rows > 1 << 28 || d->logit_rows < 1 || d->logit_rows > d->rows) return fail(-1, "vesta_pass: bad row counts");
     if (d->prompts < 0 || (d->prompts && d->logit_rows < std::min(d->rows, d->prompts))) return fail(-1, "vesta_pass: a pass over prompts needs a logit row for every prompt that can end in it");
     if (d->L < 1 || d->D < 64 || d->D % 64 || d->D > 4096 || d->H * 64 != d->D || d->F < 16 || d->F % 16 || d->N < 1 || d->tmax < 1 || d->cpos < 1) return fail(-1, "vesta_pass: sizes outside the supported family");
+    p.few = Few{};
+    if (d->exact == 2 && !few_plan(p, *d)) return fail(-1, "vesta_pass: sizes outside those of a step from packed weights");
     if (d->exact && d->rows > 16) return fail(-1, "vesta_pass: fp32-accurate operands are kept for at most 16 rows");
     p.d = *d;
     p.dev = 0;
@@ -241,7 +279,7 @@ int plan_for(Pass& p, int rows, int lrows, const Pass::Plan** out) {
     const void* w[5] = {d.qkvw, d.ow, d.fcw, d.pw, d.wte};
     const int fold[5] = {D, D, D, F, D}, pitch[5] = {D, D, D, up(F, 64), D}, feat[5] = {3 * D, D, F, D, d.N};
     const size_t op[5] = {p.o.act, p.o.att, p.o.act, p.o.gelu, p.o.fin};
-    for (int k = 0; k < 5; k++) {
+    for (int k = p.few.on ? K_LOGITS : 0; k < 5; k++) {             // (few sequences: of these contractions the logits only)
         const Tile t = q.tile[k] = tile_of(p, k, rows, lrows);
         int e;
         if (k == K_LOGITS) e = vesta_rt::fold_map(&q.w[k], w[k], D, feat[k], t.bm, k_blocks(t.bm));
@@ -252,6 +290,23 @@ int plan_for(Pass& p, int rows, int lrows, const Pass::Plan** out) {
     p.plans.push_back(q);
     *out = &p.plans.back();
     return 0;
+}
+
+FinishArgs finish(const Pass& p, int lrows) {
+    const vesta_pass_desc& d = p.d;
+    FinishArgs f = {};
+    f.rows = lrows; f.best = (u64*)(p.ws + p.o.best); f.skip = (int*)(p.ws + p.o.skip); f.bar = (const u32*)d.bar; f.next = (float*)d.next; f.pos = (const int*)(p.ws + p.o.pos);
+    f.t_stride = d.t_stride; f.tstep = d.tstep; f.N = d.N;
+    if (d.feedback && !d.prompts) { f.x = (int*)d.x; f.t = (int*)d.t; f.prompt = (const int*)d.prompt; f.plen = (const int*)d.plen; f.plen_cap = d.prompt_len; }
+    return f;
+}
+GemmArgs logits_args(const Pass& p, const Tile& t, int lrows) {
+    GemmArgs g = {};
+    g.D = p.d.D; g.rp = p.rp; g.stages = t.stages; g.status = (u32*)p.d.bar; g.limit = p.wait_ns; g.skip = (const int*)(p.ws + p.o.skip);
+    g.rows = lrows; g.kblocks = p.d.D / 64; g.kb_per = g.kblocks; g.nfeat = p.d.N;
+    g.of = (float*)p.d.logits; g.best = (u64*)(p.ws + p.o.best);
+    g.bn = t.bn; g.ftiles = (g.nfeat + t.bm - 1) / t.bm; g.rtiles = p.rp ? 1 : (g.rows + t.bn - 1) / t.bn; g.ntiles = g.ftiles * g.rtiles * t.splits;
+    return g;
 }
 
 // The launches of one pass over `rows` rows. Prompts: `tiles` runs of rows for the attention, `lrows` rows that want logits
@@ -299,10 +354,15 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
     auto mul = [&](int kind, int l) {
         const Tile& t = pl->tile[kind];
         GemmArgs g = {};
+        if (kind == K_LOGITS) {
+            g = logits_args(p, t, lrows);
+            Config c(dim3(std::min(g.ntiles, p.sms)), 0, st, true);
+            return gemm(EPI_LOGITS, t, c.c, pl->w[kind], pl->a[kind], g);
+        }
         g.layer = l; g.D = D; g.rp = p.rp; g.stages = t.stages; g.status = (u32*)d.bar; g.limit = p.wait_ns; g.skip = (const int*)u(p.o.skip);
-        g.rows = kind == K_LOGITS ? lrows : rows;
+        g.rows = rows;
         g.kblocks = kind == K_P2 ? kbf : kbd; g.kb_per = (g.kblocks + t.splits - 1) / t.splits;
-        g.nfeat = kind == K_QKV ? 3 * D : kind == K_FC ? F : kind == K_LOGITS ? d.N : D;
+        g.nfeat = kind == K_QKV ? 3 * D : kind == K_FC ? F : D;
         if (kind == K_QKV) {
             g.bias = f16(d.qkvb, (size_t)l * 3 * D); g.of = (float*)u(p.o.q); g.rowoff = (const long long*)u(p.o.rowoff);
             g.kc = (u16*)d.keys + (size_t)l * d.tmax * D; g.vc = (u16*)d.vals + (size_t)l * d.tmax * D;
@@ -310,10 +370,9 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
             if (clear) { g.lens = meta + mt.lens; g.seqs = d.prompts; g.seq_stride = (long long)L * d.tmax * D; g.tmax = d.tmax; }
         } else if (kind == K_FC) {
             g.bias = f16(d.fcb, (size_t)l * F); g.oh = (u16*)u(p.o.gelu); g.pitch = up(F, 64); g.a2 = 2 * d.gelu_a; g.k1 = d.gelu_b * 2.8853900817779268f; g.k2 = d.gelu_c * g.k1;
-        } else if (kind == K_LOGITS) { g.of = (float*)d.logits; g.best = (u64*)u(p.o.best); }
-        else { g.of = z; g.bias = kind == K_PROJ ? f16(d.ob, (size_t)l * D) : f16(d.pb, (size_t)l * D); }
+        } else { g.of = z; g.bias = kind == K_PROJ ? f16(d.ob, (size_t)l * D) : f16(d.pb, (size_t)l * D); }
         g.bn = t.bn; g.ftiles = (g.nfeat + t.bm - 1) / t.bm; g.rtiles = p.rp ? 1 : (g.rows + t.bn - 1) / t.bn; g.ntiles = g.ftiles * g.rtiles * t.splits;
-        Config c(dim3(t.bm == 64 && kind != K_LOGITS ? g.ntiles : t.bm == 256 ? 2 * std::min(g.ntiles, p.sms / 2) : std::min(g.ntiles, p.sms)), 0, st, true, t.bm == 256 ? 2 : 1, true);
+        Config c(dim3(t.bm == 64 ? g.ntiles : t.bm == 256 ? 2 * std::min(g.ntiles, p.sms / 2) : std::min(g.ntiles, p.sms)), 0, st, true, t.bm == 256 ? 2 : 1, true);
         return gemm(epi_of(kind), t, c.c, pl->w[kind], pl->a[kind], g);
     };
     auto attend = [&](int l) {
@@ -343,13 +402,114 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
         TRY(norm(l + 1 < L ? 2 : 3, l));
     }
     if (lrows) TRY(mul(K_LOGITS, 0));
-    FinishArgs f = {};
-    f.rows = lrows; f.best = (u64*)u(p.o.best); f.skip = (int*)u(p.o.skip); f.bar = (const u32*)d.bar; f.next = (float*)d.next; f.pos = (const int*)u(p.o.pos);
-    f.t_stride = d.t_stride; f.tstep = d.tstep; f.N = d.N;
+    FinishArgs f = finish(p, lrows);
     if (many) { f.dst = (const int2*)(meta + mt.dst); f.x = (int*)d.x; f.t = (int*)d.t; }
-    else if (d.feedback) { f.x = (int*)d.x; f.t = (int*)d.t; f.prompt = (const int*)d.prompt; f.plen = (const int*)d.plen; f.plen_cap = d.prompt_len; }
     Config c(dim3(1), 256, st, true);
     TRY(cudaLaunchKernelEx(&c.c, pass_finish, f));
+    return 0;
+}
+
+// one case per width (units of 256, at most) and warps per row
+#define FEW_WIDTH(X, K) X(K, 8, true) X(K, 4, true) X(K, 2, false) X(K, 1, false)
+#define FEW_EACH(X) FEW_WIDTH(X, 1) FEW_WIDTH(X, 2) FEW_WIDTH(X, 3) FEW_WIDTH(X, 4)
+cudaError_t few_launch(cudaLaunchConfig_t& c, int D, int wpr, const FewQkv& a) {
+#define ONE(K, W, F) if (D <= 256 * K && wpr == W) return cudaLaunchKernelEx(&c, few_qkv<K, W, F>, a);
+    FEW_EACH(ONE)
+#undef ONE
+    return cudaErrorInvalidValue;
+}
+cudaError_t few_launch(cudaLaunchConfig_t& c, int D, int wpr, const FewMlp& a) {
+#define ONE(K, W, F) if (D <= 256 * K && wpr == W) return cudaLaunchKernelEx(&c, few_mlp<K, W, F>, a);
+    FEW_EACH(ONE)
+#undef ONE
+    return cudaErrorInvalidValue;
+}
+// up to four sequences, fixed point
+#define FEW_ATTEND(X) X(true, true) X(true, false) X(false, false)
+cudaError_t few_launch(cudaLaunchConfig_t& c, bool four, bool fixed, const FewAttend& a) {
+#define ONE(M, F) if (four == M && fixed == F) return cudaLaunchKernelEx(&c, few_attend<M, F>, a);
+    FEW_ATTEND(ONE)
+#undef ONE
+    return cudaErrorInvalidValue;
+}
+cudaError_t few_prepare() {
+    cudaError_t e = cudaSuccess;
+    auto one = [&](auto* f, int bytes = SMEM_MAX - 1024) {
+        if (e == cudaSuccess) e = all_shared(f);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute((const void*)f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    };
+#define ONE(K, W, F) one(few_qkv<K, W, F>); one(few_mlp<K, W, F>);
+    FEW_EACH(ONE)
+#undef ONE
+#define ONE(M, F) one(few_attend<M, F>, FewAttend::bytes(1024));
+    FEW_ATTEND(ONE)
+#undef ONE
+    return e;
+}
+
+// a step of few sequences
+int enqueue_few(Pass& p, cudaStream_t st) {
+    const vesta_pass_desc& d = p.d;
+    const Few& f = p.few;
+    const int D = d.D, F = d.F, R = d.rows, wpr = R > 4 ? 1 : R > 2 ? 2 : R > 1 ? 4 : 8;
+    const Pass::Plan* pl = nullptr;
+    if (int e = plan_for(p, R, R, &pl)) return e;
+    auto u = [&](size_t off) { return p.ws + off; };
+    auto f16 = [](const void* q, size_t off) { return (const u16*)q + off; };
+    const FewPack pk(D, F);
+    int expo = 0;
+    const int pow2 = frexpf(d.scale, &expo) == 0.5f;
+    for (int l = 0; l < d.L; l++) {
+        const unsigned char* w = u(p.o.packed) + (size_t)l * pk.layer;
+        u16 *kc = (u16*)d.keys + (size_t)l * d.tmax * D, *vc = (u16*)d.vals + (size_t)l * d.tmax * D;
+        const long long ss = (long long)d.L * d.tmax * D;
+        {
+            FewQkv a = {};
+            a.n = {D, R, d.eps, u(p.o.sums[(l + 1) & 1]), f16(d.ln1w, (size_t)l * D), f16(d.ln1b, (size_t)l * D), u(p.o.z), f16(d.ob, (size_t)l * D), u(p.o.sums[l & 1])};
+            a.w = w + pk.qkv; a.bias = f16(d.qkvb, (size_t)l * 3 * D); a.tiles = 3 * D / 16; a.per = f.qkv_per; a.q = (float*)u(p.o.q); a.kc = kc; a.vc = vc; a.seq_stride = ss;
+            a.x = (const int*)d.x; a.t = (const int*)d.t; a.t_stride = d.t_stride; a.tmax = d.tmax; a.cpos = d.cpos; a.N = d.N; a.first = l == 0; a.wte = (const u16*)d.wte; a.wpe = (const u16*)d.wpe;
+            a.pos = (int*)u(p.o.pos); a.skip = (int*)u(p.o.skip); a.bar = (u32*)d.bar;
+            Config c(dim3((a.tiles + a.per - 1) / a.per), FEW_THREADS, st, l != 0);
+            c.c.dynamicSmemBytes = FewQkv::bytes(D, R, a.per);
+            TRY(few_launch(c.c, D, wpr, a));
+        }
+        {
+            FewAttend a = {};
+            a.a = {(const float*)u(p.o.q), kc, vc, ss, (const int*)d.t, d.t_stride, d.tmax, D, pow2, 0, d.scale, nullptr};
+            a.rows = R; a.chunks = wpr; a.w = w + pk.proj; a.z = u(p.o.z);
+            Config c(dim3(FEW_CLUSTER, d.H), FEW_THREADS, st, true, FEW_CLUSTER, true);
+            c.c.dynamicSmemBytes = FewAttend::bytes(D);
+            TRY(few_launch(c.c, R <= 4, f.fixed, a));
+        }
+        {
+            FewMlp a = {};
+            a.n = {D, R, d.eps, u(p.o.z), f16(d.ln2w, (size_t)l * D), f16(d.ln2b, (size_t)l * D), u(p.o.sums[l & 1]), f16(d.pb, (size_t)l * D), nullptr};
+            a.fc = w + pk.fc; a.p2 = w + pk.p2; a.bias = f16(d.fcb, (size_t)l * F); a.tiles = F / 16; a.per = f.mlp_per;
+            a.a2 = 2 * d.gelu_a; a.k1 = d.gelu_b * 2.8853900817779268f; a.k2 = d.gelu_c * a.k1;
+            Config c(dim3((a.tiles + a.per - 1) / a.per), FEW_THREADS, st, true);
+            c.c.dynamicSmemBytes = FewMlp::bytes(D, R, a.per);
+            TRY(few_launch(c.c, D, wpr, a));
+        }
+    }
+    NormArgs n = {};
+    n.D = D; n.rp = p.rp; n.eps = d.eps; n.gain = f16(d.lnfw, 0); n.shift = f16(d.lnfb, 0); n.act = (u16*)u(p.o.fin);
+    n.z = (float*)u(p.o.sums[(d.L - 1) & 1]); n.fixed = f.fixed;
+    Config cn(dim3(R), up(D / 4, 32), st, true);
+    TRY(cudaLaunchKernelEx(&cn.c, pass_norm<NORM_FINAL>, n));
+    const Tile& t = pl->tile[K_LOGITS];
+    const GemmArgs g = logits_args(p, t, R);
+    Config cg(dim3(std::min(g.ntiles, p.sms)), 0, st, true);
+    TRY(gemm(EPI_LOGITS, t, cg.c, pl->w[K_LOGITS], pl->a[K_LOGITS], g));
+    Config cf(dim3(1), 256, st, true);
+    TRY(cudaLaunchKernelEx(&cf.c, pass_finish, finish(p, R)));
+    return 0;
+}
+int step(Pass& p, cudaStream_t st) { return p.few.on ? enqueue_few(p, st) : enqueue(p, st, p.d.rows, p.d.logit_rows, 0); }
+int pack_few(const Pass& p, cudaStream_t st) {
+    const vesta_pass_desc& d = p.d;
+    const FewPackArgs a = {d.D, d.F, d.L, d.rows <= 4, (const u16*)d.qkvw, (const u16*)d.ow, (const u16*)d.fcw, (const u16*)d.pw, p.ws + p.o.packed};
+    few_pack<<<p.sms * 8, 256, 0, st>>>(a);
+    TRY(cudaGetLastError());
     return 0;
 }
 
@@ -368,7 +528,7 @@ int capture(Pass* p) {
     cudaError_t ce = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
     if (ce == cudaSuccess) ce = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
     if (ce == cudaSuccess) {
-        e = guarded([&] { return enqueue(*p, st, p->d.rows, p->d.logit_rows, 0); });      // (the capture ends whatever happens in it)
+        e = guarded([&] { return step(*p, st); });      // (the capture ends whatever happens in it)
         ce = cudaStreamEndCapture(st, &g);
     }
     if (ce == cudaSuccess && !e) ce = cudaGraphInstantiate(&ge, g, 0);
@@ -387,7 +547,7 @@ int make(Pass* p, const vesta_pass_desc* d, unsigned char* workspace, bool graph
     if (!e) e = check(*d);
     if (!e && (size_t)workspace % 256) e = fail(-1, "vesta_pass: the workspace starts on a 256-byte boundary");
     p->ws = workspace;
-    if (!e) { const cudaError_t ce = prepare_all(); if (ce != cudaSuccess) e = cuda_fail(ce, "cudaFuncSetAttribute"); }
+    if (!e) { cudaError_t ce = p->few.on ? few_prepare() : cudaSuccess; if (ce == cudaSuccess) ce = prepare_all(); if (ce != cudaSuccess) e = cuda_fail(ce, "cudaFuncSetAttribute"); }
     if (!e && d->prompts) {
         const unsigned long long D = d->D, planes = (unsigned long long)d->prompts * d->L;
         e = vesta_rt::tensor_map(&p->kmap, d->keys, D, d->tmax, planes, D * 2, D * 2 * d->tmax, 128, 1);
@@ -471,7 +631,7 @@ int pass_steps(void* pass, void* stream, int steps) {
     TRY(cudaStreamIsCapturing(st, &cap));
     return guarded([&]() -> int {
         for (int i = 0; i < steps; i++) {
-            if (cap != cudaStreamCaptureStatusNone || !p->graph) { if (int e = enqueue(*p, st, p->d.rows, p->d.logit_rows, 0)) return e; }
+            if (cap != cudaStreamCaptureStatusNone || !p->graph) { if (int e = step(*p, st)) return e; }
             else TRY(cudaGraphLaunch(p->graph, st));
         }
         return 0;
@@ -515,6 +675,14 @@ int vesta_pass_prompts(void* pass, void* stream, const int* tokens, int ld, cons
     const int e = guarded([&] { return read_prompts(p, (cudaStream_t)stream, tokens, ld, lens, status); });
     if (e) cudaStreamSynchronize((cudaStream_t)stream);                  // (the next call writes the pinned metadata that copies may still read)
     return e;
+}
+
+int vesta_pass_pack(void* pass, void* stream) {
+    Pass* p = (Pass*)pass;
+    if (!p) return fail(-1, "vesta_pass_pack: null argument");
+    if (!p->few.on) return 0;
+    const vesta_rt::OnDevice on(p->dev);
+    return pack_few(*p, (cudaStream_t)stream);
 }
 
 int vesta_pass_wait_limit(void* pass, unsigned long long ns) {

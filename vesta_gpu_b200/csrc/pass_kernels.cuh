@@ -73,6 +73,36 @@ __device__ __forceinline__ u32 elect_one() {
     return leader;
 }
 
+// The residual stream: fp32, or 64-bit fixed point (36 fractional bits: finer than fp32 below 2^27) whose integer additions give the
+// same bits in every order.
+#define STATE_SCALE 68719476736.0f
+template <bool FIXED> struct State;
+template <> struct State<false> {
+    static __device__ __forceinline__ float4 load(const void* z, size_t i) { return __ldcg(reinterpret_cast<const float4*>((const float*)z + i)); }
+    static __device__ __forceinline__ void store(void* z, size_t i, float4 v) { *reinterpret_cast<float4*>((float*)z + i) = v; }
+    static __device__ __forceinline__ void add1(void* z, size_t i, float v) { asm volatile("red.relaxed.gpu.global.add.f32 [%0], %1;" :: "l"((float*)z + i), "f"(v) : "memory"); }
+    static __device__ __forceinline__ void add(void* z, size_t i, float4 v) {
+        asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1,%2,%3,%4};" :: "l"((float*)z + i), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+    }
+};
+template <> struct State<true> {
+    static __device__ __forceinline__ float from(long long v) { return __ll2float_rn(v) * (1.0f / STATE_SCALE); }
+    static __device__ __forceinline__ float4 load(const void* z, size_t i) {
+        const longlong2* p = reinterpret_cast<const longlong2*>((const long long*)z + i);
+        const longlong2 a = __ldcg(p), b = __ldcg(p + 1);
+        return make_float4(from(a.x), from(a.y), from(b.x), from(b.y));
+    }
+    static __device__ __forceinline__ void store(void* z, size_t i, float4 v) {
+        longlong2* p = reinterpret_cast<longlong2*>((long long*)z + i);
+        p[0] = make_longlong2(__float2ll_rn(v.x * STATE_SCALE), __float2ll_rn(v.y * STATE_SCALE));
+        p[1] = make_longlong2(__float2ll_rn(v.z * STATE_SCALE), __float2ll_rn(v.w * STATE_SCALE));
+    }
+    static __device__ __forceinline__ void add1(void* z, size_t i, float v) {
+        asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" :: "l"((long long*)z + i), "l"(__float2ll_rn(v * STATE_SCALE)) : "memory");
+    }
+    static __device__ __forceinline__ void add(void* z, size_t i, float4 v) { add1(z, i, v.x); add1(z, i + 1, v.y); add1(z, i + 2, v.z); add1(z, i + 3, v.w); }
+};
+
 // Every wait gives up after `limit` nanoseconds (half a second): it leaves a code in the status word, a flag that ends the other
 // waits of the block (of the pair: `peer` is the flag of the other block) and the abort flag: this pass publishes no token or
 // position, and every later one is refused. The block runs to its end: a warp whose wait gave up goes on through the
@@ -539,6 +569,7 @@ struct NormArgs {
     int *pos, *skip;
     u32* bar;                        // [0] status, [2] abort flag
     const int* want;                 // FINAL: rows that want logits (0: all)
+    int fixed;                       // FINAL: the state is State<true>
 };
 
 // One row per block, four elements per thread (the row stays in registers). Latency bound for few rows:
@@ -576,7 +607,7 @@ __global__ void __launch_bounds__(1024) pass_norm(const __grid_constant__ NormAr
             v = make_float4(h_lo(e.x) + h_lo(p.x), h_hi(e.x) + h_hi(p.x), h_lo(e.y) + h_lo(p.y), h_hi(e.y) + h_hi(p.y));
         }
     } else if (own) {
-        v = __ldcg(reinterpret_cast<const float4*>(a.z + (size_t)row * a.D + d));
+        v = MODE == NORM_FINAL && a.fixed ? State<true>::load(a.z, (size_t)row * a.D + d) : State<false>::load(a.z, (size_t)row * a.D + d);
     }
     if (own && MODE == NORM_EMBED) *reinterpret_cast<float4*>(a.z + (size_t)row * a.D + d) = v;
     float s = (v.x + v.y) + (v.z + v.w);
@@ -679,25 +710,26 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const u32 (&a)[4], u32 b
 __device__ __forceinline__ void cp16z(u32 dst, const void* src, bool yes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(dst), "l"(src), "r"(yes ? 16 : 0) : "memory");
 }
-template <int NS>
-__global__ void __launch_bounds__(ATT_WARPS * 32) pass_attend(const __grid_constant__ AttArgs a) {
-    __shared__ float part[ATT_WARPS + 1][66];
-    extern __shared__ __align__(128) unsigned char ring_raw[];
-    const int h = blockIdx.x, row = blockIdx.y, C = gridDim.z, cr = blockIdx.z;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, pl = lane >> 3, dl = lane & 7, g = lane >> 2, t4 = lane & 3;
-    if (threadIdx.x == 0) dep_launch();
-    if (C == 2) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // (waited for before the other block's memory is written)
-    const int n = min(__ldcg(a.t + row * a.t_stride) + 1, a.tmax);
-    const u16* kp = a.kc + row * a.seq_stride + h * 64 + dl * 8;
-    const u16* vp = a.vc + row * a.seq_stride + h * 64 + dl * 8;
-    const int step = C * ATT_WARPS * ATT_RUN;
-    int p0 = (cr * ATT_WARPS + warp) * ATT_RUN;
-    // per stage 16 rows of K, then of V, 128 bytes each; the 16-byte pieces of a row swizzled (kv_off)
-    const u32 ring = smem_u32(ring_raw) + warp * (NS * 4096);
+// One warp's runs of a row's positions: from `p0`, every `step`, through its ring of NS stages of 4 KB. request_first() asks for
+// what is there since earlier steps, run() waits for nothing but that and leaves the 64 sums, the maximum and the sum of the weights
+// in `part`; run(false) does one round of the same on what there is (see FEW_DRY).
+template <int NS> struct AttRow {
+    const AttArgs& a;
+    int row, h, first, step, n;
+    u32 ring;
+    const u16 *kp, *vp;
     u32 put[4];
+    __device__ __forceinline__ AttRow(const AttArgs& args, int row_, int h_, int p0, int step_, u32 ring_) : a(args), row(row_), h(h_), first(p0), step(step_), ring(ring_) {
+        const int lane = threadIdx.x & 31, pl = lane >> 3, dl = lane & 7;
+        n = min(__ldcg(a.t + row * a.t_stride) + 1, a.tmax);
+        kp = a.kc + row * a.seq_stride + h * 64 + dl * 8;
+        vp = a.vc + row * a.seq_stride + h * 64 + dl * 8;
+        // per stage 16 rows of K, then of V, 128 bytes each; the 16-byte pieces of a row swizzled (kv_off)
 #pragma unroll
-    for (int j = 0; j < 4; j++) put[j] = ring + kv_off(j * 4 + pl, dl);
-    auto request = [&](int st, int p, int end) {
+        for (int j = 0; j < 4; j++) put[j] = ring + kv_off(j * 4 + pl, dl);
+    }
+    __device__ __forceinline__ void request(int st, int p, int end) const {
+        const int pl = (threadIdx.x & 31) >> 3;
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const int x = p + j * 4 + pl;
@@ -705,104 +737,122 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) pass_attend(const __grid_const
             cp16z(put[j] + st * 4096, kp + off, x < end);
             cp16z(put[j] + st * 4096 + 2048, vp + off, x < end);
         }
-    };
-#pragma unroll
-    for (int i = 0; i < NS; i++) {
-        if (p0 + i * step < n) request(i, p0 + i * step, n - 1);
-        asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    dep_wait();
-    u32 bq[4][2];
-    {
-        const float* qp = a.q + (size_t)row * a.D + h * 64;
-        float2 x[4][2];
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            x[k][0] = __ldcg(reinterpret_cast<const float2*>(qp + k * 16 + 2 * t4));
-            x[k][1] = __ldcg(reinterpret_cast<const float2*>(qp + k * 16 + 2 * t4 + 8));
-        }
-        // the current position, if it is in one of the runs requested above
-        u32 at = 0;
+    __device__ __forceinline__ void request_first() const {
 #pragma unroll
         for (int i = 0; i < NS; i++) {
-            const int y = n - 1 - (p0 + i * step);
-            if (y >= 0 && y < ATT_RUN && (y & 3) == pl) at = ring + i * 4096 + kv_off(y, dl);
+            if (first + i * step < n) request(i, first + i * step, n - 1);
+            asm volatile("cp.async.commit_group;" ::: "memory");
         }
-        if (at) {
-            const uint4 kc = __ldcg(reinterpret_cast<const uint4*>(kp + (size_t)(n - 1) * a.D)), vc = __ldcg(reinterpret_cast<const uint4*>(vp + (size_t)(n - 1) * a.D));
-            asm volatile("cp.async.wait_all;" ::: "memory");                       // (the zeros that were requested in its place)
-            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" :: "r"(at), "r"(kc.x), "r"(kc.y), "r"(kc.z), "r"(kc.w) : "memory");
-            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" :: "r"(at + 2048), "r"(vc.x), "r"(vc.y), "r"(vc.z), "r"(vc.w) : "memory");
-        }
-        const float sc = a.pow2 ? 1.0f / a.scale : 1.0f;
+    }
+    __device__ __forceinline__ void run(bool real, float* part) const {
+        const int lane = threadIdx.x & 31, pl = lane >> 3, dl = lane & 7, g = lane >> 2, t4 = lane & 3;
+        int p0 = first;
+        u32 bq[4][2];
+        {
+            const float* qp = a.q + (size_t)row * a.D + h * 64;
+            float2 x[4][2];
 #pragma unroll
-        for (int k = 0; k < 4; k++)
-#pragma unroll
-            for (int i = 0; i < 2; i++) {
-                const float u = x[k][i].x * sc, v = x[k][i].y * sc;
-                const u32 hi = pack_h2(u, v);
-                bq[k][i] = g & 1 ? pack_h2(u - h_lo(hi), v - h_hi(hi)) : hi;   // (every pair of columns alike: all lanes get scores)
+            for (int k = 0; k < 4; k++) {
+                x[k][0] = __ldcg(reinterpret_cast<const float2*>(qp + k * 16 + 2 * t4));
+                x[k][1] = __ldcg(reinterpret_cast<const float2*>(qp + k * 16 + 2 * t4 + 8));
             }
-    }
-    float m = -3.0e38f, den = 0.f, o[4][4];              // o[mt]: dims mt*16 + g (regs 0 + 1) and mt*16 + g + 8 (regs 2 + 3), lanes with t4 == 0
+            // the current position, if it is in one of the runs requested above
+            u32 at = 0;
 #pragma unroll
-    for (int i = 0; i < 4; i++) { o[i][0] = 0.f; o[i][1] = 0.f; o[i][2] = 0.f; o[i][3] = 0.f; }
-    int st = 0;
-    const u32 ka = ring + kv_off(lane & 15, 0), va = ring + 2048 + ((lane & 7) + ((lane >> 4) ? 8 : 0)) * 128;
-    const int kx = lane >> 4, k7 = lane & 7, vx = (lane >> 3) & 1;
+            for (int i = 0; i < NS; i++) {
+                const int y = n - 1 - (p0 + i * step);
+                if (y >= 0 && y < ATT_RUN && (y & 3) == pl) at = ring + i * 4096 + kv_off(y, dl);
+            }
+            if (at) {
+                const uint4 kc = __ldcg(reinterpret_cast<const uint4*>(kp + (size_t)(n - 1) * a.D)), vc = __ldcg(reinterpret_cast<const uint4*>(vp + (size_t)(n - 1) * a.D));
+                asm volatile("cp.async.wait_all;" ::: "memory");                       // (the zeros that were requested in its place)
+                asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" :: "r"(at), "r"(kc.x), "r"(kc.y), "r"(kc.z), "r"(kc.w) : "memory");
+                asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" :: "r"(at + 2048), "r"(vc.x), "r"(vc.y), "r"(vc.z), "r"(vc.w) : "memory");
+            }
+            const float sc = a.pow2 ? 1.0f / a.scale : 1.0f;
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    const float u = x[k][i].x * sc, v = x[k][i].y * sc;
+                    const u32 hi = pack_h2(u, v);
+                    bq[k][i] = g & 1 ? pack_h2(u - h_lo(hi), v - h_hi(hi)) : hi;   // (every pair of columns alike: all lanes get scores)
+                }
+        }
+        float m = -3.0e38f, den = 0.f, o[4][4];              // o[mt]: dims mt*16 + g (regs 0 + 1) and mt*16 + g + 8 (regs 2 + 3), lanes with t4 == 0
+#pragma unroll
+        for (int i = 0; i < 4; i++) { o[i][0] = 0.f; o[i][1] = 0.f; o[i][2] = 0.f; o[i][3] = 0.f; }
+        int st = 0;
+        const u32 ka = ring + kv_off(lane & 15, 0), va = ring + 2048 + ((lane & 7) + ((lane >> 4) ? 8 : 0)) * 128;
+        const int kx = lane >> 4, k7 = lane & 7, vx = (lane >> 3) & 1;
 #pragma unroll 1
-    while (p0 < n) {
-        asm volatile("cp.async.wait_group %0;" :: "n"(NS - 1) : "memory");
-        __syncwarp();
-        const u32 so = st * 4096;
-        float s[4] = {0.f, 0.f, 0.f, 0.f};
+        while (p0 < n) {
+            asm volatile("cp.async.wait_group %0;" :: "n"(NS - 1) : "memory");
+            __syncwarp();
+            const u32 so = st * 4096;
+            float s[4] = {0.f, 0.f, 0.f, 0.f}, x[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            u32 r[4];
-            ldsm4(r, (ka & ~127u) + so + (((k * 2 + kx) ^ k7) << 4));
-            mma16816(s, r, bq[k][0], bq[k][1]);
+            for (int k = 0; k < 4; k++) {
+                u32 r[4];
+                ldsm4(r, (ka & ~127u) + so + (((k * 2 + kx) ^ k7) << 4));
+                if (k & 1) mma16816(x, r, bq[k][0], bq[k][1]); else mma16816(s, r, bq[k][0], bq[k][1]);
+            }
+            float s0 = (s[0] + s[1]) + (x[0] + x[1]), s1 = (s[2] + s[3]) + (x[2] + x[3]);        // positions p0 + g and p0 + g + 8
+            if (!a.pow2) { s0 /= a.scale; s1 /= a.scale; }
+            if (p0 + g >= n) s0 = -3.0e38f;
+            if (p0 + g + 8 >= n) s1 = -3.0e38f;
+            // (shuffles over the eight groups: redux took longer, 16 sequences of the XL shape 1,359 -> 1,344 us per step)
+            float mx = fmaxf(s0, s1);
+#pragma unroll
+            for (int x = 4; x < 32; x <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, x));
+            if (mx > m) {                                    // (the same in the whole warp)
+                const float corr = fast_exp(m - mx);
+                m = mx;
+                den *= corr;
+#pragma unroll
+                for (int i = 0; i < 4; i++) { o[i][0] *= corr; o[i][1] *= corr; o[i][2] *= corr; o[i][3] *= corr; }
+            }
+            const float pa = s0 > -1.0e38f ? fast_exp(s0 - m) : 0.f, pb = s1 > -1.0e38f ? fast_exp(s1 - m) : 0.f;
+            den += pa + pb;
+            // the weights as operand: lane (g, t4) holds positions 2 t4, 2 t4 + 1 (and + 8); that of position r < 8 is `pa` of lane 4 r
+            const float w00 = __shfl_sync(0xffffffffu, pa, 8 * t4), w01 = __shfl_sync(0xffffffffu, pa, 8 * t4 + 4);
+            const float w10 = __shfl_sync(0xffffffffu, pb, 8 * t4), w11 = __shfl_sync(0xffffffffu, pb, 8 * t4 + 4);
+            u32 b0 = pack_h2(w00, w01), b1 = pack_h2(w10, w11);
+            if (g == 1) { b0 = pack_h2(w00 - h_lo(b0), w01 - h_hi(b0)); b1 = pack_h2(w10 - h_lo(b1), w11 - h_hi(b1)); }
+            if (g > 1) { b0 = 0; b1 = 0; }
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                u32 r[4];
+                ldsm4t(r, va + so + (((i * 2 + vx) ^ k7) << 4));
+                mma16816(o[i], r, b0, b1);
+            }
+            __syncwarp();                                    // every lane has read the stage
+            if (!real) break;
+            if (p0 + NS * step < n) request(st, p0 + NS * step, n);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            p0 += step;
+            if (++st == NS) st = 0;
         }
-        float s0 = s[0] + s[1], s1 = s[2] + s[3];        // positions p0 + g and p0 + g + 8
-        if (!a.pow2) { s0 /= a.scale; s1 /= a.scale; }
-        if (p0 + g >= n) s0 = -3.0e38f;
-        if (p0 + g + 8 >= n) s1 = -3.0e38f;
-        // (shuffles over the eight groups: redux took longer, 16 sequences of the XL shape 1,359 -> 1,344 us per step)
-        float mx = fmaxf(s0, s1);
 #pragma unroll
-        for (int x = 4; x < 32; x <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, x));
-        if (mx > m) {                                    // (the same in the whole warp)
-            const float corr = fast_exp(m - mx);
-            m = mx;
-            den *= corr;
+        for (int x = 16; x > 2; x >>= 1) den += __shfl_xor_sync(0xffffffffu, den, x);
+        if (t4 == 0)
 #pragma unroll
-            for (int i = 0; i < 4; i++) { o[i][0] *= corr; o[i][1] *= corr; o[i][2] *= corr; o[i][3] *= corr; }
-        }
-        const float pa = s0 > -1.0e38f ? fast_exp(s0 - m) : 0.f, pb = s1 > -1.0e38f ? fast_exp(s1 - m) : 0.f;
-        den += pa + pb;
-        // the weights as operand: lane (g, t4) holds positions 2 t4, 2 t4 + 1 (and + 8); that of position r < 8 is `pa` of lane 4 r
-        const float w00 = __shfl_sync(0xffffffffu, pa, 8 * t4), w01 = __shfl_sync(0xffffffffu, pa, 8 * t4 + 4);
-        const float w10 = __shfl_sync(0xffffffffu, pb, 8 * t4), w11 = __shfl_sync(0xffffffffu, pb, 8 * t4 + 4);
-        u32 b0 = pack_h2(w00, w01), b1 = pack_h2(w10, w11);
-        if (g == 1) { b0 = pack_h2(w00 - h_lo(b0), w01 - h_hi(b0)); b1 = pack_h2(w10 - h_lo(b1), w11 - h_hi(b1)); }
-        if (g > 1) { b0 = 0; b1 = 0; }
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            u32 r[4];
-            ldsm4t(r, va + so + (((i * 2 + vx) ^ k7) << 4));
-            mma16816(o[i], r, b0, b1);
-        }
-        __syncwarp();                                    // every lane has read the stage
-        if (p0 + NS * step < n) request(st, p0 + NS * step, n);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        p0 += step;
-        if (++st == NS) st = 0;
+            for (int i = 0; i < 4; i++) { part[i * 16 + g] = o[i][0] + o[i][1]; part[i * 16 + g + 8] = o[i][2] + o[i][3]; }
+        if (lane == 0) { part[64] = m; part[65] = den; }
     }
-#pragma unroll
-    for (int x = 16; x > 2; x >>= 1) den += __shfl_xor_sync(0xffffffffu, den, x);
-    if (t4 == 0)
-#pragma unroll
-        for (int i = 0; i < 4; i++) { part[warp][i * 16 + g] = o[i][0] + o[i][1]; part[warp][i * 16 + g + 8] = o[i][2] + o[i][3]; }
-    if (lane == 0) { part[warp][64] = m; part[warp][65] = den; }
+};
+template <int NS>
+__global__ void __launch_bounds__(ATT_WARPS * 32) pass_attend(const __grid_constant__ AttArgs a) {
+    __shared__ float part[ATT_WARPS + 1][66];
+    extern __shared__ __align__(128) unsigned char ring_raw[];
+    const int h = blockIdx.x, row = blockIdx.y, C = gridDim.z, cr = blockIdx.z, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) dep_launch();
+    if (C == 2) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // (waited for before the other block's memory is written)
+    AttRow<NS> r(a, row, h, (cr * ATT_WARPS + warp) * ATT_RUN, C * ATT_WARPS * ATT_RUN, smem_u32(ring_raw) + warp * (NS * 4096));
+    r.request_first();
+    dep_wait();
+    r.run(true, part[warp]);
     __syncthreads();
     float M = -3.0e38f, dd = 0.f, num = 0.f;
     if (threadIdx.x < 64) {

@@ -1,7 +1,7 @@
 """Run a Lowered program through the C ABI of libvesta_b200.so (include/vesta_b200.h) bound with ctypes: a decode step as one
-persistent kernel, compiled with NVRTC for sm_100a and launched cooperatively (few sequences, and wherever the lowering asks
-for what only it has: tune options, timing, rows of prompts), or as a chain of kernels of the library (passes.py); which of
-the two, Lowered.dims['chain'] says.
+persistent kernel, compiled with NVRTC for sm_100a and launched cooperatively (one to four wide sequences, and wherever the lowering
+asks for what only it has: tune options, timing, rows of prompts), or as a chain of kernels of the library (passes.py); which of
+the two, Lowered.dims['chain'] and, for the chain of few sequences, dims['few'] say.
 
 Mirrors the reference run-time (vesta/launch.py:10-73): `TORCH_DT`, `ok`, `compile_cubin`,
 and `Kernel` with `view`, `bind`, `launch`, `__call__` and the attributes `mod, fn, smem, sms,
@@ -61,6 +61,7 @@ def lib():
         L.vesta_pass_tiles.argtypes = [vp, ci, ci, ctypes.POINTER(ci)]
         L.vesta_pass_create.argtypes = [vp, vp, ci, ctypes.POINTER(vp)]
         L.vesta_pass_prompts.argtypes = [vp, vp, vp, ci, vp, ctypes.POINTER(cu)]
+        L.vesta_pass_pack.argtypes = [vp, vp]
         L.vesta_pass_wait_limit.argtypes = [vp, ctypes.c_ulonglong]
         L.vesta_pass_bind.argtypes = [vp, ctypes.POINTER(vp)]
         L.vesta_pass_release.argtypes = [vp]
@@ -135,6 +136,8 @@ class Kernel:
                                    f'call lower(..., grid={self.sms})')
             self.lowered = lowered
             self.chain = bool(lowered.dims.get('chain'))         # a step is a chain of kernels (passes.py), not one persistent kernel
+            self.few = bool(lowered.dims.get('few'))             # ... of three per layer, from packed weights (at most eight sequences)
+            self.graphs = self.chain or self.few
             self.smem = lowered.shared_bytes
             # The reference's signature defaults to block=256 (vesta/launch.py:30) and callers pass it along: 256 and
             # None both mean "the block size the program was lowered for" (8 consumer warps + the producer warp).
@@ -156,7 +159,7 @@ class Kernel:
             self.fuse = 16                                       # decode steps per launch in launch(steps > 1)
             self.feeds_back = '#define V_FEEDBACK 1' in lowered.src
             self.launches = 0                                    # of the persistent kernel, or of a chain's graph
-            if not self.chain:
+            if not self.graphs:
                 self._load()
 
     def _load(self):
@@ -237,15 +240,17 @@ class Kernel:
             assert t.device == self.device, (name, t.device)
         from .passes import VECTORS, WEIGHTS, aligned
         # (the persistent kernels read the matrices and the position table element by element)
-        here, copies = aligned(self.lowered, residue, WEIGHTS[1:] if self.chain else VECTORS, self._copies)
+        here, copies = aligned(self.lowered, residue, WEIGHTS[1:] if self.graphs else VECTORS, self._copies)
         if self._bound:
             L.vesta_step_release(self._bound)
             self._bound = None
         self._vals = [here[name].data_ptr() for name, _, _ in self.lowered.params] + [self.S.data_ptr(), self.bar.data_ptr(), self.TS.data_ptr()]
         self.keep, self._copies, self._args, self._tm = residue, copies, None, None
-        if self.chain:
+        if self.graphs:
             self._here = here, zeros
             self._bind_chain(graph)
+            if self.few:
+                self._pack_few()
             if self._packed is not None:
                 self.pack(residue)
         else:
@@ -266,6 +271,10 @@ class Kernel:
             self._bound, self._pass, self._work = bind_step(self, *self._here, graph)
         self._direct = not graph
 
+    def _pack_few(self):
+        with torch.cuda.device(self.device):
+            ok(lib().vesta_pass_pack(self._pass, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+
     def tensor_maps(self, residue):
         """the TMA descriptors of the step kernel, in device memory: the caches as the attention phase reads
         them (K and V with boxes of 32, 64, 96 and 128 rows of one head), then the embedding table in boxes of
@@ -283,12 +292,14 @@ class Kernel:
         return host.to(self.device)
 
     def pack(self, residue=None):
-        """(re)build the packed weight streams from the bound weights; call again after changing them (a chain reads the
+        """(re)build the packed weights from the bound ones; call again after changing them (a chain of more than few sequences reads the
         weights where they are: nothing to do but for weights that do not start on a 16-byte boundary, of which it reads a
         copy, unless its persistent kernel has been asked for)"""
         for copy, original in self._copies.values():
             copy.copy_(original)
-        if self.chain and self._packed is None:
+        if self.few:
+            self._pack_few()
+        if self.graphs and self._packed is None:
             return
         residue = residue or self.keep
         L = lib()
@@ -312,7 +323,7 @@ class Kernel:
         per = per_launch or self.fuse
         if steps > 1 and per > 1 and self.feeds_back:
             ok(lib().vesta_step_run_fused(self._bound, stream, steps, per))
-            self.launches += steps if self.chain else -(-steps // per)
+            self.launches += steps if self.graphs else -(-steps // per)
         else:
             ok(lib().vesta_step_run(self._bound, stream, steps))
             self.launches += steps
@@ -359,9 +370,9 @@ class Kernel:
 
     def clear_status(self):
         """forget a refused step or an abandoned wait: status word, abort flag and the barrier counters back to zero.
-        The status stays until this is called. After an abandoned wait, and in a chain after a refused step too, every
-        further launch returns without touching x, t or the cache; the persistent kernels run a good step after a refused
-        one. (A refused step never wrote anything; a launch in which a wait ran out may have written part of a step, so
+        The status stays until this is called. After an abandoned wait, and in a chain of more than few sequences after a refused step too, every
+        further launch returns without touching x, t or the cache; the persistent kernels and the chain of few sequences run a good step
+        after a refused one. (A refused step never wrote anything; a launch in which a wait ran out may have written part of a step, so
         reset or reload the decode state before going on.)"""
         self.bar.zero_()
 

@@ -1,7 +1,7 @@
 """Placement of a decode-step program on the 148 SMs of a B200 and assembly of the CUDA source
-of ONE persistent cooperative kernel (plus a one-time weight-packing kernel). With more than a few
-sequences a step runs as a chain of the library's own kernels instead (csrc/pass.cu; dims['chain']
-says so): the source is then compiled only for callers that ask for the persistent kernel.
+of ONE persistent cooperative kernel (plus a one-time weight-packing kernel). Where nothing asks for
+that kernel a step runs as a chain of the library's own kernels instead (csrc/pass.cu; dims['chain'],
+for few sequences dims['few'] says so): the source is then compiled only for callers that want it.
 
     lower(text, res, axis_max, batch=1, per_token=(), outputs=(), feedback=None, timing=False) -> Lowered
 
@@ -49,8 +49,8 @@ DEFAULT_SMS = 148      # B200
 @dataclass
 class Lowered:
     """What lower() makes of a program. `src`, `shared_bytes`, `barriers_per_launch`, `plan`, `sites`, `block`, `place`, `packed_bytes`
-    and the placement entries of `dims` (tc, tcl, ksplit, nch, ...) describe the persistent kernel, also where dims['chain'] is
-    set and Kernel runs steps as a chain; the tiles of a chain are the library's choice (passes.tiles)."""
+    and the placement entries of `dims` (tc, tcl, ksplit, nch, ...) describe the persistent kernel, also where dims['chain'] or
+    dims['few'] is set and Kernel runs steps as a chain; the tiles of a chain are the library's choice (passes.tiles)."""
     src: str
     params: list             # (name, dtype, emitted) in kernel argument order
     scratch: dict            # host-visible name -> (offset, axes, static shape)
@@ -523,6 +523,12 @@ def _lower_small(env, dims, res, roles, fb, B, tmax, cpos, t_per_token, t_name, 
                    dims=dict(dims, B=B, NB=1, tmax=tmax, notes=notes, WG=WG, chunk_tiles=ch, tc=False, ksplit=False, kernel='small', warps=nw,
                              nch=nch, kv_stages=kvst, ring_slots=nslot, fuse_proj=fuse, fuse_exchange=fuse_x, qkv_exchange=fuse_x2, part_exchange=fuse_x3, fuse_base=(fuse_base if fuse else 0), ordered=fixed_sums), roles=roles)
 
+def few_fits(D, F, B, sms=DEFAULT_SMS):
+    """whether a step of few sequences can run from packed weights in shared memory: at most two tiles of 16 features per SM
+    (`few_plan` of csrc/pass.cu refuses what does not fit)"""
+    return B <= 8 and D <= 1024 and 3 * D <= 32 * sms and F <= 32 * sms
+
+
 def lower(text, res, axis_max, batch=1, per_token=(), outputs=(), feedback=None, timing=False,
           grid=DEFAULT_SMS, act_lo=None, prompt_len=0, slab_tiles=None, tune=None, row_seq=False):
     """See the module docstring. `res`: name -> (shape, dtype) as the kernel sees them (batched
@@ -598,16 +604,20 @@ def lower(text, res, axis_max, batch=1, per_token=(), outputs=(), feedback=None,
     tune = dict(tune or {})
     # What a step as a chain of kernels (csrc/pass.cu) needs to know; Kernel runs that chain unless the caller asked for
     # something that only the persistent kernels have (a placement option, timing sums, rows of prompts).
-    # Up to eight sequences the small persistent kernel is the faster one at widths up to 1,024 (small shape at 200 positions: one
-    # sequence 174 against 227 us per step, four 189 against 232, eight 213 against 247, at 1,000 positions 268 against 282): its
-    # exchanges between a few CTAs cost less than kernel boundaries. The wider the rows, the less a boundary weighs and the more
+    # Up to eight sequences of widths to 1,024 a chain of three kernels per layer from packed weights (csrc/pass_few.cuh) is the
+    # fastest (small shape, per step: one sequence at 37 positions 184 in the small persistent kernel, 166 us so; eight at 128 to 144
+    # 209 and 184). Beyond (wider rows, or an MLP of more than 32 features per SM: the weights of a layer's kernels do not fit shared
+    # memory side by side) the small persistent kernel stands against the chain of seven kernels per layer:
+    # the wider the rows, the less a boundary weighs and the more
     # every CTA's norms do: width 1,280 (twelve layers) with four sequences 280 against 279, with five 293 against 286; XL shape
     # with three 1,253 against 1,168, two 1,224 against 1,165 and one 1,155 against 1,157 (left where results repeat bit for bit);
     # and with more (sequence, head) pairs than CTAs the kernel falls back on grid barriers (XL shape, eight: 1,679 against 1,245).
     persistent = B <= (8 if D <= 1024 else 4 if D <= 1280 else 2) and B * H <= grid
-    dims = dict(dims, chain=not (tune or timing or row_seq or slab_tiles or act_lo is not None) and not persistent and D <= 4096,
+    plain = not (tune or timing or row_seq or slab_tiles or act_lo is not None)
+    few = plain and persistent and few_fits(D, F, B)
+    dims = dict(dims, chain=plain and not persistent and D <= 4096, few=few,
                 step=dict(t_stride=int(t_per_token), tstep=int(fb.get(t_name, 0)), feedback=int(bool(fb)), prompt_len=int(prompt_len) if fb else 0,
-                          exact=int(B <= 8 or (B <= 16 and D <= 1024)), cpos=cpos))
+                          exact=2 if few else int(B <= 8 or (B <= 16 and D <= 1024)), cpos=cpos))
     if B <= 8 and not tune.get('large_kernel') and act_lo is None and not slab_tiles and not row_seq:
         return _lower_small(env, dims, res, roles, fb, B, tmax, cpos, t_per_token, t_name, prompt_len, timing, grid, tune)
 

@@ -1,4 +1,4 @@
-"""Forward passes as chains of kernels (csrc/pass.cu, csrc/pass_kernels.cuh): the descriptor of a pass and the dense prompt
+"""Forward passes as chains of kernels (csrc/pass.cu, csrc/pass_kernels.cuh, csrc/pass_few.cuh): the descriptor of a pass and the dense prompt
 pass behind VestaGPT2.prefill."""
 import ctypes
 import weakref
@@ -54,9 +54,10 @@ def describe(low, residue, zeros, cpos, **kw):
     return desc
 
 
-def kernels_of_a_step(layers):
-    """kernels that a decode step launches as a chain: seven per layer, the embedding with its norm, the logits, the end"""
-    return 7 * layers + 3
+def kernels_of_a_step(layers, few=False):
+    """kernels that a decode step launches as a chain: seven per layer, the embedding with its norm, the logits, the end; of few
+    sequences three per layer (the first makes the embedding), the last norm, the logits, the end"""
+    return (3 if few else 7) * layers + 3
 
 
 def tiles(desc, rows, logit_rows):
