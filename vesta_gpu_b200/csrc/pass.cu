@@ -241,11 +241,12 @@ cudaError_t prepare_all() {
     auto one = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
     one(all_shared(pass_norm<NORM_EMBED>)); one(all_shared(pass_norm<NORM_MID>)); one(all_shared(pass_norm<NORM_FINAL>));
     one(all_shared(pass_norm_rows<6>)); one(all_shared(pass_norm_rows<13>)); one(all_shared(pass_norm_rows<16>));
-    one(all_shared(pass_attend<2>)); one(all_shared(pass_attend<4>)); one(all_shared(pass_attend_many<true>)); one(all_shared(pass_attend_many<false>));
+    one(all_shared(pass_attend<2, 4>)); one(all_shared(pass_attend<2, 8>)); one(all_shared(pass_attend<3, 8>)); one(all_shared(pass_attend_many<true>)); one(all_shared(pass_attend_many<false>));
     one(gemm_prepare());
     one(cudaFuncSetAttribute((const void*)pass_attend_many<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, AM_SMEM));
     one(cudaFuncSetAttribute((const void*)pass_attend_many<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AM_SMEM));
-    one(cudaFuncSetAttribute((const void*)pass_attend<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * ATT_WARPS * 4096)); one(all_shared(pass_finish));
+    one(cudaFuncSetAttribute((const void*)pass_attend<3, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * 8 * 4096));
+    one(cudaFuncSetAttribute((const void*)pass_attend<2, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 8 * 4096)); one(all_shared(pass_finish));
     return e;
 }
 int epi_of(int kind) { return kind == K_QKV ? EPI_QKV : kind == K_FC ? EPI_GELU : kind == K_LOGITS ? EPI_LOGITS : EPI_ADD; }
@@ -325,8 +326,12 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
     // positions. Clusters of four and eight lost everywhere (XL shape, 6 sequences at 128 positions: 1,342 -> 1,337 us per
     // step with two blocks instead of four; 9 sequences, small shape, two instead of eight: 298 -> 270 us, at 1,000 positions
     // 340 -> 321), and so did two beyond that line (23 sequences at 128 positions with one block: 294 -> 277 us).
-    const int C = rows * d.H * 2 <= 3 * p.sms && d.tmax > ATT_WARPS * ATT_RUN ? 2 : 1;
-    const bool deep = rows * d.H * C <= 3 * p.sms;
+    const int C = rows * d.H * 2 <= 3 * p.sms && d.tmax > 4 * ATT_RUN ? 2 : 1;
+    // ... eight warps and deeper rings where an SM has no more than three blocks, and where it has no more than two rings that keep a third
+    // away: blocks go where there is room, which is not evenly (23 ragged sequences to 700 positions, 276 blocks: 7.05 us with four warps and
+    // rings of 64 KB, 6.15 with eight, 4.92 with eight and 96 KB; XL shape with 16, 400 blocks: 4.31, 4.30 and 6.08). Beyond, four warps: 64
+    // sequences 16.0 us, with eight 17.1.
+    const int crowd = (rows * d.H * C + p.sms - 1) / p.sms;
     const Pass::Plan* pl = nullptr;
     if (int e = plan_for(p, rows, lrows, &pl)) return e;
     auto f16 = [](const void* q, size_t off) { return (const u16*)q + off; };
@@ -386,9 +391,9 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
             return pow2 ? cudaLaunchKernelEx(&c.c, pass_attend_many<true>, p.qmap, p.kmap, p.vmap, a) : cudaLaunchKernelEx(&c.c, pass_attend_many<false>, p.qmap, p.kmap, p.vmap, a);
         }
         AttArgs a = {q, kc, vc, ss, (const int*)d.t, d.t_stride, d.tmax, D, pow2, p.rp, d.scale, att};
-        Config c(dim3(d.H, rows, C), ATT_WARPS * 32, st, true, C);
-        c.c.dynamicSmemBytes = (deep ? 4 : 2) * ATT_WARPS * 4096;
-        return deep ? cudaLaunchKernelEx(&c.c, pass_attend<4>, a) : cudaLaunchKernelEx(&c.c, pass_attend<2>, a);
+        Config c(dim3(d.H, rows, C), crowd <= 3 ? 256 : 128, st, true, C);
+        c.c.dynamicSmemBytes = (crowd <= 2 ? 24 : crowd <= 3 ? 16 : 8) * 4096;
+        return crowd <= 2 ? cudaLaunchKernelEx(&c.c, pass_attend<3, 8>, a) : crowd <= 3 ? cudaLaunchKernelEx(&c.c, pass_attend<2, 8>, a) : cudaLaunchKernelEx(&c.c, pass_attend<2, 4>, a);
     };
     TRY(norm(0, 0));
     for (int l = 0; l < L; l++) {

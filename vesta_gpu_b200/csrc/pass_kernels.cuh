@@ -685,7 +685,6 @@ struct AttArgs {
     float scale;
     u16* out;                        // [row][D] fp16 (and the remainder plane)
 };
-#define ATT_WARPS 4
 __device__ __forceinline__ int kv_off(int row, int piece) { return row * 128 + ((piece ^ (row & 7)) << 4); }
 __device__ __forceinline__ void cp16(u32 dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory"); }
 __device__ __forceinline__ void ldsm4(u32 (&r)[4], u32 p) {
@@ -842,14 +841,14 @@ template <int NS> struct AttRow {
         if (lane == 0) { part[64] = m; part[65] = den; }
     }
 };
-template <int NS>
-__global__ void __launch_bounds__(ATT_WARPS * 32) pass_attend(const __grid_constant__ AttArgs a) {
-    __shared__ float part[ATT_WARPS + 1][66];
+template <int NS, int W>
+__global__ void __launch_bounds__(W * 32) pass_attend(const __grid_constant__ AttArgs a) {
+    __shared__ float part[W + 1][66];
     extern __shared__ __align__(128) unsigned char ring_raw[];
     const int h = blockIdx.x, row = blockIdx.y, C = gridDim.z, cr = blockIdx.z, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) dep_launch();
     if (C == 2) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // (waited for before the other block's memory is written)
-    AttRow<NS> r(a, row, h, (cr * ATT_WARPS + warp) * ATT_RUN, C * ATT_WARPS * ATT_RUN, smem_u32(ring_raw) + warp * (NS * 4096));
+    AttRow<NS> r(a, row, h, (cr * W + warp) * ATT_RUN, C * W * ATT_RUN, smem_u32(ring_raw) + warp * (NS * 4096));
     r.request_first();
     dep_wait();
     r.run(true, part[warp]);
@@ -857,24 +856,24 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) pass_attend(const __grid_const
     float M = -3.0e38f, dd = 0.f, num = 0.f;
     if (threadIdx.x < 64) {
 #pragma unroll
-        for (int i = 0; i < ATT_WARPS; i++) M = fmaxf(M, part[i][64]);
+        for (int i = 0; i < W; i++) M = fmaxf(M, part[i][64]);
 #pragma unroll
-        for (int i = 0; i < ATT_WARPS; i++) { const float c = fast_exp(part[i][64] - M); dd += part[i][65] * c; num += part[i][threadIdx.x] * c; }
+        for (int i = 0; i < W; i++) { const float c = fast_exp(part[i][64] - M); dd += part[i][65] * c; num += part[i][threadIdx.x] * c; }
     }
     if (C == 2) {
         // the second block's result goes into the first one's shared memory
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         if (cr == 1 && threadIdx.x < 64) {
-            const u32 to = of_first(smem_u32(&part[ATT_WARPS][0]));
+            const u32 to = of_first(smem_u32(&part[W][0]));
             asm volatile("st.shared::cluster.f32 [%0], %1;" :: "r"(to + threadIdx.x * 4), "f"(num) : "memory");
             if (threadIdx.x == 0) asm volatile("st.shared::cluster.f32 [%0], %1;\n\tst.shared::cluster.f32 [%0+4], %2;" :: "r"(to + 64 * 4), "f"(M), "f"(dd) : "memory");
         }
         cluster_sync();
         if (cr == 1) return;
         if (threadIdx.x < 64) {
-            const float m1 = part[ATT_WARPS][64], top = fmaxf(M, m1), c0 = fast_exp(M - top), c1 = fast_exp(m1 - top);
-            dd = dd * c0 + part[ATT_WARPS][65] * c1;
-            num = num * c0 + part[ATT_WARPS][threadIdx.x] * c1;
+            const float m1 = part[W][64], top = fmaxf(M, m1), c0 = fast_exp(M - top), c1 = fast_exp(m1 - top);
+            dd = dd * c0 + part[W][65] * c1;
+            num = num * c0 + part[W][threadIdx.x] * c1;
         }
     }
     if (threadIdx.x < 64) {
