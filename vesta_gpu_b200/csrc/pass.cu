@@ -212,7 +212,7 @@ int check(const vesta_pass_desc& d) {
 template <class F> cudaError_t all_shared(F* f) { return cudaFuncSetAttribute((const void*)f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared); }
 template <int BM, int EPI>
 cudaError_t launch_gemm(cudaLaunchConfig_t& c, const Tile& t, const CUtensorMap& w, const CUtensorMap& a, const GemmArgs& g) {
-    c.dynamicSmemBytes = GemmShape<BM>::bytes(t.stages, t.bn);
+    c.dynamicSmemBytes = std::max<size_t>(GemmShape<BM>::bytes(t.stages, t.bn), c.dynamicSmemBytes);
     c.blockDim = dim3(GemmShape<BM>::THREADS + (EPI == EPI_QKV && g.seqs ? 32 : 0));
     return cudaLaunchKernelEx(&c, pass_gemm<BM, EPI>, w, a, g);
 }
@@ -327,11 +327,12 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
     // step with two blocks instead of four; 9 sequences, small shape, two instead of eight: 298 -> 270 us, at 1,000 positions
     // 340 -> 321), and so did two beyond that line (23 sequences at 128 positions with one block: 294 -> 277 us).
     const int C = rows * d.H * 2 <= 3 * p.sms && d.tmax > 4 * ATT_RUN ? 2 : 1;
-    // ... eight warps and deeper rings where an SM has no more than three blocks, and where it has no more than two rings that keep a third
-    // away: blocks go where there is room, which is not evenly (23 ragged sequences to 700 positions, 276 blocks: 7.05 us with four warps and
-    // rings of 64 KB, 6.15 with eight, 4.92 with eight and 96 KB; XL shape with 16, 400 blocks: 4.31, 4.30 and 6.08). Beyond, four warps: 64
-    // sequences 16.0 us, with eight 17.1.
-    const int crowd = (rows * d.H * C + p.sms - 1) / p.sms;
+    // ... eight warps where an SM has no more than three blocks, and rings that keep a third block away where two are due: blocks go
+    // where there is room, which is not evenly (23 ragged sequences to 700 positions, 276 blocks: 7.05 us with four warps and rings of
+    // 64 KB, 6.15 with eight, 4.92 with eight and 96 KB; 9 at 900, 216 blocks: 290, 286 and 269 us per step; XL shape with 16, 400 blocks: 4.31,
+    // 4.30 and 6.08 us; with 3, 150 blocks: 1,157, 1,162 and 1,186 us per step). Beyond, four warps: 64 sequences 16.0 us, with eight 17.1.
+    const int blocks = rows * d.H * C;
+    const bool wide = blocks <= 3 * p.sms, deep = blocks <= 2 * p.sms && 4 * blocks > 5 * p.sms;
     const Pass::Plan* pl = nullptr;
     if (int e = plan_for(p, rows, lrows, &pl)) return e;
     auto f16 = [](const void* q, size_t off) { return (const u16*)q + off; };
@@ -378,6 +379,10 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
         } else { g.of = z; g.bias = kind == K_PROJ ? f16(d.ob, (size_t)l * D) : f16(d.pb, (size_t)l * D); }
         g.bn = t.bn; g.ftiles = (g.nfeat + t.bm - 1) / t.bm; g.rtiles = p.rp ? 1 : (g.rows + t.bn - 1) / t.bn; g.ntiles = g.ftiles * g.rtiles * t.splits;
         Config c(dim3(t.bm == 64 ? g.ntiles : t.bm == 256 ? 2 * std::min(g.ntiles, p.sms / 2) : std::min(g.ntiles, p.sms)), 0, st, true, t.bm == 256 ? 2 : 1, true);
+        // The projection's blocks are small and come while the attention's leave: five of them on the first SMs that are free, none on the
+        // last. Where there is about one for every SM they ask for so much that only two fit (64 sequences, 144 blocks of 41 KB: 1,763 ->
+        // 1,721 us per four steps; 23 sequences, 72 blocks: 1,111 -> 1,122, left).
+        if (kind == K_PROJ && t.bm == 64 && 2 * g.ntiles > p.sms) c.c.dynamicSmemBytes = 110 * 1024;
         return gemm(epi_of(kind), t, c.c, pl->w[kind], pl->a[kind], g);
     };
     auto attend = [&](int l) {
@@ -391,9 +396,9 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
             return pow2 ? cudaLaunchKernelEx(&c.c, pass_attend_many<true>, p.qmap, p.kmap, p.vmap, a) : cudaLaunchKernelEx(&c.c, pass_attend_many<false>, p.qmap, p.kmap, p.vmap, a);
         }
         AttArgs a = {q, kc, vc, ss, (const int*)d.t, d.t_stride, d.tmax, D, pow2, p.rp, d.scale, att};
-        Config c(dim3(d.H, rows, C), crowd <= 3 ? 256 : 128, st, true, C);
-        c.c.dynamicSmemBytes = (crowd <= 2 ? 24 : crowd <= 3 ? 16 : 8) * 4096;
-        return crowd <= 2 ? cudaLaunchKernelEx(&c.c, pass_attend<3, 8>, a) : crowd <= 3 ? cudaLaunchKernelEx(&c.c, pass_attend<2, 8>, a) : cudaLaunchKernelEx(&c.c, pass_attend<2, 4>, a);
+        Config c(dim3(d.H, rows, C), wide ? 256 : 128, st, true, C);
+        c.c.dynamicSmemBytes = (deep ? 24 : wide ? 16 : 8) * 4096;
+        return deep ? cudaLaunchKernelEx(&c.c, pass_attend<3, 8>, a) : wide ? cudaLaunchKernelEx(&c.c, pass_attend<2, 8>, a) : cudaLaunchKernelEx(&c.c, pass_attend<2, 4>, a);
     };
     TRY(norm(0, 0));
     for (int l = 0; l < L; l++) {
