@@ -30,7 +30,7 @@ struct Tile { int bm, bn, stages, splits; };
 
 struct Layout {
     size_t z, q, act, att, gelu, fin, best, rowoff, pos, skip;
-    size_t sums[2], packed;                    // few sequences: the vectors after the MLP, in turn; the packed weights
+    size_t after[2], sums[2], packed;          // few sequences: the state after the attention and the MLP's sums, of two layers in turn; the packed weights
     size_t meta, total;                        // prompts: tokens, positions, sequences of the rows; attention runs; rows that want logits and where they go; lengths
 };
 // the metadata of a pass over prompts, as offsets in 32-bit words
@@ -136,7 +136,7 @@ Layout layout(const Pass& p, int D, int F, int rows, int lrows) {
     auto take = [&](size_t bytes) { const size_t r = at; at += (bytes + 255) / 256 * 256; return r; };
     if (p.few.on) {
         const size_t state = (size_t)rows * D * (p.few.fixed ? 8 : 4);
-        o.z = take(state); o.sums[0] = take(state); o.sums[1] = take(state);
+        for (int i = 0; i < 2; i++) { o.after[i] = take(state); o.sums[i] = take(state); }
         o.q = take((size_t)rows * D * 4);
         o.fin = take((size_t)p.fplanes * D * 2);
         o.best = take((size_t)lrows * 8);
@@ -475,7 +475,7 @@ int enqueue_few(Pass& p, cudaStream_t st) {
         const long long ss = (long long)d.L * d.tmax * D;
         {
             FewQkv a = {};
-            a.n = {D, R, d.eps, u(p.o.sums[(l + 1) & 1]), f16(d.ln1w, (size_t)l * D), f16(d.ln1b, (size_t)l * D), u(p.o.z), f16(d.ob, (size_t)l * D), u(p.o.sums[l & 1])};
+            a.n = {D, R, d.eps, u(p.o.after[(l + 1) & 1]), u(p.o.sums[(l + 1) & 1]), f16(d.ln1w, (size_t)l * D), f16(d.ln1b, (size_t)l * D), u(p.o.after[l & 1]), f16(d.ob, (size_t)l * D), u(p.o.sums[l & 1])};
             a.w = w + pk.qkv; a.bias = f16(d.qkvb, (size_t)l * 3 * D); a.tiles = 3 * D / 16; a.per = f.qkv_per; a.q = (float*)u(p.o.q); a.kc = kc; a.vc = vc; a.seq_stride = ss;
             a.x = (const int*)d.x; a.t = (const int*)d.t; a.t_stride = d.t_stride; a.tmax = d.tmax; a.cpos = d.cpos; a.N = d.N; a.first = l == 0; a.wte = (const u16*)d.wte; a.wpe = (const u16*)d.wpe;
             a.pos = (int*)u(p.o.pos); a.skip = (int*)u(p.o.skip); a.bar = (u32*)d.bar;
@@ -486,14 +486,14 @@ int enqueue_few(Pass& p, cudaStream_t st) {
         {
             FewAttend a = {};
             a.a = {(const float*)u(p.o.q), kc, vc, ss, (const int*)d.t, d.t_stride, d.tmax, D, pow2, 0, d.scale, nullptr};
-            a.rows = R; a.chunks = wpr; a.w = w + pk.proj; a.z = u(p.o.z);
+            a.rows = R; a.chunks = wpr; a.w = w + pk.proj; a.z = u(p.o.after[l & 1]);
             Config c(dim3(FEW_CLUSTER, d.H), FEW_THREADS, st, true, FEW_CLUSTER, true);
             c.c.dynamicSmemBytes = FewAttend::bytes(D);
             TRY(few_launch(c.c, R <= 4, f.fixed, a));
         }
         {
             FewMlp a = {};
-            a.n = {D, R, d.eps, u(p.o.z), f16(d.ln2w, (size_t)l * D), f16(d.ln2b, (size_t)l * D), u(p.o.sums[l & 1]), f16(d.pb, (size_t)l * D), nullptr};
+            a.n = {D, R, d.eps, u(p.o.after[l & 1]), nullptr, f16(d.ln2w, (size_t)l * D), f16(d.ln2b, (size_t)l * D), u(p.o.sums[l & 1]), f16(d.pb, (size_t)l * D), nullptr};
             a.fc = w + pk.fc; a.p2 = w + pk.p2; a.bias = f16(d.fcb, (size_t)l * F); a.tiles = F / 16; a.per = f.mlp_per;
             a.a2 = 2 * d.gelu_a; a.k1 = d.gelu_b * 2.8853900817779268f; a.k2 = d.gelu_c * a.k1;
             Config c(dim3((a.tiles + a.per - 1) / a.per), FEW_THREADS, st, true);
@@ -503,7 +503,7 @@ int enqueue_few(Pass& p, cudaStream_t st) {
     }
     NormArgs n = {};
     n.D = D; n.rp = p.rp; n.eps = d.eps; n.gain = f16(d.lnfw, 0); n.shift = f16(d.lnfb, 0); n.act = (u16*)u(p.o.fin);
-    n.z = (float*)u(p.o.sums[(d.L - 1) & 1]); n.fixed = f.fixed;
+    n.z = (float*)u(p.o.after[(d.L - 1) & 1]); n.more = u(p.o.sums[(d.L - 1) & 1]); n.fixed = f.fixed;
     Config cn(dim3(R), up(D / 4, 32), st, true);
     TRY(cudaLaunchKernelEx(&cn.c, pass_norm<NORM_FINAL>, n));
     const Tile& t = pl->tile[K_LOGITS];

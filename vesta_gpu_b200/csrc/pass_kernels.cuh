@@ -79,6 +79,10 @@ __device__ __forceinline__ u32 elect_one() {
 template <bool FIXED> struct State;
 template <> struct State<false> {
     static __device__ __forceinline__ float4 load(const void* z, size_t i) { return __ldcg(reinterpret_cast<const float4*>((const float*)z + i)); }
+    static __device__ __forceinline__ float4 load(const void* z, const void* more, size_t i) {       // the sum of two vectors
+        const float4 a = load(z, i), b = load(more, i);
+        return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+    }
     static __device__ __forceinline__ void store(void* z, size_t i, float4 v) { *reinterpret_cast<float4*>((float*)z + i) = v; }
     static __device__ __forceinline__ void add1(void* z, size_t i, float v) { asm volatile("red.relaxed.gpu.global.add.f32 [%0], %1;" :: "l"((float*)z + i), "f"(v) : "memory"); }
     static __device__ __forceinline__ void add(void* z, size_t i, float4 v) {
@@ -91,6 +95,11 @@ template <> struct State<true> {
         const longlong2* p = reinterpret_cast<const longlong2*>((const long long*)z + i);
         const longlong2 a = __ldcg(p), b = __ldcg(p + 1);
         return make_float4(from(a.x), from(a.y), from(b.x), from(b.y));
+    }
+    static __device__ __forceinline__ float4 load(const void* z, const void* more, size_t i) {
+        const longlong2 *p = reinterpret_cast<const longlong2*>((const long long*)z + i), *q = reinterpret_cast<const longlong2*>((const long long*)more + i);
+        const longlong2 a = __ldcg(p), b = __ldcg(p + 1), c = __ldcg(q), d = __ldcg(q + 1);
+        return make_float4(from(a.x + c.x), from(a.y + c.y), from(b.x + d.x), from(b.y + d.y));
     }
     static __device__ __forceinline__ void store(void* z, size_t i, float4 v) {
         longlong2* p = reinterpret_cast<longlong2*>((long long*)z + i);
@@ -569,7 +578,8 @@ struct NormArgs {
     int *pos, *skip;
     u32* bar;                        // [0] status, [2] abort flag
     const int* want;                 // FINAL: rows that want logits (0: all)
-    int fixed;                       // FINAL: the state is State<true>
+    const void* more;                // FINAL: a vector to add to the state (0: none)
+    int fixed;                       // ... and both are State<true>
 };
 
 // One row per block, four elements per thread (the row stays in registers). Latency bound for few rows:
@@ -607,7 +617,9 @@ __global__ void __launch_bounds__(1024) pass_norm(const __grid_constant__ NormAr
             v = make_float4(h_lo(e.x) + h_lo(p.x), h_hi(e.x) + h_hi(p.x), h_lo(e.y) + h_lo(p.y), h_hi(e.y) + h_hi(p.y));
         }
     } else if (own) {
-        v = MODE == NORM_FINAL && a.fixed ? State<true>::load(a.z, (size_t)row * a.D + d) : State<false>::load(a.z, (size_t)row * a.D + d);
+        const size_t at = (size_t)row * a.D + d;
+        if (MODE == NORM_FINAL && a.more) v = a.fixed ? State<true>::load(a.z, a.more, at) : State<false>::load(a.z, a.more, at);
+        else v = State<false>::load(a.z, at);
     }
     if (own && MODE == NORM_EMBED) *reinterpret_cast<float4*>(a.z + (size_t)row * a.D + d) = v;
     float s = (v.x + v.y) + (v.z + v.w);
@@ -711,7 +723,7 @@ __device__ __forceinline__ void cp16z(u32 dst, const void* src, bool yes) {
 }
 // One warp's runs of a row's positions: from `p0`, every `step`, through its ring of NS stages of 4 KB. request_first() asks for
 // what is there since earlier steps, run() waits for nothing but that and leaves the 64 sums, the maximum and the sum of the weights
-// in `part`; run(false) does one round of the same on what there is (see FEW_DRY).
+// in `part`; run(false) does one round of the same on what there is (a dry pass, see pass_few.cuh).
 template <int NS> struct AttRow {
     const AttArgs& a;
     int row, h, first, step, n;

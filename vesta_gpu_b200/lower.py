@@ -605,8 +605,8 @@ def lower(text, res, axis_max, batch=1, per_token=(), outputs=(), feedback=None,
     # What a step as a chain of kernels (csrc/pass.cu) needs to know; Kernel runs that chain unless the caller asked for
     # something that only the persistent kernels have (a placement option, timing sums, rows of prompts).
     # Up to eight sequences of widths to 1,024 a chain of three kernels per layer from packed weights (csrc/pass_few.cuh) is the
-    # fastest (small shape, per step: one sequence at 37 positions 184 in the small persistent kernel, 166 us so; eight at 128 to 144
-    # 209 and 184). Beyond (wider rows, or an MLP of more than 32 features per SM: the weights of a layer's kernels do not fit shared
+    # fastest (small shape, per step: one sequence at 37 positions 183 in the small persistent kernel, 169 us so; eight at 128 to 144
+    # 209 and 192). Beyond (wider rows, or an MLP of more than 32 features per SM: the weights of a layer's kernels do not fit shared
     # memory side by side) the small persistent kernel stands against the chain of seven kernels per layer:
     # the wider the rows, the less a boundary weighs and the more
     # every CTA's norms do: width 1,280 (twelve layers) with four sequences 280 against 279, with five 293 against 286; XL shape
