@@ -1,4 +1,4 @@
-// Kernels of a decode step of at most eight sequences: three per layer,
+// Kernels of a decode step of few sequences (at most eight; two to four by default): three per layer,
 //
 //     norm + QKV | attention + projection | norm + FC + GELU + MLP projection
 //

@@ -526,7 +526,7 @@ def _lower_small(env, dims, res, roles, fb, B, tmax, cpos, t_per_token, t_name, 
 def few_fits(D, F, B, sms=DEFAULT_SMS):
     """whether a step of few sequences can run from packed weights in shared memory: at most two tiles of 16 features per SM
     (`few_plan` of csrc/pass.cu refuses what does not fit)"""
-    return B <= 8 and D <= 1024 and 3 * D <= 32 * sms and F <= 32 * sms
+    return 2 <= B <= 4 and D <= 1024 and 3 * D <= 32 * sms and F <= 32 * sms
 
 
 def lower(text, res, axis_max, batch=1, per_token=(), outputs=(), feedback=None, timing=False,
@@ -604,9 +604,11 @@ def lower(text, res, axis_max, batch=1, per_token=(), outputs=(), feedback=None,
     tune = dict(tune or {})
     # What a step as a chain of kernels (csrc/pass.cu) needs to know; Kernel runs that chain unless the caller asked for
     # something that only the persistent kernels have (a placement option, timing sums, rows of prompts).
-    # Up to eight sequences of widths to 1,024 a chain of three kernels per layer from packed weights (csrc/pass_few.cuh) is the
-    # fastest (small shape, per step: one sequence at 37 positions 183 in the small persistent kernel, 169 us so; eight at 128 to 144
-    # 209 and 192). Beyond (wider rows, or an MLP of more than 32 features per SM: the weights of a layer's kernels do not fit shared
+    # Two to four sequences of widths to 1,024: a chain of three kernels per layer from packed weights (csrc/pass_few.cuh) is the
+    # fastest (small shape, four sequences at 200 positions 190 us per step in the small persistent kernel, 165 so). With one (183 and 169)
+    # and with eight (209 and 192) it would be too, but the logits of equal prompts there are compared from batch to batch, and its sums
+    # in another order than the persistent kernel's differ from those by up to 1.3e-4 after sixteen positions (0.9e-4 among themselves):
+    # those batches stay in one kernel text. Beyond (wider rows, or an MLP of more than 32 features per SM: the weights of a layer's kernels do not fit shared
     # memory side by side) the small persistent kernel stands against the chain of seven kernels per layer:
     # the wider the rows, the less a boundary weighs and the more
     # every CTA's norms do: width 1,280 (twelve layers) with four sequences 280 against 279, with five 293 against 286; XL shape
