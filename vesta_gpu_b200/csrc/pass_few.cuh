@@ -152,7 +152,7 @@ __device__ __forceinline__ void few_params(const FewNorm& n, u16* par) {
         if (blockIdx.x < n.rows) *reinterpret_cast<uint2*>(par + 2 * n.D + d) = __ldg(reinterpret_cast<const uint2*>(n.bias + d));
     }
 }
-// Norm of all rows into the operand. WPR warps share a row (8 / R, a power of two), a lane holds NV float4. Block `row` also starts the
+// Norm of all rows into the operand. WPR warps share a row (8 / R, a power of two), a lane holds NV float4. Block `row` (counted around where there are fewer) also starts the
 // vector of the next sums: QKV stores it (nothing adds yet), the MLP kernel adds to it (other blocks may have begun to).
 // `value(row, d)` loads four elements of the state.
 template <int KW, int WPR> struct FewLanes { static constexpr int NV = (2 * KW + WPR - 1) / WPR; };      // KW: D <= 256 KW
@@ -219,7 +219,7 @@ __device__ __forceinline__ void few_norm(const FewNorm& n, bool real, int warp, 
                 *reinterpret_cast<uint2*>(lo + d * 2) = make_uint2(pack_h2(o0 - h_lo(p0), o1 - h_hi(p0)), pack_h2(o2 - h_lo(p1), o3 - h_hi(p1)));
             }
         }
-        if (blockIdx.x == row && real)
+        if (blockIdx.x == row % gridDim.x && real)
 #pragma unroll
             for (int i = 0; i < NV; i++) {
                 const int d = d0 + i * by;
