@@ -147,6 +147,17 @@ def test_a_pass_refuses_sizes_that_would_leave_its_buffers(built_library):
         assert sizes(**bad) != 0 and L.vesta_last_error().startswith(b'vesta_pass'), bad
 
 
+def test_a_step_from_packed_weights_refuses_rows_without_logits(built_library):
+    """its end writes a row of logits and a token for every row: fewer logit rows would be written past the ends of both"""
+    from vesta_gpu_b200 import launch
+    L, n = launch.lib(), ctypes.c_size_t()
+    for rows, lrows, fine in ((4, 4, True), (4, 3, False), (2, 2, True), (2, 1, False)):
+        d = pass_desc(exact=2, rows=rows, logit_rows=lrows)
+        assert (L.vesta_pass_workspace(ctypes.byref(d), ctypes.byref(n)) == 0) == fine, (rows, lrows)
+        if not fine:
+            assert b'packed weights' in L.vesta_last_error() and 'packed weights' in create_pass(d)
+
+
 @pytest.mark.parametrize('name,exact', [('gpt2', 0), ('gpt2_xl', 0), ('tiny3', 0), ('heads20', 0), ('gpt2', 1), ('tiny', 1)])
 def test_tiles_of_a_pass_fit_a_block(built_library, name, exact):
     """every tile that is chosen is one the kernels are written for: the rows of one product, the columns of tensor memory (two

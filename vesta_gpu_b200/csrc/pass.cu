@@ -161,9 +161,10 @@ Layout layout(const Pass& p, int D, int F, int rows, int lrows) {
     return o;
 }
 
-// The tiles of a step of few sequences: about a block per SM, as far as the blocks' weights fit shared memory; false: they do not.
+// The tiles of a step of few sequences: about a block per SM, as far as the blocks' weights fit shared memory; false: they do not, or not
+// every row wants logits (the end of such a step writes a row of logits, a token and a position for each).
 bool few_plan(Pass& p, const vesta_pass_desc& d) {
-    if (d.rows > FEW_ROWS || d.prompts || d.D > 1024) return false;
+    if (d.rows > FEW_ROWS || d.logit_rows != d.rows || d.prompts || d.D > 1024) return false;
     Few f{};
     f.on = true;
     f.fixed = d.rows <= 2;
