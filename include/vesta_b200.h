@@ -106,7 +106,7 @@ int vesta_pass_workspace(const vesta_pass_desc* desc, size_t* bytes);
  * the features and rows of a tile, stages, parts of the fold and shared memory of a block: out[25]. No device needed. */
 int vesta_pass_tiles(const vesta_pass_desc* desc, int rows, int logit_rows, int* out);
 /* workspace: that many bytes of device memory, zeroed, on a 256-byte boundary (matrices, table and caches: 16 bytes, norm
- * parameters and wpe: 8 bytes; anything else is refused). graph != 0: the pass is a decode step, kept as a CUDA graph. */
+ * parameters and wpe, with exact == 2 also ob and pb: 8 bytes; anything else is refused). graph != 0: the pass is a decode step, kept as a CUDA graph. */
 int vesta_pass_create(const vesta_pass_desc* desc, void* workspace, int graph, void** pass);
 /* exact == 2: (re)makes the packed copy of the weights on `stream`; to be called before the first step and whenever the weights have
  * changed. Nothing to do for any other pass. */

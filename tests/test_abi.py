@@ -129,6 +129,10 @@ def test_a_pass_refuses_tensors_that_its_loads_cannot_reach(built_library):
         assert '8-byte boundary' in create_pass(pass_desc(**{name: 0x10002})), name
     for name in ('x', 't', 'logits', 'bar', 'qkvb', 'ob', 'fcb', 'pb'):
         assert 'missing' in create_pass(pass_desc(**{name: None})), name
+    few = dict(exact=2, rows=4, logit_rows=4)
+    for name in ('ob', 'pb'):                       # (a step from packed weights reads these four elements at a time)
+        for off in (2, 4):
+            assert '8-byte boundary' in create_pass(pass_desc(**few, **{name: 0x10000 + off})), name
     assert '256-byte boundary' in create_pass(pass_desc(), workspace=0x10010)
 
 

@@ -197,7 +197,7 @@ int plan(Pass& p, const vesta_pass_desc* d) {
 }
 
 // The weights and caches are there and start where the kernels' loads want them: 16 bytes for tensor copies and 16-byte pieces, 8 for
-// the norms' parameters and the position table
+// the norms' parameters and the position table, and for the biases that the norms of a step from packed weights start the next sums with
 int check(const vesta_pass_desc& d) {
     const void* wide[] = {d.wte, d.qkvw, d.ow, d.fcw, d.pw, d.keys, d.vals};
     const void* four[] = {d.wpe, d.ln1w, d.ln1b, d.ln2w, d.ln2b, d.lnfw, d.lnfb};
@@ -205,6 +205,7 @@ int check(const vesta_pass_desc& d) {
         if (!q) return fail(-1, "vesta_pass: a tensor is missing");
     for (const void* q : wide) if (!q || (size_t)q % 16) return fail(-1, "vesta_pass: matrices, table and caches start on a 16-byte boundary");
     for (const void* q : four) if (!q || (size_t)q % 8) return fail(-1, "vesta_pass: norm parameters and position table start on an 8-byte boundary");
+    for (const void* q : {d.ob, d.pb}) if (d.exact == 2 && (size_t)q % 8) return fail(-1, "vesta_pass: for a step from packed weights the projections' biases start on an 8-byte boundary");
     return 0;
 }
 
