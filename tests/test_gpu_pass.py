@@ -334,6 +334,38 @@ def test_weights_off_a_16_byte_boundary(batch):
         k.bind(dict(R, keys=moved(R['keys'])))
 
 
+@pytest.mark.parametrize('batch', [1, 2, 4])
+def test_packing_the_matrices_of_other_tensors(batch):
+    """pack(residue) makes the packed weights from the tensors that it is given, in the persistent kernel and in the chain of few
+    sequences, also from views off a 16-byte boundary, until pack() or bind() makes them from the bound ones again; before the first bind
+    there is nothing to keep"""
+    from vesta_gpu_b200.launch import Kernel
+    sh = shape('other')
+    m, _ = model(sh, 3, 'rich', batch, 20)
+    k = Kernel(m.low, device=m.device.index)
+    R = dict(m.k.keep)
+    k.pack(R)
+    other = dict(R, fcw=moved(R['fcw'] * 2), qkvw=R['qkvw'] * -1)
+
+    def logits(W):
+        k.bind(dict(W, x=torch.full_like(R['x'], 7), t=torch.zeros_like(R['t']), keys=torch.zeros_like(R['keys']), vals=torch.zeros_like(R['vals'])))
+        return again()
+
+    def again():
+        k.keep['t'].zero_()
+        k.keep['x'].fill_(7)
+        k.launch()
+        k.check()
+        return k.view('logit').clone()
+    plain, want = logits(R), logits(dict(other, fcw=other['fcw'].clone()))
+    assert (plain - want).abs().max() > 20 * TIGHT
+    assert (logits(R) - plain).abs().max() < TIGHT
+    k.pack(other)
+    assert (again() - want).abs().max() < TIGHT
+    k.pack()
+    assert (again() - plain).abs().max() < TIGHT
+
+
 def test_prompts_with_weights_off_a_16_byte_boundary():
     """a state dict of views (position table, output norm): prefill reads what the weights are when it is called"""
     from vesta_gpu_b200.gpt2 import VestaGPT2

@@ -271,8 +271,13 @@ class Kernel:
             self._bound, self._pass, self._work = bind_step(self, *self._here, graph)
         self._direct = not graph
 
-    def _pack_few(self):
+    def _pack_few(self, residue=None):
+        from .passes import pack_step
+        if self.keep is None:
+            return                                               # (nothing is bound yet: bind() packs)
         with torch.cuda.device(self.device):
+            if residue is not None and residue is not self.keep:
+                return pack_step(self, residue)
             ok(lib().vesta_pass_pack(self._pass, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
 
     def tensor_maps(self, residue):
@@ -292,13 +297,13 @@ class Kernel:
         return host.to(self.device)
 
     def pack(self, residue=None):
-        """(re)build the packed weights from the bound ones; call again after changing them (a chain of more than few sequences reads the
-        weights where they are: nothing to do but for weights that do not start on a 16-byte boundary, of which it reads a
+        """(re)build the packed weights from the bound ones, or from the matrices of `residue`; call again after changing them (a chain of
+        more than four sequences reads the weights where they are: nothing to do but for weights that do not start on a 16-byte boundary, of which it reads a
         copy, unless its persistent kernel has been asked for)"""
         for copy, original in self._copies.values():
             copy.copy_(original)
         if self.few:
-            self._pack_few()
+            self._pack_few(residue)
         if self.graphs and self._packed is None:
             return
         residue = residue or self.keep

@@ -81,20 +81,36 @@ def create(desc, device, graph=False, ws=None):
     return h, ws
 
 
-def bind_step(kernel, residue, zeros, graph):
-    """a decode step over the tensors of `residue` as a chain of kernels -> (handle for vesta_step_run, the pass that it owns, workspace)"""
+def step_desc(kernel, residue, zeros):
+    """the descriptor of a decode step over the tensors of `residue`"""
     low = kernel.lowered
     d, st = low.dims, low.dims['step']
     off = {n: kernel.S.data_ptr() + 4 * v[0] for n, v in low.scratch.items()}
     logit, nxt = list(off.values())
-    desc = describe(low, residue, zeros, st['cpos'], rows=d['B'], logit_rows=d['B'], exact=st['exact'], t_stride=st['t_stride'],
+    return describe(low, residue, zeros, st['cpos'], rows=d['B'], logit_rows=d['B'], exact=st['exact'], t_stride=st['t_stride'],
                     tstep=st['tstep'], feedback=st['feedback'], prompt_len=st['prompt_len'], x=residue[low.roles['x']], t=residue[low.roles['t']],
                     prompt=residue['prompt'] if st['prompt_len'] else None, plen=residue['plen'] if st['prompt_len'] else None,
                     logits=logit, next=nxt, bar=kernel.bar)
-    h, ws = create(desc, kernel.device, graph, kernel._work)
+
+
+def bind_step(kernel, residue, zeros, graph):
+    """a decode step over the tensors of `residue` as a chain of kernels -> (handle for vesta_step_run, the pass that it owns, workspace)"""
+    h, ws = create(step_desc(kernel, residue, zeros), kernel.device, graph, kernel._work)
     bound = ctypes.c_void_p()
     ok(lib().vesta_pass_bind(h, ctypes.byref(bound)))
     return bound, h, ws
+
+
+def pack_step(kernel, residue):
+    """the packed weights of a bound step of few sequences, made from the layers' matrices in `residue` instead of the bound ones"""
+    low, (bound, zeros) = kernel.lowered, kernel._here
+    names = [low.roles[r] for r in ('qkvw', 'ow', 'fcw', 'pw')]
+    here, _ = aligned(low, {**bound, **{n: residue[n] for n in names}}, WEIGHTS[1:])
+    h, _ = create(step_desc(kernel, here, zeros), kernel.device, ws=kernel._work)
+    try:
+        ok(lib().vesta_pass_pack(h, ctypes.c_void_p(torch.cuda.current_stream(kernel.device).cuda_stream)))
+    finally:
+        lib().vesta_pass_release(h)
 
 
 class PromptPass:
