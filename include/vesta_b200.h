@@ -90,7 +90,7 @@ typedef struct vesta_pass_desc {
     int rows, logit_rows;               /* most rows of a pass, most rows that want logits */
     int prompts;                        /* 0: a decode step, a row per sequence; else the number of sequences whose prompts the pass reads */
     int exact;                          /* activations enter the products at fp32 accuracy (at most 16 rows), else rounded to fp16;
-                                           2: the same for a decode step of at most eight rows, all of which want logits, from a packed copy of
+                                           2: the same for a decode step of two to four rows, all of which want logits, from a packed copy of
                                            the weights in the workspace, which vesta_pass_pack makes; sizes that do not suit it are refused */
     int t_stride, tstep, feedback, prompt_len;
     float eps, scale, gelu_a, gelu_b, gelu_c;

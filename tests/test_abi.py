@@ -151,8 +151,9 @@ def test_a_pass_refuses_sizes_that_would_leave_its_buffers(built_library):
         assert sizes(**bad) != 0 and L.vesta_last_error().startswith(b'vesta_pass'), bad
 
 
-def test_a_step_from_packed_weights_refuses_rows_without_logits(built_library):
-    """its end writes a row of logits and a token for every row: fewer logit rows would be written past the ends of both"""
+def test_a_step_from_packed_weights_refuses_what_it_is_not_written_for(built_library):
+    """fewer logit rows than rows (its end writes a row of logits and a token for every row, past the ends of both), one row and more
+    than four, wide rows, an MLP of more than 32 features per SM, prompts"""
     from vesta_gpu_b200 import launch
     L, n = launch.lib(), ctypes.c_size_t()
     for rows, lrows, fine in ((4, 4, True), (4, 3, False), (2, 2, True), (2, 1, False)):
@@ -160,6 +161,10 @@ def test_a_step_from_packed_weights_refuses_rows_without_logits(built_library):
         assert (L.vesta_pass_workspace(ctypes.byref(d), ctypes.byref(n)) == 0) == fine, (rows, lrows)
         if not fine:
             assert b'packed weights' in L.vesta_last_error() and 'packed weights' in create_pass(d)
+    for kw in (dict(rows=1, logit_rows=1), dict(rows=5, logit_rows=5), dict(rows=8, logit_rows=8), dict(rows=9, logit_rows=9), dict(D=1088, H=17), dict(F=4752),
+               dict(prompts=4)):
+        d = pass_desc(**dict(dict(exact=2, rows=4, logit_rows=4), **kw))
+        assert L.vesta_pass_workspace(ctypes.byref(d), ctypes.byref(n)) != 0 and b'packed weights' in L.vesta_last_error(), kw
 
 
 @pytest.mark.parametrize('name,exact', [('gpt2', 0), ('gpt2_xl', 0), ('tiny3', 0), ('heads20', 0), ('gpt2', 1), ('tiny', 1)])

@@ -44,7 +44,7 @@ struct Meta {
 
 // A decode step of few sequences (pass_few.cuh): tiles per block of the two kernels that cut features
 struct Few {
-    bool on, fixed;                            // fixed: the state as State<true>
+    bool on, fixed;                            // fixed: the state as State<true>, and four warps to a row instead of two
     int qkv_per, mlp_per;
 };
 const int SMEM_MAX = 227 * 1024;
@@ -164,10 +164,10 @@ Layout layout(const Pass& p, int D, int F, int rows, int lrows) {
 // The tiles of a step of few sequences: about a block per SM, as far as the blocks' weights fit shared memory; false: they do not, or not
 // every row wants logits (the end of such a step writes a row of logits, a token and a position for each).
 bool few_plan(Pass& p, const vesta_pass_desc& d) {
-    if (d.rows > FEW_ROWS || d.logit_rows != d.rows || d.prompts || d.D > 1024) return false;
+    if (d.rows < 2 || d.rows > FEW_ROWS || d.logit_rows != d.rows || d.prompts || d.D > 1024) return false;
     Few f{};
     f.on = true;
-    f.fixed = d.rows <= 2;
+    f.fixed = d.rows == 2;
     const int sms = 148;
     f.qkv_per = (3 * d.D / 16 + sms - 1) / sms;
     f.mlp_per = (d.F / 16 + sms - 1) / sms;
@@ -421,28 +421,22 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
     return 0;
 }
 
-// one case per width (units of 256, at most) and warps per row
-#define FEW_WIDTH(X, K) X(K, 8, true) X(K, 4, true) X(K, 2, false) X(K, 1, false)
-#define FEW_EACH(X) FEW_WIDTH(X, 1) FEW_WIDTH(X, 2) FEW_WIDTH(X, 3) FEW_WIDTH(X, 4)
-cudaError_t few_launch(cudaLaunchConfig_t& c, int D, int wpr, const FewQkv& a) {
-#define ONE(K, W, F) if (D <= 256 * K && wpr == W) return cudaLaunchKernelEx(&c, few_qkv<K, W, F>, a);
+// one case per width (units of 256, at most) and warps per row (four, fixed point: two rows; two, fp32: three and four)
+#define FEW_EACH(X) X(1, 4, true) X(1, 2, false) X(2, 4, true) X(2, 2, false) X(3, 4, true) X(3, 2, false) X(4, 4, true) X(4, 2, false)
+cudaError_t few_launch(cudaLaunchConfig_t& c, int D, bool fixed, const FewQkv& a) {
+#define ONE(K, W, F) if (D <= 256 * K && fixed == F) return cudaLaunchKernelEx(&c, few_qkv<K, W, F>, a);
     FEW_EACH(ONE)
 #undef ONE
     return cudaErrorInvalidValue;
 }
-cudaError_t few_launch(cudaLaunchConfig_t& c, int D, int wpr, const FewMlp& a) {
-#define ONE(K, W, F) if (D <= 256 * K && wpr == W) return cudaLaunchKernelEx(&c, few_mlp<K, W, F>, a);
+cudaError_t few_launch(cudaLaunchConfig_t& c, int D, bool fixed, const FewMlp& a) {
+#define ONE(K, W, F) if (D <= 256 * K && fixed == F) return cudaLaunchKernelEx(&c, few_mlp<K, W, F>, a);
     FEW_EACH(ONE)
 #undef ONE
     return cudaErrorInvalidValue;
 }
-// up to four sequences, fixed point
-#define FEW_ATTEND(X) X(true, true) X(true, false) X(false, false)
-cudaError_t few_launch(cudaLaunchConfig_t& c, bool four, bool fixed, const FewAttend& a) {
-#define ONE(M, F) if (four == M && fixed == F) return cudaLaunchKernelEx(&c, few_attend<M, F>, a);
-    FEW_ATTEND(ONE)
-#undef ONE
-    return cudaErrorInvalidValue;
+cudaError_t few_launch(cudaLaunchConfig_t& c, bool fixed, const FewAttend& a) {
+    return fixed ? cudaLaunchKernelEx(&c, few_attend<true>, a) : cudaLaunchKernelEx(&c, few_attend<false>, a);
 }
 cudaError_t few_prepare() {
     cudaError_t e = cudaSuccess;
@@ -453,9 +447,7 @@ cudaError_t few_prepare() {
 #define ONE(K, W, F) one(few_qkv<K, W, F>); one(few_mlp<K, W, F>);
     FEW_EACH(ONE)
 #undef ONE
-#define ONE(M, F) one(few_attend<M, F>, FewAttend::bytes(1024));
-    FEW_ATTEND(ONE)
-#undef ONE
+    one(few_attend<true>, FewAttend::bytes(1024)); one(few_attend<false>, FewAttend::bytes(1024));
     return e;
 }
 
@@ -463,7 +455,7 @@ cudaError_t few_prepare() {
 int enqueue_few(Pass& p, cudaStream_t st) {
     const vesta_pass_desc& d = p.d;
     const Few& f = p.few;
-    const int D = d.D, F = d.F, R = d.rows, wpr = R > 4 ? 1 : R > 2 ? 2 : R > 1 ? 4 : 8;
+    const int D = d.D, F = d.F, R = d.rows;
     const Pass::Plan* pl = nullptr;
     if (int e = plan_for(p, R, R, &pl)) return e;
     auto u = [&](size_t off) { return p.ws + off; };
@@ -483,15 +475,15 @@ int enqueue_few(Pass& p, cudaStream_t st) {
             a.pos = (int*)u(p.o.pos); a.skip = (int*)u(p.o.skip); a.bar = (u32*)d.bar;
             Config c(dim3((a.tiles + a.per - 1) / a.per), FEW_THREADS, st, l != 0);
             c.c.dynamicSmemBytes = FewQkv::bytes(D, R, a.per);
-            TRY(few_launch(c.c, D, wpr, a));
+            TRY(few_launch(c.c, D, f.fixed, a));
         }
         {
             FewAttend a = {};
             a.a = {(const float*)u(p.o.q), kc, vc, ss, (const int*)d.t, d.t_stride, d.tmax, D, pow2, 0, d.scale, nullptr};
-            a.rows = R; a.chunks = wpr; a.w = w + pk.proj; a.z = u(p.o.after[l & 1]);
+            a.rows = R; a.chunks = f.fixed ? 4 : 2; a.w = w + pk.proj; a.z = u(p.o.after[l & 1]);
             Config c(dim3(FEW_CLUSTER, d.H), FEW_THREADS, st, true, FEW_CLUSTER, true);
             c.c.dynamicSmemBytes = FewAttend::bytes(D);
-            TRY(few_launch(c.c, R <= 4, f.fixed, a));
+            TRY(few_launch(c.c, f.fixed, a));
         }
         {
             FewMlp a = {};
@@ -499,8 +491,10 @@ int enqueue_few(Pass& p, cudaStream_t st) {
             a.fc = w + pk.fc; a.p2 = w + pk.p2; a.bias = f16(d.fcb, (size_t)l * F); a.tiles = F / 16; a.per = f.mlp_per;
             a.a2 = 2 * d.gelu_a; a.k1 = d.gelu_b * 2.8853900817779268f; a.k2 = d.gelu_c * a.k1;
             Config c(dim3((a.tiles + a.per - 1) / a.per), FEW_THREADS, st, true);
-            c.c.dynamicSmemBytes = FewMlp::bytes(D, R, a.per);
-            TRY(few_launch(c.c, D, wpr, a));
+            // (a block of two tiles has its SM for itself, they are no more than the SMs: two sequences of the small shape, whose 114 KB would
+            // fit twice, 170.3 us per step so, 172.2 in pairs)
+            c.c.dynamicSmemBytes = std::max(FewMlp::bytes(D, R, a.per), a.per > 1 ? SMEM_MAX / 2 : 0);
+            TRY(few_launch(c.c, D, f.fixed, a));
         }
     }
     NormArgs n = {};
@@ -519,7 +513,7 @@ int enqueue_few(Pass& p, cudaStream_t st) {
 int step(Pass& p, cudaStream_t st) { return p.few.on ? enqueue_few(p, st) : enqueue(p, st, p.d.rows, p.d.logit_rows, 0); }
 int pack_few(const Pass& p, cudaStream_t st) {
     const vesta_pass_desc& d = p.d;
-    const FewPackArgs a = {d.D, d.F, d.L, d.rows <= 4, (const u16*)d.qkvw, (const u16*)d.ow, (const u16*)d.fcw, (const u16*)d.pw, p.ws + p.o.packed};
+    const FewPackArgs a = {d.D, d.F, d.L, (const u16*)d.qkvw, (const u16*)d.ow, (const u16*)d.fcw, (const u16*)d.pw, p.ws + p.o.packed};
     few_pack<<<p.sms * 8, 256, 0, st>>>(a);
     TRY(cudaGetLastError());
     return 0;

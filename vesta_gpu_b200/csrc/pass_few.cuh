@@ -1,4 +1,4 @@
-// Kernels of a decode step of few sequences (at most eight; two to four by default): three per layer,
+// Kernels of a decode step of few sequences (two to four): three per layer,
 //
 //     norm + QKV | attention + projection | norm + FC + GELU + MLP projection
 //
@@ -8,7 +8,7 @@
 // between them: GPT-2 small has 14 MB of weights per layer, 2.2 us of memory traffic, and took 15 to 17 us per layer in one persistent
 // kernel with grid barriers. So a kernel boundary (1.2 us) stands only where every SM needs sums of all the others: before the two
 // norms and before the attention, and everything else stays within a block or a cluster of eight blocks:
-//   * every block normalises all rows by itself, as they are no more than its warps (the state of eight sequences is 25 KB);
+//   * every block normalises all rows by itself, with two or four warps to a row (the state of four sequences is 12 KB);
 //   * the eight blocks of a head exchange their attention results through distributed shared memory and each applies an eighth of
 //     the head's rows of the projection to all sequences;
 //   * a block keeps the GELU output of its own features and multiplies it with their rows of the MLP projection.
@@ -17,8 +17,7 @@
 // The weights a block needs are on their way into its shared memory before it waits for its predecessor. They are a copy in the order
 // in which the lanes of mma.sync m16n8k16 hold them, so that every thread copies (cp.async) and reads back just its own 16 bytes of
 // each unit: no barrier, nothing to wait for but its own copies. The activations enter as fp16 head and remainder, whose products
-// add up to the fp32-accurate one: up to four sequences as the eight columns of operand B (sequence 0 head, remainder, sequence 1, ...)
-// with 16 features as the rows of A; more as the sixteen rows of A (eight heads, eight remainders) with twice eight features as B.
+// add up to the fp32-accurate one: the eight columns of operand B are sequence 0 head, remainder, sequence 1, ..., the rows of A 16 features.
 // (One product takes 13 to 16 cycles of a quarter of an SM, a sixth of what tcgen05 could do; but that has 64 or 128 rows, and its
 // operands would make two more trips through shared memory.)
 #pragma once
@@ -32,7 +31,8 @@ namespace vesta_pass {
 // (The compiler is not to know how often the loop runs, two copies of the code would warm nothing, and is not to move what both passes
 // compute in front of it, which costs registers.)
 __device__ __forceinline__ int few_passes(int n) { asm volatile("" : "+r"(n)); return n; }
-#define FEW_ROWS 8
+#define FEW_ROWS 4
+#define FEW_RED (FEW_ROWS * 16)          // a warp's sums of a tile
 #define FEW_WARPS 8
 #define FEW_THREADS (FEW_WARPS * 32)
 #define FEW_CLUSTER 8                 // blocks of a head
@@ -40,11 +40,9 @@ __device__ __forceinline__ int few_passes(int n) { asm volatile("" : "+r"(n)); r
 #define FEW_STAGES 2                  // stages of a warp's ring in the attention
 
 // Packed weights of a layer, in units of 512 bytes, 16 per lane (g = lane / 4, t = lane % 4):
-//   qkv, fc: [16 features][32 fold indices][2 units]: up to four sequences the unit is one half of the fold indices (operand A:
-//     fold indices 2t, 2t+1 of features g, g+8, then 2t+8, 2t+9 of both), else one half of the features (operand B: fold indices
-//     2t, 2t+1 | 2t+8, 2t+9 | 2t+16, 2t+17 | 2t+24, 2t+25 of feature g)
-//   proj, p2: [16 outputs][16 fold indices]: up to four sequences operand A as above, else operand B of outputs 4 (g / 2) + g % 2 and
-//     of that + 2 (so that a lane ends up with four consecutive outputs)
+//   qkv, fc: [16 features][32 fold indices][2 units, one half of the fold indices each]
+//   proj, p2: [16 outputs][16 fold indices]
+// every unit as operand A: fold indices 2t, 2t+1 of features g, g+8, then 2t+8, 2t+9 of both
 // proj: [head][16 outputs][4 units of the head's 64 fold indices]; p2: [16 fold indices][16 outputs]
 struct FewPack {
     size_t qkv, proj, fc, p2, layer;          // offsets in a layer, bytes of a layer
@@ -52,7 +50,7 @@ struct FewPack {
         qkv = 0; proj = qkv + (size_t)3 * D * D * 2; fc = proj + (size_t)D * D * 2; p2 = fc + (size_t)D * F * 2; layer = p2 + (size_t)D * F * 2;
     }
 };
-struct FewPackArgs { int D, F, L, four; const u16 *qkvw, *ow, *fcw, *pw; unsigned char* out; };      // four: up to four sequences
+struct FewPackArgs { int D, F, L; const u16 *qkvw, *ow, *fcw, *pw; unsigned char* out; };
 // A warp takes 1 KB of qkv / fc or a unit of proj / p2 at a time: 16 bytes per lane and load, through shared memory into the lanes' order.
 __global__ void __launch_bounds__(256) few_pack(const __grid_constant__ FewPackArgs a) {
     __shared__ __align__(16) u16 buf[8][32 * 24];
@@ -76,7 +74,7 @@ __global__ void __launch_bounds__(256) few_pack(const __grid_constant__ FewPackA
             *reinterpret_cast<uint4*>(s + lane * 24 + 8) = __ldg(reinterpret_cast<const uint4*>(src) + 1);
             __syncwarp();
             for (int j = 0; j < 2; j++) {
-                for (int q = 0; q < 4; q++) w[q] = a.four ? two(j * 16 + (q >> 1) * 8 + 2 * t, (q & 1) * 8 + g) : two(q * 8 + 2 * t, j * 8 + g);
+                for (int q = 0; q < 4; q++) w[q] = two(j * 16 + (q >> 1) * 8 + 2 * t, (q & 1) * 8 + g);
                 *reinterpret_cast<uint4*>(out + (fc ? off.fc : off.qkv) + (((size_t)tile * KP + kp) * 2 + j) * 512 + lane * 16) = make_uint4(w[0], w[1], w[2], w[3]);
             }
         } else {
@@ -87,20 +85,16 @@ __global__ void __launch_bounds__(256) few_pack(const __grid_constant__ FewPackA
             const u16* src = (p2 ? a.pw + (size_t)l * F * D : a.ow + (size_t)l * D * D) + (size_t)(kt * 16 + (lane >> 1)) * D + mt * 16 + (lane & 1) * 8;
             *reinterpret_cast<uint4*>(s + (lane >> 1) * 24 + (lane & 1) * 8) = __ldg(reinterpret_cast<const uint4*>(src));
             __syncwarp();
-            for (int q = 0; q < 4; q++) w[q] = a.four ? two((q >> 1) * 8 + 2 * t, (q & 1) * 8 + g) : two((q & 1) * 8 + 2 * t, 4 * (g >> 1) + 2 * (q >> 1) + (g & 1));
+            for (int q = 0; q < 4; q++) w[q] = two((q >> 1) * 8 + 2 * t, (q & 1) * 8 + g);
             const size_t at = p2 ? off.p2 + ((size_t)kt * MT + mt) * 512 : off.proj + (((size_t)(kt >> 2) * MT + mt) * 4 + (kt & 3)) * 512;
             *reinterpret_cast<uint4*>(out + at + lane * 16) = make_uint4(w[0], w[1], w[2], w[3]);
         }
     }
 }
 
-// Operand rows in shared memory, `ld` bytes apart: heads and remainders in turn (up to four sequences), or all heads, then all remainders
-template <bool FOUR> __device__ __forceinline__ int few_head(int row) { return FOUR ? 2 * row : row; }
-template <bool FOUR> __device__ __forceinline__ int few_rest(int row, int R) { return FOUR ? 2 * row + 1 : R + row; }
-// where a lane points ldmatrix for the first 32 (FOUR) or 16 fold indices; rows that do not exist repeat the last
-template <bool FOUR> __device__ __forceinline__ u32 few_row(u32 op, int ld, int R, int lane) {
-    return FOUR ? op + min(lane & 7, 2 * R - 1) * ld + (lane >> 3) * 16 : op + (min(lane & 7, R - 1) + ((lane >> 3) & 1) * R) * ld + (lane >> 4) * 16;
-}
+// Operand rows in shared memory, `ld` bytes apart: heads and remainders in turn. Where a lane points ldmatrix for the first 32 fold
+// indices; rows that do not exist repeat the last
+__device__ __forceinline__ u32 few_row(u32 op, int ld, int R, int lane) { return op + min(lane & 7, 2 * R - 1) * ld + (lane >> 3) * 16; }
 // a 16-byte piece of this thread's own weights
 __device__ __forceinline__ uint4 lds16(u32 p) {
     uint4 v;
@@ -111,25 +105,14 @@ __device__ __forceinline__ void few_mma(float (&c)[4], const uint4& a, u32 b0, u
     const u32 r[4] = {a.x, a.y, a.z, a.w};
     mma16816(c, r, b0, b1);
 }
-// A tile of 16 outputs over 32 fold indices (a FOUR lane has the operand in x, others in x and y): 32 x 16 per call, or two units of 16 x 16
-// (`u`, `v`); c[0], c[1]: FOUR: parts of the same sums, else the outputs' halves
-template <bool FOUR> __device__ __forceinline__ void few_pair(float (&c)[2][4], const u32 (&x)[4], const u32 (&y)[4], const uint4& u, const uint4& v) {
-    if (FOUR) { few_mma(c[0], u, x[0], x[1]); few_mma(c[1], v, x[2], x[3]); }
-    else {
-        mma16816(c[0], x, u.x, u.y); mma16816(c[1], x, u.z, u.w);
-        mma16816(c[0], y, v.x, v.y); mma16816(c[1], y, v.z, v.w);
-    }
-}
-// the sums of a tile of outputs (proj, p2) into the state
-template <bool FOUR, bool FIXED> __device__ __forceinline__ void few_add(void* z, int D, int R, int tile, const float (&c)[2][4], int lane) {
+// the sums of a tile of outputs (proj, p2; c[0] and c[1]: parts of the same sums) into the state
+template <bool FIXED> __device__ __forceinline__ void few_add(void* z, int D, int R, int tile, const float (&c)[2][4], int lane) {
     const int g = lane >> 2, t = lane & 3;
-    if (FOUR) {
-        if (t < R) {
-            const size_t at = (size_t)t * D + tile * 16 + g;
-            State<FIXED>::add1(z, at, (c[0][0] + c[0][1]) + (c[1][0] + c[1][1]));
-            State<FIXED>::add1(z, at + 8, (c[0][2] + c[0][3]) + (c[1][2] + c[1][3]));
-        }
-    } else if (g < R) State<FIXED>::add(z, (size_t)g * D + tile * 16 + 4 * t, make_float4(c[0][0] + c[0][2], c[0][1] + c[0][3], c[1][0] + c[1][2], c[1][1] + c[1][3]));
+    if (t < R) {
+        const size_t at = (size_t)t * D + tile * 16 + g;
+        State<FIXED>::add1(z, at, (c[0][0] + c[0][1]) + (c[1][0] + c[1][1]));
+        State<FIXED>::add1(z, at + 8, (c[0][2] + c[0][3]) + (c[1][2] + c[1][3]));
+    }
 }
 
 // The state between two layers is a vector that the attention's projections have been added to, and one of the MLP's sums alone: sums of
@@ -152,14 +135,13 @@ __device__ __forceinline__ void few_params(const FewNorm& n, u16* par) {
         if (blockIdx.x < n.rows) *reinterpret_cast<uint2*>(par + 2 * n.D + d) = __ldg(reinterpret_cast<const uint2*>(n.bias + d));
     }
 }
-// Norm of all rows into the operand. WPR warps share a row (8 / R, a power of two), a lane holds NV float4. Block `row` (counted around where there are fewer) also starts the
+// Norm of all rows into the operand. WPR warps share a row (four of two rows, two of three or four), a lane holds NV float4. Block `row` (counted around where there are fewer) also starts the
 // vector of the next sums: QKV stores it (nothing adds yet), the MLP kernel adds to it (other blocks may have begun to).
 // `value(row, d)` loads four elements of the state.
 template <int KW, int WPR> struct FewLanes { static constexpr int NV = (2 * KW + WPR - 1) / WPR; };      // KW: D <= 256 KW
 template <int KW, int WPR, bool FIXED, bool STORE, class Load>
 __device__ __forceinline__ void few_norm(const FewNorm& n, bool real, int warp, int lane, const u16* par, unsigned char* op, int ld, float2* red, Load value) {
     constexpr int NV = FewLanes<KW, WPR>::NV, by = WPR * 128;
-    constexpr bool FOUR = WPR > 1;
     const int row = warp / WPR, seg = warp % WPR, d0 = (seg * 32 + lane) * 4;
     const bool live = row < n.rows;
     float4 v[NV];
@@ -170,7 +152,7 @@ __device__ __forceinline__ void few_norm(const FewNorm& n, bool real, int warp, 
         return c;
     };
     const float rd = 1.0f / (float)n.D, own = (float)elements(seg), rown = own > 0.f ? 1.0f / own : 0.f;
-    const float cx = WPR > 1 ? (float)elements(lane % WPR) : 0.f, rcx = cx > 0.f ? 1.0f / cx : 0.f;
+    const float cx = (float)elements(lane % WPR), rcx = cx > 0.f ? 1.0f / cx : 0.f;
     float s = 0.f, q = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; i++) {
@@ -190,23 +172,21 @@ __device__ __forceinline__ void few_norm(const FewNorm& n, bool real, int warp, 
         }
 #pragma unroll
     for (int m = 16; m; m >>= 1) q += __shfl_xor_sync(0xffffffffu, q, m);
-    if (WPR > 1) {
-        // the row's mean, then its squared deviations: every warp's own plus its elements times (its mean - the mean)^2
-        if (lane == 0) red[warp] = make_float2(s, q);
-        __syncthreads();
-        const float2 p = red[row * WPR + lane % WPR];
-        s = p.x;
+    // the row's mean, then its squared deviations: every warp's own plus its elements times (its mean - the mean)^2
+    if (lane == 0) red[warp] = make_float2(s, q);
+    __syncthreads();
+    const float2 p = red[row * WPR + lane % WPR];
+    s = p.x;
 #pragma unroll
-        for (int m = WPR / 2; m; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
-        mean = s * rd;
-        const float dm = p.x * rcx - mean;
-        q = cx > 0.f ? p.y + cx * dm * dm : 0.f;
+    for (int m = WPR / 2; m; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+    mean = s * rd;
+    const float dm = p.x * rcx - mean;
+    q = cx > 0.f ? p.y + cx * dm * dm : 0.f;
 #pragma unroll
-        for (int m = WPR / 2; m; m >>= 1) q += __shfl_xor_sync(0xffffffffu, q, m);
-    }
+    for (int m = WPR / 2; m; m >>= 1) q += __shfl_xor_sync(0xffffffffu, q, m);
     const float rs = rsqrtf(q * rd + n.eps);
     if (live) {
-        unsigned char *hi = op + few_head<FOUR>(row) * ld, *lo = op + few_rest<FOUR>(row, n.rows) * ld;
+        unsigned char *hi = op + 2 * row * ld, *lo = hi + ld;
 #pragma unroll
         for (int i = 0; i < NV; i++) {
             const int d = d0 + i * by;
@@ -254,22 +234,21 @@ __device__ __forceinline__ void few_request(u32 slots, const unsigned char* w, i
         }
 }
 // ... and multiplies them with the operand: red[tile][warp][row][16 features]
-template <int KW, bool FOUR>
+template <int KW>
 __device__ __forceinline__ void few_fold(u32 slots, u32 a_at, int n, int KP, float* red, int warp, int lane) {
     const int KU = few_units(KP), g = lane >> 2, t = lane & 3;
-    u32 a[KW][2][4];
+    u32 a[KW][4];
 #pragma unroll
     for (int i = 0; i < KW; i++) {
         const bool yes = warp + i * FEW_WARPS < KP;
         const u32 at = a_at + (yes ? warp + i * FEW_WARPS : 0) * 64;
-        ldsm4(a[i][0], at);
-        if (!FOUR) ldsm4(a[i][1], at + 32);
+        ldsm4(a[i], at);
         if (!yes)
 #pragma unroll
-            for (int x = 0; x < 4; x++) a[i][0][x] = a[i][1][x] = 0u;
+            for (int x = 0; x < 4; x++) a[i][x] = 0u;
     }
     slots += lane * 16;
-    red += warp * 128;
+    red += warp * FEW_RED;
 #pragma unroll 1
     for (int j = 0; j < n; j++) {
         float c[2][2][4] = {};
@@ -277,29 +256,19 @@ __device__ __forceinline__ void few_fold(u32 slots, u32 a_at, int n, int KP, flo
 #pragma unroll
         for (int i = 0; i < KW; i++) { w[i][0] = lds16(slots + (j * KU + min(i, KU - 1)) * 1024); w[i][1] = lds16(slots + (j * KU + min(i, KU - 1)) * 1024 + 512); }
 #pragma unroll
-        for (int i = 0; i < KW; i++)
-            if (FOUR) few_pair<true>(c[i & 1], a[i][0], a[i][0], w[i][0], w[i][1]);
-            else {
-                mma16816(c[0][0], a[i][0], w[i][0].x, w[i][0].y); mma16816(c[1][0], a[i][0], w[i][1].x, w[i][1].y);
-                mma16816(c[0][1], a[i][1], w[i][0].z, w[i][0].w); mma16816(c[1][1], a[i][1], w[i][1].z, w[i][1].w);
-            }
-        float* to = red + j * (FEW_WARPS * 128);
-        if (FOUR) {
-            // feature g (and g + 8) of row t: head and remainder are neighbours, four accumulators hold parts of the fold
-            to[t * 16 + g] = ((c[0][0][0] + c[0][0][1]) + (c[0][1][0] + c[0][1][1])) + ((c[1][0][0] + c[1][0][1]) + (c[1][1][0] + c[1][1][1]));
-            to[t * 16 + g + 8] = ((c[0][0][2] + c[0][0][3]) + (c[0][1][2] + c[0][1][3])) + ((c[1][0][2] + c[1][0][3]) + (c[1][1][2] + c[1][1][3]));
-        } else
-#pragma unroll
-            for (int y = 0; y < 2; y++)
-                *reinterpret_cast<float2*>(to + g * 16 + y * 8 + 2 * t) = make_float2((c[y][0][0] + c[y][1][0]) + (c[y][0][2] + c[y][1][2]), (c[y][0][1] + c[y][1][1]) + (c[y][0][3] + c[y][1][3]));
+        for (int i = 0; i < KW; i++) { few_mma(c[i & 1][0], w[i][0], a[i][0], a[i][1]); few_mma(c[i & 1][1], w[i][1], a[i][2], a[i][3]); }
+        float* to = red + j * (FEW_WARPS * FEW_RED);
+        // feature g (and g + 8) of row t: head and remainder are neighbours, four accumulators hold parts of the fold
+        to[t * 16 + g] = ((c[0][0][0] + c[0][0][1]) + (c[0][1][0] + c[0][1][1])) + ((c[1][0][0] + c[1][0][1]) + (c[1][1][0] + c[1][1][1]));
+        to[t * 16 + g + 8] = ((c[0][0][2] + c[0][0][3]) + (c[0][1][2] + c[0][1][3])) + ((c[1][0][2] + c[1][0][3]) + (c[1][1][2] + c[1][1][3]));
     }
 }
-// the sum of the warps' parts of output `o` of a block: tile o / 128, row o / 16 % 8, feature o % 16
+// the sum of the warps' parts of output `o` of a block: tile o / 64, row o / 16 % 4, feature o % 16
 __device__ __forceinline__ float few_sum(const float* red, int o) {
-    const float* p = red + (o >> 7) * (FEW_WARPS * 128) + (o & 127);
+    const float* p = red + (o / FEW_RED) * (FEW_WARPS * FEW_RED) + o % FEW_RED;
     float s[FEW_WARPS];
 #pragma unroll
-    for (int i = 0; i < FEW_WARPS; i++) s[i] = p[i * 128];
+    for (int i = 0; i < FEW_WARPS; i++) s[i] = p[i * FEW_RED];
     return ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
 }
 
@@ -319,7 +288,7 @@ struct FewQkv {
     const u16 *wte, *wpe;             // first layer: the rows are embeddings
     int *pos, *skip;
     u32* bar;
-    static __host__ __device__ int bytes(int D, int rows, int per) { return per * ((D / 32 + 7) / 8) * 8192 + 2 * rows * (2 * D + 16) + per * FEW_WARPS * 512 + FewNorm::bytes(D); }
+    static __host__ __device__ int bytes(int D, int rows, int per) { return per * ((D / 32 + 7) / 8) * 8192 + 2 * rows * (2 * D + 16) + per * FEW_WARPS * FEW_RED * 4 + FewNorm::bytes(D); }
 };
 template <int KW, int WPR, bool FIXED>
 __global__ void __launch_bounds__(FEW_THREADS, 2) few_qkv(const __grid_constant__ FewQkv a) {
@@ -331,14 +300,12 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) few_qkv(const __grid_constant_
     const u32 slots = smem_u32(smem) + warp * (a.per * few_units(KP) * 1024);
     unsigned char* op = smem + a.per * few_units(KP) * (FEW_WARPS * 1024);
     float* red = reinterpret_cast<float*>(op + 2 * R * ld);
-    u16* par = reinterpret_cast<u16*>(red + a.per * FEW_WARPS * 128);
+    u16* par = reinterpret_cast<u16*>(red + a.per * FEW_WARPS * FEW_RED);
     few_request(slots, a.w + (size_t)t0 * KP * 1024, n, KP, warp, lane);
     asm volatile("cp.async.commit_group;" ::: "memory");
     if (tid == 0) dep_launch();
     few_params(a.n, par);
-    float bias[FEW_TILES / 2];                                                     // of this thread's outputs
-#pragma unroll
-    for (int x = 0; x < FEW_TILES / 2; x++) bias[x] = tid + x * FEW_THREADS < n * 128 ? h2f(__ldg(a.bias + (t0 + ((tid + x * FEW_THREADS) >> 7)) * 16 + (tid & 15))) : 0.f;
+    const float bias = tid < n * FEW_RED ? h2f(__ldg(a.bias + (t0 + tid / FEW_RED) * 16 + (tid & 15))) : 0.f;      // of this thread's output
     __syncthreads();
     bool skip = false;
 #pragma unroll 1
@@ -376,17 +343,14 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) few_qkv(const __grid_constant_
         }
         if (real) asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
-        few_fold<KW, (WPR > 1)>(slots, few_row<(WPR > 1)>(smem_u32(op), ld, R, l), n, KP, red, w, l);
+        few_fold<KW>(slots, few_row(smem_u32(op), ld, R, l), n, KP, red, w, l);
         __syncthreads();
-#pragma unroll
-        for (int x = 0; x < FEW_TILES / 2; x++) {
-            const int o = x * FEW_THREADS + w * 32 + l, row = (o >> 4) & 7, f = (t0 + (o >> 7)) * 16 + (o & 15);
-            if (row >= R || o >= n * 128) continue;
-            const float v = few_sum(red, o) + bias[x];
+        const int o = w * 32 + l, row = (o >> 4) % FEW_ROWS, f = (t0 + o / FEW_RED) * 16 + (o & 15);
+        if (row < R && o < n * FEW_RED) {
+            const float v = few_sum(red, o) + bias;
             const int part = (f >= D) + (f >= 2 * D), c = f - part * D, t = s_t[row];
-            if (!real) continue;
-            if (part == 0) a.q[(size_t)row * D + c] = v;
-            else if (!skip && t >= 0) (part == 1 ? a.kc : a.vc)[row * a.seq_stride + (size_t)t * D + c] = f2h(v);
+            if (real && part == 0) a.q[(size_t)row * D + c] = v;
+            if (real && part && !skip && t >= 0) (part == 1 ? a.kc : a.vc)[row * a.seq_stride + (size_t)t * D + c] = f2h(v);
         }
     }
 }
@@ -403,12 +367,12 @@ struct FewAttend {
 // Cluster = a head, block = a sequence or a run of its positions; see pass_attend for the attention itself. 4.5 us at eight sequences of 136
 // positions, 4.2 at one of 37: a warp's one or two rounds of 16 positions 1.6 us, the cluster's exchange 0.7.
 // (Two stages per warp: four keep the next kernel's block from the SM, eight sequences 3,080 -> 3,600 us per sixteen steps.)
-template <bool FOUR, bool FIXED>
+template <bool FIXED>
 __global__ void __launch_bounds__(FEW_THREADS) few_attend(const __grid_constant__ FewAttend a) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ float part[FEW_WARPS][66];
     __shared__ __align__(16) float all[FEW_CLUSTER][68];
-    __shared__ __align__(16) unsigned char op[16 * 144];
+    __shared__ __align__(16) unsigned char op[2 * FEW_ROWS * 144];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int h = blockIdx.y, c = blockIdx.x, row = c / a.chunks, chunk = c - row * a.chunks, D = a.a.D, MT = D / 16;
     const int nt = (MT - c + FEW_CLUSTER - 1) / FEW_CLUSTER;                       // tiles of 16 outputs: c, c + 8, ...
@@ -419,13 +383,6 @@ __global__ void __launch_bounds__(FEW_THREADS) few_attend(const __grid_constant_
         for (int k = 0; k < 4; k++) cp16(slots + (i * 4 + k) * 512 + lane * 16, a.w + (((size_t)h * MT + c + i * FEW_CLUSTER) * 4 + k) * 512 + lane * 16);
     if (tid == 0) dep_launch();
     const bool live = row < a.rows;
-    // outputs 2 lane and 2 lane + 1 of a sequence into an operand (of this or another block of the cluster)
-    auto put = [&](u32 to, int seq, float x, float y, float dd) {
-        const float u = dd > 0.f ? __fdividef(x, dd) : 0.f, v = dd > 0.f ? __fdividef(y, dd) : 0.f;   // (a sequence that has not started attends to nothing)
-        const u32 hi = pack_h2(u, v);
-        asm volatile("st.shared::cluster.u32 [%0], %1;" :: "r"(to + few_head<FOUR>(seq) * 144 + lane * 4), "r"(hi) : "memory");
-        asm volatile("st.shared::cluster.u32 [%0], %1;" :: "r"(to + few_rest<FOUR>(seq, a.rows) * 144 + lane * 4), "r"(pack_h2(u - h_lo(hi), v - h_hi(hi))) : "memory");
-    };
     AttRow<FEW_STAGES> r(a.a, live ? row : 0, h, (chunk * FEW_WARPS + warp) * ATT_RUN, a.chunks * FEW_WARPS * ATT_RUN, ring + warp * (FEW_STAGES * 4096));
     if (live) r.request_first();
 #pragma unroll 1
@@ -442,34 +399,35 @@ __global__ void __launch_bounds__(FEW_THREADS) few_attend(const __grid_constant_
             for (int i = 0; i < FEW_WARPS; i++) M = fmaxf(M, part[i][64]);
 #pragma unroll
             for (int i = 0; i < FEW_WARPS; i++) { const float e = fast_exp(part[i][64] - M); dd += part[i][65] * e; x += part[i][2 * lane] * e; y += part[i][2 * lane + 1] * e; }
-            if (FOUR) {
-                const u32 to = of_block(smem_u32(&all[c][0]), warp);
-                asm volatile("st.shared::cluster.v2.f32 [%0], {%1,%2};" :: "r"(to + lane * 8), "f"(x), "f"(y) : "memory");
-                if (lane == 0) asm volatile("st.shared::cluster.v2.f32 [%0], {%1,%2};" :: "r"(to + 256), "f"(M), "f"(dd) : "memory");
-            } else put(of_block(smem_u32(op), warp), row, x, y, dd);
+            const u32 to = of_block(smem_u32(&all[c][0]), warp);
+            asm volatile("st.shared::cluster.v2.f32 [%0], {%1,%2};" :: "r"(to + lane * 8), "f"(x), "f"(y) : "memory");
+            if (lane == 0) asm volatile("st.shared::cluster.v2.f32 [%0], {%1,%2};" :: "r"(to + 256), "f"(M), "f"(dd) : "memory");
         }
         cluster_sync();
-        if (FOUR) {
-            if (warp < a.rows) {
-                float m[FEW_CLUSTER], M = -3.0e38f, dd = 0.f, x = 0.f, y = 0.f;
+        if (warp < a.rows) {
+            // the runs of a sequence, merged: its head's outputs 2 lane and 2 lane + 1 into the operand
+            float m[FEW_CLUSTER], M = -3.0e38f, dd = 0.f, x = 0.f, y = 0.f;
 #pragma unroll
-                for (int i = 0; i < FEW_CLUSTER; i++) { m[i] = i < a.chunks ? all[warp * a.chunks + i][64] : -3.0e38f; M = fmaxf(M, m[i]); }
+            for (int i = 0; i < FEW_CLUSTER; i++) { m[i] = i < a.chunks ? all[warp * a.chunks + i][64] : -3.0e38f; M = fmaxf(M, m[i]); }
 #pragma unroll
-                for (int i = 0; i < FEW_CLUSTER; i++)
-                    if (i < a.chunks) {
-                        const float* p = all[warp * a.chunks + i];
-                        const float e = fast_exp(m[i] - M);
-                        dd += p[65] * e; x += p[2 * lane] * e; y += p[2 * lane + 1] * e;
-                    }
-                put(smem_u32(op), warp, x, y, dd);
-            }
-            __syncthreads();
+            for (int i = 0; i < FEW_CLUSTER; i++)
+                if (i < a.chunks) {
+                    const float* p = all[warp * a.chunks + i];
+                    const float e = fast_exp(m[i] - M);
+                    dd += p[65] * e; x += p[2 * lane] * e; y += p[2 * lane + 1] * e;
+                }
+            const float u = dd > 0.f ? __fdividef(x, dd) : 0.f, v = dd > 0.f ? __fdividef(y, dd) : 0.f;   // (a sequence that has not started attends to nothing)
+            const u32 hi = pack_h2(u, v);
+            unsigned char* to = op + 2 * warp * 144 + lane * 4;
+            *reinterpret_cast<u32*>(to) = hi;
+            *reinterpret_cast<u32*>(to + 144) = pack_h2(u - h_lo(hi), v - h_hi(hi));
         }
+        __syncthreads();
         if (real) asm volatile("cp.async.wait_all;" ::: "memory");
-        u32 f[4][4];
-        const u32 a_at = few_row<FOUR>(smem_u32(op), 144, a.rows, lane);
-#pragma unroll
-        for (int k = 0; k < (FOUR ? 2 : 4); k++) ldsm4(f[k], a_at + k * (FOUR ? 64 : 32));
+        u32 f[2][4];
+        const u32 a_at = few_row(smem_u32(op), 144, a.rows, lane);
+        ldsm4(f[0], a_at);
+        ldsm4(f[1], a_at + 64);
 #pragma unroll 1
         for (int i = warp; i < nt; i += FEW_WARPS) {
             float c0[2][4] = {};
@@ -477,8 +435,8 @@ __global__ void __launch_bounds__(FEW_THREADS) few_attend(const __grid_constant_
 #pragma unroll
             for (int k = 0; k < 4; k++) u[k] = lds16(slots + (i * 4 + k) * 512 + lane * 16);
 #pragma unroll
-            for (int k = 0; k < 2; k++) few_pair<FOUR>(c0, f[FOUR ? k : 2 * k], f[FOUR ? k : 2 * k + 1], u[2 * k], u[2 * k + 1]);
-            if (real) few_add<FOUR, FIXED>(a.z, D, a.rows, c + i * FEW_CLUSTER, c0, lane);
+            for (int k = 0; k < 2; k++) { few_mma(c0[0], u[2 * k], f[k][0], f[k][1]); few_mma(c0[1], u[2 * k + 1], f[k][2], f[k][3]); }
+            if (real) few_add<FIXED>(a.z, D, a.rows, c + i * FEW_CLUSTER, c0, lane);
         }
     }
 }
@@ -493,7 +451,7 @@ struct FewMlp {
     int tiles, per;                   // tiles of 16 features, tiles per block
     float a2, k1, k2;                 // gelu_tanh
     static __host__ __device__ int bytes(int D, int rows, int per) {
-        return per * ((D / 32 + 7) / 8) * 8192 + per * ((D / 16 + 7) / 8) * 4096 + 2 * rows * (2 * D + 16) + per * FEW_WARPS * 512 + 16 * (FEW_TILES * 32 + 16) + FewNorm::bytes(D);
+        return per * ((D / 32 + 7) / 8) * 8192 + per * ((D / 16 + 7) / 8) * 4096 + 2 * rows * (2 * D + 16) + per * FEW_WARPS * FEW_RED * 4 + 2 * FEW_ROWS * (FEW_TILES * 32 + 16) + FewNorm::bytes(D);
     }
 };
 template <int KW, int WPR, bool FIXED>
@@ -501,7 +459,6 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) few_mlp(const __grid_constant_
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ float2 stat[FEW_WARPS];
     constexpr int ld2 = FEW_TILES * 32 + 16;
-    constexpr bool FOUR = WPR > 1;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, D = a.n.D, R = a.n.rows, KP = D / 32, MT = D / 16, ld = 2 * D + 16;
     const int t0 = blockIdx.x * a.per, n = min(a.per, a.tiles - t0);
     // A warp's part of shared memory: its units of fc, then those of p2 (its output tiles, every eighth, x FEW_TILES tiles of the fold)
@@ -509,8 +466,8 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) few_mlp(const __grid_constant_
     const u32 slots = smem_u32(smem) + warp * ((fcu + p2u) * 512);
     unsigned char* op = smem + (fcu + p2u) * (FEW_WARPS * 512);
     unsigned char* op2 = op + 2 * R * ld;
-    float* red = reinterpret_cast<float*>(op2 + 16 * ld2);
-    u16* par = reinterpret_cast<u16*>(red + a.per * FEW_WARPS * 128);
+    float* red = reinterpret_cast<float*>(op2 + 2 * FEW_ROWS * ld2);
+    u16* par = reinterpret_cast<u16*>(red + a.per * FEW_WARPS * FEW_RED);
     few_request(slots, a.fc + (size_t)t0 * KP * 1024, n, KP, warp, lane);
     asm volatile("cp.async.commit_group;" ::: "memory");
 #pragma unroll 1
@@ -520,9 +477,7 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) few_mlp(const __grid_constant_
     asm volatile("cp.async.commit_group;" ::: "memory");
     if (tid == 0) dep_launch();
     few_params(a.n, par);
-    float bias[FEW_TILES / 2];
-#pragma unroll
-    for (int x = 0; x < FEW_TILES / 2; x++) bias[x] = tid + x * FEW_THREADS < n * 128 ? h2f(__ldg(a.bias + (t0 + ((tid + x * FEW_THREADS) >> 7)) * 16 + (tid & 15))) : 0.f;
+    const float bias = tid < n * FEW_RED ? h2f(__ldg(a.bias + (t0 + tid / FEW_RED) * 16 + (tid & 15))) : 0.f;
     __syncthreads();
 #pragma unroll 1
     for (int left = few_passes(2); left; left = few_passes(left - 1)) {
@@ -533,34 +488,29 @@ __global__ void __launch_bounds__(FEW_THREADS, 2) few_mlp(const __grid_constant_
         few_norm<KW, WPR, FIXED, false>(a.n, real, w, l, par, op, ld, stat, [&](int row, int d) { return State<FIXED>::load(z, (size_t)row * D + d); });
         if (real) asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
-        few_fold<KW, FOUR>(slots, few_row<FOUR>(smem_u32(op), ld, R, l), n, KP, red, w, l);
+        few_fold<KW>(slots, few_row(smem_u32(op), ld, R, l), n, KP, red, w, l);
         __syncthreads();
-#pragma unroll
-        for (int x = 0; x < FEW_TILES / 2; x++) {
-            const int o = x * FEW_THREADS + w * 32 + l, row = (o >> 4) & 7, f = (o >> 7) * 16 + (o & 15);
-            if (row >= R || o >= n * 128) continue;
-            const float v = gelu_tanh(few_sum(red, o) + bias[x], a.a2, a.k1, a.k2);
+        const int o = w * 32 + l, row = (o >> 4) % FEW_ROWS;
+        if (row < R && o < n * FEW_RED) {
+            const float v = gelu_tanh(few_sum(red, o) + bias, a.a2, a.k1, a.k2);
             const u16 hi = f2h(v);
-            *reinterpret_cast<u16*>(op2 + few_head<FOUR>(row) * ld2 + f * 2) = hi;
-            *reinterpret_cast<u16*>(op2 + few_rest<FOUR>(row, R) * ld2 + f * 2) = f2h(v - h2f(hi));
+            unsigned char* to = op2 + 2 * row * ld2 + ((o / FEW_RED) * 16 + (o & 15)) * 2;
+            *reinterpret_cast<u16*>(to) = hi;
+            *reinterpret_cast<u16*>(to + ld2) = f2h(v - h2f(hi));
         }
         __syncthreads();
         // (every block begins with other outputs: all of them adding to the same lines at once took longer)
-        u32 f[2][4];
-        const u32 a_at = few_row<FOUR>(smem_u32(op2), ld2, R, l), at0 = slots + fcu * 512 + l * 16;
-        ldsm4(f[0], a_at);
-        ldsm4(f[1], FOUR || n < 2 ? a_at : a_at + 32);
+        u32 f[4];
+        const u32 at0 = slots + fcu * 512 + l * 16;
+        ldsm4(f, few_row(smem_u32(op2), ld2, R, l));
         int at = cnt ? blockIdx.x % cnt : 0;
 #pragma unroll 2
         for (int x = 0; x < cnt; x++) {
             float c[2][4] = {};
             const uint4 u = lds16(at0 + at * (a.per * 512)), v = lds16(at0 + (at * a.per + n - 1) * 512);
-            if (FOUR) { few_mma(c[0], u, f[0][0], f[0][1]); if (n > 1) few_mma(c[1], v, f[0][2], f[0][3]); }
-            else {
-                mma16816(c[0], f[0], u.x, u.y); mma16816(c[1], f[0], u.z, u.w);
-                if (n > 1) { mma16816(c[0], f[1], v.x, v.y); mma16816(c[1], f[1], v.z, v.w); }
-            }
-            if (real) few_add<FOUR, FIXED>(a.n.into, D, R, w + at * FEW_WARPS, c, l);
+            few_mma(c[0], u, f[0], f[1]);
+            if (n > 1) few_mma(c[1], v, f[2], f[3]);
+            if (real) few_add<FIXED>(a.n.into, D, R, w + at * FEW_WARPS, c, l);
             at = at + 1 == cnt ? 0 : at + 1;
         }
     }

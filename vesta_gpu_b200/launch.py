@@ -136,7 +136,7 @@ class Kernel:
                                    f'call lower(..., grid={self.sms})')
             self.lowered = lowered
             self.chain = bool(lowered.dims.get('chain'))         # a step is a chain of kernels (passes.py), not one persistent kernel
-            self.few = bool(lowered.dims.get('few'))             # ... of three per layer, from packed weights (at most eight sequences)
+            self.few = bool(lowered.dims.get('few'))             # ... of three per layer, from packed weights (two to four sequences)
             self.graphs = self.chain or self.few
             self.smem = lowered.shared_bytes
             # The reference's signature defaults to block=256 (vesta/launch.py:30) and callers pass it along: 256 and
