@@ -40,6 +40,10 @@ def seeded(m, sh, ctx, seed):
     (16, dict(D=1216, H=19, F=64)),                   # a fold of 19 blocks, fp16 operands at 16 rows
     (8, dict(L=1, D=1280, H=20)),                     # 160 (sequence, head) pairs at eight sequences: a chain, not the persistent kernel
     (3, dict(L=1, D=1344, H=21)),                     # three sequences of a wide shape: the same
+    # every shape of the attention past the ends of its rings: eight warps with three stages, in clusters of two and alone, also of wide rows,
+    (35, dict(C=1200)), (80, dict(C=1200)), (13, dict(D=1216, H=19, F=64, C=1200)),
+    # with two; four warps with four stages, in clusters of two and alone, and with two
+    (16, dict(D=1216, H=19, F=64, C=1200)), (9, dict(C=1200)), (130, dict(C=1200)), (200, dict(C=1200)),
 ])
 def test_step_as_a_chain(batch, kw):
     """ragged decode steps over seeded caches, contexts from none to nearly all of the cache"""
@@ -48,8 +52,8 @@ def test_step_as_a_chain(batch, kw):
     m, hf = model(sh, 17, 'rich', batch, sh.C, per_sequence_t=True)
     assert m.low.dims['chain']
     W = O.upcast(hf.weights)
-    ctx = np.array([(37 * b) % 390 for b in range(batch)], np.int32)
-    ctx[:4] = (389, 0, 63, 64)[:batch]
+    ctx = np.array([(37 * b) % (sh.C - 10) for b in range(batch)], np.int32)
+    ctx[:4] = (sh.C - 11, 0, 63, 64)[:batch]
     caches = seeded(m, sh, ctx, 900)
     x = np.array([(b * 31 + 5) % sh.N for b in range(batch)], np.int32)
     m.t.copy_(torch.from_numpy(ctx))

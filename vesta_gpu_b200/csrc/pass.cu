@@ -243,11 +243,12 @@ cudaError_t prepare_all() {
     auto one = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
     one(all_shared(pass_norm<NORM_EMBED>)); one(all_shared(pass_norm<NORM_MID>)); one(all_shared(pass_norm<NORM_FINAL>));
     one(all_shared(pass_norm_rows<6>)); one(all_shared(pass_norm_rows<13>)); one(all_shared(pass_norm_rows<16>));
-    one(all_shared(pass_attend<2, 4>)); one(all_shared(pass_attend<2, 8>)); one(all_shared(pass_attend<3, 8>)); one(all_shared(pass_attend_many<true>)); one(all_shared(pass_attend_many<false>));
+    one(all_shared(pass_attend<2, 4>)); one(all_shared(pass_attend<4, 4>)); one(all_shared(pass_attend<2, 8>)); one(all_shared(pass_attend<3, 8>)); one(all_shared(pass_attend_many<true>)); one(all_shared(pass_attend_many<false>));
     one(gemm_prepare());
     one(cudaFuncSetAttribute((const void*)pass_attend_many<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, AM_SMEM));
     one(cudaFuncSetAttribute((const void*)pass_attend_many<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AM_SMEM));
     one(cudaFuncSetAttribute((const void*)pass_attend<3, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * 8 * 4096));
+    one(cudaFuncSetAttribute((const void*)pass_attend<4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 4 * 4096));
     one(cudaFuncSetAttribute((const void*)pass_attend<2, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 8 * 4096)); one(all_shared(pass_finish));
     return e;
 }
@@ -329,12 +330,17 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
     // step with two blocks instead of four; 9 sequences, small shape, two instead of eight: 298 -> 270 us, at 1,000 positions
     // 340 -> 321), and so did two beyond that line (23 sequences at 128 positions with one block: 294 -> 277 us).
     const int C = rows * d.H * 2 <= 3 * p.sms && d.tmax > 4 * ATT_RUN ? 2 : 1;
-    // ... eight warps where an SM has no more than three blocks, and rings that keep a third block away where two are due: blocks go
-    // where there is room, which is not evenly (23 ragged sequences to 700 positions, 276 blocks: 7.05 us with four warps and rings of
-    // 64 KB, 6.15 with eight, 4.92 with eight and 96 KB; 9 at 900, 216 blocks: 290, 286 and 269 us per step; XL shape with 16, 400 blocks: 4.31,
-    // 4.30 and 6.08 us; with 3, 150 blocks: 1,157, 1,162 and 1,186 us per step). Beyond, four warps: 64 sequences 16.0 us, with eight 17.1.
+    // Warps and stages of a block's rings. Where two blocks are due to an SM, eight warps and 96 KB, which keep a third block away: blocks
+    // go where there is room, which is not evenly (23 ragged sequences to 700 positions: 7.05 us with 4 x 4, 4.92 so; 9 at 900: 290 and 272 us per
+    // step, at 8 positions 244 and 239). Not so: clusters of two that nearly fill the SMs, whose last ones wait until both their places are
+    // free (12 sequences at 64 positions 242 us per step with 4 x 4, 248 so); wide rows with fewer blocks, where an SM with two of them
+    // has no room for the projection's block of 83 KB, which 64 KB leave (XL shape, 4 at 64: 1,149 and 1,239, 9 at 64: 1,208 and 1,223; with 10
+    // and 11, one for nearly every place, it is 0.99 to 1.06 times as fast). Elsewhere up to three blocks per SM four warps with 64 KB, which is
+    // within 1 % of eight with 64 from 300 positions and up to 2 % faster below, but for wide rows of one block per pair, where eight are 1 to 2 %
+    // faster from 64 positions (XL shape, 16 at 300: 1,372 and 1,357; at 8 1,174 and 1,185). Beyond, 32 KB: 64 sequences 16.0 us, with eight warps 17.1.
     const int blocks = rows * d.H * C;
-    const bool wide = blocks <= 3 * p.sms, deep = blocks <= 2 * p.sms && 4 * blocks > 5 * p.sms;
+    const bool some = blocks <= 3 * p.sms, deep = D <= 1024 ? 4 * blocks > 5 * p.sms : 8 * blocks > 13 * p.sms;
+    const int shape = deep && 10 * blocks <= (C == 2 ? 17 : 20) * p.sms ? 83 : !some ? 42 : D > 1024 && C == 1 ? 82 : 44;
     const Pass::Plan* pl = nullptr;
     if (int e = plan_for(p, rows, lrows, &pl)) return e;
     auto f16 = [](const void* q, size_t off) { return (const u16*)q + off; };
@@ -398,9 +404,9 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
             return pow2 ? cudaLaunchKernelEx(&c.c, pass_attend_many<true>, p.qmap, p.kmap, p.vmap, a) : cudaLaunchKernelEx(&c.c, pass_attend_many<false>, p.qmap, p.kmap, p.vmap, a);
         }
         AttArgs a = {q, kc, vc, ss, (const int*)d.t, d.t_stride, d.tmax, D, pow2, p.rp, d.scale, att};
-        Config c(dim3(d.H, rows, C), wide ? 256 : 128, st, true, C);
-        c.c.dynamicSmemBytes = (deep ? 24 : wide ? 16 : 8) * 4096;
-        return deep ? cudaLaunchKernelEx(&c.c, pass_attend<3, 8>, a) : wide ? cudaLaunchKernelEx(&c.c, pass_attend<2, 8>, a) : cudaLaunchKernelEx(&c.c, pass_attend<2, 4>, a);
+        Config c(dim3(d.H, rows, C), shape / 10 * 32, st, true, C);
+        c.c.dynamicSmemBytes = (shape / 10) * (shape % 10) * 4096;
+        return shape == 83 ? cudaLaunchKernelEx(&c.c, pass_attend<3, 8>, a) : shape == 82 ? cudaLaunchKernelEx(&c.c, pass_attend<2, 8>, a) : shape == 44 ? cudaLaunchKernelEx(&c.c, pass_attend<4, 4>, a) : cudaLaunchKernelEx(&c.c, pass_attend<2, 4>, a);
     };
     TRY(norm(0, 0));
     for (int l = 0; l < L; l++) {

@@ -802,14 +802,14 @@ template <int NS> struct AttRow {
             asm volatile("cp.async.wait_group %0;" :: "n"(NS - 1) : "memory");
             __syncwarp();
             const u32 so = st * 4096;
-            float s[4] = {0.f, 0.f, 0.f, 0.f}, x[4] = {0.f, 0.f, 0.f, 0.f};
+            float s[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int k = 0; k < 4; k++) {
                 u32 r[4];
                 ldsm4(r, (ka & ~127u) + so + (((k * 2 + kx) ^ k7) << 4));
-                if (k & 1) mma16816(x, r, bq[k][0], bq[k][1]); else mma16816(s, r, bq[k][0], bq[k][1]);
+                mma16816(s, r, bq[k][0], bq[k][1]);
             }
-            float s0 = (s[0] + s[1]) + (x[0] + x[1]), s1 = (s[2] + s[3]) + (x[2] + x[3]);        // positions p0 + g and p0 + g + 8
+            float s0 = s[0] + s[1], s1 = s[2] + s[3];        // positions p0 + g and p0 + g + 8
             if (!a.pow2) { s0 /= a.scale; s1 /= a.scale; }
             if (p0 + g >= n) s0 = -3.0e38f;
             if (p0 + g + 8 >= n) s1 = -3.0e38f;
