@@ -214,7 +214,6 @@ int check(const vesta_pass_desc& d) {
 template <class F> cudaError_t all_shared(F* f) { return cudaFuncSetAttribute((const void*)f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared); }
 template <int BM, int EPI>
 cudaError_t launch_gemm(cudaLaunchConfig_t& c, const Tile& t, const CUtensorMap& w, const CUtensorMap& a, const GemmArgs& g) {
-    c.dynamicSmemBytes = std::max<size_t>(GemmShape<BM>::bytes(t.stages, t.bn), c.dynamicSmemBytes);
     c.blockDim = dim3(GemmShape<BM>::THREADS + (EPI == EPI_QKV && g.seqs ? 32 : 0));
     return cudaLaunchKernelEx(&c, pass_gemm<BM, EPI>, w, a, g);
 }
@@ -270,6 +269,18 @@ Tile tile_of(const Pass& p, int k, int rows, int lrows) {
     const vesta_pass_desc& d = p.d;
     const int feat[5] = {3 * d.D, d.D, d.F, d.D, d.N};
     return choose(k, k == K_LOGITS ? std::max(lrows, 1) : rows, p.rp, feat[k], k == K_P2 ? (d.F + 63) / 64 : d.D / 64, p.sms);
+}
+
+// Shared memory of a block of a contraction of `ntiles` tiles. A step's projection has small blocks that come while the attention's leave: five of
+// them on the first SMs that are free, none on the last. Where there is about one for every SM and more than two would fit one, they ask for
+// so much that only two do (64 sequences, 144 blocks of 41 KB: 1,763 -> 1,721 us per four steps; 33 to 80 sequences 1 to 4 % faster; 23, 72 blocks:
+// 1,111 -> 1,122, left). Blocks of the XL shape (83 KB) are two to an SM as they are, and with more lose their place beside an attention block
+// (16 sequences at 300 positions 1,367 -> 1,355 us per step without, 8 at 300 1,309 -> 1,288). Prompts take
+// the same time either way (8 to 900 rows, within 0.5 %) and are left.
+size_t block_bytes(const Pass& p, int kind, const Tile& t, int ntiles) {
+    const int bytes = t.bm == 64 ? GemmShape<64>::bytes(t.stages, t.bn) : t.bm == 128 ? GemmShape<128>::bytes(t.stages, t.bn) : GemmShape<256>::bytes(t.stages, t.bn);
+    const bool spread = kind == K_PROJ && !p.d.prompts && t.bm == 64 && 2 * ntiles > p.sms && 3 * (bytes + 1024) <= SMEM_MAX;
+    return spread ? std::max(bytes, 110 * 1024) : bytes;
 }
 
 // The tiles and tensor maps for `rows` rows of which `lrows` want logits.
@@ -371,6 +382,7 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
         if (kind == K_LOGITS) {
             g = logits_args(p, t, lrows);
             Config c(dim3(std::min(g.ntiles, p.sms)), 0, st, true);
+            c.c.dynamicSmemBytes = block_bytes(p, kind, t, g.ntiles);
             return gemm(EPI_LOGITS, t, c.c, pl->w[kind], pl->a[kind], g);
         }
         g.layer = l; g.D = D; g.rp = p.rp; g.stages = t.stages; g.status = (u32*)d.bar; g.limit = p.wait_ns; g.skip = (const int*)u(p.o.skip);
@@ -387,10 +399,7 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
         } else { g.of = z; g.bias = kind == K_PROJ ? f16(d.ob, (size_t)l * D) : f16(d.pb, (size_t)l * D); }
         g.bn = t.bn; g.ftiles = (g.nfeat + t.bm - 1) / t.bm; g.rtiles = p.rp ? 1 : (g.rows + t.bn - 1) / t.bn; g.ntiles = g.ftiles * g.rtiles * t.splits;
         Config c(dim3(t.bm == 64 ? g.ntiles : t.bm == 256 ? 2 * std::min(g.ntiles, p.sms / 2) : std::min(g.ntiles, p.sms)), 0, st, true, t.bm == 256 ? 2 : 1, true);
-        // The projection's blocks are small and come while the attention's leave: five of them on the first SMs that are free, none on the
-        // last. Where there is about one for every SM they ask for so much that only two fit (64 sequences, 144 blocks of 41 KB: 1,763 ->
-        // 1,721 us per four steps; 23 sequences, 72 blocks: 1,111 -> 1,122, left).
-        if (kind == K_PROJ && t.bm == 64 && 2 * g.ntiles > p.sms) c.c.dynamicSmemBytes = 110 * 1024;
+        c.c.dynamicSmemBytes = block_bytes(p, kind, t, g.ntiles);
         return gemm(epi_of(kind), t, c.c, pl->w[kind], pl->a[kind], g);
     };
     auto attend = [&](int l) {
@@ -511,6 +520,7 @@ int enqueue_few(Pass& p, cudaStream_t st) {
     const Tile& t = pl->tile[K_LOGITS];
     const GemmArgs g = logits_args(p, t, R);
     Config cg(dim3(std::min(g.ntiles, p.sms)), 0, st, true);
+    cg.c.dynamicSmemBytes = block_bytes(p, K_LOGITS, t, g.ntiles);
     TRY(gemm(EPI_LOGITS, t, cg.c, pl->w[K_LOGITS], pl->a[K_LOGITS], g));
     Config cf(dim3(1), 256, st, true);
     TRY(cudaLaunchKernelEx(&cf.c, pass_finish, finish(p, R)));
@@ -667,7 +677,9 @@ int vesta_pass_tiles(const vesta_pass_desc* d, int rows, int logit_rows, int* ou
     if (int e = plan(p, d)) return e;
     for (int k = 0; k < 5; k++) {
         const Tile t = tile_of(p, k, rows, logit_rows);
-        const int v[5] = {t.bm, t.bn, t.stages, t.splits, t.bm == 64 ? GemmShape<64>::bytes(t.stages, t.bn) : t.bm == 128 ? GemmShape<128>::bytes(t.stages, t.bn) : GemmShape<256>::bytes(t.stages, t.bn)};
+        const int feat = k == K_QKV ? 3 * d->D : k == K_FC ? d->F : k == K_LOGITS ? d->N : d->D, n = k == K_LOGITS ? std::max(logit_rows, 1) : rows;
+        const int ntiles = (feat + t.bm - 1) / t.bm * (p.rp ? 1 : (n + t.bn - 1) / t.bn) * t.splits;
+        const int v[5] = {t.bm, t.bn, t.stages, t.splits, (int)block_bytes(p, k, t, ntiles)};
         std::copy(v, v + 5, out + 5 * k);
     }
     return 0;
