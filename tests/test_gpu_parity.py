@@ -347,13 +347,15 @@ def test_ragged_prompts_fed_on_the_device(B):
         assert np.array_equal(mine[:stop], ref[:stop]), i
 
 
-def test_per_sequence_positions_ragged_starts():
+@pytest.mark.parametrize('B', [4, 6])                    # (the chain of few sequences, the persistent kernel)
+def test_per_sequence_positions_ragged_starts(B):
     """every sequence at its own position: sequence b starts b*2 steps late"""
     from oracle import gpt2_numpy as O
     from vesta_gpu_b200.shapes import TINY
     from vesta_gpu_b200.synth import make_prompts
-    B, steps = 4, 12
+    steps = 12
     m, hf = model(TINY, 3, 'rich', B, steps, per_sequence_t=True, feedback=False)
+    assert m.k.graphs == (B == 4)
     W = O.upcast(hf.weights)
     feed = make_prompts(TINY, B, steps, seed=9)
     caches = [O.new_cache(TINY, steps) for _ in range(B)]
@@ -422,11 +424,13 @@ def test_tensor_core_logits_at_full_size_equal_the_mma_path():
     assert np.abs(outs[0] - outs[1]).max() < 5e-3
 
 
-def test_multi_step_launch_and_reset():
+@pytest.mark.parametrize('batch', [3, 5])                # (the chain of few sequences, the persistent kernel)
+def test_multi_step_launch_and_reset(batch):
     from vesta_gpu_b200.shapes import TINY
-    m, _ = model(TINY, 3, 'rich', 3, 32)
+    m, _ = model(TINY, 3, 'rich', batch, 32)
+    assert m.k.graphs == (batch == 3)
     def run(chunked):
-        m.reset(); m.x.copy_(torch.tensor([1, 2, 3], dtype=torch.int32))
+        m.reset(); m.x.copy_(torch.arange(1, batch + 1, dtype=torch.int32))
         if chunked:
             m.step(20)
         else:
@@ -463,11 +467,13 @@ def test_steps_inside_one_launch_equal_separate_launches(per_launch):
     assert int(m.k.bar[3]) == 0 and int(m.k.bar[32]) == 0           # step flag and barrier counter left clear
 
 
-def test_launch_of_many_steps_stops_at_the_end_of_the_cache():
+@pytest.mark.parametrize('batch', [2, 5])                # (the chain of few sequences, the persistent kernel)
+def test_launch_of_many_steps_stops_at_the_end_of_the_cache(batch):
     """a launch asked for more steps than the cache has room for stops after the last step that fits and
     says so; the steps before it are complete and the kernel is usable again afterwards"""
     from vesta_gpu_b200.shapes import TINY
-    m, _ = model(TINY, 3, 'rich', 2, 8)
+    m, _ = model(TINY, 3, 'rich', batch, 8)
+    assert m.k.graphs == (batch == 2)
     m.reset(); m.x.fill_(3)
     m.k.launch(7, per_launch=1)
     want_x, want_logits = m.x.clone(), m.logits().clone()
@@ -483,15 +489,17 @@ def test_launch_of_many_steps_stops_at_the_end_of_the_cache():
     assert torch.equal(m.x, want_x) and (m.logits() - want_logits).abs().max() < 2e-3
 
 
-def test_host_driven_step_equals_the_device_loop():
+@pytest.mark.parametrize('batch', [4, 6])                # (the chain of few sequences, the persistent kernel)
+def test_host_driven_step_equals_the_device_loop(batch):
     """vesta_step_host (tokens from pinned host memory, chosen tokens back to it, one call per step) against the
     kernel feeding itself"""
     from vesta_gpu_b200.shapes import TINY3
-    m, _ = model(TINY3, 5, 'rich', 4, 12)
-    start = torch.tensor([3, 50, 200, 331], dtype=torch.int32)
+    m, _ = model(TINY3, 5, 'rich', batch, 12)
+    assert m.k.graphs == (batch == 4)
+    start = torch.tensor([3, 50, 200, 331, 17, 90][:batch], dtype=torch.int32)
     m.reset(); m.x.copy_(start); m.k.launch(10, per_launch=1)
     want_x, want_logits = m.x.cpu(), m.logits().cpu()
-    hx, hn = start.clone().pin_memory(), torch.empty(4, dtype=torch.float32).pin_memory()
+    hx, hn = start.clone().pin_memory(), torch.empty(batch, dtype=torch.float32).pin_memory()
     m.reset()
     for _ in range(10):
         m.step_host(hx, hn)
@@ -605,18 +613,18 @@ def test_dense_prefill_at_full_size_against_the_reference(rows):
     assert compared >= 4 * B
 
 
-@pytest.mark.parametrize('batch,tune', [(3, None), (70, dict(ln_dist=True)), (70, None), (12, None)])
+@pytest.mark.parametrize('batch,tune', [(3, None), (70, dict(ln_dist=True)), (70, None), (12, None), (5, None)])
 @pytest.mark.parametrize('without', [('qkvb', 'fcb'), ('ln1b', 'qkvb', 'ob', 'ln2b', 'fcb', 'pb', 'lnfb')])
 def test_program_without_shifts_or_biases(batch, tune, without):
-    """a program that leaves out additive parameters (both kernel texts, at 70 sequences the tensor-core contractions, and the
-    chain) and the same tokens as prompts: the kernel reads zeros in their place; against the oracle with those parameters set
+    """a program that leaves out additive parameters (both kernel texts, at 70 sequences the tensor-core contractions, and both
+    chains) and the same tokens as prompts: the kernel reads zeros in their place; against the oracle with those parameters set
     to zero, which is the same arithmetic as the shorter statements"""
     from oracle import gpt2_numpy as O
     from vesta_gpu_b200.shapes import TINY
     from vesta_gpu_b200.synth import make_prompts
     steps = 5
     m, hf = model(TINY, 5, 'rich', batch, steps, without=without, tune=tune)
-    assert m.k.chain == (batch > 8 and not tune)
+    assert m.k.chain == (batch > 8 and not tune) and m.k.few == (batch == 3)
     assert m.low.dims['absent'] == sorted(without) and not set(without) & set(m.W)
     weights = dict(hf.weights)
     for n in without:
@@ -639,9 +647,11 @@ def test_program_without_shifts_or_biases(batch, tune, without):
     m.k.check()
 
 
-def test_out_of_range_inputs_are_refused_not_executed():
+@pytest.mark.parametrize('batch', [2, 5])                # (the chain of few sequences, the persistent kernel)
+def test_out_of_range_inputs_are_refused_not_executed(batch):
     from vesta_gpu_b200.shapes import TINY
-    m, _ = model(TINY, 3, 'rich', 2, 8)
+    m, _ = model(TINY, 3, 'rich', batch, 8)
+    assert m.k.graphs == (batch == 2)
     m.reset(); m.x.fill_(3); m.step()
     before = m.logits().clone()
     m.t.fill_(8)                                  # position == tmax: outside the cache

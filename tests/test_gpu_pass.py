@@ -82,8 +82,8 @@ def test_step_as_a_chain(batch, kw):
     (3, dict(L=1, D=832, H=13, F=2384)),
 ])
 def test_step_of_few_sequences(batch, kw):
-    """three kernels per layer from packed weights: ragged steps over seeded caches against the oracle; up to two sequences the same
-    bits twice; the persistent kernel takes the same step"""
+    """three kernels per layer from packed weights: ragged steps over seeded caches against the oracle; of two sequences the same bits
+    twice"""
     from oracle import gpt2_numpy as O
     sh, steps = shape('few', **kw), 2
     m, hf = model(sh, 17, 'rich', batch, sh.C, per_sequence_t=True)
@@ -110,6 +110,81 @@ def test_step_of_few_sequences(batch, kw):
         runs.append((m.logits().clone(), m.keys.clone(), m.vals.clone()))
     assert batch > 2 or all(torch.equal(a, b) for a, b in zip(*runs))
     m.k.check()
+
+
+@pytest.mark.parametrize('ctx', [(1189, 1023), (511, 1024), (1189, 512, -1), (257, 513, 767), (1189, -1, 511, 1040), (255, 256, 768, 1023)])
+def test_steps_of_few_sequences_past_the_ends_of_their_rings(ctx):
+    """contexts that take a warp's ring of two stages (of 512 positions between them with two sequences, 256 with three and four) round more
+    than once, the current position in the first round of a stage and in later ones, a sequence that starts a step later; against the oracle
+    and the persistent kernel"""
+    from oracle import gpt2_numpy as O
+    sh, batch = shape('rings', C=1200), len(ctx)
+    m, hf = model(sh, 17, 'rich', batch, sh.C, per_sequence_t=True)
+    p, _ = model(sh, 17, 'rich', batch, sh.C, per_sequence_t=True, tune=dict(wait_ns=500_000_000))
+    assert m.k.few and not p.k.graphs
+    W = O.upcast(hf.weights)
+    caches = seeded(m, sh, np.maximum(ctx, 0), 900)
+    seeded(p, sh, np.maximum(ctx, 0), 900)
+    x = np.array([(b * 31 + 5) % sh.N for b in range(batch)], np.int32)
+    for s in range(2):
+        for k in (m, p):
+            k.t.copy_(torch.tensor([c + s for c in ctx], dtype=torch.int32))
+            k.x.copy_(torch.from_numpy(x))
+            k.step()
+            k.k.check()
+        lg, other, nx = m.logits().cpu().numpy(), p.logits().cpu().numpy(), m.next().cpu().numpy()
+        for b in range(batch):
+            if ctx[b] + s < 0:
+                assert not m.keys[b].any() and not m.vals[b].any()
+                continue
+            ref, rn = O.step(sh, W, *caches[b], int(x[b]), ctx[b] + s)
+            assert np.abs(lg[b] - ref).max() < TIGHT and np.abs(lg[b] - other[b]).max() < TIGHT, (s, b)
+            assert O.margin(ref) <= MARGIN or int(nx[b]) == rn
+            x[b] = rn
+    for b in range(batch):
+        for got, ref in ((m.keys, caches[b][0]), (m.vals, caches[b][1])):
+            assert np.abs(got[b].float().cpu().numpy() - ref.astype(np.float32)).max() <= 4e-3, b
+
+
+def test_equal_prompts_are_as_exact_in_every_batch():
+    """GPT-2 small, the same sixteen tokens alone and as two to eight equal rows, in the persistent kernel and in the chain of few sequences:
+    every row against the same arithmetic in 64 bits with K and V rounded to fp16. What is left are K and V that round the other way, as
+    their sums differ from the exact ones in the last bits of fp32: over twelve prompts the persistent kernel's logits are at most 1.5 to
+    1.8e-4 off (root mean square 2e-5), the chain's at most 0.95 to 1.14e-4 (1.7e-5), so two batches differ by up to 3e-4"""
+    import math
+    from vesta_gpu_b200.gpt2 import VestaGPT2
+    from vesta_gpu_b200.shapes import GPT2_SMALL as sh
+    from vesta_gpu_b200.synth import SynthGPT2, make_prompts
+    P = 16
+    hf = SynthGPT2(sh, 0, 'baseline')
+    W = {n: torch.from_numpy(np.asarray(w)).cuda().double() for n, w in hf.weights.items()}
+    prompts = [make_prompts(sh, 1, P, seed=s)[0] for s in (5, 6, 7)]
+    toks = torch.from_numpy(np.stack(prompts).astype(np.int64)).cuda()
+
+    def norm(z, w, b):
+        m = z.mean(-1, keepdim=True)
+        return (z - m) / torch.sqrt(((z - m) ** 2).mean(-1, keepdim=True) + 1e-5) * w + b
+    heads = lambda a: a.view(len(prompts), P, sh.H, sh.E).transpose(1, 2)
+    z = W['wte'][toks] + W['wpe'][:P]
+    later = torch.full((P, P), -math.inf, device='cuda', dtype=torch.float64).triu(1)
+    for l in range(sh.L):
+        q, k, v = (norm(z, W['ln1w'][l], W['ln1b'][l]) @ W['qkvw'][l] + W['qkvb'][l]).split(sh.D, -1)
+        w = torch.softmax(heads(q) @ heads(k.half().double()).transpose(-1, -2) / 8 + later, -1)
+        z = z + (w @ heads(v.half().double())).transpose(1, 2).reshape(len(prompts), P, sh.D) @ W['ow'][l] + W['ob'][l]
+        u = norm(z, W['ln2w'][l], W['ln2b'][l]) @ W['fcw'][l] + W['fcb'][l]
+        z = z + (0.5 * u * (1 + torch.tanh(0.7978845608028654 * (u + 0.044715 * u ** 3)))) @ W['pw'][l] + W['pb'][l]
+    exact = norm(z[:, -1], W['lnfw'], W['lnfb']) @ W['wte'].T
+    for B in (1, 2, 3, 4, 5, 8):
+        m = VestaGPT2(hf, batch=B, tmax=P + 1)
+        assert m.k.few == (2 <= B <= 4) and not m.k.chain
+        for i, prompt in enumerate(prompts):
+            m.reset()
+            for t in range(P):
+                m.x.fill_(int(prompt[t]))
+                m.step()
+            off = m.logits().double() - exact[i]
+            assert off.abs().max() < 3e-4 and off.square().mean().sqrt() < 4e-5, (B, i)     # (twice and less what was seen)
+        m.k.check()
 
 
 def test_a_good_step_of_few_sequences_runs_after_a_refused_one():
@@ -306,13 +381,14 @@ def moved(t):
     return v.copy_(t)
 
 
-@pytest.mark.parametrize('batch', [3, 12])
+@pytest.mark.parametrize('batch', [3, 12, 1, 5])
 def test_weights_off_a_16_byte_boundary(batch):
-    """weights that are views into a larger buffer, in the persistent kernel and in a chain: read through aligned copies that
-    pack() renews; the caches are refused"""
+    """weights that are views into a larger buffer, in the persistent kernel (one and five sequences) and in both chains: read through aligned
+    copies that pack() renews; the caches are refused"""
     from vesta_gpu_b200.launch import Kernel
     sh = shape('moved')
     m, _ = model(sh, 3, 'rich', batch, 20)
+    assert (m.k.few, m.k.chain) == (batch == 3, batch == 12)
     k = Kernel(m.low, device=m.device.index)
     R = dict(m.k.keep)
     for role in ('ln1w', 'ln1b', 'qkvw', 'qkvb', 'ow', 'ob', 'ln2w', 'ln2b', 'fcw', 'fcb', 'pw', 'pb', 'lnfw', 'lnfb', 'wpe'):
