@@ -81,10 +81,11 @@ def test_step_as_a_chain(batch, kw):
     (2, dict(L=1, D=1024, H=16, F=4096)), (4, dict(L=1, D=1024, H=16, F=2384)),   # two tiles per block; 149 tiles, the last block has one
     (3, dict(L=1, D=832, H=13, F=2384)),
 ])
-def test_step_of_few_sequences(batch, kw):
+def test_step_of_few_sequences(batch, kw, monkeypatch):
     """three kernels per layer from packed weights: ragged steps over seeded caches against the oracle; of two sequences the same bits
     twice"""
     from oracle import gpt2_numpy as O
+    monkeypatch.setattr('vesta_gpu_b200.lower.few_pays', lambda D, F: True)          # (also where the persistent kernel is faster)
     sh, steps = shape('few', **kw), 2
     m, hf = model(sh, 17, 'rich', batch, sh.C, per_sequence_t=True)
     assert m.k.few and not m.k.chain

@@ -381,3 +381,18 @@ def test_exchanges_between_ctas_are_chosen_where_every_cta_has_at_most_one_item(
     # switched off by hand: the reference structure of one barrier per phase
     low = lower_for(GPT2_SMALL, 8, 384, tune=dict(fuse_proj=False, qkv_exchange=False))
     assert low.barriers_per_launch == 1 + 4 * 12 and not low.dims['part_exchange']
+
+
+@pytest.mark.parametrize('D,F,batch,kind', [
+    (768, 3072, 1, 'persistent'), (768, 3072, 2, 'few'), (768, 3072, 4, 'few'), (768, 3072, 5, 'persistent'), (768, 3072, 8, 'persistent'), (768, 3072, 9, 'chain'),
+    (896, 3584, 4, 'few'), (1024, 2368, 2, 'few'), (1024, 2384, 2, 'persistent'), (1024, 4096, 3, 'persistent'), (960, 3840, 2, 'persistent'),
+    (768, 4736, 3, 'few'), (768, 4752, 3, 'persistent'), (1088, 1088, 2, 'persistent'), (1280, 5120, 5, 'chain'), (1600, 6400, 3, 'chain'),
+])
+def test_which_kernels_run_a_step(D, F, batch, kind):
+    """two to four sequences take the chain of few sequences where its blocks fit beside the attention's, others one kernel or the chain of
+    seven per layer"""
+    from vesta_gpu_b200.shapes import Shape
+    low = lower_for(Shape('s', L=1, D=D, H=D // 64, E=64, F=F, N=64, C=16), batch, 16)
+    assert (low.dims['few'], low.dims['chain']) == (kind == 'few', kind == 'chain')
+    assert not low.dims['few'] or low.dims['step']['exact'] == 2
+    assert not lower_for(Shape('s', L=1, D=D, H=D // 64, E=64, F=F, N=64, C=16), batch, 16, tune=dict(wait_ns=10 ** 8)).dims['few']

@@ -529,6 +529,14 @@ def few_fits(D, F, B, sms=DEFAULT_SMS):
     return 2 <= B <= 4 and D <= 1024 and 3 * D <= 32 * sms and F <= 32 * sms
 
 
+def few_pays(D, F, sms=DEFAULT_SMS):
+    """whether such a step is faster so than in the small persistent kernel: everywhere but for blocks with two tiles of the MLP of wide rows,
+    which leave the attention's blocks no room beside them, so that the weights of neither kernel are on their way early (width 1,024 with an MLP of
+    4,096, 24 layers, two, three and four sequences at 200 positions: 408, 405 and 419 us per step in the persistent kernel, 430, 414 and
+    425 so; with an MLP of 2,368, one tile per block, twelve layers: 200, 205, 211 and 186, 178, 184; width 896 with 3,584: 202, 205, 213 and 179, 176, 207)"""
+    return D <= 896 or F <= 16 * sms
+
+
 def lower(text, res, axis_max, batch=1, per_token=(), outputs=(), feedback=None, timing=False,
           grid=DEFAULT_SMS, act_lo=None, prompt_len=0, slab_tiles=None, tune=None, row_seq=False):
     """See the module docstring. `res`: name -> (shape, dtype) as the kernel sees them (batched
@@ -604,11 +612,14 @@ def lower(text, res, axis_max, batch=1, per_token=(), outputs=(), feedback=None,
     tune = dict(tune or {})
     # What a step as a chain of kernels (csrc/pass.cu) needs to know; Kernel runs that chain unless the caller asked for
     # something that only the persistent kernels have (a placement option, timing sums, rows of prompts).
-    # Two to four sequences of widths to 1,024: a chain of three kernels per layer from packed weights (csrc/pass_few.cuh) is the
-    # fastest (small shape, four sequences at 200 positions 190 us per step in the small persistent kernel, 165 so). With one (183 and 169)
-    # and with eight (209 and 192) it would be too, but the logits of equal prompts there are compared from batch to batch, and its sums
-    # in another order than the persistent kernel's differ from those by up to 1.3e-4 after sixteen positions (0.9e-4 among themselves):
-    # those batches stay in one kernel text. Beyond (wider rows, or an MLP of more than 32 features per SM: the weights of a layer's kernels do not fit shared
+    # Two to four sequences of widths to 1,024: a chain of three kernels per layer from packed weights (csrc/pass_few.cuh), where it is the
+    # faster one (`few_pays`; small shape at 200 positions, us per step of sixteen: two 184 and 168, three 186 and 158, four 191 and 163; at 1,000: 192 and
+    # 174, 195 and 180, 208 and 185). Its logits are no further from those of 64 bits than the persistent kernel's (twelve prompts of sixteen positions: at most
+    # 0.95 to 1.14e-4, root mean square 1.6 to 1.7e-5; there 1.5 to 1.8e-4 and 1.8 to 2.0e-5), but off in other places: a prompt among two to four and the
+    # same one alone differ by up to 1.8e-4, where two batches of the persistent kernel differ by up to 1.4e-4. One sequence and five to eight stay there: a
+    # chain for them was faster (one 183 -> 169, eight 209 -> 192), but equal prompts in batches of one and eight are held to 1e-4 of each other, which needs
+    # sums that do not depend on the batch.
+    # Beyond (wider rows, or an MLP of more than 32 features per SM: the weights of a layer's kernels do not fit shared
     # memory side by side) the small persistent kernel stands against the chain of seven kernels per layer:
     # the wider the rows, the less a boundary weighs and the more
     # every CTA's norms do: width 1,280 (twelve layers) with four sequences 280 against 279, with five 293 against 286; XL shape
@@ -616,7 +627,7 @@ def lower(text, res, axis_max, batch=1, per_token=(), outputs=(), feedback=None,
     # and with more (sequence, head) pairs than CTAs the kernel falls back on grid barriers (XL shape, eight: 1,679 against 1,245).
     persistent = B <= (8 if D <= 1024 else 4 if D <= 1280 else 2) and B * H <= grid
     plain = not (tune or timing or row_seq or slab_tiles or act_lo is not None)
-    few = plain and persistent and few_fits(D, F, B)
+    few = plain and persistent and few_fits(D, F, B) and few_pays(D, F)
     dims = dict(dims, chain=plain and not persistent and D <= 4096, few=few,
                 step=dict(t_stride=int(t_per_token), tstep=int(fb.get(t_name, 0)), feedback=int(bool(fb)), prompt_len=int(prompt_len) if fb else 0,
                           exact=2 if few else int(B <= 8 or (B <= 16 and D <= 1024)), cpos=cpos))
