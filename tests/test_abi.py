@@ -193,7 +193,7 @@ def test_blocks_of_a_steps_projection_that_keep_others_away(built_library):
     from vesta_gpu_b200.passes import tiles
     from vesta_gpu_b200.shapes import SHAPES
     for name, rows, prompts, more in (('gpt2', 64, 0, True), ('gpt2', 37, 0, True), ('gpt2', 23, 0, False), ('gpt2_xl', 16, 0, False),
-                                      ('gpt2_xl', 64, 0, False), ('gpt2', 77, 1, False), ('gpt2', 300, 3, False)):
+                                      ('gpt2_xl', 64, 0, False), ('heads20', 16, 0, False), ('gpt2', 77, 1, False), ('gpt2', 300, 3, False)):
         sh = SHAPES[name]
         d = pass_desc(L=sh.L, D=sh.D, H=sh.H, F=sh.F, N=sh.N, rows=rows, logit_rows=prompts or rows, prompts=prompts)
         bm, bn, stages, parts, smem = tiles(d, rows, d.logit_rows)['proj']

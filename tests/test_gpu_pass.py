@@ -41,9 +41,9 @@ def seeded(m, sh, ctx, seed):
     (8, dict(L=1, D=1280, H=20)),                     # 160 (sequence, head) pairs at eight sequences: a chain, not the persistent kernel
     (3, dict(L=1, D=1344, H=21)),                     # three sequences of a wide shape: the same
     # every shape of the attention past the ends of its rings: eight warps with three stages, in clusters of two and alone, also of wide rows,
-    (35, dict(C=1200)), (80, dict(C=1200)), (13, dict(D=1216, H=19, F=64, C=1200)),
+    (11, dict(L=1, D=640, H=10, C=1200)), (80, dict(C=1200)), (11, dict(L=1, D=1536, H=24, F=64, C=1200)),
     # with two; four warps with four stages, in clusters of two and alone, and with two
-    (16, dict(D=1216, H=19, F=64, C=1200)), (9, dict(C=1200)), (130, dict(C=1200)), (200, dict(C=1200)),
+    (13, dict(L=1, D=1536, H=24, F=64, C=1200)), (9, dict(C=1200)), (16, dict(D=1216, H=19, F=64, C=1200)), (130, dict(C=1200)), (200, dict(C=1200)),
 ])
 def test_step_as_a_chain(batch, kw):
     """ragged decode steps over seeded caches, contexts from none to nearly all of the cache"""

@@ -275,11 +275,11 @@ Tile tile_of(const Pass& p, int k, int rows, int lrows) {
 // them on the first SMs that are free, none on the last. Where there is about one for every SM and more than two would fit one, they ask for
 // so much that only two do (64 sequences, 144 blocks of 41 KB: 1,763 -> 1,721 us per four steps; 33 to 80 sequences 1 to 4 % faster; 23, 72 blocks:
 // 1,111 -> 1,122, left). Blocks of the XL shape (83 KB) are two to an SM as they are, and with more lose their place beside an attention block
-// (16 sequences at 300 positions 1,367 -> 1,355 us per step without, 8 at 300 1,309 -> 1,288). Prompts take
+// (16 sequences at 300 positions 1,367 -> 1,355 us per step without, 8 at 300 1,309 -> 1,288), as do those of width 1,280 (16 at 128 315 -> 304). Prompts take
 // the same time either way (8 to 900 rows, within 0.5 %) and are left.
 size_t block_bytes(const Pass& p, int kind, const Tile& t, int ntiles) {
     const int bytes = t.bm == 64 ? GemmShape<64>::bytes(t.stages, t.bn) : t.bm == 128 ? GemmShape<128>::bytes(t.stages, t.bn) : GemmShape<256>::bytes(t.stages, t.bn);
-    const bool spread = kind == K_PROJ && !p.d.prompts && t.bm == 64 && 2 * ntiles > p.sms && 3 * (bytes + 1024) <= SMEM_MAX;
+    const bool spread = kind == K_PROJ && !p.d.prompts && p.d.D <= 1024 && t.bm == 64 && 2 * ntiles > p.sms && 3 * (bytes + 1024) <= SMEM_MAX;
     return spread ? std::max(bytes, 110 * 1024) : bytes;
 }
 
@@ -349,9 +349,13 @@ int enqueue(Pass& p, cudaStream_t st, int rows, int lrows, int tiles, bool clear
     // and 11, one for nearly every place, it is 0.99 to 1.06 times as fast). Elsewhere up to three blocks per SM four warps with 64 KB, which is
     // within 1 % of eight with 64 from 300 positions and up to 2 % faster below, but for wide rows of one block per pair, where eight are 1 to 2 %
     // faster from 64 positions (XL shape, 16 at 300: 1,372 and 1,357; at 8 1,174 and 1,185). Beyond, 32 KB: 64 sequences 16.0 us, with eight warps 17.1.
+    // How blocks of several kernels share an SM depends on the width: all this holds at widths of 640 to 1,024 and from 1,600 on. Width 512 loses in
+    // clusters of two (14 sequences at 64 positions 229 us per step with 4 x 4, 240 with eight warps and 96 KB), 1,280 with eight warps of either kind (13 at 128:
+    // 294 and 308, 16 at 128: 301 and 305): four warps there.
     const int blocks = rows * d.H * C;
-    const bool some = blocks <= 3 * p.sms, deep = D <= 1024 ? 4 * blocks > 5 * p.sms : 8 * blocks > 13 * p.sms;
-    const int shape = deep && 10 * blocks <= (C == 2 ? 17 : 20) * p.sms ? 83 : !some ? 42 : D > 1024 && C == 1 ? 82 : 44;
+    const bool narrow = D <= 1024, wide = D >= 1536, some = blocks <= 3 * p.sms;
+    const bool deep = (narrow && 4 * blocks > 5 * p.sms) || (wide && 8 * blocks > 13 * p.sms);
+    const int shape = deep && (C == 2 ? D > 512 && 10 * blocks <= 17 * p.sms : blocks <= 2 * p.sms) ? 83 : !some ? 42 : wide && C == 1 ? 82 : 44;
     const Pass::Plan* pl = nullptr;
     if (int e = plan_for(p, rows, lrows, &pl)) return e;
     auto f16 = [](const void* q, size_t off) { return (const u16*)q + off; };
