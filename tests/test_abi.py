@@ -188,12 +188,12 @@ def test_tiles_of_a_pass_fit_a_block(built_library, name, exact):
 
 
 def test_blocks_of_a_steps_projection_that_keep_others_away(built_library):
-    """what vesta_pass_tiles reports is what a block is launched with: in a step, more than its stages where there is a block for
-    about every SM and three would fit one; not for few blocks, wide rows or prompts"""
+    """what vesta_pass_tiles reports is what a block is launched with: more than its stages where there is a block for about every SM
+    and three would fit one; not for few blocks or wide rows"""
     from vesta_gpu_b200.passes import tiles
     from vesta_gpu_b200.shapes import SHAPES
     for name, rows, prompts, more in (('gpt2', 64, 0, True), ('gpt2', 37, 0, True), ('gpt2', 23, 0, False), ('gpt2_xl', 16, 0, False),
-                                      ('gpt2_xl', 64, 0, False), ('heads20', 16, 0, False), ('gpt2', 77, 1, False), ('gpt2', 300, 3, False)):
+                                      ('gpt2_xl', 64, 0, False), ('heads20', 16, 0, False), ('gpt2', 77, 1, True), ('gpt2_xl', 77, 1, False)):
         sh = SHAPES[name]
         d = pass_desc(L=sh.L, D=sh.D, H=sh.H, F=sh.F, N=sh.N, rows=rows, logit_rows=prompts or rows, prompts=prompts)
         bm, bn, stages, parts, smem = tiles(d, rows, d.logit_rows)['proj']

@@ -271,15 +271,15 @@ Tile tile_of(const Pass& p, int k, int rows, int lrows) {
     return choose(k, k == K_LOGITS ? std::max(lrows, 1) : rows, p.rp, feat[k], k == K_P2 ? (d.F + 63) / 64 : d.D / 64, p.sms);
 }
 
-// Shared memory of a block of a contraction of `ntiles` tiles. A step's projection has small blocks that come while the attention's leave: five of
+// Shared memory of a block of a contraction of `ntiles` tiles. The projection of few rows has small blocks that come while the attention's leave: five of
 // them on the first SMs that are free, none on the last. Where there is about one for every SM and more than two would fit one, they ask for
 // so much that only two do (64 sequences, 144 blocks of 41 KB: 1,763 -> 1,721 us per four steps; 33 to 80 sequences 1 to 4 % faster; 23, 72 blocks:
 // 1,111 -> 1,122, left). Blocks of the XL shape (83 KB) are two to an SM as they are, and with more lose their place beside an attention block
-// (16 sequences at 300 positions 1,367 -> 1,355 us per step without, 8 at 300 1,309 -> 1,288), as do those of width 1,280 (16 at 128 315 -> 304). Prompts take
-// the same time either way (8 to 900 rows, within 0.5 %) and are left.
+// (16 sequences at 300 positions 1,367 -> 1,355 us per step without, 8 at 300 1,309 -> 1,288), as do those of width 1,280 (16 at 128 315 -> 304).
+// Short prompts gain too (77 rows 368.7 -> 366.4 us, 120 rows 408.7 -> 402.1), others take the same time (100, 200 to 900 rows).
 size_t block_bytes(const Pass& p, int kind, const Tile& t, int ntiles) {
     const int bytes = t.bm == 64 ? GemmShape<64>::bytes(t.stages, t.bn) : t.bm == 128 ? GemmShape<128>::bytes(t.stages, t.bn) : GemmShape<256>::bytes(t.stages, t.bn);
-    const bool spread = kind == K_PROJ && !p.d.prompts && p.d.D <= 1024 && t.bm == 64 && 2 * ntiles > p.sms && 3 * (bytes + 1024) <= SMEM_MAX;
+    const bool spread = kind == K_PROJ && p.d.D <= 1024 && t.bm == 64 && 2 * ntiles > p.sms && 3 * (bytes + 1024) <= SMEM_MAX;
     return spread ? std::max(bytes, 110 * 1024) : bytes;
 }
 
