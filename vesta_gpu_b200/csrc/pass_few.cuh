@@ -12,8 +12,8 @@
 //   * the eight blocks of a head exchange their attention results through distributed shared memory and each applies an eighth of
 //     the head's rows of the projection to all sequences;
 //   * a block keeps the GELU output of its own features and multiplies it with their rows of the MLP projection.
-// Measured on B200 (small shape): one sequence at 37 positions 183 -> 169 us per step, eight at 128 to 144 209 -> 192; per layer 12.2 and 14.5 us,
-// of which the kernels' own chains are 9 to 10 and the rest boundaries.
+// Measured on B200 (small shape, 200 positions, steps of sixteen): two sequences 184 -> 168 us per step, three 186 -> 158, four 191 -> 163; per layer 12.9,
+// 12.3 and 12.5 us, of which 3 to 4 are boundaries and the rest the kernels' own chains.
 // The weights a block needs are on their way into its shared memory before it waits for its predecessor. They are a copy in the order
 // in which the lanes of mma.sync m16n8k16 hold them, so that every thread copies (cp.async) and reads back just its own 16 bytes of
 // each unit: no barrier, nothing to wait for but its own copies. The activations enter as fp16 head and remainder, whose products
@@ -274,7 +274,7 @@ __device__ __forceinline__ float few_sum(const float* red, int o) {
 
 // ---- norm + QKV -------------------------------------------------------------------------------------------------------
 // A tile of 16 features per block (two beyond 148 tiles): 144 blocks at width 768. Bound by its chain: state from L2, statistics, operand,
-// products, exchange between the warps. 4.2 us at eight sequences, 3.8 at one, a boundary included. (With sixteen warps 4.8 and 3.9.)
+// products, exchange between the warps. 4.6 us at two sequences (whose state is twice as wide), 4.1 at four, a boundary included.
 struct FewQkv {
     FewNorm n;
     const unsigned char* w;           // packed, of the layer
@@ -364,9 +364,9 @@ struct FewAttend {
     static __host__ __device__ int tiles(int D) { return (D / 16 + FEW_CLUSTER - 1) / FEW_CLUSTER; }
     static __host__ __device__ int bytes(int D) { return FEW_WARPS * FEW_STAGES * 4096 + tiles(D) * 2048; }
 };
-// Cluster = a head, block = a sequence or a run of its positions; see pass_attend for the attention itself. 4.5 us at eight sequences of 136
-// positions, 4.2 at one of 37: a warp's one or two rounds of 16 positions 1.6 us, the cluster's exchange 0.7.
-// (Two stages per warp: four keep the next kernel's block from the SM, eight sequences 3,080 -> 3,600 us per sixteen steps.)
+// Cluster = a head, block = a sequence or a run of its positions; see pass_attend for the attention itself. 4.3 us at two sequences of 200
+// positions, 4.0 at four, 5.8 at four of 900: a warp's rounds of 16 positions (0.8 us each), the cluster's exchange 0.7.
+// (Two stages per warp: with four, 144 KB, the next kernel's block has no room beside it.)
 template <bool FIXED>
 __global__ void __launch_bounds__(FEW_THREADS) few_attend(const __grid_constant__ FewAttend a) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -443,7 +443,7 @@ __global__ void __launch_bounds__(FEW_THREADS) few_attend(const __grid_constant_
 
 // ---- norm + FC + GELU + MLP projection ------------------------------------------------------------------------------------
 // Two tiles of 16 features per block at an MLP width of 3,072: 96 blocks; all of a block's weights (98 KB) fit beside the attention's block on an SM.
-// 5.1 us at eight sequences, 4.0 at one. The reductions of 96 blocks into the same rows are a third of it.
+// 4.1 us at two sequences, 4.4 at four; the reductions of 96 blocks into the same rows are much of it.
 struct FewMlp {
     FewNorm n;
     const unsigned char *fc, *p2;     // packed, of the layer

@@ -1,6 +1,6 @@
 """Run a Lowered program through the C ABI of libvesta_b200.so (include/vesta_b200.h) bound with ctypes: a decode step as one
-persistent kernel, compiled with NVRTC for sm_100a and launched cooperatively (one to four wide sequences, and wherever the lowering
-asks for what only it has: tune options, timing, rows of prompts), or as a chain of kernels of the library (passes.py); which of
+persistent kernel, compiled with NVRTC for sm_100a and launched cooperatively (one sequence and five to eight, two to four wide ones, and wherever the
+lowering asks for what only it has: tune options, timing, rows of prompts), or as a chain of kernels of the library (passes.py); which of
 the two, Lowered.dims['chain'] and, for the chain of few sequences, dims['few'] say.
 
 Mirrors the reference run-time (vesta/launch.py:10-73): `TORCH_DT`, `ok`, `compile_cubin`,
